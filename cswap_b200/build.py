@@ -1,4 +1,5 @@
-"""Builds libcswap_b200.so in-tree with nvcc for sm_100a (cross-compiles without a GPU)."""
+"""Builds libcswap_b200.so in-tree with nvcc for sm_100a (cross-compiles without a GPU) and the CPython extension
+behind codec.py."""
 from __future__ import annotations
 
 import os
@@ -8,6 +9,7 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libcswap_b200.so")
+ROOT = os.path.dirname(HERE)
 SOURCES = ["zfp_kernels.cu", "sparse_kernels.cu", "cswap_abi.cu", "swap_manager.cu", "cost_model.cu",
            "sparse_static.cu"]
 HEADERS = ["zfp_core.cuh", "zfp_field.cuh", "zfp_kernels.h", "sparse_kernels.h", "internal.h",
@@ -30,8 +32,14 @@ def needs_build() -> bool:
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
-    if not force and not needs_build():
-        return LIB
+    """The CUDA library and the extension module; returns the library's path."""
+    if force or needs_build():
+        _build_lib(verbose)
+    build_ext(force)
+    return LIB
+
+
+def _build_lib(verbose: bool) -> None:
     objdir = os.path.join(HERE, "build")
     os.makedirs(objdir, exist_ok=True)
     objs = []
@@ -50,7 +58,30 @@ def build(force: bool = False, verbose: bool = False) -> str:
             raise RuntimeError(f"nvcc failed on {s}")
     cmd = [_nvcc(), "-shared", "-o", LIB] + objs + ["-Xcompiler", "-fPIC"]
     subprocess.check_call(cmd)
-    return LIB
+
+
+EXT_SOURCE = os.path.join(CSRC, "codec_ext.cpp")
+EXT = os.path.join(HERE, "_codec_ext.so")
+
+
+def build_ext(force: bool = False) -> str:
+    """Compile the CPython extension behind codec.py against the installed
+    libtorch and the in-tree library (g++; needs no GPU)."""
+    deps = [EXT_SOURCE, os.path.join(ROOT, "include", "cswap_b200.h"), os.path.abspath(__file__)]
+    if not force and os.path.exists(EXT) and all(os.path.getmtime(EXT) >= os.path.getmtime(d) for d in deps):
+        return EXT
+    import sysconfig
+    import torch
+    t = os.path.dirname(torch.__file__)
+    cuda_inc = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
+    cmd = ["g++", "-std=c++17", "-O2", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           "-I", sysconfig.get_paths()["include"], "-I", os.path.join(t, "include"),
+           "-I", os.path.join(t, "include", "torch", "csrc", "api", "include"), "-I", cuda_inc,
+           EXT_SOURCE, "-o", EXT, "-L", os.path.join(t, "lib"), "-L", HERE,
+           f"-Wl,-rpath,{os.path.join(t, 'lib')}", "-Wl,-rpath,$ORIGIN",
+           "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", "-lcswap_b200"]
+    subprocess.check_call(cmd)
+    return EXT
 
 
 CPP_DRIVERS = ("execution_driver", "vgg16_step", "bert_step")

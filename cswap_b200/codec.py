@@ -1,8 +1,9 @@
 """Tensor-level front end of the codecs.
 
-Each function takes CUDA float32 tensors, passes raw device pointers and the
-current CUDA stream through the C ABI (include/cswap_b200.h) and returns
-tensors.  Nothing here computes: without the CUDA library the calls raise.
+Each function takes CUDA float32 tensors and returns tensors.  Checks, output
+allocation and the C ABI call (include/cswap_b200.h) on the current CUDA stream
+are made by the extension module built from csrc/codec_ext.cpp.  Nothing here
+computes: without the CUDA library the calls raise.
 """
 from __future__ import annotations
 
@@ -11,10 +12,27 @@ from typing import Optional, Tuple
 
 import torch
 
-from ._lib import SparseLayout, check, lib
+from ._lib import LibraryMissing, SparseLayout, check, lib
 
 # policy codes (CSWAP+/Execution.h:70,86,107,243)
 POLICY_KEEP, POLICY_DROP, POLICY_RAW, POLICY_SPARSE, POLICY_ZFP = 0, 1, 2, 3, 6
+
+
+# The extension module behind the tensor-level calls (csrc/codec_ext.cpp), loaded on first use
+_native = None
+
+
+def _load():
+    """The extension; raises LibraryMissing when it or the CUDA library has not been built."""
+    global _native
+    lib()
+    try:
+        from . import _codec_ext
+    except ImportError as e:
+        raise LibraryMissing(f"cswap_b200._codec_ext cannot be loaded ({e}): build it with "
+                             "`python -m cswap_b200.build`.") from e
+    _native = _codec_ext
+    return _native
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
@@ -55,47 +73,18 @@ def zfp_max_bytes(nx: int, ny: int, nz: int, maxbits: int) -> int:
     return out.value
 
 
-def _dims(t: torch.Tensor, dims: Optional[Tuple[int, int, int]]) -> Tuple[int, int, int]:
-    if dims is not None:
-        nx, ny, nz = dims
-        if nx * max(ny, 1) * max(nz, 1) != t.numel():
-            raise ValueError("dims do not match the tensor's element count")
-        return nx, ny, nz
-    return zfp_view(t.numel())
-
-
 def zfp_compress(t: torch.Tensor, maxbits: int = 512, dims: Optional[Tuple[int, int, int]] = None,
                  out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Fixed-rate ZFP stream (uint8 tensor) of `t` at `maxbits` bits per block.
 
     `dims` = (nx, ny, nz), x fastest, 0 for unused axes; default is the swap
     path's 32 x 32 x numel/1024 view."""
-    _require_cuda_f32(t, "t")
-    nx, ny, nz = _dims(t, dims)
-    need = zfp_max_bytes(nx, ny, nz, maxbits)
-    if out is None:
-        out = torch.empty(need, dtype=torch.uint8, device=t.device)
-    elif out.numel() * out.element_size() < need or not out.is_cuda:
-        raise ValueError("out is too small or not on the device")
-    with torch.cuda.device(t.device):
-        check(lib().csw_zfp_compress(t.data_ptr(), nx, ny, nz, maxbits, out.data_ptr(),
-                                     out.numel() * out.element_size(), None, _stream_ptr(t.device)),
-              "csw_zfp_compress")
-    return out
+    return (_native or _load()).zfp_compress(t, maxbits, dims, out)
 
 
 def zfp_decompress(stream: torch.Tensor, numel: int, maxbits: int = 512,
                    dims: Optional[Tuple[int, int, int]] = None, out: Optional[torch.Tensor] = None) -> torch.Tensor:
-    if not stream.is_cuda:
-        raise ValueError("stream must be a CUDA tensor")
-    if out is None:
-        out = torch.empty(numel, dtype=torch.float32, device=stream.device)
-    _require_cuda_f32(out, "out")
-    nx, ny, nz = _dims(out, dims)
-    with torch.cuda.device(stream.device):
-        check(lib().csw_zfp_decompress(stream.data_ptr(), stream.numel() * stream.element_size(), nx, ny, nz, maxbits,
-                                       out.data_ptr(), _stream_ptr(stream.device)), "csw_zfp_decompress")
-    return out
+    return (_native or _load()).zfp_decompress(stream, numel, maxbits, dims, out)
 
 
 # ---------------------------------------------------------------------------
@@ -120,30 +109,11 @@ def sparse_compress(t: torch.Tensor, out: Optional[torch.Tensor] = None,
 
     onepass=True reads the tensor once (csw_sparse_compress_onepass): same bitmap,
     count and per-tile contents, tile segments in schedule order."""
-    _require_cuda_f32(t, "t")
-    n = t.numel()
-    L = sparse_layout(n)
-    if out is None:
-        out = torch.empty(L.bound, dtype=torch.uint8, device=t.device)
-    if nnz_out is None:
-        nnz_out = torch.zeros(1, dtype=torch.int32, device=t.device)
-    with torch.cuda.device(t.device):
-        fn = lib().csw_sparse_compress_onepass if onepass else lib().csw_sparse_compress
-        check(fn(t.data_ptr(), n, out.data_ptr(), out.numel(), nnz_out.data_ptr(), _stream_ptr(t.device)),
-              "csw_sparse_compress")
-    return out, nnz_out
+    return (_native or _load()).sparse_compress(t, out, nnz_out, onepass)
 
 
 def sparse_decompress(packed: torch.Tensor, n: int, out: Optional[torch.Tensor] = None) -> torch.Tensor:
-    if not packed.is_cuda:
-        raise ValueError("packed must be a CUDA tensor")
-    if out is None:
-        out = torch.empty(n, dtype=torch.float32, device=packed.device)
-    _require_cuda_f32(out, "out")
-    with torch.cuda.device(packed.device):
-        check(lib().csw_sparse_decompress(packed.data_ptr(), n, out.data_ptr(), _stream_ptr(packed.device)),
-              "csw_sparse_decompress")
-    return out
+    return (_native or _load()).sparse_decompress(packed, n, out)
 
 
 # ---------------------------------------------------------------------------
