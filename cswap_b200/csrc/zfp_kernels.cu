@@ -30,6 +30,7 @@
 
 #include <cstdint>
 
+#include "pdl.cuh"
 #include "zfp_field.cuh"
 #include "zfp_kernels.h"
 
@@ -106,6 +107,10 @@ zfp_encode_slab_kernel(const float* __restrict__ in, uint32_t* __restrict__ out,
   const int t = tid >> 6, bx = tid & 7, by = (tid >> 3) & 7;
   const uint32_t zt = (blockIdx.x * (kThreads / 64) + t) * 4;  // first slab of my tile
   const int vz = zt >= nz ? 0 : (nz - zt < 4 ? (int)(nz - zt) : 4);
+  static_assert(ENC_LUT_SIZE == 2 * kThreads, "two table words per thread");
+  const uint32_t lut0 = __ldg(g_enc_table.v + tid), lut1 = __ldg(g_enc_table.v + kThreads + tid);
+  pdl_trigger();
+  pdl_wait(in);
   float f[64];
   if (vz > 0) {
     const float* my = in + (size_t)zt * kSlabFloats + by * 128 + bx * 4;
@@ -122,7 +127,8 @@ zfp_encode_slab_kernel(const float* __restrict__ in, uint32_t* __restrict__ out,
       }
     }
   }
-  for (int i = tid; i < ENC_LUT_SIZE; i += kThreads) lut[i] = __ldg(g_enc_table.v + i);
+  lut[tid] = lut0;
+  lut[kThreads + tid] = lut1;
   for (int w = 0; w < nwords; w++) stage[w * kThreads + tid] = 0u;  // coded bits are OR-ed in
   __syncthreads();  // the table is complete
   if (vz == 0) return;
@@ -176,6 +182,12 @@ zfp_decode_slab_kernel(const uint32_t* __restrict__ in, float* __restrict__ out,
   const int t = tid >> 6, bx = tid & 7, by = (tid >> 3) & 7;
   const uint32_t zt = (blockIdx.x * (kThreads / 64) + t) * 4;  // first slab of my tile
   uint32_t* col = stage + tid;
+#pragma unroll
+  for (int i = 0; i < DEC_LUT_SIZE / (4 * kThreads); i++)
+    reinterpret_cast<uint4*>(lut)[i * kThreads + tid] =
+        __ldg(reinterpret_cast<const uint4*>(g_dec_table.v) + i * kThreads + tid);
+  pdl_trigger();
+  pdl_wait(in);
   if (zt < nz) {
     const uint32_t* src = in + ((size_t)blockIdx.x * kThreads + tid) * nwords;
     if ((nwords & 3) == 0) {
@@ -192,10 +204,6 @@ zfp_decode_slab_kernel(const uint32_t* __restrict__ in, float* __restrict__ out,
   }
   // reads just past a block find zeros and need no bounds test
   for (int w = nwords; w < nwords + STAGE_SPARE_ROWS; w++) col[w * kThreads] = 0u;
-#pragma unroll
-  for (int i = 0; i < DEC_LUT_SIZE / (4 * kThreads); i++)
-    reinterpret_cast<uint4*>(lut)[i * kThreads + tid] =
-        __ldg(reinterpret_cast<const uint4*>(g_dec_table.v) + i * kThreads + tid);
   __syncthreads();  // the table is complete
   if (zt >= nz) return;
 
@@ -264,6 +272,8 @@ zfp_encode_generic_kernel(FieldGeom g, const float* __restrict__ in, uint32_t* _
                           uint64_t nblocks) {
   __shared__ uint32_t lut[ENC_LUT_SIZE];
   for (int i = threadIdx.x; i < ENC_LUT_SIZE; i += blockDim.x) lut[i] = __ldg(g_enc_table.v + i);
+  pdl_trigger();
+  pdl_wait(in);
   __syncthreads();
   const uint64_t b = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= nblocks) return;
@@ -279,6 +289,8 @@ zfp_decode_generic_kernel(FieldGeom g, const uint32_t* __restrict__ in, float* _
                           uint64_t nblocks, uint64_t total_words) {
   __shared__ uint32_t lut[DEC_LUT_SIZE];
   for (int i = threadIdx.x; i < DEC_LUT_SIZE; i += blockDim.x) lut[i] = __ldg(g_dec_table.v + i);
+  pdl_trigger();
+  pdl_wait(in);
   __syncthreads();
   const uint64_t b = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= nblocks) return;
@@ -317,9 +329,8 @@ cudaError_t zfp_encode_launch(const FieldGeom& g, const float* in, void* out, in
       if (e != cudaSuccess) return e;
     }
     const uint32_t ngroups = (g.nz + kGroupSlabs - 1) / kGroupSlabs;
-    zfp_encode_slab_kernel<<<ngroups, kThreads, smem, stream>>>(in, reinterpret_cast<uint32_t*>(out), g.nz, maxbits,
-                                                               pipe_consts());
-    return cudaGetLastError();
+    return pdl_launch(zfp_encode_slab_kernel, ngroups, kThreads, smem, stream, in, reinterpret_cast<uint32_t*>(out), g.nz,
+                      maxbits, pipe_consts());
   }
   if (maxbits & 31) {
     cudaError_t e = cudaMemsetAsync(out, 0, stream_bytes(g, (unsigned)maxbits), stream);
@@ -333,10 +344,10 @@ cudaError_t zfp_encode_launch(const FieldGeom& g, const float* in, void* out, in
   }
   const unsigned grid = (unsigned)((nblocks + 127) / 128);
   uint32_t* o = reinterpret_cast<uint32_t*>(out);
-  if (g.dims == 3) zfp_encode_generic_kernel<3><<<grid, 128, 0, stream>>>(g, in, o, maxbits, nblocks);
-  else if (g.dims == 2) zfp_encode_generic_kernel<2><<<grid, 128, 0, stream>>>(g, in, o, maxbits, nblocks);
-  else zfp_encode_generic_kernel<1><<<grid, 128, 0, stream>>>(g, in, o, maxbits, nblocks);
-  return cudaGetLastError();
+  const auto kernel = g.dims == 3   ? zfp_encode_generic_kernel<3>
+                      : g.dims == 2 ? zfp_encode_generic_kernel<2>
+                                    : zfp_encode_generic_kernel<1>;
+  return pdl_launch(kernel, grid, 128, 0, stream, g, in, o, maxbits, nblocks);
 }
 
 cudaError_t zfp_decode_launch(const FieldGeom& g, const void* in, float* out, int maxbits, cudaStream_t stream) {
@@ -350,17 +361,16 @@ cudaError_t zfp_decode_launch(const FieldGeom& g, const void* in, float* out, in
       if (e != cudaSuccess) return e;
     }
     const uint32_t ngroups = (g.nz + kGroupSlabs - 1) / kGroupSlabs;
-    zfp_decode_slab_kernel<<<ngroups, kThreads, smem, stream>>>(reinterpret_cast<const uint32_t*>(in), out, g.nz,
-                                                               maxbits, pipe_consts());
-    return cudaGetLastError();
+    return pdl_launch(zfp_decode_slab_kernel, ngroups, kThreads, smem, stream, reinterpret_cast<const uint32_t*>(in), out,
+                      g.nz, maxbits, pipe_consts());
   }
   const unsigned grid = (unsigned)((nblocks + 127) / 128);
   const uint32_t* i32 = reinterpret_cast<const uint32_t*>(in);
   const uint64_t total_words = stream_bytes(g, (unsigned)maxbits) / 4;
-  if (g.dims == 3) zfp_decode_generic_kernel<3><<<grid, 128, 0, stream>>>(g, i32, out, maxbits, nblocks, total_words);
-  else if (g.dims == 2) zfp_decode_generic_kernel<2><<<grid, 128, 0, stream>>>(g, i32, out, maxbits, nblocks, total_words);
-  else zfp_decode_generic_kernel<1><<<grid, 128, 0, stream>>>(g, i32, out, maxbits, nblocks, total_words);
-  return cudaGetLastError();
+  const auto kernel = g.dims == 3   ? zfp_decode_generic_kernel<3>
+                      : g.dims == 2 ? zfp_decode_generic_kernel<2>
+                                    : zfp_decode_generic_kernel<1>;
+  return pdl_launch(kernel, grid, 128, 0, stream, g, i32, out, maxbits, nblocks, total_words);
 }
 
 }  // namespace csw
