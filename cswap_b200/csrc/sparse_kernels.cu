@@ -13,16 +13,24 @@
 //                   round-trip exactly.
 //  count -> scan -> pack, three launches, no inter-CTA waiting; the total is
 //                   written to a caller-supplied word (device or mapped host).
+//                   16 MiB at 50 % zeros: 16.4 -> 9.2 us a call back to back
+//                   (programmatic launches; bitmap out of the counting pass).
 //  single pass    - same bitmap and per-tile contents from one read of the
 //                   tensor; tiles claim their segments with an atomic add, so
 //                   segment order follows the schedule, not the element order.
+//                   16 MiB: 8.2 -> 6.3 us, 256 MiB: 65.8 -> 62.7 us.
+//  up to 1 MiB    - one cluster, one launch for either of the two: 12.3 (6.2)
+//                   -> 3.8 ... 4.4 us, which is what launching costs.
 //  legacy format  - the reference's `begin | bitmap | values` layout with its
 //                   P-worker chunking, one warp per worker, behind the
 //                   reference's own entry-point names.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 
+#include "pdl.cuh"
 #include "sparse_kernels.h"
 
 namespace csw {
@@ -31,6 +39,7 @@ namespace {
 
 constexpr int kTile = SPARSE_TILE;        // elements per tile
 constexpr int kThreads = 256;             // 8 warps, 512 elements (16 bitmap words) each
+constexpr int kCountThreads = 128;         // 1024 elements per warp, eight 128-bit loads per lane
 constexpr int kWordsPerWarp = kTile / 32 / (kThreads / 32);  // 16
 
 __device__ __forceinline__ uint32_t lanemask_lt() {
@@ -39,54 +48,63 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
   return m;
 }
 
-// ---- pass 1: bitmap + per-tile counts ---------------------------------------------
-__global__ void __launch_bounds__(kThreads)
-sparse_count_kernel(const uint32_t* __restrict__ in, uint64_t n, uint32_t* __restrict__ bitmap,
-                    uint32_t* __restrict__ tile_cnt) {
-  __shared__ uint32_t warp_cnt[kThreads / 32];
+// ---- ordered compression, pass 1: per-tile counts -------------------------------------
+// A pure read of the tensor.  Bitmap and values are written by pass 3, which reads
+// the tensor again (from L2 where it fits).
+__global__ void __launch_bounds__(kCountThreads)
+sparse_count_kernel(const uint32_t* __restrict__ in, uint64_t n, bool vec, uint32_t* __restrict__ tile_cnt) {
+  constexpr int kWarpElems = kTile / (kCountThreads / 32);
+  __shared__ uint32_t warp_cnt[kCountThreads / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint64_t base = (uint64_t)blockIdx.x * kTile + (uint64_t)warp * (kWordsPerWarp * 32);
-  uint32_t v[kWordsPerWarp];
+  const uint64_t base = (uint64_t)blockIdx.x * kTile + (uint64_t)warp * kWarpElems;
+  pdl_wait(in);
+  pdl_trigger();  // behind the wait: what starts on it may read `in` at once
+  uint32_t c = 0;
+  if (vec && base + kWarpElems <= n) {
+    uint4 v[kWarpElems / 128];
 #pragma unroll
-  for (int j = 0; j < kWordsPerWarp; j++) {
-    const uint64_t i = base + j * 32 + lane;
-    v[j] = i < n ? __ldg(in + i) : 0u;
-  }
-  uint32_t mine = 0, cnt = 0;
+    for (int j = 0; j < kWarpElems / 128; j++) v[j] = __ldg(reinterpret_cast<const uint4*>(in + base) + j * 32 + lane);
 #pragma unroll
-  for (int j = 0; j < kWordsPerWarp; j++) {
-    const uint32_t w = __ballot_sync(0xffffffffu, v[j] != 0u);
-    cnt += __popc(w);
-    if (lane == j) mine = w;
+    for (int j = 0; j < kWarpElems / 128; j++)
+      c += (v[j].x != 0u) + (v[j].y != 0u) + (v[j].z != 0u) + (v[j].w != 0u);
+  } else {
+    for (int j = 0; j < kWarpElems / 32; j++) {
+      const uint64_t i = base + j * 32 + lane;
+      c += i < n && __ldg(in + i) != 0u;
+    }
   }
-  const uint64_t word0 = base >> 5, nwords = (n + 31) >> 5;
-  if (lane < kWordsPerWarp && word0 + lane < nwords) bitmap[word0 + lane] = mine;
-  if (lane == 0) warp_cnt[warp] = cnt;
+  c = __reduce_add_sync(0xffffffffu, c);
+  if (lane == 0) warp_cnt[warp] = c;
   __syncthreads();
   if (threadIdx.x == 0) {
     uint32_t s = 0;
 #pragma unroll
-    for (int i = 0; i < kThreads / 32; i++) s += warp_cnt[i];
+    for (int i = 0; i < kCountThreads / 32; i++) s += warp_cnt[i];
     tile_cnt[blockIdx.x] = s;
   }
 }
 
-// ---- pass 2: exclusive scan of the tile counts (one CTA) --------------------------
-// One CTA of 1024 threads scans `len` counts: off[i] = sum of cnt[0 .. i-1], the
-// total to *total.  cnt and off may be the same array (each thread reads its own
-// element before it writes it), which is how the in-place callers use it.
+// ---- pass 2: exclusive scan of the counts (one CTA) -----------------------------------
+// In place: a[i] <- sum of a[0 .. i-1], the total to *total.  A thread takes four
+// or sixteen consecutive counts, so 16384 of them (256 MiB of tensor) are one
+// round: the kernel is a chain of latencies, and rounds of 1024 cost it 7 us there.
 template <class T>
-__global__ void __launch_bounds__(1024)
-block_exclusive_scan_kernel(const T* cnt, T* off, uint32_t len, T* __restrict__ total) {
+__global__ void __launch_bounds__(1024) block_exclusive_scan_kernel(T* a, uint32_t len, T* __restrict__ total) {
   __shared__ T warp_sum[32];
-  __shared__ T carry_s;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (threadIdx.x == 0) carry_s = 0;
-  __syncthreads();
-  for (uint32_t base = 0; base < len; base += 1024) {
-    const uint32_t i = base + threadIdx.x;
-    const T c = i < len ? cnt[i] : T(0);
-    T x = c;
+  pdl_trigger();
+  pdl_wait();
+  T carry = 0;
+  for (uint32_t base = 0; base < len; base += 16384) {
+    const int per = len - base <= 4096 ? 4 : 16;
+    const uint32_t first = base + threadIdx.x * per;
+    T v[16], sum = 0;
+#pragma unroll
+    for (int q = 0; q < 16; q++) {
+      v[q] = q < per && first + q < len ? a[first + q] : T(0);
+      sum += v[q];
+    }
+    T x = sum;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
       const T y = __shfl_up_sync(0xffffffffu, x, d);
@@ -94,51 +112,121 @@ block_exclusive_scan_kernel(const T* cnt, T* off, uint32_t len, T* __restrict__ 
     }
     if (lane == 31) warp_sum[warp] = x;
     __syncthreads();
-    if (warp == 0) {
-      T s = warp_sum[lane];
+    T s = warp_sum[lane];
 #pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const T y = __shfl_up_sync(0xffffffffu, s, d);
-        if (lane >= d) s += y;
-      }
-      warp_sum[lane] = s;  // inclusive
+    for (int d = 1; d < 32; d <<= 1) {
+      const T y = __shfl_up_sync(0xffffffffu, s, d);
+      if (lane >= d) s += y;
     }
-    __syncthreads();
-    const T carry = carry_s;
-    if (i < len) off[i] = carry + (warp ? warp_sum[warp - 1] : T(0)) + x - c;
-    __syncthreads();
-    if (threadIdx.x == 1023) carry_s = carry + warp_sum[31];
-    __syncthreads();
+    const T front = __shfl_sync(0xffffffffu, s, warp - 1);  // of the warps in front of mine
+    T off = carry + (warp ? front : T(0)) + x - sum;
+    carry += __shfl_sync(0xffffffffu, s, 31);
+#pragma unroll
+    for (int q = 0; q < 16; q++) {
+      if (q < per && first + q < len) a[first + q] = off;
+      off += v[q];
+    }
+    __syncthreads();  // warp_sum is free for the next round
   }
-  if (threadIdx.x == 0) *total = carry_s;
+  if (threadIdx.x == 0) *total = carry;
 }
 
-// ---- pass 3: pack the non-zeros ----------------------------------------------------
+// ---- pass 3: bitmap and values ---------------------------------------------------------
+// The tile is loaded while the scan still runs (past L1, so that nothing a kernel
+// before left there can be met) and only its place in `values` is waited for.
 __global__ void __launch_bounds__(kThreads)
-sparse_pack_kernel(const uint32_t* __restrict__ in, uint64_t n, const uint32_t* __restrict__ tile_off,
+sparse_pack_kernel(const uint32_t* __restrict__ in, uint64_t n, uint32_t* __restrict__ bitmap, const uint32_t* tile_off,
                    uint32_t* __restrict__ values) {
   __shared__ uint32_t warp_cnt[kThreads / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint64_t base = (uint64_t)blockIdx.x * kTile + (uint64_t)warp * (kWordsPerWarp * 32);
+  pdl_trigger();
   uint32_t v[kWordsPerWarp], w[kWordsPerWarp];
 #pragma unroll
   for (int j = 0; j < kWordsPerWarp; j++) {
     const uint64_t i = base + j * 32 + lane;
-    v[j] = i < n ? __ldg(in + i) : 0u;
+    v[j] = i < n ? __ldcg(in + i) : 0u;
   }
-  uint32_t cnt = 0;
+  uint32_t mine = 0, cnt = 0;
 #pragma unroll
   for (int j = 0; j < kWordsPerWarp; j++) {
     w[j] = __ballot_sync(0xffffffffu, v[j] != 0u);
     cnt += __popc(w[j]);
+    if (lane == j) mine = w[j];
   }
+  const uint64_t word0 = base >> 5, nwords = (n + 31) >> 5;
   if (lane == 0) warp_cnt[warp] = cnt;
   __syncthreads();
+  pdl_wait();
+  if (lane < kWordsPerWarp && word0 + lane < nwords) bitmap[word0 + lane] = mine;
   uint32_t off = tile_off[blockIdx.x];
   for (int i = 0; i < warp; i++) off += warp_cnt[i];
   const uint32_t lt = lanemask_lt();
 #pragma unroll
   for (int j = 0; j < kWordsPerWarp; j++) {
+    if (v[j] != 0u) values[off + __popc(w[j] & lt)] = v[j];
+    off += __popc(w[j]);
+  }
+}
+
+// ---- small tensors: one cluster --------------------------------------------------------
+// Up to kMaxCluster CTAs of kSmallTiles tiles compress the whole tensor: bitmap,
+// counts, offsets and values from one read and one launch.  The CTAs exchange their
+// counts through distributed shared memory; three launches of 2-3 us each are what
+// bounds tensors this small otherwise.
+constexpr int kSmallThreads = 512, kMaxCluster = 16;
+template <int TILES>
+__global__ void __launch_bounds__(kSmallThreads)
+sparse_small_kernel(const uint32_t* __restrict__ in, uint64_t n, uint32_t* __restrict__ bitmap,
+                    uint32_t* __restrict__ tile_off, uint32_t* __restrict__ values, uint32_t* __restrict__ nnz_out) {
+  constexpr int W = kSmallThreads / 32, kWords = TILES * kTile / 32 / W;  // bitmap words per warp
+  __shared__ uint32_t warp_cnt[W], cta_cnt[kMaxCluster];
+  cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t cta = blockIdx.x;
+  const uint64_t base = (uint64_t)cta * (TILES * kTile) + (uint64_t)warp * (kWords * 32);
+  cl.barrier_arrive();  // that every CTA of the cluster runs is only needed further down
+  pdl_wait(in);
+  pdl_trigger();
+  uint32_t v[kWords], w[kWords];
+#pragma unroll
+  for (int j = 0; j < kWords; j++) {
+    const uint64_t i = base + j * 32 + lane;
+    v[j] = i < n ? __ldg(in + i) : 0u;
+  }
+  uint32_t mine = 0, cnt = 0;
+#pragma unroll
+  for (int j = 0; j < kWords; j++) {
+    w[j] = __ballot_sync(0xffffffffu, v[j] != 0u);
+    cnt += __popc(w[j]);
+    if (lane == j) mine = w[j];
+  }
+  const uint64_t word0 = base >> 5, nwords = (n + 31) >> 5;
+  if (lane < kWords && word0 + lane < nwords) bitmap[word0 + lane] = mine;
+  if (lane == 0) warp_cnt[warp] = cnt;
+  __syncthreads();
+  uint32_t x = lane < W ? warp_cnt[lane] : 0u;
+  const uint32_t c = x;
+#pragma unroll
+  for (int d = 1; d < W; d <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, x, d);
+    if (lane >= d) x += y;
+  }
+  const uint32_t total = __shfl_sync(0xffffffffu, x, W - 1);
+  uint32_t off = __shfl_sync(0xffffffffu, x - c, warp);
+  cl.barrier_wait();
+  if (threadIdx.x < cl.num_blocks()) cl.map_shared_rank(cta_cnt, threadIdx.x)[cta] = total;
+  cl.sync();
+  uint32_t front = 0;
+  for (uint32_t i = 0; i < cta; i++) front += cta_cnt[i];
+  off += front;
+  constexpr int kWarpsPerTile = W / TILES;
+  const uint64_t tile = (uint64_t)cta * TILES + warp / kWarpsPerTile, ntiles = (n + kTile - 1) / kTile;
+  if (lane == 0 && warp % kWarpsPerTile == 0 && tile < ntiles) tile_off[tile] = off;
+  if (threadIdx.x == 0 && cta == gridDim.x - 1) *nnz_out = front + total;
+  const uint32_t lt = lanemask_lt();
+#pragma unroll
+  for (int j = 0; j < kWords; j++) {
     if (v[j] != 0u) values[off + __popc(w[j] & lt)] = v[j];
     off += __popc(w[j]);
   }
@@ -151,6 +239,11 @@ sparse_pack_kernel(const uint32_t* __restrict__ in, uint64_t n, const uint32_t* 
 // and per-tile contents are the same as the three-pass result, but segments
 // sit in the order the tiles claimed them, so the values array (not what
 // decompression returns) can differ from run to run.  No CTA waits for another.
+__global__ void sparse_zero_kernel(uint32_t* word) {
+  pdl_wait();
+  pdl_trigger();  // behind the wait: what starts on it may read its input at once
+  *word = 0u;
+}
 __global__ void __launch_bounds__(kThreads)
 sparse_onepass_kernel(const uint32_t* __restrict__ in, uint64_t n, uint32_t* __restrict__ bitmap,
                       uint32_t* __restrict__ tile_off, uint32_t* __restrict__ values, uint32_t* __restrict__ cursor) {
@@ -158,11 +251,12 @@ sparse_onepass_kernel(const uint32_t* __restrict__ in, uint64_t n, uint32_t* __r
   __shared__ uint32_t tile_base;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint64_t base = (uint64_t)blockIdx.x * kTile + (uint64_t)warp * (kWordsPerWarp * 32);
+  pdl_trigger();
   uint32_t v[kWordsPerWarp], w[kWordsPerWarp];
 #pragma unroll
   for (int j = 0; j < kWordsPerWarp; j++) {
     const uint64_t i = base + j * 32 + lane;
-    v[j] = i < n ? __ldg(in + i) : 0u;
+    v[j] = i < n ? __ldcg(in + i) : 0u;
   }
   uint32_t mine = 0, cnt = 0;
 #pragma unroll
@@ -172,9 +266,10 @@ sparse_onepass_kernel(const uint32_t* __restrict__ in, uint64_t n, uint32_t* __r
     if (lane == j) mine = w[j];
   }
   const uint64_t word0 = base >> 5, nwords = (n + 31) >> 5;
-  if (lane < kWordsPerWarp && word0 + lane < nwords) bitmap[word0 + lane] = mine;
   if (lane == 0) warp_cnt[warp] = cnt;
   __syncthreads();
+  pdl_wait();  // the cursor is zero
+  if (lane < kWordsPerWarp && word0 + lane < nwords) bitmap[word0 + lane] = mine;
   if (threadIdx.x == 0) {
     uint32_t total = 0;
 #pragma unroll
@@ -202,6 +297,9 @@ sparse_unpack_kernel(const uint32_t* __restrict__ bitmap, const uint32_t* __rest
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint64_t base = (uint64_t)blockIdx.x * kTile + (uint64_t)warp * (kWordsPerWarp * 32);
   const uint64_t word0 = base >> 5, nwords = (n + 31) >> 5;
+  pdl_trigger();
+  pdl_wait(bitmap);
+  asm volatile("" : "+l"(values), "+l"(tile_off));  // read behind the wait as well
   const uint32_t mine = (lane < kWordsPerWarp && word0 + lane < nwords) ? __ldg(bitmap + word0 + lane) : 0u;
   // exclusive prefix of the popcounts of this warp's 16 words
   uint32_t x = __popc(mine);
@@ -243,6 +341,8 @@ __device__ __forceinline__ bool legacy_nz(uint32_t bits) { return __uint_as_floa
 
 __global__ void __launch_bounds__(kThreads)
 legacy_count_kernel(const uint32_t* __restrict__ in, int n, int chunk, int workers, int* __restrict__ count) {
+  pdl_trigger();
+  pdl_wait(in);
   const int lane = threadIdx.x & 31;
   const int i = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
   if (i >= workers) return;
@@ -260,6 +360,9 @@ legacy_count_kernel(const uint32_t* __restrict__ in, int n, int chunk, int worke
 __global__ void __launch_bounds__(kThreads)
 legacy_pack_kernel(const uint32_t* __restrict__ in, int n, int chunk, int workers, uint32_t* __restrict__ values,
                    const int* __restrict__ begin, uint32_t* __restrict__ bitmap) {
+  pdl_trigger();
+  pdl_wait(in);
+  asm volatile("" : "+l"(begin));  // read behind the wait as well
   const int lane = threadIdx.x & 31;
   const int i = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
   if (i >= workers) return;
@@ -285,6 +388,9 @@ legacy_pack_kernel(const uint32_t* __restrict__ in, int n, int chunk, int worker
 __global__ void __launch_bounds__(kThreads)
 legacy_unpack_kernel(const uint32_t* __restrict__ values, uint32_t* __restrict__ out, int n, int chunk, int workers,
                      const uint32_t* __restrict__ bitmap, const int* __restrict__ begin) {
+  pdl_trigger();
+  pdl_wait(values);
+  asm volatile("" : "+l"(bitmap), "+l"(begin));  // read behind the wait as well
   const int lane = threadIdx.x & 31;
   const int i = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
   if (i >= workers) return;
@@ -308,53 +414,91 @@ legacy_unpack_kernel(const uint32_t* __restrict__ values, uint32_t* __restrict__
 // =====================================================================================
 // launchers
 // =====================================================================================
+namespace {
+// One launch for what a cluster can hold.  Sixteen CTAs in a cluster are more than the
+// portable eight and need opting in, once per device.
+template <int TILES>
+cudaError_t small_launch(const uint32_t* in, uint64_t n, uint32_t* bitmap, uint32_t* values, uint32_t* tile_off,
+                         uint32_t* nnz_out, cudaStream_t stream) {
+  static std::atomic<uint64_t> allowed{0};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const uint64_t bit = dev < 64 ? (uint64_t)1 << dev : 0;
+  if (!(allowed.load(std::memory_order_acquire) & bit)) {
+    e = cudaFuncSetAttribute(sparse_small_kernel<TILES>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return e;
+    allowed.fetch_or(bit, std::memory_order_release);
+  }
+  const uint32_t ctas = n ? (uint32_t)((n + TILES * kTile - 1) / (TILES * kTile)) : 1u;
+  cudaLaunchAttribute attr[2]{};
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = ctas;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(kSmallThreads);
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  return cudaLaunchKernelEx(&cfg, sparse_small_kernel<TILES>, in, n, bitmap, tile_off, values, nnz_out);
+}
+// true (and *e set) when the tensor is small enough for one cluster
+bool small_compress(const uint32_t* in, uint64_t n, uint32_t* bitmap, uint32_t* values, uint32_t* tile_off,
+                    uint32_t* nnz_out, cudaStream_t stream, cudaError_t* e) {
+  if (n <= (uint64_t)kMaxCluster * kTile) *e = small_launch<1>(in, n, bitmap, values, tile_off, nnz_out, stream);
+  else if (n <= (uint64_t)kMaxCluster * 2 * kTile) *e = small_launch<2>(in, n, bitmap, values, tile_off, nnz_out, stream);
+  else if (n <= (uint64_t)kMaxCluster * 4 * kTile) *e = small_launch<4>(in, n, bitmap, values, tile_off, nnz_out, stream);
+  else return false;
+  return true;
+}
+}  // namespace
+
 cudaError_t sparse_compress_launch(const float* in, uint64_t n, uint32_t* bitmap, float* values, uint32_t* tile_off,
                                    uint32_t* nnz_out, cudaStream_t stream) {
   const uint32_t ntiles = (uint32_t)((n + kTile - 1) / kTile);
-  if (ntiles) {
-    sparse_count_kernel<<<ntiles, kThreads, 0, stream>>>(reinterpret_cast<const uint32_t*>(in), n, bitmap, tile_off);
-  }
-  block_exclusive_scan_kernel<uint32_t><<<1, 1024, 0, stream>>>(tile_off, tile_off, ntiles, nnz_out);
-  if (ntiles) {
-    sparse_pack_kernel<<<ntiles, kThreads, 0, stream>>>(reinterpret_cast<const uint32_t*>(in), n, tile_off,
-                                                        reinterpret_cast<uint32_t*>(values));
-  }
-  return cudaGetLastError();
+  const uint32_t* src = reinterpret_cast<const uint32_t*>(in);
+  uint32_t* val = reinterpret_cast<uint32_t*>(values);
+  cudaError_t e;
+  if (small_compress(src, n, bitmap, val, tile_off, nnz_out, stream, &e)) return e;
+  const bool vec = (reinterpret_cast<uintptr_t>(in) & 15) == 0;
+  e = pdl_launch(sparse_count_kernel, ntiles, kCountThreads, 0, stream, src, n, vec, tile_off);
+  if (e == cudaSuccess) e = pdl_launch(block_exclusive_scan_kernel<uint32_t>, 1, 1024, 0, stream, tile_off, ntiles, nnz_out);
+  if (e == cudaSuccess) e = pdl_launch(sparse_pack_kernel, ntiles, kThreads, 0, stream, src, n, bitmap, tile_off, val);
+  return e;
 }
 
-cudaError_t sparse_compress_scratch_launch(const float* in, uint64_t n, uint32_t* bitmap, float* values,
-                                           uint32_t* tile_off, uint32_t* tile_cnt_scratch, uint32_t* nnz_out,
-                                           cudaStream_t stream) {
-  const uint32_t ntiles = (uint32_t)((n + kTile - 1) / kTile);
-  if (ntiles) {
-    sparse_count_kernel<<<ntiles, kThreads, 0, stream>>>(reinterpret_cast<const uint32_t*>(in), n, bitmap,
-                                                         tile_cnt_scratch);
-  }
-  block_exclusive_scan_kernel<uint32_t><<<1, 1024, 0, stream>>>(tile_cnt_scratch, tile_off, ntiles, nnz_out);
-  if (ntiles) {
-    sparse_pack_kernel<<<ntiles, kThreads, 0, stream>>>(reinterpret_cast<const uint32_t*>(in), n, tile_off,
-                                                        reinterpret_cast<uint32_t*>(values));
-  }
-  return cudaGetLastError();
+cudaError_t sparse_compress_preload() {
+  cudaFuncAttributes a;
+  cudaError_t e = cudaFuncGetAttributes(&a, sparse_small_kernel<1>);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, sparse_small_kernel<2>);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, sparse_small_kernel<4>);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, sparse_count_kernel);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, block_exclusive_scan_kernel<uint32_t>);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, sparse_pack_kernel);
+  return e;
 }
 
 cudaError_t sparse_compress_onepass_launch(const float* in, uint64_t n, uint32_t* bitmap, float* values,
                                            uint32_t* tile_off, uint32_t* nnz_out, cudaStream_t stream) {
   const uint32_t ntiles = (uint32_t)((n + kTile - 1) / kTile);
-  cudaError_t e = cudaMemsetAsync(nnz_out, 0, sizeof(uint32_t), stream);  // the cursor, then the total
-  if (e != cudaSuccess || !ntiles) return e;
-  sparse_onepass_kernel<<<ntiles, kThreads, 0, stream>>>(reinterpret_cast<const uint32_t*>(in), n, bitmap, tile_off,
-                                                         reinterpret_cast<uint32_t*>(values), nnz_out);
-  return cudaGetLastError();
+  const uint32_t* src = reinterpret_cast<const uint32_t*>(in);
+  uint32_t* val = reinterpret_cast<uint32_t*>(values);
+  cudaError_t e;
+  if (small_compress(src, n, bitmap, val, tile_off, nnz_out, stream, &e)) return e;
+  e = pdl_launch(sparse_zero_kernel, 1, 1, 0, stream, nnz_out);  // the cursor, then the total
+  if (e == cudaSuccess) e = pdl_launch(sparse_onepass_kernel, ntiles, kThreads, 0, stream, src, n, bitmap, tile_off, val, nnz_out);
+  return e;
 }
 
 cudaError_t sparse_decompress_launch(const uint32_t* bitmap, const float* values, const uint32_t* tile_off, uint64_t n,
                                      float* out, cudaStream_t stream) {
   const uint32_t ntiles = (uint32_t)((n + kTile - 1) / kTile);
   if (!ntiles) return cudaSuccess;
-  sparse_unpack_kernel<<<ntiles, kThreads, 0, stream>>>(bitmap, reinterpret_cast<const uint32_t*>(values), tile_off, n,
-                                                        reinterpret_cast<uint32_t*>(out));
-  return cudaGetLastError();
+  return pdl_launch(sparse_unpack_kernel, ntiles, kThreads, 0, stream, bitmap, reinterpret_cast<const uint32_t*>(values),
+                    tile_off, n, reinterpret_cast<uint32_t*>(out));
 }
 
 static int ceil_div_i(int a, int b) { return a % b == 0 ? a / b : a / b + 1; }
@@ -362,33 +506,27 @@ static int ceil_div_i(int a, int b) { return a % b == 0 ? a / b : a / b + 1; }
 cudaError_t legacy_count_launch(int n, int workers, const float* in, int* count, cudaStream_t stream) {
   if (n <= 0 || workers <= 0) return cudaSuccess;
   const int chunk = ceil_div_i(n, workers);
-  legacy_count_kernel<<<(workers + 7) / 8, kThreads, 0, stream>>>(reinterpret_cast<const uint32_t*>(in), n, chunk,
-                                                                  workers, count);
-  return cudaGetLastError();
+  return pdl_launch(legacy_count_kernel, (workers + 7) / 8, kThreads, 0, stream, reinterpret_cast<const uint32_t*>(in), n,
+                    chunk, workers, count);
 }
 cudaError_t legacy_scan_launch(int* idx, int len, int* num, cudaStream_t stream) {
   if (len <= 0) return cudaSuccess;
   // in-place scan of the first `len` counts, total to num[0] (compression.cu:9-19)
-  block_exclusive_scan_kernel<int><<<1, 1024, 0, stream>>>(idx, idx, (uint32_t)len, num);
-  return cudaGetLastError();
+  return pdl_launch(block_exclusive_scan_kernel<int>, 1, 1024, 0, stream, idx, (uint32_t)len, num);
 }
 cudaError_t legacy_pack_launch(int n, int workers, const float* in, float* values, const int* begin, uint32_t* bitmap,
                                cudaStream_t stream) {
   if (n <= 0 || workers <= 0) return cudaSuccess;
   const int chunk = ceil_div_i(n, workers);
-  legacy_pack_kernel<<<(workers + 7) / 8, kThreads, 0, stream>>>(reinterpret_cast<const uint32_t*>(in), n, chunk,
-                                                                 workers, reinterpret_cast<uint32_t*>(values), begin,
-                                                                 bitmap);
-  return cudaGetLastError();
+  return pdl_launch(legacy_pack_kernel, (workers + 7) / 8, kThreads, 0, stream, reinterpret_cast<const uint32_t*>(in), n,
+                    chunk, workers, reinterpret_cast<uint32_t*>(values), begin, bitmap);
 }
 cudaError_t legacy_unpack_launch(const float* values, float* out, int n, int workers, const uint32_t* bitmap,
                                  const int* begin, cudaStream_t stream) {
   if (n <= 0 || workers <= 0) return cudaSuccess;
   const int chunk = ceil_div_i(n, workers);
-  legacy_unpack_kernel<<<(workers + 7) / 8, kThreads, 0, stream>>>(reinterpret_cast<const uint32_t*>(values),
-                                                                   reinterpret_cast<uint32_t*>(out), n, chunk, workers,
-                                                                   bitmap, begin);
-  return cudaGetLastError();
+  return pdl_launch(legacy_unpack_kernel, (workers + 7) / 8, kThreads, 0, stream, reinterpret_cast<const uint32_t*>(values),
+                    reinterpret_cast<uint32_t*>(out), n, chunk, workers, bitmap, begin);
 }
 
 }  // namespace csw

@@ -9,15 +9,12 @@ namespace csw {
 constexpr int SPARSE_TILE = 4096;  // elements per independently decodable tile
 
 // Native format.  tile_off must hold ceil(n/4096) words (it is used as the
-// count buffer first), bitmap ceil(n/32) words, values up to n floats.
-// *nnz_out (device or mapped host memory) receives the number of values.
+// count buffer first), bitmap ceil(n/32) words, values up to n floats; no other
+// memory is used.  *nnz_out (device or mapped host memory) receives the number of values.
 cudaError_t sparse_compress_launch(const float* in, uint64_t n, uint32_t* bitmap, float* values, uint32_t* tile_off,
                                    uint32_t* nnz_out, cudaStream_t stream);
-// Same result, with the per-tile counts kept in a scratch array the caller owns
-// (ceil(n/4096) words) instead of passing through tile_off.
-cudaError_t sparse_compress_scratch_launch(const float* in, uint64_t n, uint32_t* bitmap, float* values,
-                                           uint32_t* tile_off, uint32_t* tile_cnt_scratch, uint32_t* nnz_out,
-                                           cudaStream_t stream);
+// Makes the driver load every kernel sparse_compress_launch may use on the current device.
+cudaError_t sparse_compress_preload();
 // Single pass over the tensor: same bitmap, same per-tile contents, but the
 // tiles' value segments are laid out in the order the tiles claimed them
 // (tile_off says where each one starts).  *nnz_out must be DEVICE memory: it is

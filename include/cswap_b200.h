@@ -141,25 +141,20 @@ csw_status csw_sparse_compress_onepass(const float* d_in, size_t n, void* d_out,
  * hook invoked while the framework's allocator is locked or has just failed
  * (the moment swapping is most wanted), a callback where cudaMalloc's implicit
  * synchronisation would stall unrelated streams, or a host program that gets a
- * fixed memory budget at start-up.  The compressor's per-tile counters sit in
- * a fixed 256 KiB array inside the library image (present on every GPU that
- * loads the library until the process exits); the call performs no cudaMalloc,
- * cudaFree or other allocating call, and writes the same bytes to d_out and
- * the same count to *nnz_out as csw_sparse_compress.
+ * fixed memory budget at start-up.  The compressor keeps its
+ * working state in d_out; the call performs no cudaMalloc, cudaFree or other
+ * allocating call, and writes the same bytes to d_out and the same count to
+ * *nnz_out as csw_sparse_compress.
  *
  *  - n may be at most CSW_SPARSE_STATIC_MAX_ELEMS; larger inputs return
  *    CSW_ERR_LIMIT and launch nothing.
- *  - The first call on each device looks up the array's device address.  With
- *    the CUDA runtime's default lazy loading that first lookup (or launch) is
- *    also when the driver loads the library's kernels and the array itself
- *    onto the device, which does take device memory and can fail when none is
- *    left.  So make one warm-up call per device (n = 0 is enough) at start-up,
- *    outside any stream capture and before memory is tight; later calls on
- *    that device touch no allocator of any kind.
- *  - All calls share the one array: two calls whose kernels may run at the same
- *    time on the same GPU (different streams, no ordering between them) race
- *    and corrupt each other's output.  Calls ordered on one stream, or by
- *    events, are fine; nothing needs clearing between them. */
+ *  - With the CUDA runtime's default lazy loading the first launch of a kernel
+ *    on a device is also when the driver loads it there, which does take device
+ *    memory and can fail when none is left.  So make one warm-up call per
+ *    device with n = 0 at start-up, outside any stream capture and before memory
+ *    is tight: it loads every kernel of the compressor; later calls on that
+ *    device touch no allocator of any kind.
+ *  - Calls do not share anything: any number of them may be in flight. */
 #define CSW_SPARSE_STATIC_MAX_ELEMS 268435456u /* 65536 tiles of 4096 floats = 1 GiB of input */
 csw_status csw_sparse_compress_static(const float* d_in, size_t n, void* d_out, size_t cap, uint32_t* nnz_out,
                                       csw_stream_t stream);

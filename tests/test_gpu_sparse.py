@@ -210,3 +210,25 @@ def test_reference_layout(cs, oracle, n, dimsize):
     got = out0.cpu().numpy()
     keep = ~np.isnan(a)
     assert np.array_equal(got[keep], a[keep] + np.float32(0.0)) and np.isnan(got[~keep]).all()
+
+
+@pytest.mark.parametrize("n", [4095, 16 * 4096, 16 * 4096 + 1, 32 * 4096, 32 * 4096 + 1, 64 * 4096, 64 * 4096 + 1,
+                               16384 * 4096 // 64 + 4097])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_compress_at_the_edges_of_the_launch_rule(cs, oracle, n, offset):
+    """One cluster with one, two and four tiles per CTA, the three launches behind it; a tensor that starts on
+    and off a 16-byte boundary."""
+    import torch
+    a = util.relu_normal(n + offset, 0.5, seed=n + offset)[offset:]
+    t = torch.from_numpy(np.concatenate([np.zeros(offset, np.float32), a])).cuda()[offset:]
+    bitmap, values, tile_off, nnz = oracle.sparse_compress(a)
+    L = cs.sparse_layout(n)
+    for onepass in (False, True):
+        packed, nnz_t = cs.sparse_compress(t, onepass=onepass)
+        assert int(nnz_t.item()) == nnz
+        buf = packed.cpu().numpy()
+        assert np.array_equal(buf[L.bitmap:L.bitmap + 4 * bitmap.size].view(np.uint32), bitmap)
+        if not onepass:
+            assert np.array_equal(buf[:4 * tile_off.size].view(np.uint32), tile_off)
+            assert np.array_equal(buf[L.values:L.values + 4 * nnz].view(np.uint32), values.view(np.uint32))
+        assert torch.equal(cs.sparse_decompress(packed, n).view(torch.int32), t.view(torch.int32))
