@@ -140,7 +140,6 @@ sparse_pack_kernel(const uint32_t* __restrict__ in, uint64_t n, uint32_t* __rest
   __shared__ uint32_t warp_cnt[kThreads / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint64_t base = (uint64_t)blockIdx.x * kTile + (uint64_t)warp * (kWordsPerWarp * 32);
-  pdl_trigger();
   uint32_t v[kWordsPerWarp], w[kWordsPerWarp];
 #pragma unroll
   for (int j = 0; j < kWordsPerWarp; j++) {
@@ -187,7 +186,6 @@ sparse_small_kernel(const uint32_t* __restrict__ in, uint64_t n, uint32_t* __res
   const uint64_t base = (uint64_t)cta * (TILES * kTile) + (uint64_t)warp * (kWords * 32);
   cl.barrier_arrive();  // that every CTA of the cluster runs is only needed further down
   pdl_wait(in);
-  pdl_trigger();
   uint32_t v[kWords], w[kWords];
 #pragma unroll
   for (int j = 0; j < kWords; j++) {
@@ -251,7 +249,6 @@ sparse_onepass_kernel(const uint32_t* __restrict__ in, uint64_t n, uint32_t* __r
   __shared__ uint32_t tile_base;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint64_t base = (uint64_t)blockIdx.x * kTile + (uint64_t)warp * (kWordsPerWarp * 32);
-  pdl_trigger();
   uint32_t v[kWordsPerWarp], w[kWordsPerWarp];
 #pragma unroll
   for (int j = 0; j < kWordsPerWarp; j++) {
@@ -297,7 +294,6 @@ sparse_unpack_kernel(const uint32_t* __restrict__ bitmap, const uint32_t* __rest
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint64_t base = (uint64_t)blockIdx.x * kTile + (uint64_t)warp * (kWordsPerWarp * 32);
   const uint64_t word0 = base >> 5, nwords = (n + 31) >> 5;
-  pdl_trigger();
   pdl_wait(bitmap);
   asm volatile("" : "+l"(values), "+l"(tile_off));  // read behind the wait as well
   const uint32_t mine = (lane < kWordsPerWarp && word0 + lane < nwords) ? __ldg(bitmap + word0 + lane) : 0u;
@@ -341,7 +337,6 @@ __device__ __forceinline__ bool legacy_nz(uint32_t bits) { return __uint_as_floa
 
 __global__ void __launch_bounds__(kThreads)
 legacy_count_kernel(const uint32_t* __restrict__ in, int n, int chunk, int workers, int* __restrict__ count) {
-  pdl_trigger();
   pdl_wait(in);
   const int lane = threadIdx.x & 31;
   const int i = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
@@ -360,7 +355,6 @@ legacy_count_kernel(const uint32_t* __restrict__ in, int n, int chunk, int worke
 __global__ void __launch_bounds__(kThreads)
 legacy_pack_kernel(const uint32_t* __restrict__ in, int n, int chunk, int workers, uint32_t* __restrict__ values,
                    const int* __restrict__ begin, uint32_t* __restrict__ bitmap) {
-  pdl_trigger();
   pdl_wait(in);
   asm volatile("" : "+l"(begin));  // read behind the wait as well
   const int lane = threadIdx.x & 31;
@@ -388,7 +382,6 @@ legacy_pack_kernel(const uint32_t* __restrict__ in, int n, int chunk, int worker
 __global__ void __launch_bounds__(kThreads)
 legacy_unpack_kernel(const uint32_t* __restrict__ values, uint32_t* __restrict__ out, int n, int chunk, int workers,
                      const uint32_t* __restrict__ bitmap, const int* __restrict__ begin) {
-  pdl_trigger();
   pdl_wait(values);
   asm volatile("" : "+l"(bitmap), "+l"(begin));  // read behind the wait as well
   const int lane = threadIdx.x & 31;

@@ -109,7 +109,6 @@ zfp_encode_slab_kernel(const float* __restrict__ in, uint32_t* __restrict__ out,
   const int vz = zt >= nz ? 0 : (nz - zt < 4 ? (int)(nz - zt) : 4);
   static_assert(ENC_LUT_SIZE == 2 * kThreads, "two table words per thread");
   const uint32_t lut0 = __ldg(g_enc_table.v + tid), lut1 = __ldg(g_enc_table.v + kThreads + tid);
-  pdl_trigger();
   pdl_wait(in);
   float f[64];
   if (vz > 0) {
@@ -186,7 +185,6 @@ zfp_decode_slab_kernel(const uint32_t* __restrict__ in, float* __restrict__ out,
   for (int i = 0; i < DEC_LUT_SIZE / (4 * kThreads); i++)
     reinterpret_cast<uint4*>(lut)[i * kThreads + tid] =
         __ldg(reinterpret_cast<const uint4*>(g_dec_table.v) + i * kThreads + tid);
-  pdl_trigger();
   pdl_wait(in);
   if (zt < nz) {
     const uint32_t* src = in + ((size_t)blockIdx.x * kThreads + tid) * nwords;
@@ -272,7 +270,6 @@ zfp_encode_generic_kernel(FieldGeom g, const float* __restrict__ in, uint32_t* _
                           uint64_t nblocks) {
   __shared__ uint32_t lut[ENC_LUT_SIZE];
   for (int i = threadIdx.x; i < ENC_LUT_SIZE; i += blockDim.x) lut[i] = __ldg(g_enc_table.v + i);
-  pdl_trigger();
   pdl_wait(in);
   __syncthreads();
   const uint64_t b = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -289,7 +286,6 @@ zfp_decode_generic_kernel(FieldGeom g, const uint32_t* __restrict__ in, float* _
                           uint64_t nblocks, uint64_t total_words) {
   __shared__ uint32_t lut[DEC_LUT_SIZE];
   for (int i = threadIdx.x; i < DEC_LUT_SIZE; i += blockDim.x) lut[i] = __ldg(g_dec_table.v + i);
-  pdl_trigger();
   pdl_wait(in);
   __syncthreads();
   const uint64_t b = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
