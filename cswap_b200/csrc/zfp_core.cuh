@@ -447,8 +447,8 @@ struct SigState {
   }
 };
 
-// ---- encoder: one plane -----------------------------------------------------------
-// Codes plane word hi:lo (coefficient i at bit i, N coefficients) given the
+// ---- encoder: one plane of a 3-D block ----------------------------------------------
+// Codes plane word hi:lo (coefficient i at bit i, N = 64 coefficients) given the
 // significance state (encode.cuh:336-343).  Emission ignores the bit budget:
 // the stream is an exact prefix of the unlimited-budget stream, so the caller
 // stops once total() reaches maxbits and the emitter drops the overrun.
@@ -471,7 +471,7 @@ CSW_HD void encode_plane(uint32_t lo, uint32_t hi, SigState& sg, Emitter<WordSin
   const bool any = (xl | xh) != 0u;
   em.emit64((lo & sg.mlo) | (any ? sg.glo : 0u), (hi & sg.mhi) | (any ? sg.ghi : 0u), n + 1);
   if (!any) return;
-  const int top = (int)((N == 64 ? hi >> 31 : lo >> (N - 1)) & 1u);  // last position set: its 1 is implied
+  const int top = (int)(hi >> 31);  // last position set: its 1 is implied
   bool more;
   do {
     const uint32_t e = enc_lut[xl & 0xffu];
@@ -487,6 +487,44 @@ CSW_HD void encode_plane(uint32_t lo, uint32_t hi, SigState& sg, Emitter<WordSin
   } while (more);
   const int msb = hi ? 64 - clz32(hi) : 32 - clz32(lo);
   sg.set(msb);  // xs != 0, so the top set bit lies at or above n
+}
+
+// ---- encoder: one plane of a small block ---------------------------------------------
+// N = 4 or 16 coefficients: the whole code of a plane - verbatim prefix, group
+// test, expansions - is at most 32 bits (n verbatim bits, one test, two bits for
+// each of the N - n positions less the implied end), so it is put together
+// without a loop from one table entry per eight positions and appended at once.
+template <int N, class WordSink>
+CSW_HD void encode_plane_small(uint32_t x, int& n, Emitter<WordSink>& em, const uint32_t* enc_lut) {
+  static_assert(N == 16 || N == 4, "block size");
+  if (n >= N) {  // everything significant: the plane is copied verbatim
+    em.emit32(x, N);
+    return;
+  }
+  const uint32_t r = x >> n;
+  const int top = (int)(x >> (N - 1)) & 1;  // last position set: its 1 is implied
+  const uint32_t e0 = enc_lut[r & 0xffu];
+  uint32_t code = 0;
+  int len = 0;
+  if constexpr (N == 16) {
+    const uint32_t e1 = enc_lut[r >> 8];
+    const bool more = (r >> 8) != 0u;
+    const int len0 = more ? (int)((e0 >> 16) & 0x1fu) : (int)(e0 >> 24) - 2 * top;
+    const int len1 = more ? (int)(e1 >> 24) - 2 * top : 0;
+    code = e0 & (more ? 0xffffu : low_mask32(len0 + top - 1));
+    code |= (e1 & (more ? low_mask32(len1 + top - 1) : 0u)) << len0;
+    len = len0 + len1;
+  } else {
+    len = (int)(e0 >> 24) - 2 * top;
+    code = e0 & low_mask32(len + top - 1);
+  }
+  const uint32_t head = x & ((1u << n) - 1u);
+  if (r == 0u) {  // a failed group test
+    em.emit32(head, n + 1);
+    return;
+  }
+  em.emit32(head | (1u << n) | (code << (n + 1)), n + 1 + len);
+  n = 32 - clz32(x);
 }
 
 // ---- encoder: whole block ---------------------------------------------------------
@@ -516,23 +554,31 @@ CSW_HD void encode_block(const float (&f)[1 << (2 * DIMS)], int maxbits, WordSin
   uint32_t u[N];
   fwd_order<DIMS>(v, u, std::make_integer_sequence<int, N>{});
 
-  SigState sg;
-  sg.set(0);
-  for (int c = 3; c >= 0; c--) {  // planes 8c+7 .. 8c
-    const uint32_t sel = (uint32_t)c | ((uint32_t)(4 + c) << 4);
-    uint32_t lo[8], hi[8];
-    planes_of_byte<0>(u, sel, lo);
-    if constexpr (N == 64) {
+  if constexpr (N == 64) {
+    SigState sg;
+    sg.set(0);
+    for (int c = 3; c >= 0; c--) {  // planes 8c+7 .. 8c
+      const uint32_t sel = (uint32_t)c | ((uint32_t)(4 + c) << 4);
+      uint32_t lo[8], hi[8];
+      planes_of_byte<0>(u, sel, lo);
       planes_of_byte<1>(u, sel, hi);
-    } else {
 #pragma unroll
-      for (int k = 0; k < 8; k++) hi[k] = 0u;
+      for (int k = 7; k >= 0; k--) {
+        if (em.total() < maxbits) encode_plane<N>(lo[k], hi[k], sg, em, enc_lut);
+      }
+      if (em.total() >= maxbits) break;
     }
+  } else {
+    int n = 0;
+    for (int c = 3; c >= 0; c--) {
+      uint32_t x[8];
+      planes_of_byte<0>(u, (uint32_t)c | ((uint32_t)(4 + c) << 4), x);
 #pragma unroll
-    for (int k = 7; k >= 0; k--) {
-      if (em.total() < maxbits) encode_plane<N>(lo[k], hi[k], sg, em, enc_lut);
+      for (int k = 7; k >= 0; k--) {
+        if (em.total() < maxbits) encode_plane_small<N>(x[k], n, em, enc_lut);
+      }
+      if (em.total() >= maxbits) break;
     }
-    if (em.total() >= maxbits) break;
   }
   em.finish();
 }
@@ -776,7 +822,7 @@ struct Reader {
   }
 };
 
-// ---- decoder: one plane -----------------------------------------------------------
+// ---- decoder: one plane of a 3-D block ----------------------------------------------
 // decode.cuh:141-165 for one plane; returns the plane word.
 template <int N, class WordSource>
 CSW_HD uint64_t decode_plane(Reader<WordSource>& rd, int& n, int& bits, const uint32_t* dec_lut) {
@@ -814,36 +860,80 @@ CSW_HD uint64_t decode_plane(Reader<WordSource>& rd, int& n, int& bits, const ui
   return x;
 }
 
+// ---- decoder: one plane of a small block ----------------------------------------------
+// The code of a plane of N = 4 or 16 coefficients is at most 32 bits: one window
+// of the stream, consumed from the bottom, holds all of it.
+template <int N>
+CSW_HD uint32_t decode_plane_small(uint32_t win, int& n, int& left, const uint32_t* dec_lut) {
+  const int m = n < left ? n : left;
+  uint32_t x = win & low_mask32(m);
+  win >>= m;
+  left -= m;
+  if (n < N) {
+    int st = 0;
+    do {
+      const int lim = N - st - n;
+      int L = lim < 8 ? lim : 8;
+      L = left < L ? left : L;
+      const uint32_t e = dec_lut[dec_lut_index(L, st, win & 0xffu)];
+      const int used = dec_lut_used(e);
+      x |= dec_lut_pattern(e) << n;
+      n += dec_lut_advance(e);
+      win >>= used;
+      left -= used;
+      st = dec_lut_state(e);
+    } while (st != 2);
+  }
+  return x;
+}
+
 // ---- decoder: whole block ---------------------------------------------------------
 template <int DIMS, class WordSource>
 CSW_HD void decode_block(WordSource& src, int maxbits, float (&f)[1 << (2 * DIMS)], const uint32_t* dec_lut) {
   constexpr int N = 1 << (2 * DIMS);
-  Reader<WordSource> rd(src);
-  if (!(rd.peek() & 1u)) {  // zero block (decode.cuh:240-243, decode3.cuh:72-73)
+  const uint32_t head = src.get(0);
+  if (!(head & 1u)) {  // zero block (decode.cuh:240-243, decode3.cuh:72-73)
 #pragma unroll
     for (int i = 0; i < N; i++) f[i] = 0.0f;
     return;
   }
-  const uint32_t e = (rd.peek() >> 1) & 0xffu;
-  rd.skip(9);
-  int bits = maxbits - 9, n = 0;
+  const uint32_t e = (head >> 1) & 0xffu;
   uint32_t u[N];
 #pragma unroll
   for (int i = 0; i < N; i++) u[i] = 0;
-  for (int c = 3; c >= 0; c--) {
-    uint32_t lo[8], hi[8];
+  int left = maxbits - 9, n = 0;
+  if constexpr (N == 64) {
+    Reader<WordSource> rd(src);
+    rd.skip(9);
+    for (int c = 3; c >= 0; c--) {
+      uint32_t lo[8], hi[8];
 #pragma unroll
-    for (int k = 7; k >= 0; k--) {
-      uint64_t x = 0;
-      if (bits > 0) x = decode_plane<N>(rd, n, bits, dec_lut);
-      lo[k] = (uint32_t)x;
-      hi[k] = (uint32_t)(x >> 32);
+      for (int k = 7; k >= 0; k--) {
+        uint64_t x = 0;
+        if (left > 0) x = decode_plane<N>(rd, n, left, dec_lut);
+        lo[k] = (uint32_t)x;
+        hi[k] = (uint32_t)(x >> 32);
+      }
+      const uint32_t sel0 = (0x3210u & ~(0xfu << (4 * c))) | (4u << (4 * c));
+      const uint32_t step = 1u << (4 * c);
+      bytes_from_planes<0>(lo, sel0, step, u);
+      bytes_from_planes<1>(hi, sel0, step, u);
+      if (left <= 0) break;
     }
-    const uint32_t sel0 = (0x3210u & ~(0xfu << (4 * c))) | (4u << (4 * c));
-    const uint32_t step = 1u << (4 * c);
-    bytes_from_planes<0>(lo, sel0, step, u);
-    if constexpr (N == 64) bytes_from_planes<1>(hi, sel0, step, u);
-    if (bits <= 0) break;
+  } else {
+    for (int c = 3; c >= 0; c--) {
+      uint32_t x[8];
+#pragma unroll
+      for (int k = 7; k >= 0; k--) {
+        x[k] = 0u;
+        if (left > 0) {
+          const int pos = maxbits - left;
+          x[k] = decode_plane_small<N>(funnel_r(src.get(pos >> 5), src.get((pos >> 5) + 1), pos), n, left, dec_lut);
+        }
+      }
+      bytes_from_planes<0>(x, (0x3210u & ~(0xfu << (4 * c))) | (4u << (4 * c)), 1u << (4 * c), u);
+      if (left <= 0) break;
+    }
   }
   int v[N];
   inv_order<DIMS>(u, v, std::make_integer_sequence<int, N>{});

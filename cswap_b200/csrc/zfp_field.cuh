@@ -2,7 +2,8 @@
 // replicate padding of partial blocks, scatter, and stream sizing.
 // Follows CSWAP+/zfp/encode3.cuh:12-47,78-105, encode2.cuh, encode1.cuh,
 // encode.cuh:17-38 (pad_block), decode3.cuh:10-39 and shared.h:39-84.
-// Plain scalar code, shared by the generic CUDA kernels and host-side tests.
+// The geometry is shared by the kernels and the host; the scalar gather and
+// scatter drive the block coders in host-side tests.
 #pragma once
 #include <cstddef>
 #include <cstdint>

@@ -22,7 +22,7 @@
 //    took 168 us (32 KB more shared memory per CTA, 196 bytes of spills, and
 //    the CTAs of an SM marching through the same phase together); asking L2
 //    for the successor CTA's lines ahead of time cost 3 % in either kernel.
-//  * generic kernels, one thread per block straight from/to global memory, for
+//  * generic kernels, one thread per block with the same coders and staging, for
 //    any 1-D/2-D/3-D extents, strides, partial blocks and bit budgets.
 //
 // No kernel here waits on another CTA, a flag or a copy engine.
@@ -223,77 +223,266 @@ zfp_decode_slab_kernel(const uint32_t* __restrict__ in, float* __restrict__ out,
 }
 
 // =====================================================================================
-// generic kernels: one thread per block
+// generic kernels: one thread per block, any extents, strides and budgets
 // =====================================================================================
+// The same coders and the same word-major staging as the slab kernels; what differs
+// is how a lane finds its block and, for budgets that are not whole words, how the
+// stream is put together: 128 blocks of any budget are a whole number of words, so a
+// CTA's part of the stream is its own and is assembled from the staged columns -
+// no atomics, no zeroed stream.  (One thread per block reading and writing global
+// memory word by word, with plane-by-plane coders whose lanes wait for each other,
+// took 28.7 + 33.4 us a call for 31 x 33 x 4096 at 512 bits and 22.6 + 26.7 us for
+// 768 x 4096 at 128; these take 13.1 + 14.3 and 12.8 + 13.4.  They are bound as the
+// slab kernels are, by the number of instructions a block costs.)
 namespace {
 
-// Words of block b go to bit offset b * maxbits.  With whole words per block
-// they are plain stores; otherwise neighbours share words, the stream is
-// zeroed beforehand and words are OR-ed in.
-struct GlobalSink {
-  uint32_t* out;
-  uint64_t bit0;    // first bit of the block
-  int maxbits;
-  bool aligned;
-  __device__ __forceinline__ void put(int w, uint32_t v) {
-    const int left = maxbits - 32 * w;
-    if (left < 32) v &= (1u << left) - 1u;
-    const uint64_t p = bit0 + 32u * (uint32_t)w;
-    if (aligned) {
-      out[p >> 5] = v;
+// Where a block lies and how much of it: offsets of its four positions along an
+// axis, with the replicate padding of partial blocks (encode.cuh:17-38) folded in.
+__device__ __forceinline__ int pad_src(int i, int valid) { return i < valid ? i : (i == 3 ? 0 : valid - 1); }
+
+template <int DIMS>
+struct BlockAt {
+  int64_t base;
+  int vx, vy, vz;
+  __device__ __forceinline__ BlockAt(const FieldGeom& g, uint64_t b) {
+    uint32_t x, y = 0, z = 0;
+    if (DIMS == 1) {
+      x = (uint32_t)b;
+    } else if (b <= 0xffffffffu) {
+      const uint32_t i = (uint32_t)b, r = i / g.bx;
+      x = i - r * g.bx;
+      z = DIMS == 3 ? r / g.by : 0u;
+      y = r - z * (DIMS == 3 ? g.by : 0u);
     } else {
-      const uint32_t s = (uint32_t)(p & 31);
-      if (v << s) atomicOr(out + (p >> 5), v << s);
-      if (s && (v >> (32 - s))) atomicOr(out + (p >> 5) + 1, v >> (32 - s));
+      const uint64_t r = b / g.bx;
+      x = (uint32_t)(b - r * g.bx);
+      z = DIMS == 3 ? (uint32_t)(r / g.by) : 0u;
+      y = (uint32_t)(r - (uint64_t)z * (DIMS == 3 ? g.by : 0u));
     }
+    x *= 4; y *= 4; z *= 4;
+    vx = g.nx - x < 4 ? (int)(g.nx - x) : 4;
+    vy = DIMS >= 2 && g.ny - y < 4 ? (int)(g.ny - y) : 4;
+    vz = DIMS >= 3 && g.nz - z < 4 ? (int)(g.nz - z) : 4;
+    base = (int64_t)x * g.sx + (int64_t)y * g.sy + (int64_t)z * g.sz;
   }
 };
-struct GlobalSource {
-  const uint32_t* in;
-  uint64_t bit0;
-  uint64_t total_words;
-  int nwords;
-  __device__ __forceinline__ uint32_t get(int w) const {
-    if (w >= nwords) return 0u;
-    const uint64_t p = bit0 + 32u * (uint32_t)w, i = p >> 5;
-    const uint32_t s = (uint32_t)(p & 31);
-    uint32_t lo = i < total_words ? in[i] : 0u;
-    if (!s) return lo;
-    uint32_t hi = i + 1 < total_words ? in[i + 1] : 0u;
-    return (lo >> s) | (hi << (32 - s));
+
+// `vec`: rows of four values that start on a 16-byte boundary (decided for the whole field)
+template <int DIMS>
+__device__ __forceinline__ void load_block(const FieldGeom& g, const float* in, bool vec, const BlockAt<DIMS>& at,
+                                           float (&f)[1 << (2 * DIMS)]) {
+  const float* p = in + at.base;
+  if (vec && at.vx == 4) {
+#pragma unroll
+    for (int r = 0; r < (1 << (2 * DIMS)) / 4; r++) {
+      const float4 v = __ldg(reinterpret_cast<const float4*>(p + (DIMS >= 2 ? pad_src(r & 3, at.vy) * g.sy : 0) +
+                                                             (DIMS >= 3 ? pad_src(r >> 2, at.vz) * g.sz : 0)));
+      f[4 * r] = v.x;
+      f[4 * r + 1] = v.y;
+      f[4 * r + 2] = v.z;
+      f[4 * r + 3] = v.w;
+    }
+  } else {
+    int64_t ox[4];
+#pragma unroll
+    for (int x = 0; x < 4; x++) ox[x] = pad_src(x, at.vx) * g.sx;
+#pragma unroll
+    for (int r = 0; r < (1 << (2 * DIMS)) / 4; r++) {
+      const float* row = p + (DIMS >= 2 ? pad_src(r & 3, at.vy) * g.sy : 0) + (DIMS >= 3 ? pad_src(r >> 2, at.vz) * g.sz : 0);
+#pragma unroll
+      for (int x = 0; x < 4; x++) f[4 * r + x] = __ldg(row + ox[x]);
+    }
   }
+}
+template <int DIMS>
+__device__ __forceinline__ void store_block(const FieldGeom& g, float* out, bool vec, const BlockAt<DIMS>& at,
+                                            const float (&f)[1 << (2 * DIMS)]) {
+  float* p = out + at.base;
+#pragma unroll
+  for (int r = 0; r < (1 << (2 * DIMS)) / 4; r++) {
+    if ((DIMS < 2 || (r & 3) < at.vy) && (DIMS < 3 || (r >> 2) < at.vz)) {
+      float* row = p + (DIMS >= 2 ? (r & 3) * g.sy : 0) + (DIMS >= 3 ? (r >> 2) * g.sz : 0);
+      if (vec && at.vx == 4) {
+        *reinterpret_cast<float4*>(row) = make_float4(f[4 * r], f[4 * r + 1], f[4 * r + 2], f[4 * r + 3]);
+      } else {
+#pragma unroll
+        for (int x = 0; x < 4; x++)
+          if (x < at.vx) row[x * g.sx] = f[4 * r + x];
+      }
+    }
+  }
+}
+
+// 3-D blocks whose rows do not start on 16-byte boundaries, x contiguous: the rows of a
+// warp's 32 blocks go through shared memory so that a store instruction writes 32
+// neighbouring values (lanes storing their own values one by one write 4 of every
+// 16 bytes: four times the write transactions; 31 x 33 x 4096 at 512 bits 17.9 -> 14.3
+// us, 7 x 7 x 65536 21.1 -> 13.5).  `buf`: 512 words of the warp's own;
+// every lane of the warp calls.
+__device__ __forceinline__ void store_rows3(const FieldGeom& g, float* out, const BlockAt<3>& at, bool valid, float* buf,
+                                            const float (&f)[64]) {
+  const int lane = threadIdx.x & 31, x = lane & 3;
+  const int have = valid ? at.vx | at.vy << 4 | at.vz << 8 : 0;
+  float* dst[4];
+  int vy[4], vz[4];
+#pragma unroll
+  for (int q = 0; q < 4; q++) {  // pass q stores value x of block 8q + lane / 4
+    const int src = 8 * q + (lane >> 2), h = __shfl_sync(0xffffffffu, have, src);
+    dst[q] = out + __shfl_sync(0xffffffffu, at.base, src) + x;
+    vy[q] = x < (h & 15) ? h >> 4 & 15 : 0;
+    vz[q] = h >> 8;
+  }
+#pragma unroll
+  for (int z = 0; z < 4; z++) {
+#pragma unroll
+    for (int y = 0; y < 4; y++)
+      *reinterpret_cast<float4*>(buf + 128 * y + 4 * lane) =
+          make_float4(f[16 * z + 4 * y], f[16 * z + 4 * y + 1], f[16 * z + 4 * y + 2], f[16 * z + 4 * y + 3]);
+    __syncwarp();
+#pragma unroll
+    for (int y = 0; y < 4; y++)
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+        if (y < vy[q] && z < vz[q]) dst[q][y * g.sy + z * g.sz] = buf[128 * y + 32 * q + lane];
+    __syncwarp();
+  }
+}
+
+// a lane's column of the staging area as a word sink / source of the small-block coders
+struct ColumnSink {
+  uint32_t* p;
+  __device__ __forceinline__ void put(int w, uint32_t v) { p[w * kThreads] = v; }
+};
+struct ColumnSource {
+  const uint32_t* p;
+  __device__ __forceinline__ uint32_t get(int w) const { return p[w * kThreads]; }
 };
 
 template <int DIMS>
-__global__ void __launch_bounds__(128)
-zfp_encode_generic_kernel(FieldGeom g, const float* __restrict__ in, uint32_t* __restrict__ out, int maxbits,
-                          uint64_t nblocks) {
-  __shared__ uint32_t lut[ENC_LUT_SIZE];
-  for (int i = threadIdx.x; i < ENC_LUT_SIZE; i += blockDim.x) lut[i] = __ldg(g_enc_table.v + i);
+__global__ void __launch_bounds__(kThreads, DIMS == 3 ? kEncCtasPerSm : 8)
+zfp_encode_generic_kernel(const FieldGeom g, const float* __restrict__ in, bool vec, uint32_t* __restrict__ out,
+                          int maxbits, uint64_t nblocks, uint64_t total_words, const PipeConsts kc) {
+  extern __shared__ __align__(16) uint32_t smem_words[];
+  const int nwords = (maxbits + 31) >> 5, tid = threadIdx.x;
+  uint32_t* stage = smem_words;
+  uint32_t* queue = stage + (nwords + STAGE_SPARE_ROWS) * kThreads;
+  uint32_t* lut = queue + (DIMS == 3 ? QUEUE_SLOTS * QUEUE_FIELDS * kThreads : 0);
+  const uint32_t lut0 = __ldg(g_enc_table.v + tid), lut1 = __ldg(g_enc_table.v + kThreads + tid);
+  const uint64_t b0 = (uint64_t)blockIdx.x * kThreads, b = b0 + tid;
   pdl_wait(in);
-  __syncthreads();
-  const uint64_t b = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= nblocks) return;
   float f[1 << (2 * DIMS)];
-  gather_block<DIMS>(g, in, b, f);
-  GlobalSink sink{out, b * (uint64_t)maxbits, maxbits, (maxbits & 31) == 0};
-  encode_block<DIMS>(f, maxbits, sink, lut);
+  if (b < nblocks) load_block<DIMS>(g, in, vec, BlockAt<DIMS>(g, b), f);
+  lut[tid] = lut0;
+  lut[kThreads + tid] = lut1;
+  uint32_t* col = stage + tid;
+  if (DIMS == 3) {
+    for (int w = 0; w < nwords; w++) col[w * kThreads] = 0u;  // coded bits are OR-ed in
+  }
+  __syncthreads();  // the table is complete
+  if (b < nblocks) {
+    if constexpr (DIMS == 3) {
+      SmemStage st{col, queue + tid};
+      encode_block3_staged(f, maxbits, st, lut, kc);
+    } else {
+      ColumnSink sink{col};
+      encode_block<DIMS>(f, maxbits, sink, lut);
+    }
+  }
+  if ((maxbits & 31) == 0) {  // whole words per block: every lane writes its own
+    if (b < nblocks) {
+      uint32_t* dst = out + b * nwords;
+      if ((nwords & 3) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0) {
+        for (int w = 0; w < nwords; w += 4)
+          *reinterpret_cast<uint4*>(dst + w) = make_uint4(col[w * kThreads], col[(w + 1) * kThreads],
+                                                          col[(w + 2) * kThreads], col[(w + 3) * kThreads]);
+      } else {
+        for (int w = 0; w < nwords; w++) dst[w] = col[w * kThreads];
+      }
+      // the stream is whole 64-bit words: the last 32 bits may belong to no block
+      if (b == nblocks - 1 && nblocks * nwords < total_words) dst[nwords] = 0u;
+    }
+    return;
+  }
+  __syncthreads();  // every column is complete
+  const uint64_t first = b0 * (uint64_t)maxbits >> 5;  // of this CTA's words; b0 * maxbits is a multiple of 32
+  const int here = nblocks - b0 < kThreads ? (int)(nblocks - b0) : kThreads;
+  const uint64_t left = total_words - first;
+  const int mine = here < kThreads ? (int)left : 4 * maxbits;
+  for (int w = tid; w < mine; w += kThreads) {
+    uint32_t v = 0;
+    int blk = 32 * w / maxbits, off = 32 * w - blk * maxbits;
+    for (int have = 0; have < 32 && blk < here; blk++, off = 0) {
+      const uint32_t* c = stage + blk + (off >> 5) * kThreads;  // the row behind the last one exists
+      const int take = maxbits - off < 32 - have ? maxbits - off : 32 - have;
+      v |= (funnel_r(c[0], c[kThreads], off) & low_mask32(take)) << have;
+      have += take;
+    }
+    out[first + w] = v;
+  }
 }
 
 template <int DIMS>
-__global__ void __launch_bounds__(128)
-zfp_decode_generic_kernel(FieldGeom g, const uint32_t* __restrict__ in, float* __restrict__ out, int maxbits,
-                          uint64_t nblocks, uint64_t total_words) {
-  __shared__ uint32_t lut[DEC_LUT_SIZE];
-  for (int i = threadIdx.x; i < DEC_LUT_SIZE; i += blockDim.x) lut[i] = __ldg(g_dec_table.v + i);
+__global__ void __launch_bounds__(kThreads, DIMS == 3 ? kDecCtasPerSm : 8)
+zfp_decode_generic_kernel(const FieldGeom g, const uint32_t* __restrict__ in, float* __restrict__ out, bool vec,
+                          int maxbits, uint64_t nblocks, uint64_t total_words, const PipeConsts kc) {
+  extern __shared__ __align__(16) uint32_t smem_words[];
+  const int nwords = (maxbits + 31) >> 5, tid = threadIdx.x;
+  uint32_t* stage = smem_words;
+  uint32_t* lut = stage + (nwords + STAGE_SPARE_ROWS) * kThreads;
+  uint32_t* col = stage + tid;
+#pragma unroll
+  for (int i = 0; i < DEC_LUT_SIZE / (4 * kThreads); i++)
+    reinterpret_cast<uint4*>(lut)[i * kThreads + tid] =
+        __ldg(reinterpret_cast<const uint4*>(g_dec_table.v) + i * kThreads + tid);
+  // reads just past a block find zeros and need no bounds test
+  for (int w = nwords; w < nwords + STAGE_SPARE_ROWS; w++) col[w * kThreads] = 0u;
+  __syncthreads();  // the table is complete
   pdl_wait(in);
-  __syncthreads();
-  const uint64_t b = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= nblocks) return;
-  float f[1 << (2 * DIMS)];
-  GlobalSource source{in, b * (uint64_t)maxbits, total_words, (maxbits + 31) >> 5};
-  decode_block<DIMS>(source, maxbits, f, lut);
-  scatter_block<DIMS>(g, out, b, f);
+  // whole warps go round: the 3-D parser takes a minimum over all lanes
+  for (uint64_t wb = (uint64_t)blockIdx.x * kThreads + (tid & ~31); wb < nblocks; wb += (uint64_t)gridDim.x * kThreads) {
+    const uint64_t b = wb + (tid & 31), bit0 = b * (uint64_t)maxbits, w0 = bit0 >> 5;
+    const int s = (int)(bit0 & 31);
+    if (b >= nblocks) {
+      col[0] = 0u;  // an empty block, not stored
+    } else if ((maxbits & 127) == 0 && (reinterpret_cast<uintptr_t>(in) & 15) == 0) {
+      for (int w = 0; w < nwords; w += 4) {
+        const uint4 v = __ldg(reinterpret_cast<const uint4*>(in + w0 + w));
+        col[w * kThreads] = v.x;
+        col[(w + 1) * kThreads] = v.y;
+        col[(w + 2) * kThreads] = v.z;
+        col[(w + 3) * kThreads] = v.w;
+      }
+    } else {
+      uint32_t lo = __ldg(in + w0);
+      for (int w = 0; w < nwords; w++) {
+        const uint32_t hi = w0 + w + 1 < total_words ? __ldg(in + w0 + w + 1) : 0u;
+        col[w * kThreads] = funnel_r(lo, hi, s);
+        lo = hi;
+      }
+    }
+    float f[1 << (2 * DIMS)];
+    if constexpr (DIMS == 3) {
+      StageWords source{col};
+      decode_block3_pos(source, maxbits, f, lut, kc);
+    } else {
+      ColumnSource source{col};
+      decode_block<DIMS>(source, maxbits, f, lut);
+    }
+    const BlockAt<DIMS> at(g, b < nblocks ? b : nblocks - 1);
+    if constexpr (DIMS == 3) {
+      if (!vec && g.sx == 1) {
+        store_rows3(g, out, at, b < nblocks, reinterpret_cast<float*>(lut + DEC_LUT_SIZE) + 512 * (tid >> 5), f);
+        continue;
+      }
+    }
+    if (b < nblocks) store_block<DIMS>(g, out, vec, at, f);
+  }
+}
+
+// rows of four values start on 16-byte boundaries
+bool vector_rows(const FieldGeom& g, const void* field) {
+  return g.sx == 1 && (g.dims < 2 || g.sy % 4 == 0) && (g.dims < 3 || g.sz % 4 == 0) &&
+         (reinterpret_cast<uintptr_t>(field) & 15) == 0;
 }
 
 }  // namespace
@@ -302,10 +491,19 @@ zfp_decode_generic_kernel(FieldGeom g, const uint32_t* __restrict__ in, float* _
 // launchers
 // =====================================================================================
 constexpr size_t kDefaultDynamicSmem = 48 * 1024;  // what a kernel may ask for without opting in
-static size_t slab_smem_bytes(int maxbits, bool decode) {
-  if (decode)
-    return (size_t)((maxbits >> 5) + STAGE_SPARE_ROWS) * kThreads * 4 + DEC_LUT_SIZE * 4;
-  return (size_t)((maxbits >> 5) + STAGE_SPARE_ROWS + QUEUE_SLOTS * QUEUE_FIELDS) * kThreads * 4 + ENC_LUT_SIZE * 4;
+constexpr uint64_t kFullGrid = 148 * 8;             // CTAs the device holds at eight per SM
+constexpr int kMostBits = 4096;                    // largest budget the library accepts
+static size_t staged_smem_bytes(int maxbits, bool decode, int dims, bool rowbuf = false) {
+  const size_t rows = ((size_t)maxbits + 31) / 32 + STAGE_SPARE_ROWS;
+  if (decode) return rows * kThreads * 4 + DEC_LUT_SIZE * 4 + (rowbuf ? kThreads * 16 * 4 : 0);
+  return (rows + (dims == 3 ? QUEUE_SLOTS * QUEUE_FIELDS : 0)) * kThreads * 4 + ENC_LUT_SIZE * 4;
+}
+// Only the largest budgets need it; the call costs host time on every launch.
+template <class K>
+static cudaError_t allow_smem(K* kernel, size_t smem, bool decode, int dims) {
+  if (smem <= kDefaultDynamicSmem) return cudaSuccess;
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)staged_smem_bytes(kMostBits, decode, dims, true));
 }
 
 bool zfp_slab_eligible(const FieldGeom& g, const void* field, const void* stream, int maxbits) {
@@ -314,59 +512,61 @@ bool zfp_slab_eligible(const FieldGeom& g, const void* field, const void* stream
          (reinterpret_cast<uintptr_t>(stream) & 15) == 0;
 }
 
+template <int DIMS>
+static cudaError_t encode_generic(const FieldGeom& g, const float* in, uint32_t* out, int maxbits, uint64_t nblocks,
+                                  cudaStream_t stream) {
+  const size_t smem = staged_smem_bytes(maxbits, false, DIMS);
+  cudaError_t e = allow_smem(zfp_encode_generic_kernel<DIMS>, smem, false, DIMS);
+  if (e != cudaSuccess) return e;
+  return pdl_launch(zfp_encode_generic_kernel<DIMS>, (unsigned)((nblocks + kThreads - 1) / kThreads), kThreads, smem, stream,
+                    g, in, vector_rows(g, in), out, maxbits, nblocks, (uint64_t)stream_bytes(g, (unsigned)maxbits) / 4,
+                    pipe_consts());
+}
+template <int DIMS>
+static cudaError_t decode_generic(const FieldGeom& g, const uint32_t* in, float* out, int maxbits, uint64_t nblocks,
+                                  cudaStream_t stream) {
+  const size_t smem = staged_smem_bytes(maxbits, true, DIMS, DIMS == 3);
+  cudaError_t e = allow_smem(zfp_decode_generic_kernel<DIMS>, smem, true, DIMS);
+  if (e != cudaSuccess) return e;
+  const uint64_t ctas = (nblocks + kThreads - 1) / kThreads;
+  // The parser table is 18 KiB and 128 small blocks are 8 KiB of field or less: once
+  // every SM has its eight CTAs, a CTA takes up to eight rounds of blocks.
+  const uint64_t rounds = DIMS == 3 || ctas < 2 * kFullGrid ? 1 : ctas / kFullGrid < 8 ? ctas / kFullGrid : 8;
+  return pdl_launch(zfp_decode_generic_kernel<DIMS>, (unsigned)((ctas + rounds - 1) / rounds), kThreads, smem, stream,
+                    g, in, out, vector_rows(g, out), maxbits, nblocks, (uint64_t)stream_bytes(g, (unsigned)maxbits) / 4,
+                    pipe_consts());
+}
+
 cudaError_t zfp_encode_launch(const FieldGeom& g, const float* in, void* out, int maxbits, cudaStream_t stream) {
   const uint64_t nblocks = geom_blocks(g);
   if (nblocks == 0) return cudaSuccess;
+  uint32_t* o = reinterpret_cast<uint32_t*>(out);
   if (zfp_slab_eligible(g, in, out, maxbits)) {
-    const size_t smem = slab_smem_bytes(maxbits, false);
-    if (smem > kDefaultDynamicSmem) {  // only the largest budgets: the call costs host time on every launch
-      cudaError_t e = cudaFuncSetAttribute(zfp_encode_slab_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)slab_smem_bytes(2048, false));
-      if (e != cudaSuccess) return e;
-    }
-    const uint32_t ngroups = (g.nz + kGroupSlabs - 1) / kGroupSlabs;
-    return pdl_launch(zfp_encode_slab_kernel, ngroups, kThreads, smem, stream, in, reinterpret_cast<uint32_t*>(out), g.nz,
+    const size_t smem = staged_smem_bytes(maxbits, false, 3);
+    cudaError_t e = allow_smem(zfp_encode_slab_kernel, smem, false, 3);
+    if (e != cudaSuccess) return e;
+    return pdl_launch(zfp_encode_slab_kernel, (g.nz + kGroupSlabs - 1) / kGroupSlabs, kThreads, smem, stream, in, o, g.nz,
                       maxbits, pipe_consts());
   }
-  if (maxbits & 31) {
-    cudaError_t e = cudaMemsetAsync(out, 0, stream_bytes(g, (unsigned)maxbits), stream);
-    if (e != cudaSuccess) return e;
-  } else if ((nblocks * (uint64_t)maxbits) & 63) {
-    // whole 32-bit words per block but an odd number of them in total: the
-    // stream is sized in 64-bit words, so its last 32 bits belong to no block
-    const size_t nbytes = stream_bytes(g, (unsigned)maxbits);
-    cudaError_t e = cudaMemsetAsync(static_cast<char*>(out) + nbytes - 8, 0, 8, stream);
-    if (e != cudaSuccess) return e;
-  }
-  const unsigned grid = (unsigned)((nblocks + 127) / 128);
-  uint32_t* o = reinterpret_cast<uint32_t*>(out);
-  const auto kernel = g.dims == 3   ? zfp_encode_generic_kernel<3>
-                      : g.dims == 2 ? zfp_encode_generic_kernel<2>
-                                    : zfp_encode_generic_kernel<1>;
-  return pdl_launch(kernel, grid, 128, 0, stream, g, in, o, maxbits, nblocks);
+  return g.dims == 3   ? encode_generic<3>(g, in, o, maxbits, nblocks, stream)
+         : g.dims == 2 ? encode_generic<2>(g, in, o, maxbits, nblocks, stream)
+                       : encode_generic<1>(g, in, o, maxbits, nblocks, stream);
 }
 
 cudaError_t zfp_decode_launch(const FieldGeom& g, const void* in, float* out, int maxbits, cudaStream_t stream) {
   const uint64_t nblocks = geom_blocks(g);
   if (nblocks == 0) return cudaSuccess;
-  if (zfp_slab_eligible(g, out, in, maxbits)) {
-    const size_t smem = slab_smem_bytes(maxbits, true);
-    if (smem > kDefaultDynamicSmem) {
-      cudaError_t e = cudaFuncSetAttribute(zfp_decode_slab_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)slab_smem_bytes(2048, true));
-      if (e != cudaSuccess) return e;
-    }
-    const uint32_t ngroups = (g.nz + kGroupSlabs - 1) / kGroupSlabs;
-    return pdl_launch(zfp_decode_slab_kernel, ngroups, kThreads, smem, stream, reinterpret_cast<const uint32_t*>(in), out,
-                      g.nz, maxbits, pipe_consts());
-  }
-  const unsigned grid = (unsigned)((nblocks + 127) / 128);
   const uint32_t* i32 = reinterpret_cast<const uint32_t*>(in);
-  const uint64_t total_words = stream_bytes(g, (unsigned)maxbits) / 4;
-  const auto kernel = g.dims == 3   ? zfp_decode_generic_kernel<3>
-                      : g.dims == 2 ? zfp_decode_generic_kernel<2>
-                                    : zfp_decode_generic_kernel<1>;
-  return pdl_launch(kernel, grid, 128, 0, stream, g, i32, out, maxbits, nblocks, total_words);
+  if (zfp_slab_eligible(g, out, in, maxbits)) {
+    const size_t smem = staged_smem_bytes(maxbits, true, 3);
+    cudaError_t e = allow_smem(zfp_decode_slab_kernel, smem, true, 3);
+    if (e != cudaSuccess) return e;
+    return pdl_launch(zfp_decode_slab_kernel, (g.nz + kGroupSlabs - 1) / kGroupSlabs, kThreads, smem, stream, i32, out, g.nz,
+                      maxbits, pipe_consts());
+  }
+  return g.dims == 3   ? decode_generic<3>(g, i32, out, maxbits, nblocks, stream)
+         : g.dims == 2 ? decode_generic<2>(g, i32, out, maxbits, nblocks, stream)
+                       : decode_generic<1>(g, i32, out, maxbits, nblocks, stream);
 }
 
 }  // namespace csw

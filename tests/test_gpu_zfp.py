@@ -92,6 +92,24 @@ def test_generic_odd_word_count_writes_every_byte(cs, oracle, dims, maxbits):
     assert np.array_equal(out.cpu().numpy().view(np.uint64), ref)
 
 
+@pytest.mark.parametrize("dims", [(4 * 127, 0, 0), (4 * 129 - 1, 0, 0), (31, 62, 0), (4 * 16, 4 * 8, 0), (4 * 16, 36, 0),
+                                  (16, 16, 31), (15, 16, 32), (13, 40, 13)])
+@pytest.mark.parametrize("maxbits", [9, 33, 128, 300, 2048, 4096])
+def test_generic_cta_edges(cs, oracle, dims, maxbits):
+    """127, 128 and 129 blocks and ragged warps: the last CTA's part of the stream, budgets that share
+    words between blocks, the smallest and the largest budget; the buffer holds other bytes before."""
+    import torch
+    nx, ny, nz = dims
+    n = nx * max(ny, 1) * max(nz, 1)
+    a = util.block_zoo((n + 63) // 64 * 64, seed=n + maxbits)[:n]
+    out = torch.full((cs.zfp_max_bytes(nx, ny, nz, maxbits),), 0xFF, dtype=torch.uint8, device="cuda")
+    cs.zfp_compress(torch.from_numpy(a).cuda(), maxbits, dims, out=out)
+    ref = oracle.zfp_encode(a, nx, ny, nz, maxbits)
+    assert np.array_equal(out.cpu().numpy().view(np.uint64), ref)
+    back = cs.zfp_decompress(out, n, maxbits, dims).cpu().numpy()
+    assert np.array_equal(back.view(np.uint32), oracle.zfp_decode(ref, nx, ny, nz, maxbits).view(np.uint32))
+
+
 def test_special_values(cs, oracle):
     n = 1024 * 16
     a = np.zeros(n, dtype=np.float32)
