@@ -363,3 +363,26 @@ def test_decode_arbitrary_streams(cs, oracle, dims, maxbits):
         got = cs.zfp_decompress(stream, nx * ny * nz, maxbits, dims).cpu().numpy()
         assert np.array_equal(got.view(np.uint32), ref.view(np.uint32))
     assert cs.lib().csw_device_status(None) == 0
+
+
+@pytest.mark.parametrize("nx,ny,nz,maxbits", [(32, 32, 3071, 512), (32, 32, 3072, 512), (32, 32, 3073, 1024),
+                                              (32, 32, 16387, 256), (1000, 500, 9, 512), (70, 50, 1003, 64)])
+def test_host_calls_cut_anywhere(cs, nx, ny, nz, maxbits):
+    """Host field and host stream just below and above the size from which the calls are cut into
+    chunks, slab counts that no chunk divides, slabs larger than a chunk: the stream and the values
+    are those of the call on device memory."""
+    import ctypes as C
+    import torch
+    from cswap_b200._lib import Bitstream, ZfpField, ZfpStream
+    L = cs.lib()
+    t = torch.from_numpy(util.tanh_normal(nx * ny * nz, seed=nz))
+    want = cs.zfp_compress(t.cuda(), maxbits, (nx, ny, nz)).cpu()
+    stream, back = torch.empty_like(want).pin_memory(), torch.empty_like(t).pin_memory()
+    p = stream.data_ptr()
+    bs = Bitstream(64, 0, p, p, p + stream.numel())
+    zs = ZfpStream(maxbits, maxbits, 32, -1074, C.pointer(bs))
+    src, dst = (ZfpField(3, nx, ny, nz, 0, 0, 0, 0, 0, x.data_ptr()) for x in (t, back))
+    assert L.cuda_compress(C.byref(zs), C.byref(src)) == stream.numel()
+    assert torch.equal(stream, want)
+    L.cuda_decompress(C.byref(zs), C.byref(dst))
+    assert torch.equal(back, cs.zfp_decompress(want.cuda(), t.numel(), maxbits, (nx, ny, nz)).cpu())
