@@ -6,7 +6,7 @@
 //
 //  * slab kernels for the swap path's view (nx = ny = 32, contiguous, whole
 //    32-bit words per block): one CTA per group of 8 z-slabs (32 KiB, 128
-//    blocks), four (encoder) or five (decoder) CTAs per SM, lane = zfp block
+//    blocks; fewer when the tensor is small), four (encoder) or five (decoder) CTAs per SM, lane = zfp block
 //    held in registers.  A lane moves its block with sixteen 128-bit accesses
 //    (eight neighbouring lanes cover one 128-byte row segment, so a warp
 //    access touches four whole lines); stream words sit word-major in shared
@@ -40,7 +40,6 @@ namespace {
 
 constexpr int kThreads = 128;                  // zfp blocks (lanes) per CTA
 constexpr int kSlabFloats = 1024;              // one 32x32 z-slab
-constexpr int kGroupSlabs = kThreads / 16;      // z-slabs per CTA: kThreads / 64 tiles of four
 constexpr int kEncCtasPerSm = 4;                // 128 registers per thread: the encoder needs 122
 constexpr int kDecCtasPerSm = 5;                // 96 registers: the decoder fits without spills, and a fifth
                                                 // CTA hides more of its dependent shared-memory reads
@@ -79,6 +78,15 @@ constexpr EncTable make_enc_table() {
 }
 __device__ const EncTable g_enc_table = make_enc_table();
 
+// Block of this thread: a warp takes 1 << lsh neighbouring blocks.  With lsh < 5 the lanes
+// above do the work of the ones below a second time - the same data, so they cost
+// nothing - and store nothing (blocks_per_warp says when).
+__device__ __forceinline__ uint64_t block_of_thread(int lsh) {
+  const uint64_t warp = (uint64_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
+  return (warp << lsh) + (threadIdx.x & ((1u << lsh) - 1u));
+}
+__device__ __forceinline__ bool is_copy(int lsh) { return ((threadIdx.x & 31) >> lsh) != 0; }
+
 // z-slab that feeds row z of a block with vz valid slabs (encode.cuh:17-38
 // applied along z: a,a,a,a / a,b,b,a / a,b,c,a)
 __device__ __forceinline__ int pad_src_z(int z, int vz) { return z < vz ? z : (z == 3 ? 0 : vz - 1); }
@@ -88,13 +96,14 @@ __device__ __forceinline__ int pad_src_z(int z, int vz) { return z < vz ? z : (z
 // =====================================================================================
 // slab encoder
 // =====================================================================================
-// One CTA per group of 8 z-slabs (128 blocks, lane = block).  A lane reads its
+// One CTA per group of 8 z-slabs (128 blocks, lane = block; blocks_per_warp when the tensor is
+// small).  A lane reads its
 // 4x4x4 block with sixteen 128-bit loads (eight neighbouring lanes cover one
 // 128-byte row segment, so a warp load touches four full lines), codes it into
 // its own column of the word-major staging area and writes its own words out:
 // after the table is built no warp waits for another.
 __global__ void __launch_bounds__(kThreads, kEncCtasPerSm)
-zfp_encode_slab_kernel(const float* __restrict__ in, uint32_t* __restrict__ out, uint32_t nz, int maxbits,
+zfp_encode_slab_kernel(const float* __restrict__ in, uint32_t* __restrict__ out, uint32_t nz, int maxbits, int lsh,
                        const PipeConsts kc) {
   extern __shared__ __align__(16) uint32_t smem_words[];
   const int nwords = maxbits >> 5;
@@ -103,9 +112,10 @@ zfp_encode_slab_kernel(const float* __restrict__ in, uint32_t* __restrict__ out,
   uint32_t* lut = queue + QUEUE_SLOTS * QUEUE_FIELDS * kThreads;
 
   const int tid = threadIdx.x;
-  // my block: tile t of the group (4 slabs), block (bx, by) of its 8x8 grid
-  const int t = tid >> 6, bx = tid & 7, by = (tid >> 3) & 7;
-  const uint32_t zt = (blockIdx.x * (kThreads / 64) + t) * 4;  // first slab of my tile
+  // my block: (bx, by) of the 8x8 grid of its tile of four slabs
+  const uint32_t b = (uint32_t)block_of_thread(lsh);
+  const int bx = b & 7, by = (b >> 3) & 7;
+  const uint32_t zt = (b >> 6) * 4;  // first slab of my tile
   const int vz = zt >= nz ? 0 : (nz - zt < 4 ? (int)(nz - zt) : 4);
   static_assert(ENC_LUT_SIZE == 2 * kThreads, "two table words per thread");
   const uint32_t lut0 = __ldg(g_enc_table.v + tid), lut1 = __ldg(g_enc_table.v + kThreads + tid);
@@ -136,7 +146,8 @@ zfp_encode_slab_kernel(const float* __restrict__ in, uint32_t* __restrict__ out,
   encode_block3_staged(f, maxbits, st, lut, kc);
 
   // a lane's words sit in its own column: no barrier before reading them back
-  uint32_t* dst = out + ((size_t)blockIdx.x * kThreads + tid) * nwords;
+  if (is_copy(lsh)) return;
+  uint32_t* dst = out + (size_t)b * nwords;
   const uint32_t* col = stage + tid;
   if ((nwords & 3) == 0) {
     for (int w = 0; w < nwords; w += 4)
@@ -170,7 +181,7 @@ static_assert(DEC_LUT_SIZE % (4 * kThreads) == 0, "table copy assumes whole 128-
 // area, parses them by bit position and stores the rebuilt 4x4x4 block with
 // sixteen 128-bit stores.  The only barrier is the one after the table copy.
 __global__ void __launch_bounds__(kThreads, kDecCtasPerSm)
-zfp_decode_slab_kernel(const uint32_t* __restrict__ in, float* __restrict__ out, uint32_t nz, int maxbits,
+zfp_decode_slab_kernel(const uint32_t* __restrict__ in, float* __restrict__ out, uint32_t nz, int maxbits, int lsh,
                        const PipeConsts kc) {
   extern __shared__ __align__(16) uint32_t smem_words[];
   const int nwords = maxbits >> 5;
@@ -178,8 +189,9 @@ zfp_decode_slab_kernel(const uint32_t* __restrict__ in, float* __restrict__ out,
   uint32_t* lut = stage + (nwords + STAGE_SPARE_ROWS) * kThreads;
 
   const int tid = threadIdx.x;
-  const int t = tid >> 6, bx = tid & 7, by = (tid >> 3) & 7;
-  const uint32_t zt = (blockIdx.x * (kThreads / 64) + t) * 4;  // first slab of my tile
+  const uint32_t b = (uint32_t)block_of_thread(lsh);
+  const int bx = b & 7, by = (b >> 3) & 7;
+  const uint32_t zt = (b >> 6) * 4;  // first slab of my tile
   uint32_t* col = stage + tid;
 #pragma unroll
   for (int i = 0; i < DEC_LUT_SIZE / (4 * kThreads); i++)
@@ -187,7 +199,7 @@ zfp_decode_slab_kernel(const uint32_t* __restrict__ in, float* __restrict__ out,
         __ldg(reinterpret_cast<const uint4*>(g_dec_table.v) + i * kThreads + tid);
   pdl_wait(in);
   if (zt < nz) {
-    const uint32_t* src = in + ((size_t)blockIdx.x * kThreads + tid) * nwords;
+    const uint32_t* src = in + (size_t)b * nwords;
     if ((nwords & 3) == 0) {
       for (int w = 0; w < nwords; w += 4) {
         const uint4 v = __ldg(reinterpret_cast<const uint4*>(src + w));
@@ -208,6 +220,7 @@ zfp_decode_slab_kernel(const uint32_t* __restrict__ in, float* __restrict__ out,
   float f[64];
   StageWords source{col};
   decode_block3_pos(source, maxbits, f, lut, kc);
+  if (is_copy(lsh)) return;
   // eight neighbouring lanes cover one 128-byte row segment, so every store
   // instruction of a warp writes four full lines: no staging of the output
   const int vz = nz - zt < 4 ? (int)(nz - zt) : 4;
@@ -361,14 +374,14 @@ struct ColumnSource {
 template <int DIMS>
 __global__ void __launch_bounds__(kThreads, DIMS == 3 ? kEncCtasPerSm : 8)
 zfp_encode_generic_kernel(const FieldGeom g, const float* __restrict__ in, bool vec, uint32_t* __restrict__ out,
-                          int maxbits, uint64_t nblocks, uint64_t total_words, const PipeConsts kc) {
+                          int maxbits, uint64_t nblocks, uint64_t total_words, int lsh, const PipeConsts kc) {
   extern __shared__ __align__(16) uint32_t smem_words[];
   const int nwords = (maxbits + 31) >> 5, tid = threadIdx.x;
   uint32_t* stage = smem_words;
   uint32_t* queue = stage + (nwords + STAGE_SPARE_ROWS) * kThreads;
   uint32_t* lut = queue + (DIMS == 3 ? QUEUE_SLOTS * QUEUE_FIELDS * kThreads : 0);
   const uint32_t lut0 = __ldg(g_enc_table.v + tid), lut1 = __ldg(g_enc_table.v + kThreads + tid);
-  const uint64_t b0 = (uint64_t)blockIdx.x * kThreads, b = b0 + tid;
+  const uint64_t b0 = (uint64_t)blockIdx.x * kThreads, b = block_of_thread(lsh);  // lsh < 5: whole words only
   pdl_wait(in);
   float f[1 << (2 * DIMS)];
   if (b < nblocks) load_block<DIMS>(g, in, vec, BlockAt<DIMS>(g, b), f);
@@ -389,7 +402,7 @@ zfp_encode_generic_kernel(const FieldGeom g, const float* __restrict__ in, bool 
     }
   }
   if ((maxbits & 31) == 0) {  // whole words per block: every lane writes its own
-    if (b < nblocks) {
+    if (b < nblocks && !is_copy(lsh)) {
       uint32_t* dst = out + b * nwords;
       if ((nwords & 3) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0) {
         for (int w = 0; w < nwords; w += 4)
@@ -424,7 +437,7 @@ zfp_encode_generic_kernel(const FieldGeom g, const float* __restrict__ in, bool 
 template <int DIMS>
 __global__ void __launch_bounds__(kThreads, DIMS == 3 ? kDecCtasPerSm : 8)
 zfp_decode_generic_kernel(const FieldGeom g, const uint32_t* __restrict__ in, float* __restrict__ out, bool vec,
-                          int maxbits, uint64_t nblocks, uint64_t total_words, const PipeConsts kc) {
+                          int maxbits, uint64_t nblocks, uint64_t total_words, int lsh, const PipeConsts kc) {
   extern __shared__ __align__(16) uint32_t smem_words[];
   const int nwords = (maxbits + 31) >> 5, tid = threadIdx.x;
   uint32_t* stage = smem_words;
@@ -439,8 +452,9 @@ zfp_decode_generic_kernel(const FieldGeom g, const uint32_t* __restrict__ in, fl
   __syncthreads();  // the table is complete
   pdl_wait(in);
   // whole warps go round: the 3-D parser takes a minimum over all lanes
-  for (uint64_t wb = (uint64_t)blockIdx.x * kThreads + (tid & ~31); wb < nblocks; wb += (uint64_t)gridDim.x * kThreads) {
-    const uint64_t b = wb + (tid & 31), bit0 = b * (uint64_t)maxbits, w0 = bit0 >> 5;
+  const uint64_t mine = block_of_thread(lsh), my_lane = tid & ((1u << lsh) - 1u);
+  for (uint64_t wb = mine - my_lane; wb < nblocks; wb += (uint64_t)gridDim.x * kThreads) {
+    const uint64_t b = wb + my_lane, bit0 = b * (uint64_t)maxbits, w0 = bit0 >> 5;
     const int s = (int)(bit0 & 31);
     if (b >= nblocks) {
       col[0] = 0u;  // an empty block, not stored
@@ -471,11 +485,11 @@ zfp_decode_generic_kernel(const FieldGeom g, const uint32_t* __restrict__ in, fl
     const BlockAt<DIMS> at(g, b < nblocks ? b : nblocks - 1);
     if constexpr (DIMS == 3) {
       if (!vec && g.sx == 1) {
-        store_rows3(g, out, at, b < nblocks, reinterpret_cast<float*>(lut + DEC_LUT_SIZE) + 512 * (tid >> 5), f);
+        store_rows3(g, out, at, b < nblocks && !is_copy(lsh), reinterpret_cast<float*>(lut + DEC_LUT_SIZE) + 512 * (tid >> 5), f);
         continue;
       }
     }
-    if (b < nblocks) store_block<DIMS>(g, out, vec, at, f);
+    if (b < nblocks && !is_copy(lsh)) store_block<DIMS>(g, out, vec, at, f);
   }
 }
 
@@ -492,6 +506,7 @@ bool vector_rows(const FieldGeom& g, const void* field) {
 // =====================================================================================
 constexpr size_t kDefaultDynamicSmem = 48 * 1024;  // what a kernel may ask for without opting in
 constexpr uint64_t kFullGrid = 148 * 8;             // CTAs the device holds at eight per SM
+constexpr uint64_t kSchedulers = 148 * 4;
 constexpr int kMostBits = 4096;                    // largest budget the library accepts
 static size_t staged_smem_bytes(int maxbits, bool decode, int dims, bool rowbuf = false) {
   const size_t rows = ((size_t)maxbits + 31) / 32 + STAGE_SPARE_ROWS;
@@ -506,6 +521,24 @@ static cudaError_t allow_smem(K* kernel, size_t smem, bool decode, int dims) {
                               (int)staged_smem_bytes(kMostBits, decode, dims, true));
 }
 
+static uint64_t slab_blocks(const FieldGeom& g) { return ((uint64_t)g.nz + 3) / 4 * 64; }
+// log2 of the blocks a warp takes.  While every scheduler of the device has at most one
+// warp, a call lasts as long as one warp does, and a warp waits, plane by plane, for
+// the one of its blocks with the most group tests: the fewer blocks, the shorter.  So blocks
+// are spread until there is a warp for each of the 4 x 148 schedulers.  64 KiB at 512 bits
+// 5.4 -> 4.4 us (encode) and 7.3 -> 5.2 (decode), 1 MiB at 1024 bits 6.4 -> 5.8 and 8.7 -> 7.8.
+// From two warps a scheduler on the copies cost more issue slots than they save: 4 MiB with
+// 16 blocks a warp 5.6 -> 6.6 and 7.3 -> 7.8.
+static int blocks_per_warp(uint64_t nblocks) {
+  int lsh = 0;
+  while (lsh < 5 && (nblocks >> lsh) > kSchedulers) lsh++;
+  return lsh;
+}
+static unsigned ctas_of(uint64_t nblocks, int lsh) {
+  const uint64_t per = (uint64_t)(kThreads / 32) << lsh;
+  return (unsigned)((nblocks + per - 1) / per);
+}
+
 bool zfp_slab_eligible(const FieldGeom& g, const void* field, const void* stream, int maxbits) {
   return g.dims == 3 && g.nx == 32 && g.ny == 32 && g.sx == 1 && g.sy == 32 && g.sz == 1024 && (maxbits & 31) == 0 &&
          maxbits >= 32 && maxbits <= 2048 && (reinterpret_cast<uintptr_t>(field) & 15) == 0 &&
@@ -518,8 +551,10 @@ static cudaError_t encode_generic(const FieldGeom& g, const float* in, uint32_t*
   const size_t smem = staged_smem_bytes(maxbits, false, DIMS);
   cudaError_t e = allow_smem(zfp_encode_generic_kernel<DIMS>, smem, false, DIMS);
   if (e != cudaSuccess) return e;
-  return pdl_launch(zfp_encode_generic_kernel<DIMS>, (unsigned)((nblocks + kThreads - 1) / kThreads), kThreads, smem, stream,
-                    g, in, vector_rows(g, in), out, maxbits, nblocks, (uint64_t)stream_bytes(g, (unsigned)maxbits) / 4,
+  // blocks that share words are put together by a CTA of 128
+  const int lsh = DIMS == 3 && maxbits % 32 == 0 ? blocks_per_warp(nblocks) : 5;
+  return pdl_launch(zfp_encode_generic_kernel<DIMS>, ctas_of(nblocks, lsh), kThreads, smem, stream, g, in,
+                    vector_rows(g, in), out, maxbits, nblocks, (uint64_t)stream_bytes(g, (unsigned)maxbits) / 4, lsh,
                     pipe_consts());
 }
 template <int DIMS>
@@ -528,12 +563,13 @@ static cudaError_t decode_generic(const FieldGeom& g, const uint32_t* in, float*
   const size_t smem = staged_smem_bytes(maxbits, true, DIMS, DIMS == 3);
   cudaError_t e = allow_smem(zfp_decode_generic_kernel<DIMS>, smem, true, DIMS);
   if (e != cudaSuccess) return e;
-  const uint64_t ctas = (nblocks + kThreads - 1) / kThreads;
+  const int lsh = DIMS == 3 ? blocks_per_warp(nblocks) : 5;
+  const uint64_t ctas = ctas_of(nblocks, lsh);
   // The parser table is 18 KiB and 128 small blocks are 8 KiB of field or less: once
   // every SM has its eight CTAs, a CTA takes up to eight rounds of blocks.
   const uint64_t rounds = DIMS == 3 || ctas < 2 * kFullGrid ? 1 : ctas / kFullGrid < 8 ? ctas / kFullGrid : 8;
   return pdl_launch(zfp_decode_generic_kernel<DIMS>, (unsigned)((ctas + rounds - 1) / rounds), kThreads, smem, stream,
-                    g, in, out, vector_rows(g, out), maxbits, nblocks, (uint64_t)stream_bytes(g, (unsigned)maxbits) / 4,
+                    g, in, out, vector_rows(g, out), maxbits, nblocks, (uint64_t)stream_bytes(g, (unsigned)maxbits) / 4, lsh,
                     pipe_consts());
 }
 
@@ -545,8 +581,10 @@ cudaError_t zfp_encode_launch(const FieldGeom& g, const float* in, void* out, in
     const size_t smem = staged_smem_bytes(maxbits, false, 3);
     cudaError_t e = allow_smem(zfp_encode_slab_kernel, smem, false, 3);
     if (e != cudaSuccess) return e;
-    return pdl_launch(zfp_encode_slab_kernel, (g.nz + kGroupSlabs - 1) / kGroupSlabs, kThreads, smem, stream, in, o, g.nz,
-                      maxbits, pipe_consts());
+    const uint64_t blocks = slab_blocks(g);
+    const int lsh = blocks_per_warp(blocks);
+    return pdl_launch(zfp_encode_slab_kernel, ctas_of(blocks, lsh), kThreads, smem, stream, in, o, g.nz, maxbits, lsh,
+                      pipe_consts());
   }
   return g.dims == 3   ? encode_generic<3>(g, in, o, maxbits, nblocks, stream)
          : g.dims == 2 ? encode_generic<2>(g, in, o, maxbits, nblocks, stream)
@@ -561,8 +599,10 @@ cudaError_t zfp_decode_launch(const FieldGeom& g, const void* in, float* out, in
     const size_t smem = staged_smem_bytes(maxbits, true, 3);
     cudaError_t e = allow_smem(zfp_decode_slab_kernel, smem, true, 3);
     if (e != cudaSuccess) return e;
-    return pdl_launch(zfp_decode_slab_kernel, (g.nz + kGroupSlabs - 1) / kGroupSlabs, kThreads, smem, stream, i32, out, g.nz,
-                      maxbits, pipe_consts());
+    const uint64_t blocks = slab_blocks(g);
+    const int lsh = blocks_per_warp(blocks);
+    return pdl_launch(zfp_decode_slab_kernel, ctas_of(blocks, lsh), kThreads, smem, stream, i32, out, g.nz, maxbits, lsh,
+                      pipe_consts());
   }
   return g.dims == 3   ? decode_generic<3>(g, i32, out, maxbits, nblocks, stream)
          : g.dims == 2 ? decode_generic<2>(g, i32, out, maxbits, nblocks, stream)

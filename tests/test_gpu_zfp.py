@@ -386,3 +386,13 @@ def test_host_calls_cut_anywhere(cs, nx, ny, nz, maxbits):
     assert torch.equal(stream, want)
     L.cuda_decompress(C.byref(zs), C.byref(dst))
     assert torch.equal(back, cs.zfp_decompress(want.cuda(), t.numel(), maxbits, (nx, ny, nz)).cpu())
+
+
+@pytest.mark.parametrize("nz", [33, 36, 37, 73, 76, 77, 148, 149, 295, 296, 297, 592, 593])
+def test_blocks_spread_over_warps(cs, oracle, nz):
+    """Slab counts on either side of where a warp takes 1, 2, 4, 8, 16 or 32 blocks (one warp per
+    scheduler: 592 << k blocks), for the slab view and, with a field of as many blocks, the generic kernels."""
+    for maxbits in (256, 512):
+        _roundtrip(cs, oracle, util.tanh_normal(1024 * nz, seed=nz), (32, 32, nz), maxbits)
+        _roundtrip(cs, oracle, util.normal(31 * 30 * nz, seed=nz), (31, 30, nz), maxbits)
+        _roundtrip(cs, oracle, util.normal(64 * 16 * nz, seed=nz), (64, 16, nz), maxbits)
