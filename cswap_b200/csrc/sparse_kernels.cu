@@ -133,13 +133,17 @@ __global__ void __launch_bounds__(1024) block_exclusive_scan_kernel(T* a, uint32
 
 // ---- pass 3: bitmap and values ---------------------------------------------------------
 // The tile is loaded while the scan still runs (past L1, so that nothing a kernel
-// before left there can be met) and only its place in `values` is waited for.
+// before left there can be met) and only its place in `values` is waited for.  Tiles are
+// taken from the end: what pass 1 read last is what L2 still holds of a tensor larger than
+// itself (126 MB).  256 MiB, the whole call: 126 -> 118 us at 50 % zeros, 116 -> 106 at 90 %;
+// tensors that fit into L2 take the same time either way.
 __global__ void __launch_bounds__(kThreads)
 sparse_pack_kernel(const uint32_t* __restrict__ in, uint64_t n, uint32_t* __restrict__ bitmap, const uint32_t* tile_off,
                    uint32_t* __restrict__ values) {
   __shared__ uint32_t warp_cnt[kThreads / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint64_t base = (uint64_t)blockIdx.x * kTile + (uint64_t)warp * (kWordsPerWarp * 32);
+  const uint32_t tile = gridDim.x - 1 - blockIdx.x;
+  const uint64_t base = (uint64_t)tile * kTile + (uint64_t)warp * (kWordsPerWarp * 32);
   uint32_t v[kWordsPerWarp], w[kWordsPerWarp];
 #pragma unroll
   for (int j = 0; j < kWordsPerWarp; j++) {
@@ -158,7 +162,7 @@ sparse_pack_kernel(const uint32_t* __restrict__ in, uint64_t n, uint32_t* __rest
   __syncthreads();
   pdl_wait();
   if (lane < kWordsPerWarp && word0 + lane < nwords) bitmap[word0 + lane] = mine;
-  uint32_t off = tile_off[blockIdx.x];
+  uint32_t off = tile_off[tile];
   for (int i = 0; i < warp; i++) off += warp_cnt[i];
   const uint32_t lt = lanemask_lt();
 #pragma unroll
@@ -287,6 +291,11 @@ sparse_onepass_kernel(const uint32_t* __restrict__ in, uint64_t n, uint32_t* __r
 }
 
 // ---- decompression -----------------------------------------------------------------
+// A CTA is a chain of two loads from memory - bitmap word and tile offset, then values -
+// and bound by how many of them an SM has in flight.  (With the offset loaded behind the
+// barrier, a chain of three: 256 MiB 70.6 -> 69.3 us at 50 % zeros, 63.1 -> 61.1 at 75 %.  One
+// set of CTAs that loads the next tile's words ahead is slower, 80 and 73 us: its CTAs march
+// through load and store phases together, those of a plain grid are spread over them.)
 __global__ void __launch_bounds__(kThreads)
 sparse_unpack_kernel(const uint32_t* __restrict__ bitmap, const uint32_t* __restrict__ values,
                      const uint32_t* __restrict__ tile_off, uint64_t n, uint32_t* __restrict__ out) {
@@ -297,6 +306,7 @@ sparse_unpack_kernel(const uint32_t* __restrict__ bitmap, const uint32_t* __rest
   pdl_wait(bitmap);
   asm volatile("" : "+l"(values), "+l"(tile_off));  // read behind the wait as well
   const uint32_t mine = (lane < kWordsPerWarp && word0 + lane < nwords) ? __ldg(bitmap + word0 + lane) : 0u;
+  uint32_t off = __ldg(tile_off + blockIdx.x);  // on its way together with the bitmap
   // exclusive prefix of the popcounts of this warp's 16 words
   uint32_t x = __popc(mine);
   const uint32_t c = x;
@@ -307,7 +317,6 @@ sparse_unpack_kernel(const uint32_t* __restrict__ bitmap, const uint32_t* __rest
   }
   if (lane == kWordsPerWarp - 1) warp_cnt[warp] = x;
   __syncthreads();
-  uint32_t off = tile_off[blockIdx.x];
   for (int i = 0; i < warp; i++) off += warp_cnt[i];
   const uint32_t my_off = off + x - c;
   const uint32_t lt = lanemask_lt();
