@@ -115,6 +115,18 @@ CSW_HD uint32_t low_mask32(int n) {  // n in 0..32
   return n >= 32 ? 0xffffffffu : ((1u << n) - 1u);
 }
 
+// low min(max(n, 0), 32) bits set, for any n
+CSW_HD uint32_t low_mask_sat(int n) {
+  const int k = n > 0 ? n : 0;
+#if defined(__CUDA_ARCH__)
+  uint32_t m;
+  asm("bmsk.clamp.b32 %0, 0, %1;" : "=r"(m) : "r"(k));
+  return m;
+#else
+  return k >= 32 ? 0xffffffffu : ((1u << k) - 1u);
+#endif
+}
+
 // ---- sequency order (constants.h:8-131), entries are x + 4y + 16z ---------------
 constexpr int perm3(int i) {
   constexpr unsigned char t[64] = {
@@ -130,7 +142,7 @@ constexpr int perm2(int i) {
 }
 template <int DIMS, int I>
 struct PermAt {
-  static constexpr int v = DIMS == 3 ? perm3(I & 63) : DIMS == 2 ? perm2(I & 15) : I;
+  static constexpr int v = DIMS == 3 ? perm3(I & 63) : perm2(I & 15);
 };
 
 // ---- lifting (encode.cuh:73-99, shared.h:221-250) --------------------------------
@@ -166,13 +178,11 @@ CSW_HD void fwd_xform(int (&v)[1 << (2 * DIMS)]) {
         fwd_lift(v[16 * z + x], v[16 * z + x + 4], v[16 * z + x + 8], v[16 * z + x + 12]);
 #pragma unroll
     for (int i = 0; i < 16; i++) fwd_lift(v[i], v[i + 16], v[i + 32], v[i + 48]);
-  } else if constexpr (DIMS == 2) {
+  } else {
 #pragma unroll
     for (int y = 0; y < 4; y++) fwd_lift(v[4 * y], v[4 * y + 1], v[4 * y + 2], v[4 * y + 3]);
 #pragma unroll
     for (int x = 0; x < 4; x++) fwd_lift(v[x], v[x + 4], v[x + 8], v[x + 12]);
-  } else {
-    fwd_lift(v[0], v[1], v[2], v[3]);
   }
 }
 
@@ -188,13 +198,11 @@ CSW_HD void inv_xform(int (&v)[1 << (2 * DIMS)]) {
         inv_lift(v[16 * z + x], v[16 * z + x + 4], v[16 * z + x + 8], v[16 * z + x + 12]);
 #pragma unroll
     for (int i = 0; i < 16; i++) inv_lift(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-  } else if constexpr (DIMS == 2) {
+  } else {
 #pragma unroll
     for (int x = 0; x < 4; x++) inv_lift(v[x], v[x + 4], v[x + 8], v[x + 12]);
 #pragma unroll
     for (int y = 0; y < 4; y++) inv_lift(v[4 * y], v[4 * y + 1], v[4 * y + 2], v[4 * y + 3]);
-  } else {
-    inv_lift(v[0], v[1], v[2], v[3]);
   }
 }
 
@@ -262,17 +270,15 @@ CSW_HD void transpose8(uint32_t (&r)[8]) {
 // sel = c | (4 + c) << 4 picks byte c of both PRMT operands.
 template <int G, int N>
 CSW_HD void planes_of_byte(const uint32_t (&u)[N], uint32_t sel, uint32_t (&p)[8]) {
-  static_assert(N == 64 || N == 16 || N == 4, "block size");
+  static_assert(N == 64 || N == 16, "block size");
 #pragma unroll
   for (int j = 0; j < 8; j++) {
     if constexpr (N == 64) {
       uint32_t t0 = byte_perm(u[32 * G + j], u[32 * G + 8 + j], sel);
       uint32_t t1 = byte_perm(u[32 * G + 16 + j], u[32 * G + 24 + j], sel);
       p[j] = byte_perm(t0, t1, 0x5410);
-    } else if constexpr (N == 16) {
-      p[j] = byte_perm(u[j], u[8 + j], sel) & 0xffffu;
     } else {
-      p[j] = j < 4 ? (byte_perm(u[j & 3], 0, sel) & 0xffu) : 0u;
+      p[j] = byte_perm(u[j], u[8 + j], sel) & 0xffffu;
     }
   }
   transpose8(p);
@@ -289,11 +295,9 @@ CSW_HD void bytes_from_planes(uint32_t (&p)[8], uint32_t sel0, uint32_t step, ui
     if constexpr (N == 64) {
 #pragma unroll
       for (int m = 0; m < 4; m++) u[32 * G + 8 * m + j] = byte_perm(u[32 * G + 8 * m + j], p[j], sel0 + m * step);
-    } else if constexpr (N == 16) {
+    } else {
       u[j] = byte_perm(u[j], p[j], sel0);
       u[8 + j] = byte_perm(u[8 + j], p[j], sel0 + step);
-    } else {
-      if (j < 4) u[j & 3] = byte_perm(u[j & 3], p[j], sel0);
     }
   }
 }
@@ -362,6 +366,42 @@ CSW_HD int dec_lut_used(uint32_t e) { return (int)(e & 0xffu); }
 CSW_HD int dec_lut_advance(uint32_t e) { return (int)byte_perm(e, 0u, 0x4441u); }
 CSW_HD uint32_t dec_lut_pattern(uint32_t e) { return byte_perm(e, 0u, 0x4442u); }
 CSW_HD int dec_lut_state(uint32_t e) { return (int)(e >> 24); }
+
+// Blocks of four values: a plane is a nibble and its whole code at most eight bits, so one
+// entry holds a plane.  Encoder: entry for (n significant so far, nibble): code in bits
+// 0..7, its length in 8..11, n afterwards in 16..18.  Decoder: entry for (n, next eight stream
+// bits): nibble in bits 0..3, stream bits read in 4..7, n afterwards in 8..10.
+constexpr int ENC1_LUT_SIZE = 5 * 16, DEC1_LUT_SIZE = 5 * 256;
+constexpr CSW_HD uint32_t enc1_lut_entry(int idx) {
+  int n = idx >> 4, len = n;
+  uint32_t x = (uint32_t)idx & 15u, code = x & ((1u << n) - 1u);
+  x >>= n;
+  while (n < 4) {  // encode.cuh:336-343
+    code |= (x != 0u ? 1u : 0u) << len++;
+    if (x == 0u) break;
+    while (n < 3) {
+      const uint32_t b = x & 1u;
+      code |= b << len++;
+      if (b) break;
+      x >>= 1;
+      n++;
+    }
+    x >>= 1;
+    n++;
+  }
+  return code | ((uint32_t)len << 8) | ((uint32_t)n << 16);
+}
+constexpr CSW_HD uint16_t dec1_lut_entry(int idx) {
+  int n = idx >> 8, len = n;
+  const uint32_t s = (uint32_t)idx & 255u;
+  uint32_t x = s & ((1u << n) - 1u);
+  while (n < 4) {  // decode.cuh:147-164
+    if (!((s >> len++) & 1u)) break;
+    while (n < 3 && !((s >> len++) & 1u)) n++;
+    x |= 1u << n++;
+  }
+  return (uint16_t)(x | ((uint32_t)len << 4) | ((uint32_t)n << 8));
+}
 
 // ---- bit emitter ------------------------------------------------------------------
 // WordSink::put(w, word) receives the block's w-th 32-bit stream word; words
@@ -490,41 +530,102 @@ CSW_HD void encode_plane(uint32_t lo, uint32_t hi, SigState& sg, Emitter<WordSin
 }
 
 // ---- encoder: one plane of a small block ---------------------------------------------
-// N = 4 or 16 coefficients: the whole code of a plane - verbatim prefix, group
+// N = 16 coefficients: the whole code of a plane - verbatim prefix, group
 // test, expansions - is at most 32 bits (n verbatim bits, one test, two bits for
 // each of the N - n positions less the implied end), so it is put together
 // without a loop from one table entry per eight positions and appended at once.
-template <int N, class WordSink>
-CSW_HD void encode_plane_small(uint32_t x, int& n, Emitter<WordSink>& em, const uint32_t* enc_lut) {
-  static_assert(N == 16 || N == 4, "block size");
-  if (n >= N) {  // everything significant: the plane is copied verbatim
+// One path and one append for every lane (with n == 16 nothing is left over, r == 0,
+// and no group test is coded), but for planes that the whole warp copies.
+template <class WordSink>
+CSW_HD void encode_plane2(uint32_t x, int& n, Emitter<WordSink>& em, const uint32_t* enc_lut) {
+  constexpr int N = 16;
+  if (warp_all(n >= N)) {
     em.emit32(x, N);
     return;
   }
   const uint32_t r = x >> n;
-  const int top = (int)(x >> (N - 1)) & 1;  // last position set: its 1 is implied
-  const uint32_t e0 = enc_lut[r & 0xffu];
-  uint32_t code = 0;
-  int len = 0;
-  if constexpr (N == 16) {
-    const uint32_t e1 = enc_lut[r >> 8];
-    const bool more = (r >> 8) != 0u;
-    const int len0 = more ? (int)((e0 >> 16) & 0x1fu) : (int)(e0 >> 24) - 2 * top;
-    const int len1 = more ? (int)(e1 >> 24) - 2 * top : 0;
-    code = e0 & (more ? 0xffffu : low_mask32(len0 + top - 1));
-    code |= (e1 & (more ? low_mask32(len1 + top - 1) : 0u)) << len0;
-    len = len0 + len1;
-  } else {
-    len = (int)(e0 >> 24) - 2 * top;
-    code = e0 & low_mask32(len + top - 1);
+  const int top = (int)(x >> (N - 1));  // last position set: its 1 is implied
+  const uint32_t e0 = enc_lut[r & 0xffu], e1 = enc_lut[r >> 8];
+  const bool two = r > 0xffu;
+  const uint32_t last = two ? e1 : e0;           // of the byte with the last set bit
+  const int len1 = (int)(last >> 24) - 2 * top;  // meaningless, and not used, when r == 0
+  const int len0 = two ? (int)((e0 >> 16) & 0x1fu) : 0;
+  const uint32_t code = ((last & low_mask_sat(len1 + top - 1)) << len0) | (two ? e0 & 0xffffu : 0u);
+  const uint32_t head = x & low_mask_sat(n);
+  const int plain = n + 1 < N ? n + 1 : N;
+  em.emit32(r ? head | ((2u * code + 1u) << n) : head, r ? n + 1 + len0 + len1 : plain);
+  if (r) n = 32 - clz32(x);
+}
+
+// ---- blocks of four values: all planes at once ------------------------------------------
+// Bits 4k .. 4k+3 of w[c] <-> bit 8c+k of the four coefficients.  One bit transpose of
+// the four words covers all 32 planes: its word k holds plane 8m+k in byte m.
+CSW_HD void transpose_bytes4(uint32_t (&w)[4]) {  // byte i of word m <-> byte m of word i
+  const uint32_t a = byte_perm(w[0], w[1], 0x5140), b = byte_perm(w[2], w[3], 0x5140);
+  const uint32_t c = byte_perm(w[0], w[1], 0x7362), d = byte_perm(w[2], w[3], 0x7362);
+  w[0] = byte_perm(a, b, 0x5410);
+  w[1] = byte_perm(a, b, 0x7632);
+  w[2] = byte_perm(c, d, 0x5410);
+  w[3] = byte_perm(c, d, 0x7632);
+}
+CSW_HD void nibbles_of_planes(const uint32_t (&u)[4], uint32_t (&w)[4]) {
+  uint32_t r[8] = {u[0], u[1], u[2], u[3], 0u, 0u, 0u, 0u};
+  transpose8(r);
+#pragma unroll
+  for (int i = 0; i < 4; i++) w[i] = r[2 * i] | (r[2 * i + 1] << 4);
+  transpose_bytes4(w);
+}
+CSW_HD void planes_of_nibbles(uint32_t (&w)[4], uint32_t (&u)[4]) {
+  transpose_bytes4(w);
+  uint32_t r[8];
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    r[2 * i] = w[i] & 0x0f0f0f0fu;
+    r[2 * i + 1] = (w[i] >> 4) & 0x0f0f0f0fu;
   }
-  const uint32_t head = x & ((1u << n) - 1u);
-  if (r == 0u) {  // a failed group test
-    em.emit32(head, n + 1);
+  transpose8(r);
+#pragma unroll
+  for (int i = 0; i < 4; i++) u[i] = r[i];
+}
+
+template <class WordSink>
+CSW_HD void encode_block1(const float (&f)[4], int maxbits, WordSink& sink, const uint32_t* lut) {
+  Emitter<WordSink> em(sink, (maxbits + 31) >> 5);
+  float m = 0.0f;
+#pragma unroll
+  for (int i = 0; i < 4; i++) m = fmaxf(m, fabsf(f[i]));
+  const uint32_t e = biased_emax(m);
+  if (e == 0) {  // all-zero block: nothing is coded (encode.cuh:356-357)
+    em.finish();
     return;
   }
-  em.emit32(head | (1u << n) | (code << (n + 1)), n + 1 + len);
-  n = 32 - clz32(x);
+  int v[4];
+  const float s = quant_scale(e);
+#pragma unroll
+  for (int i = 0; i < 4; i++) v[i] = f2i_rz(s * f[i]);
+  fwd_lift(v[0], v[1], v[2], v[3]);
+  uint32_t u[4], w[4];
+#pragma unroll
+  for (int i = 0; i < 4; i++) u[i] = int2uint(v[i]);
+  nibbles_of_planes(u, w);
+  const int lead = clz32(u[0] | u[1] | u[2] | u[3]);  // empty planes: a failed group test each
+  em.emit32((2u * e + 1u) & 0x1ffu, 9);
+  em.emit32(0u, lead);
+  int n = 0;
+  for (int c = 3; c >= 0; c--) {
+    const uint32_t now = w[3];
+    w[3] = w[2]; w[2] = w[1]; w[1] = w[0];
+#pragma unroll
+    for (int k = 7; k >= 0; k--) {
+      if (8 * c + k < 32 - lead && em.total() < maxbits) {
+        const uint32_t en = lut[16 * n + ((now >> (4 * k)) & 15u)];
+        em.emit32(en & 0xffu, (int)((en >> 8) & 15u));
+        n = (int)(en >> 16);
+      }
+    }
+    if (em.total() >= maxbits) break;
+  }
+  em.finish();
 }
 
 // ---- encoder: whole block ---------------------------------------------------------
@@ -533,6 +634,7 @@ CSW_HD void encode_plane_small(uint32_t x, int& n, Emitter<WordSink>& em, const 
 // when maxbits is not a multiple of 32).
 template <int DIMS, class WordSink>
 CSW_HD void encode_block(const float (&f)[1 << (2 * DIMS)], int maxbits, WordSink& sink, const uint32_t* enc_lut) {
+  static_assert(DIMS > 1, "encode_block1");
   constexpr int N = 1 << (2 * DIMS);
   Emitter<WordSink> em(sink, (maxbits + 31) >> 5);
   float m = 0.0f;
@@ -575,7 +677,7 @@ CSW_HD void encode_block(const float (&f)[1 << (2 * DIMS)], int maxbits, WordSin
       planes_of_byte<0>(u, (uint32_t)c | ((uint32_t)(4 + c) << 4), x);
 #pragma unroll
       for (int k = 7; k >= 0; k--) {
-        if (em.total() < maxbits) encode_plane_small<N>(x[k], n, em, enc_lut);
+        if (em.total() < maxbits) encode_plane2(x[k], n, em, enc_lut);
       }
       if (em.total() >= maxbits) break;
     }
@@ -861,12 +963,12 @@ CSW_HD uint64_t decode_plane(Reader<WordSource>& rd, int& n, int& bits, const ui
 }
 
 // ---- decoder: one plane of a small block ----------------------------------------------
-// The code of a plane of N = 4 or 16 coefficients is at most 32 bits: one window
+// The code of a plane of 16 coefficients is at most 32 bits: one window
 // of the stream, consumed from the bottom, holds all of it.
-template <int N>
-CSW_HD uint32_t decode_plane_small(uint32_t win, int& n, int& left, const uint32_t* dec_lut) {
+CSW_HD uint32_t decode_plane2(uint32_t win, int& n, int& left, const uint32_t* dec_lut) {
+  constexpr int N = 16;
   const int m = n < left ? n : left;
-  uint32_t x = win & low_mask32(m);
+  uint32_t x = win & low_mask_sat(m);
   win >>= m;
   left -= m;
   if (n < N) {
@@ -885,6 +987,63 @@ CSW_HD uint32_t decode_plane_small(uint32_t win, int& n, int& left, const uint32
     } while (st != 2);
   }
   return x;
+}
+
+// Leading empty planes of a block whose first two words are given, `budget` bits of which
+// follow the header: while no coefficient is significant a plane is a single '0' bit (the
+// group test of decode.cuh:147 fails at n = 0), so the zeros that follow the header are
+// whole planes.
+CSW_HD int leading_empty_planes(uint32_t head, uint32_t second, int budget) {
+  const uint32_t first = funnel_r(head, second, 9);  // stream bits 9..40
+  const int zeros = first ? ctz32(first) : 32;
+  return zeros < budget ? zeros : budget;
+}
+
+// ---- decoder: blocks of four values ---------------------------------------------------
+// One table entry per plane.  The last plane may be cut by the budget: the entry is
+// then read with the missing bits as zeros, which is right (decode.cuh:141-165) but for a
+// run of zeros that is cut: its one belongs where the bits ran out, while the entry ran on
+// to the last position, where it is implied.
+template <class WordSource>
+CSW_HD void decode_block1(WordSource& src, int maxbits, float (&f)[4], const uint16_t* lut) {
+  const uint32_t head = src.get(0);
+  if (!(head & 1u)) {  // zero block (decode.cuh:240-243)
+#pragma unroll
+    for (int i = 0; i < 4; i++) f[i] = 0.0f;
+    return;
+  }
+  const uint32_t e = (head >> 1) & 0xffu;
+  int left = maxbits - 9, n = 0;
+  const int lead = leading_empty_planes(head, src.get(1), left);
+  left -= lead;
+  uint32_t w[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+  for (int c = 3; c >= 0; c--) {
+#pragma unroll
+    for (int k = 7; k >= 0; k--) {
+      if (8 * c + k < 32 - lead && left > 0) {
+        const int pos = maxbits - left;
+        const uint32_t win = funnel_r(src.get(pos >> 5), src.get((pos >> 5) + 1), pos) & low_mask_sat(left < 8 ? left : 8);
+        const uint32_t en = lut[256 * n + win];
+        const int over = (int)((en >> 4) & 15u) - left;
+        uint32_t x = en & 15u;
+        if (over > 0 && n < 4 && (en >> 8) == 4u) x = (x & 7u) | (8u >> over);
+        w[c] |= x << (4 * k);
+        left = -over;
+        n = (int)(en >> 8);
+      }
+    }
+    if (left <= 0) break;
+  }
+  uint32_t u[4];
+  planes_of_nibbles(w, u);
+  int v[4];
+#pragma unroll
+  for (int i = 0; i < 4; i++) v[i] = uint2int(u[i]);
+  inv_lift(v[0], v[1], v[2], v[3]);
+  const float scale = dequant_scale(e);
+#pragma unroll
+  for (int i = 0; i < 4; i++) f[i] = scale * (float)v[i];
 }
 
 // ---- decoder: whole block ---------------------------------------------------------
@@ -921,14 +1080,16 @@ CSW_HD void decode_block(WordSource& src, int maxbits, float (&f)[1 << (2 * DIMS
       if (left <= 0) break;
     }
   } else {
+    const int lead = leading_empty_planes(src.get(0), src.get(1), left);
+    left -= lead;
     for (int c = 3; c >= 0; c--) {
       uint32_t x[8];
 #pragma unroll
       for (int k = 7; k >= 0; k--) {
         x[k] = 0u;
-        if (left > 0) {
+        if (8 * c + k < 32 - lead && left > 0) {
           const int pos = maxbits - left;
-          x[k] = decode_plane_small<N>(funnel_r(src.get(pos >> 5), src.get((pos >> 5) + 1), pos), n, left, dec_lut);
+          x[k] = decode_plane2(funnel_r(src.get(pos >> 5), src.get((pos >> 5) + 1), pos), n, left, dec_lut);
         }
       }
       bytes_from_planes<0>(x, (0x3210u & ~(0xfu << (4 * c))) | (4u << (4 * c)), 1u << (4 * c), u);
@@ -954,17 +1115,6 @@ template <class WordSrc>
 CSW_HD uint32_t peek_at(const WordSrc& src, int pos) {
   const int w = pos >> 5;
   return funnel_r(src.word(w), src.word(w + 1), pos);  // the shift uses pos mod 32
-}
-// low min(max(n, 0), 32) bits set, for any n
-CSW_HD uint32_t low_mask_sat(int n) {
-  const int k = n > 0 ? n : 0;
-#if defined(__CUDA_ARCH__)
-  uint32_t m;
-  asm("bmsk.clamp.b32 %0, 0, %1;" : "=r"(m) : "r"(k));
-  return m;
-#else
-  return k >= 32 ? 0xffffffffu : ((1u << k) - 1u);
-#endif
 }
 // (h:l) rotated right by r, r in 0..31
 CSW_HD void ror64_small(uint32_t& l, uint32_t& h, int r) {
@@ -1042,18 +1192,12 @@ template <class WordSrc>
 CSW_HD void decode_block3_pos(const WordSrc& src, int maxbits, float (&f)[64], const uint32_t* dec_lut,
                               const PipeConsts& kc) {
   const uint32_t head = src.word(0);
-  // While no coefficient is significant a plane is a single '0' bit (the group
-  // test of decode.cuh:147 fails at n = 0), so the zeros that follow the header
-  // are whole planes.  The count common to the warp (at most the first slice)
-  // is skipped in one go; a lane's further empty planes go through the loop
-  // like any other.
+  // The empty planes common to the warp (at most the first slice) are skipped in one go; a
+  // lane's further ones go through the loop like any other.
   int lead = 8;
   if (head & 1u) {
-    const uint32_t first = funnel_r(head, src.word(1), 9);  // stream bits 9..40
-    const int zeros = first ? ctz32(first) : 32;
-    const int budget = maxbits - 9;
+    const int zeros = leading_empty_planes(head, src.word(1), maxbits - 9);
     lead = zeros < lead ? zeros : lead;
-    lead = budget < lead ? budget : lead;
   }
   lead = warp_min(lead);  // every lane of the warp is here: the tile test before the call is warp-uniform
   if (!(head & 1u)) {  // zero block

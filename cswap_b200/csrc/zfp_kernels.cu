@@ -245,7 +245,7 @@ zfp_decode_slab_kernel(const uint32_t* __restrict__ in, float* __restrict__ out,
 // no atomics, no zeroed stream.  (One thread per block reading and writing global
 // memory word by word, with plane-by-plane coders whose lanes wait for each other,
 // took 28.7 + 33.4 us a call for 31 x 33 x 4096 at 512 bits and 22.6 + 26.7 us for
-// 768 x 4096 at 128; these take 13.1 + 14.3 and 12.8 + 13.4.  They are bound as the
+// 768 x 4096 at 128; these take 12.9 + 14.5 and 11.4 + 13.2.  They are bound as the
 // slab kernels are, by the number of instructions a block costs.)
 namespace {
 
@@ -361,6 +361,28 @@ __device__ __forceinline__ void store_rows3(const FieldGeom& g, float* out, cons
   }
 }
 
+// Tables of the 1-D coders.  A plane of four values is one entry, and one bit transpose serves
+// all 32 planes: 4 Mi values at 32 bits 26.8 + 37.2 -> 18.9 + 23.9 us against the step tables of
+// the larger blocks and a transpose for every eight planes.
+struct Enc1Table {
+  uint32_t v[ENC1_LUT_SIZE];
+};
+constexpr Enc1Table make_enc1_table() {
+  Enc1Table t{};
+  for (int i = 0; i < ENC1_LUT_SIZE; i++) t.v[i] = enc1_lut_entry(i);
+  return t;
+}
+__device__ const Enc1Table g_enc1_table = make_enc1_table();
+struct alignas(16) Dec1Table {
+  uint16_t v[DEC1_LUT_SIZE];
+};
+constexpr Dec1Table make_dec1_table() {
+  Dec1Table t{};
+  for (int i = 0; i < DEC1_LUT_SIZE; i++) t.v[i] = dec1_lut_entry(i);
+  return t;
+}
+__device__ const Dec1Table g_dec1_table = make_dec1_table();
+
 // a lane's column of the staging area as a word sink / source of the small-block coders
 struct ColumnSink {
   uint32_t* p;
@@ -380,13 +402,21 @@ zfp_encode_generic_kernel(const FieldGeom g, const float* __restrict__ in, bool 
   uint32_t* stage = smem_words;
   uint32_t* queue = stage + (nwords + STAGE_SPARE_ROWS) * kThreads;
   uint32_t* lut = queue + (DIMS == 3 ? QUEUE_SLOTS * QUEUE_FIELDS * kThreads : 0);
-  const uint32_t lut0 = __ldg(g_enc_table.v + tid), lut1 = __ldg(g_enc_table.v + kThreads + tid);
-  const uint64_t b0 = (uint64_t)blockIdx.x * kThreads, b = block_of_thread(lsh);  // lsh < 5: whole words only
+  static_assert(ENC1_LUT_SIZE <= kThreads && ENC_LUT_SIZE == 2 * kThreads, "one or two table words per thread");
+  uint32_t lut0 = 0, lut1 = 0;
+  if (DIMS == 1) {
+    if (tid < ENC1_LUT_SIZE) lut0 = __ldg(g_enc1_table.v + tid);
+  } else {
+    lut0 = __ldg(g_enc_table.v + tid);
+    lut1 = __ldg(g_enc_table.v + kThreads + tid);
+  }
+  const uint32_t per_cta = (kThreads / 32) << lsh;
+  const uint64_t b0 = (uint64_t)blockIdx.x * per_cta, b = block_of_thread(lsh);
   pdl_wait(in);
   float f[1 << (2 * DIMS)];
   if (b < nblocks) load_block<DIMS>(g, in, vec, BlockAt<DIMS>(g, b), f);
   lut[tid] = lut0;
-  lut[kThreads + tid] = lut1;
+  if (DIMS > 1) lut[kThreads + tid] = lut1;
   uint32_t* col = stage + tid;
   if (DIMS == 3) {
     for (int w = 0; w < nwords; w++) col[w * kThreads] = 0u;  // coded bits are OR-ed in
@@ -398,7 +428,8 @@ zfp_encode_generic_kernel(const FieldGeom g, const float* __restrict__ in, bool 
       encode_block3_staged(f, maxbits, st, lut, kc);
     } else {
       ColumnSink sink{col};
-      encode_block<DIMS>(f, maxbits, sink, lut);
+      if constexpr (DIMS == 2) encode_block<2>(f, maxbits, sink, lut);
+      else encode_block1(f, maxbits, sink, lut);
     }
   }
   if ((maxbits & 31) == 0) {  // whole words per block: every lane writes its own
@@ -418,14 +449,15 @@ zfp_encode_generic_kernel(const FieldGeom g, const float* __restrict__ in, bool 
   }
   __syncthreads();  // every column is complete
   const uint64_t first = b0 * (uint64_t)maxbits >> 5;  // of this CTA's words; b0 * maxbits is a multiple of 32
-  const int here = nblocks - b0 < kThreads ? (int)(nblocks - b0) : kThreads;
+  const int here = nblocks - b0 < per_cta ? (int)(nblocks - b0) : (int)per_cta;
   const uint64_t left = total_words - first;
-  const int mine = here < kThreads ? (int)left : 4 * maxbits;
+  const int mine = nblocks - b0 <= per_cta ? (int)left : (int)(per_cta / 32) * maxbits;  // the last CTA: to the end
   for (int w = tid; w < mine; w += kThreads) {
     uint32_t v = 0;
     int blk = 32 * w / maxbits, off = 32 * w - blk * maxbits;
     for (int have = 0; have < 32 && blk < here; blk++, off = 0) {
-      const uint32_t* c = stage + blk + (off >> 5) * kThreads;  // the row behind the last one exists
+      const int owner = (blk >> lsh) * 32 + (blk & ((1 << lsh) - 1));  // its first thread
+      const uint32_t* c = stage + owner + (off >> 5) * kThreads;       // the row behind the last one exists
       const int take = maxbits - off < 32 - have ? maxbits - off : 32 - have;
       v |= (funnel_r(c[0], c[kThreads], off) & low_mask32(take)) << have;
       have += take;
@@ -443,10 +475,15 @@ zfp_decode_generic_kernel(const FieldGeom g, const uint32_t* __restrict__ in, fl
   uint32_t* stage = smem_words;
   uint32_t* lut = stage + (nwords + STAGE_SPARE_ROWS) * kThreads;
   uint32_t* col = stage + tid;
+  if (DIMS == 1) {
+    for (int i = tid; i < DEC1_LUT_SIZE / 8; i += kThreads)
+      reinterpret_cast<uint4*>(lut)[i] = __ldg(reinterpret_cast<const uint4*>(g_dec1_table.v) + i);
+  } else {
 #pragma unroll
-  for (int i = 0; i < DEC_LUT_SIZE / (4 * kThreads); i++)
-    reinterpret_cast<uint4*>(lut)[i * kThreads + tid] =
-        __ldg(reinterpret_cast<const uint4*>(g_dec_table.v) + i * kThreads + tid);
+    for (int i = 0; i < DEC_LUT_SIZE / (4 * kThreads); i++)
+      reinterpret_cast<uint4*>(lut)[i * kThreads + tid] =
+          __ldg(reinterpret_cast<const uint4*>(g_dec_table.v) + i * kThreads + tid);
+  }
   // reads just past a block find zeros and need no bounds test
   for (int w = nwords; w < nwords + STAGE_SPARE_ROWS; w++) col[w * kThreads] = 0u;
   __syncthreads();  // the table is complete
@@ -480,7 +517,8 @@ zfp_decode_generic_kernel(const FieldGeom g, const uint32_t* __restrict__ in, fl
       decode_block3_pos(source, maxbits, f, lut, kc);
     } else {
       ColumnSource source{col};
-      decode_block<DIMS>(source, maxbits, f, lut);
+      if constexpr (DIMS == 2) decode_block<2>(source, maxbits, f, lut);
+      else decode_block1(source, maxbits, f, reinterpret_cast<const uint16_t*>(lut));
     }
     const BlockAt<DIMS> at(g, b < nblocks ? b : nblocks - 1);
     if constexpr (DIMS == 3) {
@@ -510,6 +548,7 @@ constexpr uint64_t kSchedulers = 148 * 4;
 constexpr int kMostBits = 4096;                    // largest budget the library accepts
 static size_t staged_smem_bytes(int maxbits, bool decode, int dims, bool rowbuf = false) {
   const size_t rows = ((size_t)maxbits + 31) / 32 + STAGE_SPARE_ROWS;
+  if (decode && dims == 1) return rows * kThreads * 4 + DEC1_LUT_SIZE * 2;
   if (decode) return rows * kThreads * 4 + DEC_LUT_SIZE * 4 + (rowbuf ? kThreads * 16 * 4 : 0);
   return (rows + (dims == 3 ? QUEUE_SLOTS * QUEUE_FIELDS : 0)) * kThreads * 4 + ENC_LUT_SIZE * 4;
 }
@@ -551,8 +590,8 @@ static cudaError_t encode_generic(const FieldGeom& g, const float* in, uint32_t*
   const size_t smem = staged_smem_bytes(maxbits, false, DIMS);
   cudaError_t e = allow_smem(zfp_encode_generic_kernel<DIMS>, smem, false, DIMS);
   if (e != cudaSuccess) return e;
-  // blocks that share words are put together by a CTA of 128
-  const int lsh = DIMS == 3 && maxbits % 32 == 0 ? blocks_per_warp(nblocks) : 5;
+  int lsh = DIMS == 3 ? blocks_per_warp(nblocks) : 5;
+  if (maxbits % 32 && lsh < 3) lsh = 3;  // a CTA puts whole words together: 32 blocks at least
   return pdl_launch(zfp_encode_generic_kernel<DIMS>, ctas_of(nblocks, lsh), kThreads, smem, stream, g, in,
                     vector_rows(g, in), out, maxbits, nblocks, (uint64_t)stream_bytes(g, (unsigned)maxbits) / 4, lsh,
                     pipe_consts());

@@ -31,6 +31,22 @@ std::vector<uint32_t> dec_lut() {
   for (int i = 0; i < csw::DEC_LUT_SIZE; i++) t[i] = csw::dec_lut_entry(i);
   return t;
 }
+const std::vector<uint32_t>& enc1_lut() {
+  static const std::vector<uint32_t> t = [] {
+    std::vector<uint32_t> v(csw::ENC1_LUT_SIZE);
+    for (int i = 0; i < csw::ENC1_LUT_SIZE; i++) v[i] = csw::enc1_lut_entry(i);
+    return v;
+  }();
+  return t;
+}
+const std::vector<uint16_t>& dec1_lut() {
+  static const std::vector<uint16_t> t = [] {
+    std::vector<uint16_t> v(csw::DEC1_LUT_SIZE);
+    for (int i = 0; i < csw::DEC1_LUT_SIZE; i++) v[i] = csw::dec1_lut_entry(i);
+    return v;
+  }();
+  return t;
+}
 
 template <int DIMS>
 void encode_field(const csw::FieldGeom& g, const float* in, int maxbits, uint32_t* out) {
@@ -41,7 +57,8 @@ void encode_field(const csw::FieldGeom& g, const float* in, int maxbits, uint32_
     float q[1 << (2 * DIMS)];
     csw::gather_block<DIMS>(g, in, b, q);
     VecSink s{out + b * nw};
-    csw::encode_block<DIMS>(q, maxbits, s, lut.data());
+    if constexpr (DIMS == 1) csw::encode_block1(q, maxbits, s, enc1_lut().data());
+    else csw::encode_block<DIMS>(q, maxbits, s, lut.data());
   }
 }
 template <int DIMS>
@@ -52,7 +69,8 @@ void decode_field(const csw::FieldGeom& g, const uint32_t* in, int maxbits, floa
   for (size_t b = 0; b < nb; b++) {
     float q[1 << (2 * DIMS)];
     VecSource s{in + b * nw, nw};
-    csw::decode_block<DIMS>(s, maxbits, q, lut.data());
+    if constexpr (DIMS == 1) csw::decode_block1(s, maxbits, q, dec1_lut().data());
+    else csw::decode_block<DIMS>(s, maxbits, q, lut.data());
     csw::scatter_block<DIMS>(g, out, b, q);
   }
 }

@@ -396,3 +396,19 @@ def test_blocks_spread_over_warps(cs, oracle, nz):
         _roundtrip(cs, oracle, util.tanh_normal(1024 * nz, seed=nz), (32, 32, nz), maxbits)
         _roundtrip(cs, oracle, util.normal(31 * 30 * nz, seed=nz), (31, 30, nz), maxbits)
         _roundtrip(cs, oracle, util.normal(64 * 16 * nz, seed=nz), (64, 16, nz), maxbits)
+
+
+@pytest.mark.parametrize("dims", [(4, 0, 0), (4099, 0, 0), (130, 37, 0)])
+@pytest.mark.parametrize("maxbits", [9, 10, 11, 14, 17, 25, 32, 37, 64, 100, 160])
+def test_small_blocks_cut_anywhere(cs, oracle, dims, maxbits):
+    """1-D and 2-D blocks whose last plane is cut at any place of its code - in its verbatim bits, in a
+    group test, in a run - for values of every kind and for bits that no encoder wrote."""
+    import torch
+    nx, ny, nz = dims
+    n = nx * max(ny, 1)
+    _roundtrip(cs, oracle, util.block_zoo((n + 63) // 64 * 64, seed=maxbits)[:n], dims, maxbits)
+    nbytes = oracle.zfp_stream_bytes(nx, ny, nz, maxbits)
+    for sw in util.arbitrary_streams(nbytes // 4, maxbits + nx):
+        ref = oracle.zfp_decode(np.ascontiguousarray(sw).view(np.uint64), nx, ny, nz, maxbits)
+        got = cs.zfp_decompress(torch.from_numpy(sw.view(np.uint8).copy()).cuda(), n, maxbits, dims).cpu().numpy()
+        assert np.array_equal(got.view(np.uint32), ref.view(np.uint32))
