@@ -12,7 +12,7 @@
 //    (PRMT gathers + 3 masked swap stages), eight planes at a time, instead of
 //    a 64-step gather per plane;
 //  * the group-test phase of a plane is expanded (encoder) or parsed (decoder)
-//    eight positions / stream bits per step through small tables held in
+//    eight to eleven positions / stream bits per step through small tables held in
 //    shared memory instead of one stream bit per step;
 //  * coded bits are assembled in a 64-bit register window and leave as whole
 //    32-bit words - no atomics and no pre-zeroed output.
@@ -124,6 +124,26 @@ CSW_HD uint32_t low_mask_sat(int n) {
   return m;
 #else
   return k >= 32 ? 0xffffffffu : ((1u << k) - 1u);
+#endif
+}
+// 1 << n, 0 for n outside 0..31
+CSW_HD uint32_t bit_or_none(int n) {
+#if defined(__CUDA_ARCH__)
+  uint32_t m;
+  asm("shl.b32 %0, 1, %1;" : "=r"(m) : "r"(n));  // counts above 31, unsigned, shift everything out
+  return m;
+#else
+  return (uint32_t)n < 32u ? 1u << n : 0u;
+#endif
+}
+// (s * a, s * b), one instruction on the device
+CSW_HD void mul2(float s, float a, float b, float& x, float& y) {
+#if defined(__CUDA_ARCH__)
+  asm("{\n\t.reg .b64 p, q;\n\tmov.b64 p, {%2, %2};\n\tmov.b64 q, {%3, %4};\n\tmul.rn.f32x2 p, p, q;\n\tmov.b64 {%0, %1}, p;\n\t}"
+      : "=f"(x), "=f"(y) : "f"(s), "f"(a), "f"(b));
+#else
+  x = s * a;
+  y = s * b;
 #endif
 }
 
@@ -328,6 +348,23 @@ constexpr CSW_HD uint32_t enc_lut_entry(uint32_t v) {
   return pat | ((uint32_t)len << 16) | (lf << 24);
 }
 
+// The same for the eleven positions of the 3-D staged encoder: pattern in bits 0..21, the
+// length 11 + popc(v) in 22..26, the length of a last piece in 27..31: no bit is left over.
+constexpr int ENC3_BITS = 11, ENC3_LUT_SIZE = 1 << ENC3_BITS;
+constexpr CSW_HD uint32_t enc3_lut_entry(uint32_t v) {
+  uint32_t pat = 0, len = 0, last = 0;
+  for (int i = 0; i < ENC3_BITS; i++) {
+    if ((v >> i) & 1u) {
+      pat |= 3u << len;
+      len += 2;
+      last = len;
+    } else {
+      len += 1;
+    }
+  }
+  return pat | (len << 22) | (last << 27);
+}
+
 // Decoder: entry for (limit L in 0..8, state, next stream byte).  Simulates the
 // group-test parser of decode.cuh:147-164 over at most L stream bits.
 // State 0: expecting a group-test bit; state 1: inside a unary run (expecting
@@ -474,16 +511,16 @@ struct Emitter {
 // ---- encoder: coefficient-count state ----------------------------------------------
 // n coefficients are significant so far; the masks select plane bits below n
 // and the single bit at position n (zero when n == 64).
-struct SigState {
+struct SigState {  // by mask and shift instructions that saturate: a dozen fewer per plane than selects
   int n;
   uint32_t mlo, mhi;  // low n bits of a 64-bit plane word
   uint32_t glo, ghi;  // bit n
   CSW_HD void set(int nn) {
     n = nn;
-    mlo = nn >= 32 ? 0xffffffffu : ((1u << nn) - 1u);
-    mhi = nn <= 32 ? 0u : low_mask32(nn - 32);
-    glo = nn < 32 ? (1u << nn) : 0u;
-    ghi = (nn >= 32 && nn < 64) ? (1u << (nn - 32)) : 0u;
+    mlo = low_mask_sat(nn);
+    mhi = low_mask_sat(nn - 32);
+    glo = bit_or_none(nn);
+    ghi = bit_or_none(nn - 32);
   }
 };
 
@@ -810,7 +847,12 @@ CSW_HD void encode_block3_staged(const float (&f)[64], int maxbits, Stage& st, c
   {
     const float s = quant_scale(e);
 #pragma unroll
-    for (int i = 0; i < 64; i++) v[i] = f2i_rz(s * f[i]);
+    for (int i = 0; i < 64; i += 2) {
+      float a, b;
+      mul2(s, f[i], f[i + 1], a, b);
+      v[i] = f2i_rz(a);
+      v[i + 1] = f2i_rz(b);
+    }
   }
   fwd_xform3_bal(v, kc);
   uint32_t u[64];
@@ -830,23 +872,22 @@ CSW_HD void encode_block3_staged(const float (&f)[64], int maxbits, Stage& st, c
       if (off < maxbits) {
         // one path for every lane: with n == 64 the masks select the whole
         // word, no position is left over and no group test is coded
-        const int n = sg.n, s = n & 31;
-        const uint32_t fl = funnel_r(lo[k], hi[k], s), sh = hi[k] >> s;
-        const uint32_t xl = n >= 64 ? 0u : (n < 32 ? fl : sh);
-        const uint32_t xh = n < 32 ? sh : 0u;
-        const bool any = (xl | xh) != 0u;
+        const int n = sg.n;
+        const uint32_t above_lo = lo[k] & ~sg.mlo, above_hi = hi[k] & ~sg.mhi;
+        const bool any = (above_lo | above_hi) != 0u;
         stage_put64(st, off, (lo[k] & sg.mlo) | (any ? sg.glo : 0u), (hi[k] & sg.mhi) | (any ? sg.ghi : 0u));
-        off += n < 64 ? n + 1 : 64;
+        off += n + 1 < 64 ? n + 1 : 64;
         if (any) {
           const int top = (int)(hi[k] >> 31);
           const int msb = hi[k] ? 64 - clz32(hi[k]) : 32 - clz32(lo[k]);
           if (off < maxbits) {
-            st.q_put(count, 0, xl);
-            st.q_put(count, 1, xh);
+            const uint32_t fl = funnel_r(lo[k], hi[k], n), sh = hi[k] >> (n & 31);
+            st.q_put(count, 0, n < 32 ? fl : sh);
+            st.q_put(count, 1, n < 32 ? sh : 0u);
             st.q_put(count, 2, (uint32_t)off | ((uint32_t)top << 31));
             count++;
           }
-          off += (msb - n) + popc32(xl) + popc32(xh) - 2 * top;
+          off += (msb - n) + popc32(above_lo) + popc32(above_hi) - 2 * top;
           sg.set(msb);
         }
       }
@@ -864,13 +905,13 @@ CSW_HD void encode_block3_staged(const float (&f)[64], int maxbits, Stage& st, c
       top = (int)(meta >> 31);
     }
     while (have) {
-      const uint32_t en = enc_lut[xl & 0xffu];
-      xl = funnel_r(xl, xh, 8);
-      xh >>= 8;
+      const uint32_t en = enc_lut[xl & (ENC3_LUT_SIZE - 1)];
+      xl = funnel_r(xl, xh, ENC3_BITS);
+      xh >>= ENC3_BITS;
       const bool more = (xl | xh) != 0u;
-      const int lf = (int)(en >> 24);
-      const int len = more ? (int)((en >> 16) & 0x1fu) : lf - 2 * top;
-      const uint32_t keep = more ? 0xffffu : low_mask32(lf - 1 - top);
+      const int lf = (int)(en >> 27);
+      const int len = more ? (int)((en >> 22) & 0x1fu) : lf - 2 * top;
+      const uint32_t keep = more ? 0x3fffffu : low_mask_sat(lf - 1 - top);
       const uint32_t pat = en & keep;
       const int s = boff & 31, w = boff >> 5;
       st.or_word(w, pat << s);
@@ -1228,7 +1269,7 @@ CSW_HD void decode_block3_pos(const WordSrc& src, int maxbits, float (&f)[64], c
   inv_xform<3>(v);
   const float w = dequant_scale(e);
 #pragma unroll
-  for (int i = 0; i < 64; i++) f[i] = w * (float)v[i];
+  for (int i = 0; i < 64; i += 2) mul2(w, (float)v[i], (float)v[i + 1], f[i], f[i + 1]);
 }
 
 }  // namespace csw

@@ -66,8 +66,8 @@ struct SmemStage {
   }
 };
 
-// The expansion table, evaluated at compile time: a CTA copies it to shared
-// memory (two words per thread) instead of computing 256 entries per launch.
+// The expansion tables, evaluated at compile time: a CTA copies its own to shared
+// memory instead of computing the entries per launch.
 struct EncTable {
   uint32_t v[ENC_LUT_SIZE];
 };
@@ -77,6 +77,25 @@ constexpr EncTable make_enc_table() {
   return t;
 }
 __device__ const EncTable g_enc_table = make_enc_table();
+// 3-D: eleven positions a step where the table of eight takes one.  Steps are what the lanes
+// of a warp differ in, so each one saved is saved by the warp: 256 MiB at 512 / 1024 bits
+// 110.6 / 145.2 -> 104.7 / 136.3 us.  (Twelve positions do not fit an entry's 32 bits.)
+struct alignas(16) Enc3Table {
+  uint32_t v[ENC3_LUT_SIZE];
+};
+constexpr Enc3Table make_enc3_table() {
+  Enc3Table t{};
+  for (int i = 0; i < ENC3_LUT_SIZE; i++) t.v[i] = enc3_lut_entry((uint32_t)i);
+  return t;
+}
+__device__ const Enc3Table g_enc3_table = make_enc3_table();
+static_assert(ENC3_LUT_SIZE % (4 * kThreads) == 0, "table copy assumes whole 128-bit rounds");
+__device__ __forceinline__ void copy_enc3_table(uint32_t* lut) {
+#pragma unroll
+  for (int i = 0; i < ENC3_LUT_SIZE / (4 * kThreads); i++)
+    reinterpret_cast<uint4*>(lut)[i * kThreads + threadIdx.x] =
+        __ldg(reinterpret_cast<const uint4*>(g_enc3_table.v) + i * kThreads + threadIdx.x);
+}
 
 // Block of this thread: a warp takes 1 << lsh neighbouring blocks.  With lsh < 5 the lanes
 // above do the work of the ones below a second time - the same data, so they cost
@@ -117,8 +136,7 @@ zfp_encode_slab_kernel(const float* __restrict__ in, uint32_t* __restrict__ out,
   const int bx = b & 7, by = (b >> 3) & 7;
   const uint32_t zt = (b >> 6) * 4;  // first slab of my tile
   const int vz = zt >= nz ? 0 : (nz - zt < 4 ? (int)(nz - zt) : 4);
-  static_assert(ENC_LUT_SIZE == 2 * kThreads, "two table words per thread");
-  const uint32_t lut0 = __ldg(g_enc_table.v + tid), lut1 = __ldg(g_enc_table.v + kThreads + tid);
+  copy_enc3_table(lut);
   pdl_wait(in);
   float f[64];
   if (vz > 0) {
@@ -136,8 +154,6 @@ zfp_encode_slab_kernel(const float* __restrict__ in, uint32_t* __restrict__ out,
       }
     }
   }
-  lut[tid] = lut0;
-  lut[kThreads + tid] = lut1;
   for (int w = 0; w < nwords; w++) stage[w * kThreads + tid] = 0u;  // coded bits are OR-ed in
   __syncthreads();  // the table is complete
   if (vz == 0) return;
@@ -245,7 +261,7 @@ zfp_decode_slab_kernel(const uint32_t* __restrict__ in, float* __restrict__ out,
 // no atomics, no zeroed stream.  (One thread per block reading and writing global
 // memory word by word, with plane-by-plane coders whose lanes wait for each other,
 // took 28.7 + 33.4 us a call for 31 x 33 x 4096 at 512 bits and 22.6 + 26.7 us for
-// 768 x 4096 at 128; these take 12.9 + 14.5 and 11.4 + 13.2.  They are bound as the
+// 768 x 4096 at 128; these take 11.9 + 14.5 and 11.4 + 13.2.  They are bound as the
 // slab kernels are, by the number of instructions a block costs.)
 namespace {
 
@@ -406,17 +422,19 @@ zfp_encode_generic_kernel(const FieldGeom g, const float* __restrict__ in, bool 
   uint32_t lut0 = 0, lut1 = 0;
   if (DIMS == 1) {
     if (tid < ENC1_LUT_SIZE) lut0 = __ldg(g_enc1_table.v + tid);
-  } else {
+  } else if (DIMS == 2) {
     lut0 = __ldg(g_enc_table.v + tid);
     lut1 = __ldg(g_enc_table.v + kThreads + tid);
+  } else {
+    copy_enc3_table(lut);
   }
   const uint32_t per_cta = (kThreads / 32) << lsh;
   const uint64_t b0 = (uint64_t)blockIdx.x * per_cta, b = block_of_thread(lsh);
   pdl_wait(in);
   float f[1 << (2 * DIMS)];
   if (b < nblocks) load_block<DIMS>(g, in, vec, BlockAt<DIMS>(g, b), f);
-  lut[tid] = lut0;
-  if (DIMS > 1) lut[kThreads + tid] = lut1;
+  if (DIMS < 3) lut[tid] = lut0;
+  if (DIMS == 2) lut[kThreads + tid] = lut1;
   uint32_t* col = stage + tid;
   if (DIMS == 3) {
     for (int w = 0; w < nwords; w++) col[w * kThreads] = 0u;  // coded bits are OR-ed in
@@ -550,7 +568,7 @@ static size_t staged_smem_bytes(int maxbits, bool decode, int dims, bool rowbuf 
   const size_t rows = ((size_t)maxbits + 31) / 32 + STAGE_SPARE_ROWS;
   if (decode && dims == 1) return rows * kThreads * 4 + DEC1_LUT_SIZE * 2;
   if (decode) return rows * kThreads * 4 + DEC_LUT_SIZE * 4 + (rowbuf ? kThreads * 16 * 4 : 0);
-  return (rows + (dims == 3 ? QUEUE_SLOTS * QUEUE_FIELDS : 0)) * kThreads * 4 + ENC_LUT_SIZE * 4;
+  return (rows + (dims == 3 ? QUEUE_SLOTS * QUEUE_FIELDS : 0)) * kThreads * 4 + (dims == 3 ? ENC3_LUT_SIZE : ENC_LUT_SIZE) * 4;
 }
 // Only the largest budgets need it; the call costs host time on every launch.
 template <class K>

@@ -88,7 +88,8 @@ extern "C" {
 // the staged 3-D encoder of the slab kernel (nx, ny, nz arbitrary here; whole words per block)
 void core_encode_staged(const float* in, size_t nx, size_t ny, size_t nz, int maxbits, uint32_t* out) {
   csw::FieldGeom g = csw::make_geom(nx, ny, nz, 0, 0, 0);
-  auto lut = enc_lut();
+  std::vector<uint32_t> lut(csw::ENC3_LUT_SIZE);
+  for (int i = 0; i < csw::ENC3_LUT_SIZE; i++) lut[i] = csw::enc3_lut_entry((uint32_t)i);
   const csw::PipeConsts kc = csw::pipe_consts();
   const int nw = maxbits / 32;
   std::vector<uint32_t> rows(nw + csw::STAGE_SPARE_ROWS);
