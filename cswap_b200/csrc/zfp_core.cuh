@@ -112,7 +112,13 @@ CSW_HD int ctz32(uint32_t x) {  // x != 0
 #endif
 }
 CSW_HD uint32_t low_mask32(int n) {  // n in 0..32
+#if defined(__CUDA_ARCH__)
+  uint32_t m;
+  asm("bmsk.clamp.b32 %0, 0, %1;" : "=r"(m) : "r"(n));
+  return m;
+#else
   return n >= 32 ? 0xffffffffu : ((1u << n) - 1u);
+#endif
 }
 
 // low min(max(n, 0), 32) bits set, for any n
@@ -438,6 +444,36 @@ constexpr CSW_HD uint16_t dec1_lut_entry(int idx) {
     x |= 1u << n++;
   }
   return (uint16_t)(x | ((uint32_t)len << 4) | ((uint32_t)n << 8));
+}
+
+// The same for up to ten stream bits, for the 3-D decoder: of a row with limit L only the
+// first L bits matter, so its entries are the 1 << L ones behind entry (1 << L) of the
+// state's half.  Bits 0..9: plane bits found; 16..23: positions advanced; 24..27: stream bits
+// consumed; 30..31: state afterwards.
+constexpr int DEC3_BITS = 10, DEC3_LUT_SIZE = 2 << (DEC3_BITS + 1);
+constexpr CSW_HD uint32_t dec3_lut_entry(int idx) {
+  const int half = idx & ((2 << DEC3_BITS) - 1);
+  int st = idx >> (DEC3_BITS + 1), L = 0;
+  while ((2 << L) <= half) L++;
+  const uint32_t bits = (uint32_t)(half - (1 << L));
+  int c = 0, dn = 0;
+  uint32_t pat = 0;
+  if (L == 0) {
+    if (st == 1) { pat = 1u; dn = 1; }
+    st = 2;
+  }
+  while (c < L) {
+    const uint32_t bit = (bits >> c) & 1u;
+    c++;
+    if (st == 0) {
+      if (bit) st = 1;
+      else { st = 2; break; }
+    } else {
+      if (bit) { pat |= 1u << dn; st = 0; }
+      dn++;
+    }
+  }
+  return pat | ((uint32_t)dn << 16) | ((uint32_t)c << 24) | ((uint32_t)st << 30);
 }
 
 // ---- bit emitter ------------------------------------------------------------------
@@ -1194,7 +1230,7 @@ CSW_HD void decode_slice3(const WordSrc& src, int maxbits, const uint32_t* dec_l
       xl = funnel_r(w0, w1, pos) & low_mask_sat(m);
       xh = funnel_r(w1, w2, pos) & low_mask_sat(m - 32);
       pos += m;
-      // group tests and unary runs (decode.cuh:147-164), up to eight stream
+      // group tests and unary runs (decode.cuh:147-164), up to ten stream
       // bits per step; none once every coefficient is significant.  The bits
       // found are gathered in (ah:al), kept rotated so that position n is bit
       // 0: a step ORs its pattern in at the bottom and rotates by the positions
@@ -1203,21 +1239,22 @@ CSW_HD void decode_slice3(const WordSrc& src, int maxbits, const uint32_t* dec_l
         uint32_t al = 0u, ah = 0u;
         int st = 0;
         do {
-          // stream bits this step may read: up to eight, no further than the
+          // stream bits this step may read: up to ten, no further than the
           // last open position (a run's final one is implied, so it stops one
           // short) and no further than the block's budget; none at all ends
           // the plane through the table's L = 0 rows
           const int left = maxbits - pos;
           const int lim = 64 - st - n;
-          int L = lim < 8 ? lim : 8;
+          int L = lim < DEC3_BITS ? lim : DEC3_BITS;
           L = left < L ? left : L;
-          const uint32_t en = dec_lut[dec_lut_index(L, st, peek_at(src, pos) & 0xffu)];
-          const int dn = dec_lut_advance(en);
-          al |= dec_lut_pattern(en);
+          const uint32_t mask = low_mask32(L);
+          const uint32_t en = dec_lut[(st << (DEC3_BITS + 1)) + (int)mask + 1 + (int)(peek_at(src, pos) & mask)];
+          const int dn = (int)byte_perm(en, 0u, 0x4442u);
+          al |= en & ((1u << DEC3_BITS) - 1u);
           ror64_small(al, ah, dn);
           n += dn;
-          pos += dec_lut_used(en);
-          st = dec_lut_state(en);
+          pos += (int)((en >> 24) & 15u);
+          st = (int)(en >> 30);
         } while (st != 2);
         rol64(al, ah, n);  // position 0 back to bit 0
         xl |= al;

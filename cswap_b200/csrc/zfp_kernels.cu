@@ -66,6 +66,14 @@ struct SmemStage {
   }
 };
 
+template <int SIZE>
+__device__ __forceinline__ void copy_table(uint32_t* to, const uint32_t* from) {
+  static_assert(SIZE % (4 * kThreads) == 0, "table copy assumes whole 128-bit rounds");
+#pragma unroll
+  for (int i = 0; i < SIZE / (4 * kThreads); i++)
+    reinterpret_cast<uint4*>(to)[i * kThreads + threadIdx.x] =
+        __ldg(reinterpret_cast<const uint4*>(from) + i * kThreads + threadIdx.x);
+}
 // The expansion tables, evaluated at compile time: a CTA copies its own to shared
 // memory instead of computing the entries per launch.
 struct EncTable {
@@ -89,13 +97,6 @@ constexpr Enc3Table make_enc3_table() {
   return t;
 }
 __device__ const Enc3Table g_enc3_table = make_enc3_table();
-static_assert(ENC3_LUT_SIZE % (4 * kThreads) == 0, "table copy assumes whole 128-bit rounds");
-__device__ __forceinline__ void copy_enc3_table(uint32_t* lut) {
-#pragma unroll
-  for (int i = 0; i < ENC3_LUT_SIZE / (4 * kThreads); i++)
-    reinterpret_cast<uint4*>(lut)[i * kThreads + threadIdx.x] =
-        __ldg(reinterpret_cast<const uint4*>(g_enc3_table.v) + i * kThreads + threadIdx.x);
-}
 
 // Block of this thread: a warp takes 1 << lsh neighbouring blocks.  With lsh < 5 the lanes
 // above do the work of the ones below a second time - the same data, so they cost
@@ -136,7 +137,7 @@ zfp_encode_slab_kernel(const float* __restrict__ in, uint32_t* __restrict__ out,
   const int bx = b & 7, by = (b >> 3) & 7;
   const uint32_t zt = (b >> 6) * 4;  // first slab of my tile
   const int vz = zt >= nz ? 0 : (nz - zt < 4 ? (int)(nz - zt) : 4);
-  copy_enc3_table(lut);
+  copy_table<ENC3_LUT_SIZE>(lut, g_enc3_table.v);
   pdl_wait(in);
   float f[64];
   if (vz > 0) {
@@ -178,9 +179,9 @@ zfp_encode_slab_kernel(const float* __restrict__ in, uint32_t* __restrict__ out,
 // slab decoder
 // =====================================================================================
 namespace {
-// The parser table, evaluated at compile time: a CTA copies it to shared memory
-// with four 128-bit loads per thread instead of rebuilding 4096 entries.
-struct DecTable {
+// The parser tables (2-D; 3-D), evaluated at compile time: a CTA copies its own to shared
+// memory with 128-bit loads instead of rebuilding the entries.
+struct alignas(16) DecTable {
   uint32_t v[DEC_LUT_SIZE];
 };
 constexpr DecTable make_dec_table() {
@@ -189,7 +190,20 @@ constexpr DecTable make_dec_table() {
   return t;
 }
 __device__ const DecTable g_dec_table = make_dec_table();
-static_assert(DEC_LUT_SIZE % (4 * kThreads) == 0, "table copy assumes whole 128-bit rounds");
+// 3-D: up to ten stream bits a step (16 KiB; every row with eight took 18).  256 MiB at 256 / 512
+// / 1024 bits 101.2 / 128.1 / 162.5 -> 96.1 / 123.1 / 158.6 us; nine bits 96.8 / 123.4 / 157.6, but
+// 32 MiB at 1024 bits 24.8 against 24.0; eleven (32 KiB: four CTAs per SM at 1024 bits) 99.2 /
+// 131.8 / 176.6.
+struct alignas(16) Dec3Table {
+  uint32_t v[DEC3_LUT_SIZE];
+};
+constexpr Dec3Table make_dec3_table() {
+  Dec3Table t{};
+  for (int i = 0; i < DEC3_LUT_SIZE; i++)
+    if (i & ((2 << DEC3_BITS) - 1)) t.v[i] = dec3_lut_entry(i);
+  return t;
+}
+__device__ const Dec3Table g_dec3_table = make_dec3_table();
 }  // namespace
 
 // One CTA per group of 8 z-slabs, lane = block, mirror image of the encoder: a
@@ -209,10 +223,7 @@ zfp_decode_slab_kernel(const uint32_t* __restrict__ in, float* __restrict__ out,
   const int bx = b & 7, by = (b >> 3) & 7;
   const uint32_t zt = (b >> 6) * 4;  // first slab of my tile
   uint32_t* col = stage + tid;
-#pragma unroll
-  for (int i = 0; i < DEC_LUT_SIZE / (4 * kThreads); i++)
-    reinterpret_cast<uint4*>(lut)[i * kThreads + tid] =
-        __ldg(reinterpret_cast<const uint4*>(g_dec_table.v) + i * kThreads + tid);
+  copy_table<DEC3_LUT_SIZE>(lut, g_dec3_table.v);
   pdl_wait(in);
   if (zt < nz) {
     const uint32_t* src = in + (size_t)b * nwords;
@@ -261,7 +272,7 @@ zfp_decode_slab_kernel(const uint32_t* __restrict__ in, float* __restrict__ out,
 // no atomics, no zeroed stream.  (One thread per block reading and writing global
 // memory word by word, with plane-by-plane coders whose lanes wait for each other,
 // took 28.7 + 33.4 us a call for 31 x 33 x 4096 at 512 bits and 22.6 + 26.7 us for
-// 768 x 4096 at 128; these take 11.9 + 14.5 and 11.4 + 13.2.  They are bound as the
+// 768 x 4096 at 128; these take 11.9 + 14.3 and 11.4 + 13.2.  They are bound as the
 // slab kernels are, by the number of instructions a block costs.)
 namespace {
 
@@ -426,7 +437,7 @@ zfp_encode_generic_kernel(const FieldGeom g, const float* __restrict__ in, bool 
     lut0 = __ldg(g_enc_table.v + tid);
     lut1 = __ldg(g_enc_table.v + kThreads + tid);
   } else {
-    copy_enc3_table(lut);
+    copy_table<ENC3_LUT_SIZE>(lut, g_enc3_table.v);
   }
   const uint32_t per_cta = (kThreads / 32) << lsh;
   const uint64_t b0 = (uint64_t)blockIdx.x * per_cta, b = block_of_thread(lsh);
@@ -496,11 +507,10 @@ zfp_decode_generic_kernel(const FieldGeom g, const uint32_t* __restrict__ in, fl
   if (DIMS == 1) {
     for (int i = tid; i < DEC1_LUT_SIZE / 8; i += kThreads)
       reinterpret_cast<uint4*>(lut)[i] = __ldg(reinterpret_cast<const uint4*>(g_dec1_table.v) + i);
+  } else if (DIMS == 2) {
+    copy_table<DEC_LUT_SIZE>(lut, g_dec_table.v);
   } else {
-#pragma unroll
-    for (int i = 0; i < DEC_LUT_SIZE / (4 * kThreads); i++)
-      reinterpret_cast<uint4*>(lut)[i * kThreads + tid] =
-          __ldg(reinterpret_cast<const uint4*>(g_dec_table.v) + i * kThreads + tid);
+    copy_table<DEC3_LUT_SIZE>(lut, g_dec3_table.v);
   }
   // reads just past a block find zeros and need no bounds test
   for (int w = nwords; w < nwords + STAGE_SPARE_ROWS; w++) col[w * kThreads] = 0u;
@@ -541,7 +551,7 @@ zfp_decode_generic_kernel(const FieldGeom g, const uint32_t* __restrict__ in, fl
     const BlockAt<DIMS> at(g, b < nblocks ? b : nblocks - 1);
     if constexpr (DIMS == 3) {
       if (!vec && g.sx == 1) {
-        store_rows3(g, out, at, b < nblocks && !is_copy(lsh), reinterpret_cast<float*>(lut + DEC_LUT_SIZE) + 512 * (tid >> 5), f);
+        store_rows3(g, out, at, b < nblocks && !is_copy(lsh), reinterpret_cast<float*>(lut + DEC3_LUT_SIZE) + 512 * (tid >> 5), f);
         continue;
       }
     }
@@ -567,7 +577,7 @@ constexpr int kMostBits = 4096;                    // largest budget the library
 static size_t staged_smem_bytes(int maxbits, bool decode, int dims, bool rowbuf = false) {
   const size_t rows = ((size_t)maxbits + 31) / 32 + STAGE_SPARE_ROWS;
   if (decode && dims == 1) return rows * kThreads * 4 + DEC1_LUT_SIZE * 2;
-  if (decode) return rows * kThreads * 4 + DEC_LUT_SIZE * 4 + (rowbuf ? kThreads * 16 * 4 : 0);
+  if (decode) return (rows * kThreads + (dims == 3 ? DEC3_LUT_SIZE : DEC_LUT_SIZE)) * 4 + (rowbuf ? kThreads * 16 * 4 : 0);
   return (rows + (dims == 3 ? QUEUE_SLOTS * QUEUE_FIELDS : 0)) * kThreads * 4 + (dims == 3 ? ENC3_LUT_SIZE : ENC_LUT_SIZE) * 4;
 }
 // Only the largest budgets need it; the call costs host time on every launch.

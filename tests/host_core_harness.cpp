@@ -111,7 +111,9 @@ struct PadSource {
 };
 void core_decode_pos(const uint32_t* in, size_t nx, size_t ny, size_t nz, int maxbits, float* out) {
   csw::FieldGeom g = csw::make_geom(nx, ny, nz, 0, 0, 0);
-  auto lut = dec_lut();
+  std::vector<uint32_t> lut(csw::DEC3_LUT_SIZE);
+  for (int i = 0; i < csw::DEC3_LUT_SIZE; i++)
+    if (i % (2 << csw::DEC3_BITS)) lut[i] = csw::dec3_lut_entry(i);
   const int nw = maxbits / 32;
   size_t nb = csw::geom_blocks(g);
   for (size_t b = 0; b < nb; b++) {
