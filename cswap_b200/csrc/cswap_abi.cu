@@ -341,9 +341,12 @@ struct Pipeline {
 };
 Pipeline g_pipe;
 
-// Bytes of field.  Up to 8 MiB one copy each way is as fast as a pipeline (218 + 220 us
-// against 226 + 224); 16 MiB gains 4 %, 64 MiB 8 %.
-constexpr size_t kMinPipelined = size_t(12) << 20, kMinChunk = size_t(2) << 20, kMaxChunk = size_t(16) << 20;
+// Bytes of field and of stream from which a call is cut.  What a pipeline hides is the smaller
+// direction, the stream, and what it costs is some microseconds per chunk: the two calls
+// uncut against cut take 629 / 621 us at 12 MiB and 1017 / 962 at 20 MiB with 512 bits, 657 / 689
+// at 14 MiB, 823 / 842 at 18, 913 / 911 at 20 and 1091 / 1074 at 24 MiB with 256.
+constexpr size_t kMinPipelined = size_t(12) << 20, kMinPipelinedStream = size_t(3) << 20;
+constexpr size_t kMinChunk = size_t(2) << 20, kMaxChunk = size_t(16) << 20;
 
 // true when the call was handled here (ok tells how it went)
 bool pipelined_host_call(bool compress, const csw_zfp_field* f, void* h_stream, unsigned maxbits, size_t bytes,
@@ -351,7 +354,7 @@ bool pipelined_host_call(bool compress, const csw_zfp_field* f, void* h_stream, 
   const size_t slab = f->nx * f->ny;                      // values per z-slab
   const size_t blocks_per_4 = ((f->nx + 3) / 4) * ((f->ny + 3) / 4);
   const size_t fb = slab * f->nz * 4;
-  if (maxbits % 64 || !contiguous(f) || fb < kMinPipelined) return false;
+  if (maxbits % 64 || !contiguous(f) || fb < kMinPipelined || bytes < kMinPipelinedStream) return false;
   // Chunk boundaries, in slabs.  A copy costs some microseconds of set-up and its stretch
   // of the pipeline; what is not overlapped is the small direction's chunk at the far end
   // (compression) or at the near end (decompression), so chunks are an eighth of the field

@@ -366,7 +366,9 @@ def test_decode_arbitrary_streams(cs, oracle, dims, maxbits):
 
 
 @pytest.mark.parametrize("nx,ny,nz,maxbits", [(32, 32, 3071, 512), (32, 32, 3072, 512), (32, 32, 3073, 1024),
-                                              (32, 32, 16387, 256), (1000, 500, 9, 512), (70, 50, 1003, 64)])
+                                              (32, 32, 6143, 256), (32, 32, 6148, 256),
+                                              (32, 32, 16387, 256), (1000, 500, 9, 512), (70, 50, 1003, 64),
+                                              (70, 50, 1003, 128)])
 def test_host_calls_cut_anywhere(cs, nx, ny, nz, maxbits):
     """Host field and host stream just below and above the size from which the calls are cut into
     chunks, slab counts that no chunk divides, slabs larger than a chunk: the stream and the values
