@@ -61,6 +61,24 @@ bool as_size(PyObject* o, size_t* v) {
 struct Field {
   size_t nx = 0, ny = 0, nz = 0;
 };
+// An extent; one that is negative or beyond 63 bits fits no tensor.
+bool as_extent(PyObject* o, size_t* v) {
+  const Py_ssize_t x = PyNumber_AsSsize_t(o, nullptr);  // saturates, so that the product below cannot be met
+  if (x == -1 && PyErr_Occurred()) return false;
+  if (x < 0) return value_error("dims do not match the tensor's element count");
+  *v = (size_t)x;
+  return true;
+}
+// Whether the extents, 0 counting as 1 behind the first, multiply to numel.  A product that has
+// passed numel (below 2^63) is not multiplied on, so nothing wraps.
+bool covers(const Field& f, size_t numel) {
+  unsigned __int128 p = f.nx;
+  for (const size_t v : {f.ny, f.nz}) {
+    if (p > numel) return false;
+    p *= v ? v : 1;
+  }
+  return p == numel;
+}
 // (nx, ny, nz) of the call: the caller's, or the swap path's view
 bool field_of(PyObject* dims, size_t numel, Field* f) {
   if (dims == Py_None) return status_ok(csw_zfp_view(numel, &f->nx, &f->ny, &f->nz), "csw_zfp_view");
@@ -68,10 +86,10 @@ bool field_of(PyObject* dims, size_t numel, Field* f) {
   if (!seq) return false;
   bool ok = PySequence_Fast_GET_SIZE(seq) == 3;
   if (!ok) value_error("dims must be (nx, ny, nz)");
-  ok = ok && as_size(PySequence_Fast_GET_ITEM(seq, 0), &f->nx) && as_size(PySequence_Fast_GET_ITEM(seq, 1), &f->ny) &&
-       as_size(PySequence_Fast_GET_ITEM(seq, 2), &f->nz);
+  ok = ok && as_extent(PySequence_Fast_GET_ITEM(seq, 0), &f->nx) &&
+       as_extent(PySequence_Fast_GET_ITEM(seq, 1), &f->ny) && as_extent(PySequence_Fast_GET_ITEM(seq, 2), &f->nz);
   Py_DECREF(seq);
-  if (ok && f->nx * (f->ny ? f->ny : 1) * (f->nz ? f->nz : 1) != numel)
+  if (ok && !covers(*f, numel))
     return value_error("dims do not match the tensor's element count");
   return ok;
 }

@@ -104,16 +104,22 @@ csw_status csw_device_status(csw_stream_t stream) {
 }
 
 // ---- ZFP --------------------------------------------------------------------------
-csw_status csw_zfp_max_bytes(size_t nx, size_t ny, size_t nz, unsigned maxbits, size_t* bytes) {
-  if (!bytes || !valid_maxbits(maxbits)) return CSW_ERR_ARG;
+// Extents and budget of a call.
+static csw_status check_field(size_t nx, size_t ny, size_t nz, unsigned maxbits) {
+  if (!valid_maxbits(maxbits)) return CSW_ERR_ARG;
   if (nx == 0 || (ny == 0 && nz != 0)) return CSW_ERR_ARG;
   if (nx > 0xfffffffcu || ny > 0xfffffffcu || nz > 0xfffffffcu) return CSW_ERR_ARG;  // extents are 32-bit inside
   const FieldGeom g = make_geom(nx, ny, nz, 0, 0, 0);
-  // blocks * maxbits must not wrap a 64-bit count of bits
+  // blocks * maxbits must not wrap a 64-bit count of bits: the size of the stream would come out too small
   const unsigned __int128 bits = (unsigned __int128)g.bx * g.by * g.bz * maxbits;
-  if (bits > ((unsigned __int128)1 << 62)) return CSW_ERR_ARG;
-  *bytes = stream_bytes(g, maxbits);
-  return CSW_OK;
+  return bits > ((unsigned __int128)1 << 62) ? CSW_ERR_ARG : CSW_OK;
+}
+
+csw_status csw_zfp_max_bytes(size_t nx, size_t ny, size_t nz, unsigned maxbits, size_t* bytes) {
+  if (!bytes) return CSW_ERR_ARG;
+  const csw_status st = check_field(nx, ny, nz, maxbits);
+  if (st == CSW_OK) *bytes = stream_bytes(make_geom(nx, ny, nz, 0, 0, 0), maxbits);
+  return st;
 }
 
 csw_status csw_zfp_view(size_t numel, size_t* nx, size_t* ny, size_t* nz) {
@@ -122,13 +128,6 @@ csw_status csw_zfp_view(size_t numel, size_t* nx, size_t* ny, size_t* nz) {
   *nx = 32;
   *ny = 32;
   *nz = numel / 1024;
-  return CSW_OK;
-}
-
-static csw_status check_field(size_t nx, size_t ny, size_t nz, unsigned maxbits) {
-  if (!valid_maxbits(maxbits)) return CSW_ERR_ARG;
-  if (nx == 0 || (ny == 0 && nz != 0)) return CSW_ERR_ARG;
-  if (nx > 0xfffffffcu || ny > 0xfffffffcu || nz > 0xfffffffcu) return CSW_ERR_ARG;
   return CSW_OK;
 }
 

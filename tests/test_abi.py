@@ -57,6 +57,22 @@ def test_sizing_and_layout_without_a_device(L):
     assert L.csw_version().count(b".") == 2
 
 
+def test_fields_whose_size_wraps_are_refused(L):
+    """Extents whose element count (and with it the stream's size) wraps 64 bits: 2^64 + 1024 and 2^64 + 4352
+    values, which would pass for a stream of 128 and 544 bytes.  Refused as an argument before any launch."""
+    b = C.c_size_t()
+    buf = (C.c_char * 65536)()
+    p = C.addressof(buf)
+    for dims in ((4, 1073872904, 4294443040), (2788552, 2841636, 2327944)):
+        for maxbits in (9, 64, 4096):  # at 9 bits the stream's size does not wrap: too large for the buffer
+            st = 2 if maxbits == 9 else 1
+            assert L.csw_zfp_max_bytes(*dims, maxbits, C.byref(b)) == (0 if maxbits == 9 else 1)
+            assert L.csw_zfp_compress(p, *dims, maxbits, p, 65536, None, None) == st
+            assert L.csw_zfp_compress_strided(p, *dims, 1, 4, 16, maxbits, p, 65536, None, None) == st
+            assert L.csw_zfp_decompress(p, 65536, *dims, maxbits, p, None) == st
+            assert L.csw_zfp_decompress_strided(p, 65536, *dims, 1, 4, 16, maxbits, p, None) == st
+
+
 def test_cost_decision_is_pure_host_logic(L):
     import cswap_b200 as cs
     cm = cs.CostModel(zfp_enc_b=2.5e-13, zfp_dec_b=2.5e-13, sparse_enc_b=2e-13, sparse_dec_b=1.5e-13,

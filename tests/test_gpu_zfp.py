@@ -203,6 +203,21 @@ def test_errors_do_not_launch(cs):
     assert torch.count_nonzero(out).item() == 0
 
 
+def test_dims_that_multiply_past_64_bits_are_refused(cs):
+    """The element count of `dims` is compared as an exact integer: products of 2^64 + numel, of two negative
+    extents and of extents no integer register holds are all a ValueError, and nothing is launched."""
+    import torch
+    s = torch.zeros(544, dtype=torch.uint8, device="cuda")
+    t = torch.zeros(1024, device="cuda")
+    for numel, dims in ((1024, (4, 1073872904, 4294443040)), (4352, (2788552, 2841636, 2327944)),
+                        (1024, (-32, -32, 0)), (1024, (-1024, -1, 1)), (1024, (1 << 70, 0, 0)),
+                        (1024, (1 << 62, 4, 1 << 10)), (1024, (32, 32)), (1024, (32, 32, 2))):
+        with pytest.raises(ValueError):
+            cs.zfp_decompress(s, numel, 64, dims)
+        with pytest.raises(ValueError):
+            cs.zfp_compress(t, 64, dims)
+
+
 def test_strided_field(cs, oracle):
     """A 3-D window of a larger array through the strided entry point."""
     import torch
