@@ -34,6 +34,13 @@ __device__ __forceinline__ void pdl_wait(T* __restrict__& p) {
   asm volatile("griddepcontrol.wait;" : "+l"(p)::"memory");
 }
 
+// An error that a call returns is its caller's to report: left pending in the runtime as well,
+// the next cudaGetLastError of the process (torch's after a launch of its own, say) would meet it.
+inline cudaError_t taken(cudaError_t e) {
+  if (e != cudaSuccess) cudaGetLastError();
+  return e;
+}
+
 template <class... P, class... A>
 inline cudaError_t pdl_launch(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream,
                               A&&... args) {
@@ -47,7 +54,7 @@ inline cudaError_t pdl_launch(void (*kernel)(P...), unsigned grid, unsigned bloc
   cfg.stream = stream;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, P(std::forward<A>(args))...);
+  return taken(cudaLaunchKernelEx(&cfg, kernel, P(std::forward<A>(args))...));
 }
 
 }  // namespace csw

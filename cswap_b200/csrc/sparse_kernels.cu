@@ -424,11 +424,11 @@ cudaError_t small_launch(const uint32_t* in, uint64_t n, uint32_t* bitmap, uint3
                          uint32_t* nnz_out, cudaStream_t stream) {
   static std::atomic<uint64_t> allowed{0};
   int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
+  cudaError_t e = taken(cudaGetDevice(&dev));
   if (e != cudaSuccess) return e;
   const uint64_t bit = dev < 64 ? (uint64_t)1 << dev : 0;
   if (!(allowed.load(std::memory_order_acquire) & bit)) {
-    e = cudaFuncSetAttribute(sparse_small_kernel<TILES>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    e = taken(cudaFuncSetAttribute(sparse_small_kernel<TILES>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     if (e != cudaSuccess) return e;
     allowed.fetch_or(bit, std::memory_order_release);
   }
@@ -445,7 +445,7 @@ cudaError_t small_launch(const uint32_t* in, uint64_t n, uint32_t* bitmap, uint3
   cfg.stream = stream;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  return cudaLaunchKernelEx(&cfg, sparse_small_kernel<TILES>, in, n, bitmap, tile_off, values, nnz_out);
+  return taken(cudaLaunchKernelEx(&cfg, sparse_small_kernel<TILES>, in, n, bitmap, tile_off, values, nnz_out));
 }
 // true (and *e set) when the tensor is small enough for one cluster
 bool small_compress(const uint32_t* in, uint64_t n, uint32_t* bitmap, uint32_t* values, uint32_t* tile_off,
@@ -480,7 +480,7 @@ cudaError_t sparse_compress_preload() {
   if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, sparse_count_kernel);
   if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, block_exclusive_scan_kernel<uint32_t>);
   if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, sparse_pack_kernel);
-  return e;
+  return taken(e);
 }
 
 cudaError_t sparse_compress_onepass_launch(const float* in, uint64_t n, uint32_t* bitmap, float* values,

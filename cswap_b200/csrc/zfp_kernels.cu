@@ -584,8 +584,8 @@ static size_t staged_smem_bytes(int maxbits, bool decode, int dims, bool rowbuf 
 template <class K>
 static cudaError_t allow_smem(K* kernel, size_t smem, bool decode, int dims) {
   if (smem <= kDefaultDynamicSmem) return cudaSuccess;
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)staged_smem_bytes(kMostBits, decode, dims, true));
+  return taken(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)staged_smem_bytes(kMostBits, decode, dims, true)));
 }
 
 static uint64_t slab_blocks(const FieldGeom& g) { return ((uint64_t)g.nz + 3) / 4 * 64; }

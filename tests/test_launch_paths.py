@@ -1,0 +1,80 @@
+"""What the launchers do when the runtime refuses something, and which kernels they
+choose, without a GPU: the library's object files linked against a stand-in for
+the CUDA runtime (tests/fake_cudart.cpp) that records launches and copies.  No
+kernel runs; what the kernels compute is tested on the GPU."""
+import ctypes as C
+import os
+import subprocess
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+OBJECTS = ("sparse_kernels", "zfp_kernels", "cswap_abi", "sparse_static")
+
+
+class Fake:
+    def __init__(self, path):
+        self.lib = C.CDLL(path)
+        self.lib.fake_log.restype = C.c_char_p
+        # stands for every device buffer: no kernel runs, so only the address is looked at
+        self._mem = (C.c_char * (1 << 16))()
+        self.buf = (C.addressof(self._mem) + 255) // 256 * 256
+
+    def log(self):
+        return self.lib.fake_log().decode().splitlines()
+
+    def kernels(self):
+        """Names of the kernels that were launched, in order."""
+        names = ("sparse_small", "sparse_count", "block_exclusive_scan", "sparse_pack", "sparse_zero",
+                 "sparse_onepass", "sparse_unpack", "zfp_encode_slab", "zfp_decode_slab", "zfp_encode_generic",
+                 "zfp_decode_generic")
+        return [next(n for n in names if n in line) for line in self.log() if line.startswith("launch")]
+
+    def compress(self, n, onepass=False):
+        fn = self.lib.csw_sparse_compress_onepass if onepass else self.lib.csw_sparse_compress
+        p = C.c_void_p(self.buf)
+        return fn(p, C.c_size_t(n), p, C.c_size_t(1 << 40), p, None)
+
+    def zfp(self, dims, maxbits, decode=False):
+        p, d = C.c_void_p(self.buf), [C.c_size_t(v) for v in dims]
+        if decode:
+            return self.lib.csw_zfp_decompress(p, C.c_size_t(1 << 40), *d, maxbits, p, None)
+        return self.lib.csw_zfp_compress(p, *d, maxbits, p, C.c_size_t(1 << 40), None, None)
+
+
+@pytest.fixture(scope="module")
+def fake_library(tmp_path_factory):
+    from cswap_b200 import build
+    build.build()
+    objs = [os.path.join(build.HERE, "build", o + ".o") for o in OBJECTS]
+    if not all(os.path.exists(o) for o in objs):
+        build.build(force=True)
+    so = str(tmp_path_factory.mktemp("fake") / "libfake.so")
+    subprocess.check_call(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I", os.path.join(CUDA, "include"), "-o", so,
+                           os.path.join(HERE, "fake_cudart.cpp")] + objs + ["-Wl,-Bsymbolic", "-Wl,-z,defs"])
+    return Fake(so)
+
+
+@pytest.fixture
+def fake(fake_library):
+    fake_library.lib.fake_reset()
+    return fake_library
+
+
+def test_a_refused_launch_leaves_no_error_behind(fake):
+    """A call whose launch is refused says so itself; the runtime's last error, which the next caller of
+    cudaGetLastError in the process would take for its own, is clear again."""
+    calls = [lambda: fake.compress(1 << 20), lambda: fake.compress(1 << 20, onepass=True),
+             lambda: fake.zfp((32, 32, 64), 512), lambda: fake.zfp((32, 32, 64), 512, decode=True),
+             lambda: fake.zfp((33, 7, 0), 128), lambda: fake.zfp((33, 7, 0), 128, decode=True),
+             lambda: fake.lib.csw_sparse_decompress(C.c_void_p(fake.buf), C.c_size_t(5000), C.c_void_p(fake.buf), None)]
+    for call in calls:
+        fake.lib.fake_reset()
+        fake.lib.fake_fail_launches(100)
+        assert call() == 3 and fake.lib.fake_pending_error() == 0
+        assert fake.lib.csw_last_cuda_error() == 701  # cudaErrorLaunchOutOfResources
+    for decode in (False, True):  # more shared memory than a kernel may use without opting in
+        fake.lib.fake_reset()
+        fake.lib.fake_fail_attributes(100)
+        assert fake.zfp((32, 32, 64), 2048, decode) == 3 and fake.lib.fake_pending_error() == 0
