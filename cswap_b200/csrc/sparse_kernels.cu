@@ -447,14 +447,16 @@ cudaError_t small_launch(const uint32_t* in, uint64_t n, uint32_t* bitmap, uint3
   cfg.numAttrs = 2;
   return taken(cudaLaunchKernelEx(&cfg, sparse_small_kernel<TILES>, in, n, bitmap, tile_off, values, nnz_out));
 }
-// true (and *e set) when the tensor is small enough for one cluster
+// true when the tensor is small enough for one cluster and its launch went through.  A cluster needs
+// its CTAs' SMs in one GPC, all at a time: a process that has only part of a GPC (a partition, a
+// green context) may be refused the launch, and is served by the ordinary ones.
 bool small_compress(const uint32_t* in, uint64_t n, uint32_t* bitmap, uint32_t* values, uint32_t* tile_off,
-                    uint32_t* nnz_out, cudaStream_t stream, cudaError_t* e) {
-  if (n <= (uint64_t)kMaxCluster * kTile) *e = small_launch<1>(in, n, bitmap, values, tile_off, nnz_out, stream);
-  else if (n <= (uint64_t)kMaxCluster * 2 * kTile) *e = small_launch<2>(in, n, bitmap, values, tile_off, nnz_out, stream);
-  else if (n <= (uint64_t)kMaxCluster * 4 * kTile) *e = small_launch<4>(in, n, bitmap, values, tile_off, nnz_out, stream);
-  else return false;
-  return true;
+                    uint32_t* nnz_out, cudaStream_t stream) {
+  cudaError_t e = cudaErrorNotSupported;
+  if (n <= (uint64_t)kMaxCluster * kTile) e = small_launch<1>(in, n, bitmap, values, tile_off, nnz_out, stream);
+  else if (n <= (uint64_t)kMaxCluster * 2 * kTile) e = small_launch<2>(in, n, bitmap, values, tile_off, nnz_out, stream);
+  else if (n <= (uint64_t)kMaxCluster * 4 * kTile) e = small_launch<4>(in, n, bitmap, values, tile_off, nnz_out, stream);
+  return e == cudaSuccess;
 }
 }  // namespace
 
@@ -463,12 +465,13 @@ cudaError_t sparse_compress_launch(const float* in, uint64_t n, uint32_t* bitmap
   const uint32_t ntiles = (uint32_t)((n + kTile - 1) / kTile);
   const uint32_t* src = reinterpret_cast<const uint32_t*>(in);
   uint32_t* val = reinterpret_cast<uint32_t*>(values);
-  cudaError_t e;
-  if (small_compress(src, n, bitmap, val, tile_off, nnz_out, stream, &e)) return e;
+  if (small_compress(src, n, bitmap, val, tile_off, nnz_out, stream)) return cudaSuccess;
   const bool vec = (reinterpret_cast<uintptr_t>(in) & 15) == 0;
-  e = pdl_launch(sparse_count_kernel, ntiles, kCountThreads, 0, stream, src, n, vec, tile_off);
+  cudaError_t e = cudaSuccess;
+  if (ntiles) e = pdl_launch(sparse_count_kernel, ntiles, kCountThreads, 0, stream, src, n, vec, tile_off);
   if (e == cudaSuccess) e = pdl_launch(block_exclusive_scan_kernel<uint32_t>, 1, 1024, 0, stream, tile_off, ntiles, nnz_out);
-  if (e == cudaSuccess) e = pdl_launch(sparse_pack_kernel, ntiles, kThreads, 0, stream, src, n, bitmap, tile_off, val);
+  if (e == cudaSuccess && ntiles)
+    e = pdl_launch(sparse_pack_kernel, ntiles, kThreads, 0, stream, src, n, bitmap, tile_off, val);
   return e;
 }
 
@@ -488,10 +491,10 @@ cudaError_t sparse_compress_onepass_launch(const float* in, uint64_t n, uint32_t
   const uint32_t ntiles = (uint32_t)((n + kTile - 1) / kTile);
   const uint32_t* src = reinterpret_cast<const uint32_t*>(in);
   uint32_t* val = reinterpret_cast<uint32_t*>(values);
-  cudaError_t e;
-  if (small_compress(src, n, bitmap, val, tile_off, nnz_out, stream, &e)) return e;
-  e = pdl_launch(sparse_zero_kernel, 1, 1, 0, stream, nnz_out);  // the cursor, then the total
-  if (e == cudaSuccess) e = pdl_launch(sparse_onepass_kernel, ntiles, kThreads, 0, stream, src, n, bitmap, tile_off, val, nnz_out);
+  if (small_compress(src, n, bitmap, val, tile_off, nnz_out, stream)) return cudaSuccess;
+  cudaError_t e = pdl_launch(sparse_zero_kernel, 1, 1, 0, stream, nnz_out);  // the cursor, then the total
+  if (e == cudaSuccess && ntiles)
+    e = pdl_launch(sparse_onepass_kernel, ntiles, kThreads, 0, stream, src, n, bitmap, tile_off, val, nnz_out);
   return e;
 }
 

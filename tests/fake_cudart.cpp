@@ -67,7 +67,7 @@ cudaError_t __cudaPopCallConfiguration(dim3*, dim3*, size_t*, void*) { return cu
 
 // ---- launches ------------------------------------------------------------------------
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* fn, void**) {
-  unsigned cluster = 1;
+  unsigned cluster = 0;  // an ordinary launch
   for (unsigned i = 0; i < c->numAttrs; i++)
     if (c->attrs[i].id == cudaLaunchAttributeClusterDimension) cluster = c->attrs[i].val.clusterDim.x;
   cudaError_t e = cudaSuccess;
@@ -82,7 +82,7 @@ cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* fn, voi
   return done(e);
 }
 cudaError_t cudaLaunchKernel(const void* fn, dim3 g, dim3 b, void**, size_t smem, cudaStream_t) {
-  note("launch %s grid %u block %u smem %zu cluster 1\n", g_names[fn].c_str(), g.x, b.x, smem);
+  note("launch %s grid %u block %u smem %zu cluster 0\n", g_names[fn].c_str(), g.x, b.x, smem);
   return cudaSuccess;
 }
 cudaError_t cudaFuncSetAttribute(const void*, cudaFuncAttribute, int) {

@@ -78,3 +78,20 @@ def test_a_refused_launch_leaves_no_error_behind(fake):
         fake.lib.fake_reset()
         fake.lib.fake_fail_attributes(100)
         assert fake.zfp((32, 32, 64), 2048, decode) == 3 and fake.lib.fake_pending_error() == 0
+
+
+@pytest.mark.parametrize("most", [0, 8])  # CTAs of the largest cluster that can be placed
+@pytest.mark.parametrize("n", [0, 1, 4096, 9 * 4096, 16 * 4096, 100003, 64 * 4096])
+def test_a_cluster_that_cannot_be_placed_is_replaced(fake, n, most):
+    """Where a process has only part of a GPC a cluster launch is refused: the call then makes the ordinary
+    launches, which need nothing of the sort, and succeeds."""
+    tiles = -(-n // 4096)
+    for onepass, ordinary in ((False, ["sparse_count", "block_exclusive_scan", "sparse_pack"]),
+                              (True, ["sparse_zero", "sparse_onepass"])):
+        if not tiles:  # nothing to count or pack, only the total to write
+            ordinary = [k for k in ordinary if k in ("block_exclusive_scan", "sparse_zero")]
+        fake.lib.fake_reset()
+        fake.lib.fake_max_cluster(most)
+        assert fake.compress(n, onepass) == 0
+        assert fake.kernels() == (["sparse_small"] if max(tiles, 1) <= most else ordinary)
+        assert fake.lib.fake_pending_error() == 0
