@@ -19,8 +19,10 @@
 //                   tensor; tiles claim their segments with an atomic add, so
 //                   segment order follows the schedule, not the element order.
 //                   16 MiB: 8.2 -> 6.3 us, 256 MiB: 65.8 -> 62.7 us.
-//  up to 1 MiB    - one cluster, one launch for either of the two: 12.3 (6.2)
-//                   -> 3.8 ... 4.4 us, which is what launching costs.
+//  small tensors  - one cluster, one launch: up to 1 MiB in place of the three
+//                   launches (12.3 -> 2.4 ... 4.4 us back to back, which is what
+//                   launching costs), up to 512 KiB in place of the single pass
+//                   (7.5 -> 2.4 ... 3.1; its launcher says why no further).
 //  legacy format  - the reference's `begin | bitmap | values` layout with its
 //                   P-worker chunking, one warp per worker, behind the
 //                   reference's own entry-point names.
@@ -173,7 +175,7 @@ sparse_pack_kernel(const uint32_t* __restrict__ in, uint64_t n, uint32_t* __rest
 }
 
 // ---- small tensors: one cluster --------------------------------------------------------
-// Up to kMaxCluster CTAs of kSmallTiles tiles compress the whole tensor: bitmap,
+// Up to kMaxCluster CTAs of TILES tiles compress the whole tensor: bitmap,
 // counts, offsets and values from one read and one launch.  The CTAs exchange their
 // counts through distributed shared memory; three launches of 2-3 us each are what
 // bounds tensors this small otherwise.
@@ -417,6 +419,7 @@ legacy_unpack_kernel(const uint32_t* __restrict__ values, uint32_t* __restrict__
 // launchers
 // =====================================================================================
 namespace {
+constexpr uint64_t kOnepassClusterElems = (uint64_t)kMaxCluster * 2 * kTile;
 // One launch for what a cluster can hold.  Sixteen CTAs in a cluster are more than the
 // portable eight and need opting in, once per device.
 template <int TILES>
@@ -491,7 +494,14 @@ cudaError_t sparse_compress_onepass_launch(const float* in, uint64_t n, uint32_t
   const uint32_t ntiles = (uint32_t)((n + kTile - 1) / kTile);
   const uint32_t* src = reinterpret_cast<const uint32_t*>(in);
   uint32_t* val = reinterpret_cast<uint32_t*>(values);
-  if (small_compress(src, n, bitmap, val, tile_off, nnz_out, stream)) return cudaSuccess;
+  // Not up to 1 MiB as the ordered compressor: with four tiles each the cluster's CTAs (512 threads of 120
+  // registers) fit no SM that runs anything else, and the two launches are short.  180000 elements 4.3 us in the
+  // cluster, 3.5 in two launches, back to back; 262144 elements 4.4 and 3.3, and beside matrix products of another
+  // stream (which is where the swap manager calls) 15.3 us at the median but 300 at the 90th percentile, a
+  // product's whole run, against 14.1 and 16.8.  131072 elements 3.1 and 3.4 idle, 15.6 and 13.7 beside products,
+  // 13.2 and 13.3 beside a convolution, 41 and 30 beside elementwise kernels that keep every SM full; 16384
+  // elements 2.5 and 3.4, 14.0 and 13.3, 11.6 and 12.7, 36 and 28.
+  if (n <= kOnepassClusterElems && small_compress(src, n, bitmap, val, tile_off, nnz_out, stream)) return cudaSuccess;
   cudaError_t e = pdl_launch(sparse_zero_kernel, 1, 1, 0, stream, nnz_out);  // the cursor, then the total
   if (e == cudaSuccess && ntiles)
     e = pdl_launch(sparse_onepass_kernel, ntiles, kThreads, 0, stream, src, n, bitmap, tile_off, val, nnz_out);

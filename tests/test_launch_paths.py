@@ -95,3 +95,14 @@ def test_a_cluster_that_cannot_be_placed_is_replaced(fake, n, most):
         assert fake.compress(n, onepass) == 0
         assert fake.kernels() == (["sparse_small"] if max(tiles, 1) <= most else ordinary)
         assert fake.lib.fake_pending_error() == 0
+
+
+def test_the_single_pass_compressor_leaves_its_cluster_at_512_kib(fake):
+    """Above, the cluster's blocks want an SM each, and two launches are shorter; the ordered compressor, whose
+    alternative is three dependent launches, keeps it up to 1 MiB."""
+    for n in (1, 4096, 65536, 65537, 131072, 131073, 180000, 262144, 262145):
+        for onepass, most, ordinary in ((False, 262144, ["sparse_count", "block_exclusive_scan", "sparse_pack"]),
+                                        (True, 131072, ["sparse_zero", "sparse_onepass"])):
+            fake.lib.fake_reset()
+            assert fake.compress(n, onepass) == 0
+            assert fake.kernels() == (["sparse_small"] if n <= most else ordinary)
