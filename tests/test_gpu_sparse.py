@@ -232,3 +232,30 @@ def test_compress_at_the_edges_of_the_launch_rule(cs, oracle, n, offset):
             assert np.array_equal(buf[:4 * tile_off.size].view(np.uint32), tile_off)
             assert np.array_equal(buf[L.values:L.values + 4 * nnz].view(np.uint32), values.view(np.uint32))
         assert torch.equal(cs.sparse_decompress(packed, n).view(torch.int32), t.view(torch.int32))
+
+
+@pytest.mark.parametrize("count", [1, 4095, 4096, 4097, 16384, 16385, 20480, 40000, 2 * 16384 + 4097])
+def test_scan_goes_round(cs, count):
+    """The one-CTA scan behind PreAcc and ordered compression takes 16384 counts a round (the last one with 4
+    or 16 a thread): in place, the total apart, and nothing behind the last count touched."""
+    import torch
+    rng = np.random.default_rng(count)
+    a = rng.integers(0, 4097, count + 3).astype(np.int32)
+    t = torch.from_numpy(a).cuda()
+    total = torch.full((1,), -1, dtype=torch.int32, device="cuda")
+    cs.lib().PreAcc(t.data_ptr(), count, total.data_ptr(), 1, 1, torch.cuda.current_stream().cuda_stream)
+    sums = np.cumsum(a[:count], dtype=np.int32)
+    got = t.cpu().numpy()
+    assert int(total.item()) == sums[-1]
+    assert np.array_equal(got[:count], sums - a[:count]) and np.array_equal(got[count:], a[count:])
+
+
+@pytest.mark.parametrize("tiles", [4097, 16385])
+def test_ordered_compress_with_many_tiles(cs, oracle, tiles):
+    """Enough tiles for sixteen counts a thread, and for a second round of the scan."""
+    n = tiles * 4096 - 5
+    rng = np.random.default_rng(tiles)
+    a = rng.standard_normal(n, dtype=np.float32)
+    a[rng.random(n, dtype=np.float32) < 0.7] = 0.0
+    a[4096 * 100:4096 * 103] = 0.0  # empty tiles
+    _check_native(cs, oracle, a)
