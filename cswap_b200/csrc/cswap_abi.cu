@@ -354,6 +354,10 @@ bool pipelined_host_call(bool compress, const csw_zfp_field* f, void* h_stream, 
   const size_t blocks_per_4 = ((f->nx + 3) / 4) * ((f->ny + 3) / 4);
   const size_t fb = slab * f->nz * 4;
   if (maxbits % 64 || !contiguous(f) || fb < kMinPipelined || bytes < kMinPipelinedStream) return false;
+  // Results of the first chunks are written while later ones are still to be read: where the
+  // caller's field and stream share memory, all of it has to be read first.
+  const char* field = static_cast<const char*>(f->data);
+  if (field < static_cast<const char*>(h_stream) + bytes && static_cast<const char*>(h_stream) < field + fb) return false;
   // Chunk boundaries, in slabs.  A copy costs some microseconds of set-up and its stretch
   // of the pipeline; what is not overlapped is the small direction's chunk at the far end
   // (compression) or at the near end (decompression), so chunks are an eighth of the field

@@ -405,6 +405,27 @@ def test_host_calls_cut_anywhere(cs, nx, ny, nz, maxbits):
     assert torch.equal(back, cs.zfp_decompress(want.cuda(), t.numel(), maxbits, (nx, ny, nz)).cpu())
 
 
+def test_host_call_in_place(cs):
+    """A 16 MiB field decoded into, and coded from, the memory that holds its stream."""
+    import torch
+    from cswap_b200._lib import Bitstream, ZfpField, ZfpStream
+    L = cs.lib()
+    nz = 4096
+    t = torch.from_numpy(util.tanh_normal(1024 * nz, seed=9))
+    want = cs.zfp_compress(t.cuda(), 512).cpu()
+    mem = torch.empty(4 * t.numel() + 4096, dtype=torch.uint8).pin_memory()
+    for shift in (0, 4096):  # of the stream against the field
+        p = mem.data_ptr() + shift
+        bs = Bitstream(64, 0, p, p, p + want.numel())
+        zs = ZfpStream(512, 512, 32, -1074, C.pointer(bs))
+        f = ZfpField(3, 32, 32, nz, 0, 0, 0, 0, 0, mem.data_ptr())
+        mem[:4 * t.numel()].copy_(t.view(torch.uint8))
+        assert L.cuda_compress(C.byref(zs), C.byref(f)) == want.numel()
+        assert torch.equal(mem[shift:shift + want.numel()], want)
+        L.cuda_decompress(C.byref(zs), C.byref(f))
+        assert torch.equal(mem[:4 * t.numel()].view(torch.float32), cs.zfp_decompress(want.cuda(), t.numel()).cpu())
+
+
 @pytest.mark.parametrize("nz", [33, 36, 37, 73, 76, 77, 148, 149, 295, 296, 297, 592, 593])
 def test_blocks_spread_over_warps(cs, oracle, nz):
     """Slab counts on either side of where a warp takes 1, 2, 4, 8, 16 or 32 blocks (one warp per

@@ -106,3 +106,31 @@ def test_the_single_pass_compressor_leaves_its_cluster_at_512_kib(fake):
             fake.lib.fake_reset()
             assert fake.compress(n, onepass) == 0
             assert fake.kernels() == (["sparse_small"] if n <= most else ordinary)
+
+
+@pytest.mark.parametrize("decode", [False, True])
+@pytest.mark.parametrize("where", ["apart", "touching", "in place", "at the field's end", "at the stream's end"])
+def test_host_calls_on_overlapping_buffers_are_not_cut(fake, decode, where):
+    """Large host-to-host calls run in chunks whose results are written while later chunks are still to be read.
+    Where the host's field and stream share memory everything is read first, as the reference reads it."""
+    from cswap_b200._lib import Bitstream, ZfpField, ZfpStream
+    nz, maxbits = 4096, 512
+    field_bytes, stream_bytes = 4096 * nz, nz // 4 * 64 * maxbits // 8
+    mem = (C.c_char * (2 * field_bytes))()
+    field = C.addressof(mem) + stream_bytes
+    begin = field + {"apart": field_bytes + 4096, "touching": field_bytes, "in place": 0,
+                     "at the field's end": field_bytes - 8, "at the stream's end": 8 - stream_bytes}[where]
+    bs = Bitstream(64, 0, begin, begin, begin + stream_bytes)
+    zs, f = ZfpStream(maxbits, maxbits, 32, -1074, C.pointer(bs)), ZfpField(3, 32, 32, nz, 0, 0, 0, 0, 0, field)
+    fake.lib.fake_host_pointers()
+    fake.lib.cuda_compress.restype = C.c_size_t
+    if decode:
+        fake.lib.cuda_decompress(C.byref(zs), C.byref(f))
+    else:
+        assert fake.lib.cuda_compress(C.byref(zs), C.byref(f)) == stream_bytes
+    read, written = (stream_bytes, field_bytes) if decode else (field_bytes, stream_bytes)
+    copies = [line.split()[1:] for line in fake.log() if line.startswith("copy")]
+    assert sum(int(n) for k, n in copies if k == "h2d") == read and sum(int(n) for k, n in copies if k == "d2h") == written
+    assert (len(copies) == 2) == (where not in ("apart", "touching"))
+    assert len(copies) != 2 or [k for k, _ in copies] == ["h2d", "d2h"]
+    assert bs.bits == 64 and bs.ptr == begin + stream_bytes
