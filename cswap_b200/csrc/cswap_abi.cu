@@ -3,6 +3,7 @@
 // include/cswap_compat.h.
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
@@ -11,6 +12,7 @@
 #include "../../include/cswap_b200.h"
 #include "../../include/cswap_compat.h"
 #include "internal.h"
+#include "pdl.cuh"
 #include "sparse_kernels.h"
 #include "zfp_kernels.h"
 
@@ -23,11 +25,10 @@ csw_status cuda_fail(cudaError_t e) {
   return CSW_ERR_CUDA;
 }
 
-// ---- per-device state: SM count and the device status word ----------------------
+// ---- per-device state: the device status word, the SM count ----------------------
 namespace {
 struct DeviceState {
   bool ready = false;
-  int sm_count = 0;
   int* d_status = nullptr;  // one int, zero when healthy
 };
 constexpr int kMaxDevices = 64;
@@ -35,7 +36,7 @@ DeviceState g_dev[kMaxDevices];
 std::mutex g_dev_mu;
 }  // namespace
 
-csw_status device_state(int* sm_count, int** d_status) {
+csw_status device_state(int** d_status) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return cuda_fail(e);
@@ -43,17 +44,25 @@ csw_status device_state(int* sm_count, int** d_status) {
   std::lock_guard<std::mutex> lk(g_dev_mu);
   DeviceState& s = g_dev[dev];
   if (!s.ready) {
-    e = cudaDeviceGetAttribute(&s.sm_count, cudaDevAttrMultiProcessorCount, dev);
-    if (e != cudaSuccess) return cuda_fail(e);
     e = cudaMalloc(&s.d_status, sizeof(int));
     if (e != cudaSuccess) return cuda_fail(e);
     e = cudaMemset(s.d_status, 0, sizeof(int));
     if (e != cudaSuccess) return cuda_fail(e);
     s.ready = true;
   }
-  if (sm_count) *sm_count = s.sm_count;
   if (d_status) *d_status = s.d_status;
   return CSW_OK;
+}
+
+int sm_count() {
+  constexpr int kWhole = 148;
+  static std::atomic<int> known[kMaxDevices];
+  int dev = 0, n = kWhole;
+  if (taken(cudaGetDevice(&dev)) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return kWhole;
+  if (const int have = known[dev].load(std::memory_order_relaxed)) return have;
+  if (taken(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess || n < 1) return kWhole;
+  known[dev].store(n, std::memory_order_relaxed);
+  return n;
 }
 
 static bool valid_maxbits(unsigned maxbits) {
@@ -88,7 +97,7 @@ const char* csw_version(void) { return "0.1.0"; }
 
 csw_status csw_device_status(csw_stream_t stream) {
   int* d_status = nullptr;
-  csw_status st = device_state(nullptr, &d_status);
+  csw_status st = device_state(&d_status);
   if (st != CSW_OK) return st;
   cudaError_t e = cudaStreamSynchronize(stream);
   if (e != cudaSuccess) return cuda_fail(e);

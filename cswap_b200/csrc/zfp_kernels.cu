@@ -30,6 +30,7 @@
 
 #include <cstdint>
 
+#include "internal.h"
 #include "pdl.cuh"
 #include "zfp_field.cuh"
 #include "zfp_kernels.h"
@@ -571,8 +572,7 @@ bool vector_rows(const FieldGeom& g, const void* field) {
 // launchers
 // =====================================================================================
 constexpr size_t kDefaultDynamicSmem = 48 * 1024;  // what a kernel may ask for without opting in
-constexpr uint64_t kFullGrid = 148 * 8;             // CTAs the device holds at eight per SM
-constexpr uint64_t kSchedulers = 148 * 4;
+constexpr uint64_t kSchedulersPerSm = 4;
 constexpr int kMostBits = 4096;                    // largest budget the library accepts
 static size_t staged_smem_bytes(int maxbits, bool decode, int dims, bool rowbuf = false) {
   const size_t rows = ((size_t)maxbits + 31) / 32 + STAGE_SPARE_ROWS;
@@ -592,13 +592,14 @@ static uint64_t slab_blocks(const FieldGeom& g) { return ((uint64_t)g.nz + 3) / 
 // log2 of the blocks a warp takes.  While every scheduler of the device has at most one
 // warp, a call lasts as long as one warp does, and a warp waits, plane by plane, for
 // the one of its blocks with the most group tests: the fewer blocks, the shorter.  So blocks
-// are spread until there is a warp for each of the 4 x 148 schedulers.  64 KiB at 512 bits
+// are spread until there is a warp for each of the schedulers, 4 x 148.  64 KiB at 512 bits
 // 5.4 -> 4.4 us (encode) and 7.3 -> 5.2 (decode), 1 MiB at 1024 bits 6.4 -> 5.8 and 8.7 -> 7.8.
 // From two warps a scheduler on the copies cost more issue slots than they save: 4 MiB with
 // 16 blocks a warp 5.6 -> 6.6 and 7.3 -> 7.8.
 static int blocks_per_warp(uint64_t nblocks) {
+  const uint64_t schedulers = kSchedulersPerSm * (unsigned)sm_count();
   int lsh = 0;
-  while (lsh < 5 && (nblocks >> lsh) > kSchedulers) lsh++;
+  while (lsh < 5 && (nblocks >> lsh) > schedulers) lsh++;
   return lsh;
 }
 static unsigned ctas_of(uint64_t nblocks, int lsh) {
@@ -634,7 +635,8 @@ static cudaError_t decode_generic(const FieldGeom& g, const uint32_t* in, float*
   const uint64_t ctas = ctas_of(nblocks, lsh);
   // The parser table is 18 KiB and 128 small blocks are 8 KiB of field or less: once
   // every SM has its eight CTAs, a CTA takes up to eight rounds of blocks.
-  const uint64_t rounds = DIMS == 3 || ctas < 2 * kFullGrid ? 1 : ctas / kFullGrid < 8 ? ctas / kFullGrid : 8;
+  const uint64_t full = 8 * (uint64_t)sm_count();
+  const uint64_t rounds = DIMS == 3 || ctas < 2 * full ? 1 : ctas / full < 8 ? ctas / full : 8;
   return pdl_launch(zfp_decode_generic_kernel<DIMS>, (unsigned)((ctas + rounds - 1) / rounds), kThreads, smem, stream,
                     g, in, out, vector_rows(g, out), maxbits, nblocks, (uint64_t)stream_bytes(g, (unsigned)maxbits) / 4, lsh,
                     pipe_consts());

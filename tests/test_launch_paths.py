@@ -44,7 +44,7 @@ class Fake:
 
 
 @pytest.fixture(scope="module")
-def fake_library(tmp_path_factory):
+def fake_path(tmp_path_factory):
     from cswap_b200 import build
     build.build()
     objs = [os.path.join(build.HERE, "build", o + ".o") for o in OBJECTS]
@@ -53,7 +53,12 @@ def fake_library(tmp_path_factory):
     so = str(tmp_path_factory.mktemp("fake") / "libfake.so")
     subprocess.check_call(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I", os.path.join(CUDA, "include"), "-o", so,
                            os.path.join(HERE, "fake_cudart.cpp")] + objs + ["-Wl,-Bsymbolic", "-Wl,-z,defs"])
-    return Fake(so)
+    return so
+
+
+@pytest.fixture(scope="module")
+def fake_library(fake_path):
+    return Fake(fake_path)
 
 
 @pytest.fixture
@@ -134,3 +139,25 @@ def test_host_calls_on_overlapping_buffers_are_not_cut(fake, decode, where):
     assert (len(copies) == 2) == (where not in ("apart", "touching"))
     assert len(copies) != 2 or [k for k, _ in copies] == ["h2d", "d2h"]
     assert bs.bits == 64 and bs.ptr == begin + stream_bytes
+
+
+@pytest.mark.parametrize("sms", [148, 74, 18])
+def test_grids_follow_the_devices_own_sms(fake_path, tmp_path, sms):
+    """Blocks are spread over warps until there is one for each scheduler of the device at hand, and 2-D decoders
+    take several rounds from twice as many CTAs as it holds: a partition has fewer SMs than the whole chip."""
+    import shutil
+    so = str(tmp_path / "libfake.so")  # a library of its own: the count of a device is asked for once
+    shutil.copy(fake_path, so)
+    fake = Fake(so)
+    fake.lib.fake_reset()
+    fake.lib.fake_sms(sms)
+    for dims in ((32, 32, 148), (31, 30, 148), (32, 32, 8192)):
+        blocks = -(-dims[0] // 4) * -(-dims[1] // 4) * -(-dims[2] // 4)
+        per_warp = next((1 << k for k in range(5) if blocks >> k <= 4 * sms), 32)
+        for decode in (False, True):
+            assert fake.zfp(dims, 512, decode) == 0
+            assert int(fake.log()[-1].split("grid ")[1].split()[0]) == -(-blocks // (4 * per_warp))
+    ctas = 768 * 4096 // 16 // 128
+    rounds = 1 if ctas < 16 * sms else min(ctas // (8 * sms), 8)
+    assert fake.zfp((768, 4096, 0), 128, decode=True) == 0
+    assert int(fake.log()[-1].split("grid ")[1].split()[0]) == -(-ctas // rounds)
