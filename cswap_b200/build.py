@@ -2,9 +2,11 @@
 behind codec.py."""
 from __future__ import annotations
 
+import importlib.metadata
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -32,14 +34,16 @@ def needs_build() -> bool:
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
-    """The CUDA library and the extension module; returns the library's path."""
-    if force or needs_build():
-        _build_lib(verbose)
+    """The CUDA library and, where torch is installed, the extension module; returns the library's path."""
+    build_library(force, verbose)
     build_ext(force)
     return LIB
 
 
-def _build_lib(verbose: bool) -> None:
+def build_library(force: bool = False, verbose: bool = False) -> str:
+    """The CUDA library alone: needs nvcc, neither torch nor Python's headers."""
+    if not force and not needs_build():
+        return LIB
     objdir = os.path.join(HERE, "build")
     os.makedirs(objdir, exist_ok=True)
     objs = []
@@ -58,20 +62,44 @@ def _build_lib(verbose: bool) -> None:
             raise RuntimeError(f"nvcc failed on {s}")
     cmd = [_nvcc(), "-shared", "-o", LIB] + objs + ["-Xcompiler", "-fPIC"]
     subprocess.check_call(cmd)
+    return LIB
 
 
 EXT_SOURCE = os.path.join(CSRC, "codec_ext.cpp")
 EXT = os.path.join(HERE, "_codec_ext.so")
+EXT_STAMP = os.path.join(HERE, "build", "_codec_ext.built_for")
 
 
-def build_ext(force: bool = False) -> str:
-    """Compile the CPython extension behind codec.py against the installed
-    libtorch and the in-tree library (g++; needs no GPU)."""
+def _built_for() -> str:
+    """What an extension module is good for: the interpreter and the torch it was compiled against."""
+    try:
+        torch_version = importlib.metadata.version("torch")
+    except importlib.metadata.PackageNotFoundError:
+        torch_version = "none"
+    return f"{sysconfig.get_config_var('SOABI')} torch {torch_version}"
+
+
+def _ext_up_to_date() -> bool:
     deps = [EXT_SOURCE, os.path.join(ROOT, "include", "cswap_b200.h"), os.path.abspath(__file__)]
-    if not force and os.path.exists(EXT) and all(os.path.getmtime(EXT) >= os.path.getmtime(d) for d in deps):
+    if not os.path.exists(EXT) or not os.path.exists(EXT_STAMP):
+        return False
+    if any(os.path.getmtime(EXT) < os.path.getmtime(d) for d in deps):
+        return False
+    with open(EXT_STAMP) as f:
+        return f.read() == _built_for()
+
+
+def build_ext(force: bool = False) -> str | None:
+    """Compile the CPython extension behind codec.py against the installed
+    libtorch and the in-tree library (g++; needs no GPU).  Without torch there
+    is nothing it could serve: None."""
+    if not force and _ext_up_to_date():
         return EXT
-    import sysconfig
-    import torch
+    try:
+        import torch
+    except ImportError:
+        sys.stderr.write("cswap_b200: torch is not installed, so the extension behind codec.py is not built\n")
+        return None
     t = os.path.dirname(torch.__file__)
     cuda_inc = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
     cmd = ["g++", "-std=c++17", "-O2", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
@@ -81,6 +109,9 @@ def build_ext(force: bool = False) -> str:
            f"-Wl,-rpath,{os.path.join(t, 'lib')}", "-Wl,-rpath,$ORIGIN",
            "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", "-lcswap_b200"]
     subprocess.check_call(cmd)
+    os.makedirs(os.path.dirname(EXT_STAMP), exist_ok=True)
+    with open(EXT_STAMP, "w") as f:
+        f.write(_built_for())
     return EXT
 
 
@@ -124,4 +155,5 @@ if __name__ == "__main__":
     if "--cpp" in sys.argv:
         print(build_cpp_drivers(force="--force" in sys.argv))
         sys.exit(0)
-    print(build(force="--force" in sys.argv, verbose="-v" in sys.argv))
+    make = build_library if "--library" in sys.argv else build
+    print(make(force="--force" in sys.argv, verbose="-v" in sys.argv))
