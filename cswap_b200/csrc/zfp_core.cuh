@@ -42,13 +42,6 @@ CSW_HD uint32_t byte_perm(uint32_t a, uint32_t b, uint32_t s) {
   return r;
 #endif
 }
-CSW_HD int clz64(uint64_t x) {
-#if defined(__CUDA_ARCH__)
-  return __clzll((long long)x);
-#else
-  return x ? __builtin_clzll(x) : 64;
-#endif
-}
 CSW_HD int clz32(uint32_t x) {
 #if defined(__CUDA_ARCH__)
   return __clz((int)x);
@@ -192,24 +185,11 @@ CSW_HD void inv_lift(int& x, int& y, int& z, int& w) {
   w = wadd(w, x); x = twice_minus(x, w);
 }
 
-template <int DIMS>
-CSW_HD void fwd_xform(int (&v)[1 << (2 * DIMS)]) {
-  if constexpr (DIMS == 3) {
+CSW_HD void fwd_xform2(int (&v)[16]) {
 #pragma unroll
-    for (int i = 0; i < 16; i++) fwd_lift(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+  for (int y = 0; y < 4; y++) fwd_lift(v[4 * y], v[4 * y + 1], v[4 * y + 2], v[4 * y + 3]);
 #pragma unroll
-    for (int z = 0; z < 4; z++)
-#pragma unroll
-      for (int x = 0; x < 4; x++)
-        fwd_lift(v[16 * z + x], v[16 * z + x + 4], v[16 * z + x + 8], v[16 * z + x + 12]);
-#pragma unroll
-    for (int i = 0; i < 16; i++) fwd_lift(v[i], v[i + 16], v[i + 32], v[i + 48]);
-  } else {
-#pragma unroll
-    for (int y = 0; y < 4; y++) fwd_lift(v[4 * y], v[4 * y + 1], v[4 * y + 2], v[4 * y + 3]);
-#pragma unroll
-    for (int x = 0; x < 4; x++) fwd_lift(v[x], v[x + 4], v[x + 8], v[x + 12]);
-  }
+  for (int x = 0; x < 4; x++) fwd_lift(v[x], v[x + 4], v[x + 8], v[x + 12]);
 }
 
 template <int DIMS>
@@ -236,13 +216,13 @@ CSW_HD void inv_xform(int (&v)[1 << (2 * DIMS)]) {
 CSW_HD uint32_t int2uint(int x) { return ((uint32_t)x + 0xaaaaaaaau) ^ 0xaaaaaaaau; }
 CSW_HD int uint2int(uint32_t x) { return (int)((x ^ 0xaaaaaaaau) - 0xaaaaaaaau); }
 
-template <int DIMS, int... I>
-CSW_HD void fwd_order(const int (&v)[sizeof...(I)], uint32_t (&u)[sizeof...(I)], std::integer_sequence<int, I...>) {
-  ((u[I] = int2uint(v[PermAt<DIMS, I>::v])), ...);
+template <int... I>
+CSW_HD void fwd_order2(const int (&v)[16], uint32_t (&u)[16], std::integer_sequence<int, I...>) {
+  ((u[I] = int2uint(v[PermAt<2, I>::v])), ...);
 }
-template <int DIMS, int... I>
-CSW_HD void inv_order(const uint32_t (&u)[sizeof...(I)], int (&v)[sizeof...(I)], std::integer_sequence<int, I...>) {
-  ((v[PermAt<DIMS, I>::v] = uint2int(u[I])), ...);
+template <int... I>
+CSW_HD void inv_order2(const uint32_t (&u)[16], int (&v)[16], std::integer_sequence<int, I...>) {
+  ((v[PermAt<2, I>::v] = uint2int(u[I])), ...);
 }
 
 // ---- block exponent and cast (encode.cuh:40-71,120-149) ---------------------------
@@ -290,23 +270,12 @@ CSW_HD void transpose8(uint32_t (&r)[8]) {
   for (int j = 0; j < 8; j += 2) tswap<1, 0x55555555u>(r[j], r[j + 1]);
 }
 
-// p[k] (k = 0..7) <- bit (8c + k) of coefficients 32G .. 32G+31, coefficient
-// 32G + i at bit i.  Byte m of gather word j holds coefficient 8m + j, so after
-// the transpose bit 8m + j of a plane word is coefficient 8m + j.
-// sel = c | (4 + c) << 4 picks byte c of both PRMT operands.
-template <int G, int N>
-CSW_HD void planes_of_byte(const uint32_t (&u)[N], uint32_t sel, uint32_t (&p)[8]) {
-  static_assert(N == 64 || N == 16, "block size");
+// p[k] (k = 0..7) <- bit (8c + k) of the sixteen coefficients of a 2-D block, coefficient i at
+// bit i.  Byte m of gather word j holds coefficient 8m + j, so after the transpose bit 8m + j
+// of a plane word is coefficient 8m + j.  sel = c | (4 + c) << 4 picks byte c of both PRMT operands.
+CSW_HD void planes_of_byte2(const uint32_t (&u)[16], uint32_t sel, uint32_t (&p)[8]) {
 #pragma unroll
-  for (int j = 0; j < 8; j++) {
-    if constexpr (N == 64) {
-      uint32_t t0 = byte_perm(u[32 * G + j], u[32 * G + 8 + j], sel);
-      uint32_t t1 = byte_perm(u[32 * G + 16 + j], u[32 * G + 24 + j], sel);
-      p[j] = byte_perm(t0, t1, 0x5410);
-    } else {
-      p[j] = byte_perm(u[j], u[8 + j], sel) & 0xffffu;
-    }
-  }
+  for (int j = 0; j < 8; j++) p[j] = byte_perm(u[j], u[8 + j], sel) & 0xffffu;
   transpose8(p);
 }
 
@@ -521,23 +490,6 @@ struct Emitter {
     }
     fill = nf;
   }
-  // append the low `len` (0..64) bits of hi:lo; bits at and above len must be zero
-  CSW_HD void emit64(uint32_t lo, uint32_t hi, int len) {
-    uint32_t t1 = funnel_l(lo, hi, fill);
-    const uint32_t t2 = funnel_l(hi, 0u, fill);
-    a0 |= lo << fill;
-    int nf = fill + len;
-    if (nf >= 32) {
-      flush_word(t1);
-      t1 = t2;
-      nf -= 32;
-    }
-    if (nf >= 32) {
-      flush_word(t1);
-      nf -= 32;
-    }
-    fill = nf;
-  }
   // hand over whatever is buffered and zero-fill the rest of the block
   CSW_HD void finish() {
     while (wpos < nwords) flush_word(0u);
@@ -559,48 +511,6 @@ struct SigState {  // by mask and shift instructions that saturate: a dozen fewe
     ghi = bit_or_none(nn - 32);
   }
 };
-
-// ---- encoder: one plane of a 3-D block ----------------------------------------------
-// Codes plane word hi:lo (coefficient i at bit i, N = 64 coefficients) given the
-// significance state (encode.cuh:336-343).  Emission ignores the bit budget:
-// the stream is an exact prefix of the unlimited-budget stream, so the caller
-// stops once total() reaches maxbits and the emitter drops the overrun.
-//
-// The first group-test bit rides on the verbatim prefix (it is bit n of the
-// same word).  The rest of the group-test phase is produced eight positions
-// per step from enc_lut; the loop body has no branches, so lanes only differ
-// in how many steps they take.
-template <int N, class WordSink>
-CSW_HD void encode_plane(uint32_t lo, uint32_t hi, SigState& sg, Emitter<WordSink>& em, const uint32_t* enc_lut) {
-  if (sg.n >= N) {  // everything significant: the plane is copied verbatim
-    em.emit64(lo, hi, N);
-    return;
-  }
-  // remaining positions xs = x >> n (n < 64)
-  const int n = sg.n, s = n & 31;
-  const uint32_t fl = funnel_r(lo, hi, s), sh = hi >> s;
-  uint32_t xl = n < 32 ? fl : sh;
-  uint32_t xh = n < 32 ? sh : 0u;
-  const bool any = (xl | xh) != 0u;
-  em.emit64((lo & sg.mlo) | (any ? sg.glo : 0u), (hi & sg.mhi) | (any ? sg.ghi : 0u), n + 1);
-  if (!any) return;
-  const int top = (int)(hi >> 31);  // last position set: its 1 is implied
-  bool more;
-  do {
-    const uint32_t e = enc_lut[xl & 0xffu];
-    xl = funnel_r(xl, xh, 8);
-    xh >>= 8;
-    more = (xl | xh) != 0u;
-    // a byte that holds the plane's last set bit ends with the '0' terminator
-    // (dropped from the pattern) or, on the last position, with nothing at all
-    const int lf = (int)(e >> 24);
-    const int len = more ? (int)((e >> 16) & 0x1fu) : lf - 2 * top;
-    const uint32_t keep = more ? 0xffffu : low_mask32(lf - 1 - top);
-    em.emit32(e & keep, len);
-  } while (more);
-  const int msb = hi ? 64 - clz32(hi) : 32 - clz32(lo);
-  sg.set(msb);  // xs != 0, so the top set bit lies at or above n
-}
 
 // ---- encoder: one plane of a small block ---------------------------------------------
 // N = 16 coefficients: the whole code of a plane - verbatim prefix, group
@@ -701,65 +611,46 @@ CSW_HD void encode_block1(const float (&f)[4], int maxbits, WordSink& sink, cons
   em.finish();
 }
 
-// ---- encoder: whole block ---------------------------------------------------------
-// f: the block's values, x fastest (index x + 4y + 16z).  Produces exactly
-// ceil(maxbits/32) words through the sink (the last one masked by the caller
-// when maxbits is not a multiple of 32).
-template <int DIMS, class WordSink>
-CSW_HD void encode_block(const float (&f)[1 << (2 * DIMS)], int maxbits, WordSink& sink, const uint32_t* enc_lut) {
-  static_assert(DIMS > 1, "encode_block1");
-  constexpr int N = 1 << (2 * DIMS);
+// ---- encoder: 2-D block -------------------------------------------------------------
+// f: the block's values, x fastest (index x + 4y).  Produces exactly ceil(maxbits/32) words
+// through the sink (the last one masked by the caller when maxbits is not a multiple of 32).
+template <class WordSink>
+CSW_HD void encode_block2(const float (&f)[16], int maxbits, WordSink& sink, const uint32_t* enc_lut) {
   Emitter<WordSink> em(sink, (maxbits + 31) >> 5);
   float m = 0.0f;
 #pragma unroll
-  for (int i = 0; i < N; i++) m = fmaxf(m, fabsf(f[i]));
+  for (int i = 0; i < 16; i++) m = fmaxf(m, fabsf(f[i]));
   const uint32_t e = biased_emax(m);
   if (e == 0) {  // all-zero block: nothing is coded (encode.cuh:356-357)
     em.finish();
     return;
   }
   em.emit32((2u * e + 1u) & 0x1ffu, 9);
-  int v[N];
+  int v[16];
   {
     const float s = quant_scale(e);
 #pragma unroll
-    for (int i = 0; i < N; i++) v[i] = f2i_rz(s * f[i]);
+    for (int i = 0; i < 16; i++) v[i] = f2i_rz(s * f[i]);
   }
-  fwd_xform<DIMS>(v);
-  uint32_t u[N];
-  fwd_order<DIMS>(v, u, std::make_integer_sequence<int, N>{});
+  fwd_xform2(v);
+  uint32_t u[16];
+  fwd_order2(v, u, std::make_integer_sequence<int, 16>{});
 
-  if constexpr (N == 64) {
-    SigState sg;
-    sg.set(0);
-    for (int c = 3; c >= 0; c--) {  // planes 8c+7 .. 8c
-      const uint32_t sel = (uint32_t)c | ((uint32_t)(4 + c) << 4);
-      uint32_t lo[8], hi[8];
-      planes_of_byte<0>(u, sel, lo);
-      planes_of_byte<1>(u, sel, hi);
+  int n = 0;
+  for (int c = 3; c >= 0; c--) {  // planes 8c+7 .. 8c
+    uint32_t x[8];
+    planes_of_byte2(u, (uint32_t)c | ((uint32_t)(4 + c) << 4), x);
 #pragma unroll
-      for (int k = 7; k >= 0; k--) {
-        if (em.total() < maxbits) encode_plane<N>(lo[k], hi[k], sg, em, enc_lut);
-      }
-      if (em.total() >= maxbits) break;
+    for (int k = 7; k >= 0; k--) {
+      if (em.total() < maxbits) encode_plane2(x[k], n, em, enc_lut);
     }
-  } else {
-    int n = 0;
-    for (int c = 3; c >= 0; c--) {
-      uint32_t x[8];
-      planes_of_byte<0>(u, (uint32_t)c | ((uint32_t)(4 + c) << 4), x);
-#pragma unroll
-      for (int k = 7; k >= 0; k--) {
-        if (em.total() < maxbits) encode_plane2(x[k], n, em, enc_lut);
-      }
-      if (em.total() >= maxbits) break;
-    }
+    if (em.total() >= maxbits) break;
   }
   em.finish();
 }
 
-// ---- staged encoder (3-D blocks, whole words per block) ----------------------------
-// Same stream as encode_block, produced in a way that suits a warp whose lanes
+// ---- staged encoder (3-D blocks, any budget) ----------------------------------------
+// The stream of encode.cuh:306-368, produced in a way that suits a warp whose lanes
 // code 32 different blocks:
 //
 //  * every plane's bit offset is known before its bits are made: a plane costs
@@ -835,6 +726,8 @@ CSW_HD void transpose8_bal(uint32_t (&r)[8], const PipeConsts& k) {
 #pragma unroll
   for (int j = 0; j < 8; j += 2) tswap_bal<1, 0x55555555u>(r[j], r[j + 1], k.p1);
 }
+// p[k] (k = 0..7) <- bit (8c + k) of coefficients 32G .. 32G+31 of a 3-D block, coefficient
+// 32G + i at bit i, gathered as planes_of_byte2 does
 template <int G>
 CSW_HD void planes_of_byte_bal(const uint32_t (&u)[64], uint32_t sel, uint32_t (&p)[8], const PipeConsts& k) {
 #pragma unroll
@@ -969,76 +862,6 @@ CSW_HD void encode_block3_staged(const float (&f)[64], int maxbits, Stage& st, c
   }
 }
 
-// ---- bit reader -------------------------------------------------------------------
-// WordSource::get(w) returns the block's w-th 32-bit stream word (0 past the
-// end of the block).
-template <class WordSource>
-struct Reader {
-  uint64_t win;
-  int avail;  // valid bits in win, >= 32 between calls
-  int wi;     // next word to fetch
-  WordSource& src;
-  CSW_HD Reader(WordSource& s) : win(0), avail(0), wi(0), src(s) {
-    win = src.get(0);
-    win |= (uint64_t)src.get(1) << 32;
-    avail = 64;
-    wi = 2;
-  }
-  CSW_HD uint32_t peek() const { return (uint32_t)win; }
-  CSW_HD void skip(int nb) {  // nb in 0..32
-    win >>= nb;
-    avail -= nb;
-    if (avail < 32) {
-      win |= (uint64_t)src.get(wi) << avail;
-      wi++;
-      avail += 32;
-    }
-  }
-  CSW_HD uint32_t take(int nb) {  // nb in 0..32
-    uint32_t r = peek() & low_mask32(nb);
-    skip(nb);
-    return r;
-  }
-};
-
-// ---- decoder: one plane of a 3-D block ----------------------------------------------
-// decode.cuh:141-165 for one plane; returns the plane word.
-template <int N, class WordSource>
-CSW_HD uint64_t decode_plane(Reader<WordSource>& rd, int& n, int& bits, const uint32_t* dec_lut) {
-  // step 1: first min(n, bits) bits verbatim
-  int m = n < bits ? n : bits;
-  bits -= m;
-  uint64_t x;
-  if (m <= 32) {
-    x = rd.take(m);
-  } else {
-    x = rd.take(32);
-    x |= (uint64_t)rd.take(m - 32) << 32;
-  }
-  // step 2: group tests + unary runs
-  int st = 0;
-  for (;;) {
-    if (st == 1 && (n == N - 1 || bits == 0)) {  // run cut short: the one is implied
-      x |= (uint64_t)1 << n;
-      n++;
-      st = 0;
-    }
-    if (st == 0 && (n >= N || bits == 0)) break;
-    int lim = (st == 0 ? N : N - 1) - n;
-    int L = lim < 8 ? lim : 8;
-    L = bits < L ? bits : L;
-    uint32_t e = dec_lut[dec_lut_index(L, st, rd.peek() & 0xffu)];
-    int used = dec_lut_used(e);
-    x |= (uint64_t)dec_lut_pattern(e) << n;
-    n += dec_lut_advance(e);
-    bits -= used;
-    rd.skip(used);
-    st = dec_lut_state(e);
-    if (st == 2) break;
-  }
-  return x;
-}
-
 // ---- decoder: one plane of a small block ----------------------------------------------
 // The code of a plane of 16 coefficients is at most 32 bits: one window
 // of the stream, consumed from the bottom, holds all of it.
@@ -1123,66 +946,46 @@ CSW_HD void decode_block1(WordSource& src, int maxbits, float (&f)[4], const uin
   for (int i = 0; i < 4; i++) f[i] = scale * (float)v[i];
 }
 
-// ---- decoder: whole block ---------------------------------------------------------
-template <int DIMS, class WordSource>
-CSW_HD void decode_block(WordSource& src, int maxbits, float (&f)[1 << (2 * DIMS)], const uint32_t* dec_lut) {
-  constexpr int N = 1 << (2 * DIMS);
+// ---- decoder: 2-D block -------------------------------------------------------------
+// WordSource::get(w) returns the block's w-th 32-bit stream word (0 past the end of the block).
+template <class WordSource>
+CSW_HD void decode_block2(WordSource& src, int maxbits, float (&f)[16], const uint32_t* dec_lut) {
   const uint32_t head = src.get(0);
-  if (!(head & 1u)) {  // zero block (decode.cuh:240-243, decode3.cuh:72-73)
+  if (!(head & 1u)) {  // zero block (decode.cuh:240-243)
 #pragma unroll
-    for (int i = 0; i < N; i++) f[i] = 0.0f;
+    for (int i = 0; i < 16; i++) f[i] = 0.0f;
     return;
   }
   const uint32_t e = (head >> 1) & 0xffu;
-  uint32_t u[N];
+  uint32_t u[16];
 #pragma unroll
-  for (int i = 0; i < N; i++) u[i] = 0;
+  for (int i = 0; i < 16; i++) u[i] = 0;
   int left = maxbits - 9, n = 0;
-  if constexpr (N == 64) {
-    Reader<WordSource> rd(src);
-    rd.skip(9);
-    for (int c = 3; c >= 0; c--) {
-      uint32_t lo[8], hi[8];
+  const int lead = leading_empty_planes(head, src.get(1), left);
+  left -= lead;
+  for (int c = 3; c >= 0; c--) {
+    uint32_t x[8];
 #pragma unroll
-      for (int k = 7; k >= 0; k--) {
-        uint64_t x = 0;
-        if (left > 0) x = decode_plane<N>(rd, n, left, dec_lut);
-        lo[k] = (uint32_t)x;
-        hi[k] = (uint32_t)(x >> 32);
+    for (int k = 7; k >= 0; k--) {
+      x[k] = 0u;
+      if (8 * c + k < 32 - lead && left > 0) {
+        const int pos = maxbits - left;
+        x[k] = decode_plane2(funnel_r(src.get(pos >> 5), src.get((pos >> 5) + 1), pos), n, left, dec_lut);
       }
-      const uint32_t sel0 = (0x3210u & ~(0xfu << (4 * c))) | (4u << (4 * c));
-      const uint32_t step = 1u << (4 * c);
-      bytes_from_planes<0>(lo, sel0, step, u);
-      bytes_from_planes<1>(hi, sel0, step, u);
-      if (left <= 0) break;
     }
-  } else {
-    const int lead = leading_empty_planes(src.get(0), src.get(1), left);
-    left -= lead;
-    for (int c = 3; c >= 0; c--) {
-      uint32_t x[8];
-#pragma unroll
-      for (int k = 7; k >= 0; k--) {
-        x[k] = 0u;
-        if (8 * c + k < 32 - lead && left > 0) {
-          const int pos = maxbits - left;
-          x[k] = decode_plane2(funnel_r(src.get(pos >> 5), src.get((pos >> 5) + 1), pos), n, left, dec_lut);
-        }
-      }
-      bytes_from_planes<0>(x, (0x3210u & ~(0xfu << (4 * c))) | (4u << (4 * c)), 1u << (4 * c), u);
-      if (left <= 0) break;
-    }
+    bytes_from_planes<0>(x, (0x3210u & ~(0xfu << (4 * c))) | (4u << (4 * c)), 1u << (4 * c), u);
+    if (left <= 0) break;
   }
-  int v[N];
-  inv_order<DIMS>(u, v, std::make_integer_sequence<int, N>{});
-  inv_xform<DIMS>(v);
+  int v[16];
+  inv_order2(u, v, std::make_integer_sequence<int, 16>{});
+  inv_xform<2>(v);
   const float w = dequant_scale(e);
 #pragma unroll
-  for (int i = 0; i < N; i++) f[i] = w * (float)v[i];
+  for (int i = 0; i < 16; i++) f[i] = w * (float)v[i];
 }
 
-// ---- decoder for the slab kernel (3-D blocks, whole words per block) ----------------
-// Same result as decode_block<3>.  Instead of shifting a 64-bit window along
+// ---- 3-D decoder (any budget) --------------------------------------------------------
+// The values of decode.cuh:232-288.  Instead of shifting a 64-bit window along
 // the stream (integer-pipe work on every read), the parser keeps one bit
 // position and fetches what it needs from the staged words with two or three
 // shared-memory loads and a funnel shift; the bit budget is simply

@@ -458,7 +458,7 @@ zfp_encode_generic_kernel(const FieldGeom g, const float* __restrict__ in, bool 
       encode_block3_staged(f, maxbits, st, lut, kc);
     } else {
       ColumnSink sink{col};
-      if constexpr (DIMS == 2) encode_block<2>(f, maxbits, sink, lut);
+      if constexpr (DIMS == 2) encode_block2(f, maxbits, sink, lut);
       else encode_block1(f, maxbits, sink, lut);
     }
   }
@@ -546,7 +546,7 @@ zfp_decode_generic_kernel(const FieldGeom g, const uint32_t* __restrict__ in, fl
       decode_block3_pos(source, maxbits, f, lut, kc);
     } else {
       ColumnSource source{col};
-      if constexpr (DIMS == 2) decode_block<2>(source, maxbits, f, lut);
+      if constexpr (DIMS == 2) decode_block2(source, maxbits, f, lut);
       else decode_block1(source, maxbits, f, reinterpret_cast<const uint16_t*>(lut));
     }
     const BlockAt<DIMS> at(g, b < nblocks ? b : nblocks - 1);

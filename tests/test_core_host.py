@@ -27,35 +27,25 @@ def _run(core, O, a, dims, maxbits):
     nx, ny, nz = dims
     a = np.ascontiguousarray(a, dtype=np.float32)
     s = O.zfp_encode(a, nx, ny, nz, maxbits)
-    nb = ((nx + 3) // 4) * max((ny + 3) // 4, 1) * max((nz + 3) // 4, 1)
-    words = nb * maxbits // 32
-    out = np.zeros(words + 4, dtype=np.uint32)
+    out = np.zeros(s.size * 2 + 4, dtype=np.uint32)
     core.core_encode(a.ctypes.data_as(C.c_void_p), C.c_size_t(nx), C.c_size_t(ny), C.c_size_t(nz), maxbits,
                      out.ctypes.data_as(C.c_void_p))
-    sw = s.view(np.uint32)
-    assert np.array_equal(out[:words], sw[:words])
-    if nz:  # the slab kernel's staged encoder must produce the same words
-        out2 = np.zeros(words + 4, dtype=np.uint32)
-        core.core_encode_staged(a.ctypes.data_as(C.c_void_p), C.c_size_t(nx), C.c_size_t(ny), C.c_size_t(nz), maxbits,
-                                out2.ctypes.data_as(C.c_void_p))
-        assert np.array_equal(out2[:words], sw[:words])
+    assert np.array_equal(out[:s.size * 2], s.view(np.uint32)) and not out[s.size * 2:].any()
+    _check_decode(core, O, s, dims, maxbits)
+
+
+def _check_decode(core, O, s, dims, maxbits):
+    nx, ny, nz = dims
     d = O.zfp_decode(s, nx, ny, nz, maxbits)
-    d2 = np.zeros(a.size, dtype=np.float32)
-    inw = np.zeros(words + 4, dtype=np.uint32)
-    inw[:sw.size] = sw
-    core.core_decode(inw.ctypes.data_as(C.c_void_p), C.c_size_t(nx), C.c_size_t(ny), C.c_size_t(nz), maxbits,
+    d2 = np.zeros(d.size, dtype=np.float32)
+    core.core_decode(s.ctypes.data_as(C.c_void_p), C.c_size_t(nx), C.c_size_t(ny), C.c_size_t(nz), maxbits,
                      d2.ctypes.data_as(C.c_void_p))
     assert np.array_equal(d.view(np.uint32), d2.view(np.uint32))
-    if nz:  # the slab kernel's position-based decoder
-        d3 = np.zeros(a.size, dtype=np.float32)
-        core.core_decode_pos(inw.ctypes.data_as(C.c_void_p), C.c_size_t(nx), C.c_size_t(ny), C.c_size_t(nz), maxbits,
-                             d3.ctypes.data_as(C.c_void_p))
-        assert np.array_equal(d.view(np.uint32), d3.view(np.uint32))
 
 
 @pytest.mark.parametrize("dims", [(32, 32, 16), (32, 32, 7), (9, 5, 3), (4, 4, 4), (13, 0, 0), (64, 0, 0),
                                   (12, 10, 0), (32, 32, 0), (5, 5, 5)])
-@pytest.mark.parametrize("maxbits", [32, 64, 96, 128, 256, 512, 1024, 2048])
+@pytest.mark.parametrize("maxbits", [9, 10, 32, 33, 37, 64, 95, 96, 128, 256, 300, 512, 1024, 2048, 4095, 4096])
 def test_core_matches_oracle(core, oracle, dims, maxbits):
     nx, ny, nz = dims
     n = nx * max(ny, 1) * max(nz, 1)
@@ -70,7 +60,7 @@ def test_core_matches_oracle(core, oracle, dims, maxbits):
 
 def test_core_on_awkward_blocks(core, oracle):
     a = util.block_zoo(32 * 32 * 12, seed=4)
-    for maxbits in (64, 512, 1024):
+    for maxbits in (64, 512, 1024, 9, 33, 300, 777, 4095):
         _run(core, oracle, a, (32, 32, 12), maxbits)
 
 
@@ -82,22 +72,11 @@ def test_stream_sizes_agree(core, oracle):
             assert got == oracle.zfp_stream_bytes(*dims, maxbits)
 
 
-@pytest.mark.parametrize("maxbits", [32, 64, 128, 512, 1024])
-def test_decoders_agree_on_arbitrary_streams(core, oracle, maxbits):
+@pytest.mark.parametrize("maxbits", [9, 32, 33, 64, 100, 128, 300, 512, 1024, 4095])
+@pytest.mark.parametrize("dims", [(32, 32, 8), (130, 37, 0), (4099, 0, 0)])
+def test_decoders_agree_on_arbitrary_streams(core, oracle, maxbits, dims):
     """Decoding is defined for any bit string (a swapped-out tensor may come
-    back from a file): both decoders of the library's core must produce what
+    back from a file): the decoders of the library's core must produce what
     the oracle produces, bit for bit, also for streams no encoder wrote."""
-    nx, ny, nz = 32, 32, 8
-    nb = 8 * 8 * 2
-    words = nb * maxbits // 32
-    for sw in util.arbitrary_streams(words, maxbits):
-        s64 = np.zeros((words + 1) // 2, dtype=np.uint64)
-        s64.view(np.uint32)[:words] = sw
-        d = oracle.zfp_decode(s64, nx, ny, nz, maxbits)
-        inw = np.zeros(words + 4, dtype=np.uint32)
-        inw[:words] = sw
-        for fn in (core.core_decode, core.core_decode_pos):
-            out = np.zeros(nx * ny * nz, dtype=np.float32)
-            fn(inw.ctypes.data_as(C.c_void_p), C.c_size_t(nx), C.c_size_t(ny), C.c_size_t(nz), maxbits,
-               out.ctypes.data_as(C.c_void_p))
-            assert np.array_equal(d.view(np.uint32), out.view(np.uint32))
+    for sw in util.arbitrary_streams(oracle.zfp_stream_bytes(*dims, maxbits) // 4, maxbits):
+        _check_decode(core, oracle, np.ascontiguousarray(sw).view(np.uint64), dims, maxbits)
