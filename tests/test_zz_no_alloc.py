@@ -1,9 +1,9 @@
 """csw_sparse_compress_static - the entry point for callers that cannot
 allocate device memory when they need to compress (allocator locked or
-exhausted, callbacks that must not synchronise, fixed memory budgets).  Its
-scratch is a fixed array inside the library; this checks, through the C ABI,
-that it produces exactly what csw_sparse_compress produces, on two calls in a
-row that share that array."""
+exhausted, callbacks that must not synchronise, fixed memory budgets).  The
+compressor's working state lives in the output buffer; this checks, through the
+C ABI, that it produces exactly what csw_sparse_compress produces, on two calls
+in a row, and that a warmed call takes no device memory."""
 import ctypes as C
 
 import numpy as np
@@ -34,8 +34,7 @@ def test_static_scratch_entry_point_matches_the_allocating_one():
     import cswap_b200 as cs
     lib = cs.lib()
     rng = np.random.default_rng(77)
-    # second call is smaller and sparser than the first: stale counters of the
-    # first call's extra tiles stay in the shared array and must not matter
+    # second call is smaller and sparser than the first: nothing of the first may show
     for n, keep in ((3 * 4096 * 37 + 123, 0.5), (4096 * 5 + 7, 0.1)):
         a = (rng.standard_normal(n) * (rng.random(n) < keep)).astype(np.float32)
         a[1] = -0.0
@@ -61,7 +60,7 @@ def test_static_scratch_entry_point_matches_the_allocating_one():
     # exactly the limit passes the limit check (capacity 0 then stops it before any launch)
     st = lib.csw_sparse_compress_static(t.data_ptr(), C.c_size_t(268435456), out_keep.data_ptr(), 0, z.data_ptr(), None)
     assert st == 2
-    # beyond the fixed array: refused, nothing launched
+    # beyond the limit: refused, nothing launched
     big = C.c_size_t(268435456 + 1)
     st = lib.csw_sparse_compress_static(t.data_ptr(), big, t.data_ptr(), 0, t.data_ptr(), None)
     assert st == 8 and b"fixed limit" in lib.csw_status_string(st)
