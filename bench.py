@@ -3,7 +3,8 @@
 
 One "step" = ZFP fixed-rate compress + decompress of one float32 tensor
 (default 256 MiB, rate 8, values tanh(N(0,1)), viewed 32 x 32 x numel/1024) on
-each GPU.  Prints ONE JSON line:
+each GPU.  Prints ONE JSON line of some 2 KB; the side measurements, which are
+twenty times as long, go to standard error as a line of their own ("extra: {...}"):
 
   value     uncompressed GB/s through the round trip, all GPUs together:
             n_gpus * 2 * 4N bytes / (time of K steps / K), inputs resident in HBM
@@ -14,7 +15,7 @@ each GPU.  Prints ONE JSON line:
             (host->device and device->host copies inside the timed region)
   cpu_baseline  the CPU codec (oracle port, OpenMP over blocks) on a bounded
             sample of the same data, on this host's cores
-  extra     reference_cuda (the reference's own CUDA kernels on the same tensors,
+  extra     (standard error) reference_cuda (the reference's own CUDA kernels on the same tensors,
             when their build is present), link (plain pinned-copy ceiling with
             all ranks copying at once), zfp_sweep (64 KiB .. 512 MiB x rates x
             distributions), sparse codec at 50/75/90 % zeros, swap-manager
@@ -827,8 +828,11 @@ def main():
             "steps": args.steps, "warmup": max(args.warmup, 3), "ms_per_step": ms_per_step, "higher_is_better": True,
             "scaling": "weak", "vs_baseline": None, "dtype": "f32->i32/u64", "data": "synthetic",
             "config": workload_config(args), "roofline": roofline, "cpu_baseline": cpu, "e2e": e2e,
-            "gpu_launches": 2 * args.steps, "clocks": clocks, "sustained": sustained, "extra": extra,
+            "gpu_launches": 2 * args.steps, "clocks": clocks, "sustained": sustained,
         }
+        if extra:
+            line["speedup_over_reference_cuda"] = extra["speedup_over_reference_cuda"]
+            print("extra: " + json.dumps(extra), file=sys.stderr, flush=True)
         emit(line)
     if world > 1:
         dist.destroy_process_group()
