@@ -89,10 +89,18 @@ CSW_HD bool warp_all(bool p) {
   return p;
 #endif
 }
-// smallest value over the lanes of the warp, all of which must call (host: the one "lane")
-CSW_HD int warp_min(int v) {
+// true when it holds on some lane of the warp, all of which must call (host: the one "lane")
+CSW_HD bool warp_any(bool p) {
 #if defined(__CUDA_ARCH__)
-  return __reduce_min_sync(0xffffffffu, v);
+  return __any_sync(0xffffffffu, p);
+#else
+  return p;
+#endif
+}
+// largest value over the lanes of the warp, all of which must call
+CSW_HD int warp_max(int v) {
+#if defined(__CUDA_ARCH__)
+  return __reduce_max_sync(0xffffffffu, v);
 #else
   return v;
 #endif
@@ -146,6 +154,51 @@ CSW_HD void mul2(float s, float a, float b, float& x, float& y) {
 #endif
 }
 
+// pairs of floats: two operations in one instruction on the device
+struct F2 {
+  float x, y;
+};
+CSW_HD float fma1(float a, float b, float c) {
+#if defined(__CUDA_ARCH__)
+  return __fmaf_rn(a, b, c);
+#else
+  return __builtin_fmaf(a, b, c);
+#endif
+}
+CSW_HD F2 fma2(F2 a, float s, F2 c) {
+#if defined(__CUDA_ARCH__)
+  F2 d;
+  asm("{\n\t.reg .b64 p, q, r;\n\tmov.b64 p, {%2, %3};\n\tmov.b64 q, {%4, %4};\n\tmov.b64 r, {%5, %6};\n\t"
+      "fma.rn.f32x2 p, p, q, r;\n\tmov.b64 {%0, %1}, p;\n\t}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(s), "f"(c.x), "f"(c.y));
+  return d;
+#else
+  return F2{fma1(a.x, s, c.x), fma1(a.y, s, c.y)};
+#endif
+}
+CSW_HD F2 add2(F2 a, F2 b) {
+#if defined(__CUDA_ARCH__)
+  F2 d;
+  asm("{\n\t.reg .b64 p, q;\n\tmov.b64 p, {%2, %3};\n\tmov.b64 q, {%4, %5};\n\t"
+      "add.rn.f32x2 p, p, q;\n\tmov.b64 {%0, %1}, p;\n\t}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+#else
+  return F2{a.x + b.x, a.y + b.y};
+#endif
+}
+
+// largest magnitude of three
+CSW_HD float max_abs3(float a, float b, float c) {
+#if defined(__CUDA_ARCH__)
+  float d;
+  asm("max.abs.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+#else
+  return fmaxf(fmaxf(fabsf(a), fabsf(b)), fabsf(c));
+#endif
+}
+
 // ---- sequency order (constants.h:8-131), entries are x + 4y + 16z ---------------
 constexpr int perm3(int i) {
   constexpr unsigned char t[64] = {
@@ -192,24 +245,22 @@ CSW_HD void fwd_xform2(int (&v)[16]) {
   for (int x = 0; x < 4; x++) fwd_lift(v[x], v[x + 4], v[x + 8], v[x + 12]);
 }
 
-template <int DIMS>
-CSW_HD void inv_xform(int (&v)[1 << (2 * DIMS)]) {
-  if constexpr (DIMS == 3) {
+CSW_HD void inv_xform3(int (&v)[64]) {
 #pragma unroll
-    for (int i = 0; i < 16; i++) inv_lift(v[i], v[i + 16], v[i + 32], v[i + 48]);
+  for (int i = 0; i < 16; i++) inv_lift(v[i], v[i + 16], v[i + 32], v[i + 48]);
 #pragma unroll
-    for (int z = 0; z < 4; z++)
+  for (int z = 0; z < 4; z++)
 #pragma unroll
-      for (int x = 0; x < 4; x++)
-        inv_lift(v[16 * z + x], v[16 * z + x + 4], v[16 * z + x + 8], v[16 * z + x + 12]);
+    for (int x = 0; x < 4; x++)
+      inv_lift(v[16 * z + x], v[16 * z + x + 4], v[16 * z + x + 8], v[16 * z + x + 12]);
 #pragma unroll
-    for (int i = 0; i < 16; i++) inv_lift(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-  } else {
+  for (int i = 0; i < 16; i++) inv_lift(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+}
+CSW_HD void inv_xform2(int (&v)[16]) {
 #pragma unroll
-    for (int x = 0; x < 4; x++) inv_lift(v[x], v[x + 4], v[x + 8], v[x + 12]);
+  for (int x = 0; x < 4; x++) inv_lift(v[x], v[x + 4], v[x + 8], v[x + 12]);
 #pragma unroll
-    for (int y = 0; y < 4; y++) inv_lift(v[4 * y], v[4 * y + 1], v[4 * y + 2], v[4 * y + 3]);
-  }
+  for (int y = 0; y < 4; y++) inv_lift(v[4 * y], v[4 * y + 1], v[4 * y + 2], v[4 * y + 3]);
 }
 
 // ---- negabinary (shared.h:176-181, decode.cuh:33-37) ------------------------------
@@ -415,34 +466,49 @@ constexpr CSW_HD uint16_t dec1_lut_entry(int idx) {
   return (uint16_t)(x | ((uint32_t)len << 4) | ((uint32_t)n << 8));
 }
 
-// The same for up to ten stream bits, for the 3-D decoder: of a row with limit L only the
-// first L bits matter, so its entries are the 1 << L ones behind entry (1 << L) of the
-// state's half.  Bits 0..9: plane bits found; 16..23: positions advanced; 24..27: stream bits
-// consumed; 30..31: state afterwards.
-constexpr int DEC3_BITS = 10, DEC3_LUT_SIZE = 2 << (DEC3_BITS + 1);
+// The same for up to nine stream bits, for the 3-D decoder, whose steps are limited by the open
+// positions alone (its words are zero past the budget).  With L < 9 exactly L positions are open,
+// with L = 9 at least as many; a row of limit L has an entry for each value of L stream bits, behind
+// entry (1 << L) of the state's half.  A run reads one bit less: the last position's one is implied.
+// Bits 0..8: plane bits found; 9: the plane is finished; 10: a run is open (the other half is
+// next; the bits from 9 on are never shifted into what was found); 16..23: stream bits consumed;
+// 24..31: positions advanced.
+constexpr int DEC3_BITS = 9, DEC3_LUT_SIZE = 2 << (DEC3_BITS + 1);
+constexpr uint32_t DEC3_END = 1u << DEC3_BITS, DEC3_RUN = 2u << DEC3_BITS;
 constexpr CSW_HD uint32_t dec3_lut_entry(int idx) {
   const int half = idx & ((2 << DEC3_BITS) - 1);
-  int st = idx >> (DEC3_BITS + 1), L = 0;
+  bool run = (idx >> (DEC3_BITS + 1)) != 0, end = false;
+  int L = 0;
   while ((2 << L) <= half) L++;
   const uint32_t bits = (uint32_t)(half - (1 << L));
+  const int last = L < DEC3_BITS ? L - 1 : 1000;  // the last open position, where it is known
+  const int most = run && L > 0 ? L - 1 : L;      // bits to read
   int c = 0, dn = 0;
   uint32_t pat = 0;
-  if (L == 0) {
-    if (st == 1) { pat = 1u; dn = 1; }
-    st = 2;
-  }
-  while (c < L) {
-    const uint32_t bit = (bits >> c) & 1u;
-    c++;
-    if (st == 0) {
-      if (bit) st = 1;
-      else { st = 2; break; }
+  while (!end) {
+    if (dn > last) {
+      end = dn > 0;  // no position open at all is no plane: nothing happens
+      break;
+    } else if (run && dn == last) {
+      pat |= 1u << dn++;
+      run = false;
+    } else if (c == most) {
+      break;
     } else {
-      if (bit) { pat |= 1u << dn; st = 0; }
-      dn++;
+      const uint32_t bit = (bits >> c++) & 1u;
+      if (!run) {
+        if (bit) run = true;
+        else end = true;
+      } else {
+        if (bit) {
+          pat |= 1u << dn;
+          run = false;
+        }
+        dn++;
+      }
     }
   }
-  return pat | ((uint32_t)dn << 16) | ((uint32_t)c << 24) | ((uint32_t)st << 30);
+  return pat | (end ? DEC3_END : 0u) | (run ? DEC3_RUN : 0u) | ((uint32_t)c << 16) | ((uint32_t)dn << 24);
 }
 
 // ---- bit emitter ------------------------------------------------------------------
@@ -978,138 +1044,456 @@ CSW_HD void decode_block2(WordSource& src, int maxbits, float (&f)[16], const ui
   }
   int v[16];
   inv_order2(u, v, std::make_integer_sequence<int, 16>{});
-  inv_xform<2>(v);
+  inv_xform2(v);
   const float w = dequant_scale(e);
 #pragma unroll
   for (int i = 0; i < 16; i++) f[i] = w * (float)v[i];
 }
 
 // ---- 3-D decoder (any budget) --------------------------------------------------------
-// The values of decode.cuh:232-288.  Instead of shifting a 64-bit window along
-// the stream (integer-pipe work on every read), the parser keeps one bit
-// position and fetches what it needs from the staged words with two or three
-// shared-memory loads and a funnel shift; the bit budget is simply
-// maxbits - pos.  WordSrc::word(w) returns the block's w-th 32-bit word and 0
-// for the two rows past the end.
-template <class WordSrc>
-CSW_HD uint32_t peek_at(const WordSrc& src, int pos) {
-  const int w = pos >> 5;
-  return funnel_r(src.word(w), src.word(w + 1), pos);  // the shift uses pos mod 32
-}
-// (h:l) rotated right by r, r in 0..31
-CSW_HD void ror64_small(uint32_t& l, uint32_t& h, int r) {
-  const uint32_t t = funnel_r(l, h, r);
-  h = funnel_r(h, l, r);
-  l = t;
-}
-// (h:l) rotated left by r, r in 0..63
+// The values of decode.cuh:232-288.  A warp's lanes decode 32 different blocks, whose group
+// tests lie in different planes and take different numbers of steps, so nothing here goes
+// plane by plane for the warp as a whole:
+//
+//  * Planes are counted from a block's own first one that is not empty (the empty ones ahead
+//    of it are one '0' bit each), and taken in chunks of eight.
+//  * In a chunk every lane first runs through the group tests of its own planes, as long as
+//    it has coefficients that are not significant, and parks a mark at the end of each: where
+//    the next plane begins and how many of its bits are verbatim.  The loop lasts as long as the lane
+//    with the most steps, not the sum over planes of the longest (15.7 steps against 33.7 at
+//    512 bits, counted on the CPU for tanh of normal values).  What the tests find needs no slots:
+//    a position becomes significant once, so the bits of all planes fit into one word.
+//  * Then the eight planes are put together by all lanes in step - a funnel shift of staged
+//    words, the found bits, masks - and transposed.
+//
+// WordSrc::word(w) returns the block's w-th 32-bit word, with zeros for the bits past the
+// budget and for DEC3_SPARE_ROWS words behind it: a group test that finds no bits ends its plane,
+// as it must, and only a run cut by the budget needs a correction (decode_tests3).
+// Park: mark(j) is the lane's slot j, j <= DEC3_CHUNK + 1.
+constexpr int DEC3_SPARE_ROWS = 4, DEC3_CHUNK = 8;
+
+// (h:l) rotated left by r, r in 0..64
 CSW_HD void rol64(uint32_t& l, uint32_t& h, int r) {
   const uint32_t a = (r & 32) ? h : l, b = (r & 32) ? l : h;  // halves after a rotation by 32
   l = funnel_l(b, a, r);
   h = funnel_l(a, b, r);
 }
 
-template <int... I>
-CSW_HD void inv_order3_sub(const uint32_t (&u)[64], int (&v)[64], uint32_t nb, int mone,
-                           std::integer_sequence<int, I...>) {
-  ((v[PermAt<3, I>::v] = imad((int)nb, mone, (int)u[I])), ...);  // u - 0xaaaaaaaa on the multiply-add pipe
+// A place in the stream: bit position in the low half, significant coefficients in the high one.
+CSW_HD int mark_pos(uint32_t m) { return (int)(m & 0xffffu); }
+CSW_HD int mark_n(uint32_t m) { return (int)(m >> 16); }
+
+// What the group tests of a block have found so far: position p of n is bit 64 - n + p of (hi:lo).
+struct Found {
+  uint32_t lo, hi;
+};
+
+// The group tests and unary runs (decode.cuh:147-164) of up to eight planes from `m` on, up to
+// nine stream bits per step.  Returns how many planes had any; m moves behind them.  All lanes of
+// the warp go round together, with a vote at every step: left to itself the compiler makes two
+// loops of this one, the inner one a plane's steps, and the lanes wait at its end.
+template <class WordSrc, class Park>
+CSW_HD int decode_tests3(const WordSrc& src, Park& park, int maxbits, const uint32_t* dec_lut, uint32_t& m, Found& found) {
+  constexpr uint32_t kDone = 64u << 16;  // no open position: steps change nothing
+  int j = 0;
+  park.put_mark(0, m);
+  uint32_t at = m + (m >> 16), run = 0u;
+  if (m >= kDone || mark_pos(m) >= maxbits) at = kDone;
+  while (warp_any(at < kDone)) {
+    const int open = 64 - (int)(at >> 16);
+    const uint32_t mask = low_mask32(open < DEC3_BITS ? open : DEC3_BITS);
+    const int w = mark_pos(at) >> 5;
+    const uint32_t win = funnel_r(src.word(w), src.word(w + 1), (int)at);
+    const uint32_t en = dec_lut[run + mask + 1u + (win & mask)];
+    const int dn = (int)(en >> 24);
+    found.lo = funnel_r(found.lo, found.hi, dn);
+    found.hi = funnel_r(found.hi, en, dn);
+    at += byte_perm(en, 0u, 0x4342u);
+    run = en & DEC3_RUN;
+    park.put_mark(j + 1, at);  // stays when the plane is finished
+    const bool end = (en & DEC3_END) != 0u;
+    j += end ? 1 : 0;
+    uint32_t next = at + (at >> 16);  // behind the verbatim bits
+    next = (int)(j == DEC3_CHUNK) | (int)(mark_pos(at) >= maxbits) ? kDone : next;
+    next = at >= kDone ? kDone : next;
+    at = end ? next : at;
+  }
+  m = park.mark(j);
+  // A run cut by the budget: its one belongs where the bits ran out, but it ran on through the
+  // zeros behind them to the last position, where it is implied.
+  const int over = mark_pos(m) - maxbits;
+  if (over > 0 && m >= kDone && j > 0) {
+    found.hi &= 0x7fffffffu;
+    if (over < 32) found.hi |= 0x80000000u >> over;
+    else found.lo |= 0x80000000u >> (over - 32);
+  }
+  return j;
 }
-// Planes 8c+7 .. 8c of one block: (hi[k]:lo[k]) <- plane 8c+k, odd planes
-// complemented (the xor half of the inverse negabinary map, applied to planes
-// instead of coefficients).  `skip` leading planes of the slice are known to be
-// empty and have been stepped over already (warp-uniform).
-template <class WordSrc>
-CSW_HD void decode_slice3(const WordSrc& src, int maxbits, const uint32_t* dec_lut, int skip, int& pos, int& n,
-                          uint32_t (&lo)[8], uint32_t (&hi)[8]) {
+
+// Eight planes, transposed: byte b of w[8 * g + i] holds coefficient 32g + 8b + i (in sequency
+// order), the first plane in its top bit, odd bits complemented (the xor half of the inverse negabinary
+// map).  `tests` of them have group tests, which decode_tests3 found; `m` is what it left, and moves
+// behind the chunk.  left: planes of the block that begin within the budget, from this chunk on (nine when
+// there are more than eight).  NARROW: look out for warps none of whose coefficients from the 32nd on
+// is significant yet.
+template <bool NARROW, class WordSrc, class Park>
+CSW_HD void decode_rows3(const WordSrc& src, const Park& park, int maxbits, int tests, uint32_t& m, const Found& found,
+                         int& left, uint32_t (&w)[16]) {
+  const int nwords = (maxbits + 31) >> 5;
+  uint32_t at = park.mark(0);
+  {
+    const int rest = maxbits - mark_pos(m);
+    left = tests + (rest > 0 ? (mark_n(m) == 64 ? (rest + 63) >> 6 : 1) : 0);
+  }
+  const int warp_tests = warp_max(tests), warp_left = warp_max(left);
+  uint32_t fl = found.lo, fh = found.hi;
+  rol64(fl, fh, mark_n(m));  // position p at bit p
+  uint32_t ml = low_mask_sat(mark_n(at)), mh = low_mask_sat(mark_n(at) - 32);
+  if (warp_left == 1 && warp_tests == 0) {
+    // A plane is left, the usual case behind eight or sixteen of a budget of whole values: no transpose.
+    int i = mark_pos(at) >> 5;
+    i = i < nwords ? i : nwords;
+    const uint32_t w0 = src.word(i), w1 = src.word(i + 1), w2 = src.word(i + 2);
+    const uint32_t xl = ~funnel_r(w0, w1, (int)at), xh = ~funnel_r(w1, w2, (int)at);
 #pragma unroll
-  for (int k = 7; k >= 0; k--) {
+    for (int k = 0; k < 8; k++) {
+      w[k] = ((xl << (7 - k)) & 0x80808080u) | 0x2a2a2a2au;
+      w[8 + k] = ((xh << (7 - k)) & 0x80808080u) | 0x2a2a2a2au;
+    }
+    m = at + 64u * DEC3_CHUNK;
+    return;
+  }
+  uint32_t lo[8], hi[8];
+  if (NARROW && warp_max(mark_n(m)) <= 32) {
+#pragma unroll
+    for (int j = 0; j < DEC3_CHUNK; j++) {
+      uint32_t xl = 0u;
+      if (j < warp_tests) {
+        int i = mark_pos(at) >> 5;
+        i = i < nwords ? i : nwords;
+        xl = funnel_r(src.word(i), src.word(i + 1), (int)at);
+        if (j < tests) at = park.mark(j + 1);
+        xl = (xl & ml) | (fl & ~ml);
+        ml = low_mask_sat(mark_n(at));
+        xl &= ml;
+      }
+      lo[7 - j] = (j & 1) ? xl : ~xl;
+    }
+    transpose8(lo);
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      w[i] = lo[i];
+      w[8 + i] = 0xaaaaaaaau;
+    }
+    m = at;
+    return;
+  }
+#pragma unroll
+  for (int j = 0; j < DEC3_CHUNK; j++) {
     uint32_t xl = 0u, xh = 0u;
-    if (7 - k >= skip && pos < maxbits) {
-      // first min(n, budget) bits verbatim (decode.cuh:143-145)
-      const int left0 = maxbits - pos;
-      const int m = n < left0 ? n : left0;
-      const int w = pos >> 5;
-      const uint32_t w0 = src.word(w), w1 = src.word(w + 1), w2 = src.word(w + 2);
-      xl = funnel_r(w0, w1, pos) & low_mask_sat(m);
-      xh = funnel_r(w1, w2, pos) & low_mask_sat(m - 32);
-      pos += m;
-      // group tests and unary runs (decode.cuh:147-164), up to ten stream
-      // bits per step; none once every coefficient is significant.  The bits
-      // found are gathered in (ah:al), kept rotated so that position n is bit
-      // 0: a step ORs its pattern in at the bottom and rotates by the positions
-      // it advanced.
-      if (n < 64) {
-        uint32_t al = 0u, ah = 0u;
-        int st = 0;
-        do {
-          // stream bits this step may read: up to ten, no further than the
-          // last open position (a run's final one is implied, so it stops one
-          // short) and no further than the block's budget; none at all ends
-          // the plane through the table's L = 0 rows
-          const int left = maxbits - pos;
-          const int lim = 64 - st - n;
-          int L = lim < DEC3_BITS ? lim : DEC3_BITS;
-          L = left < L ? left : L;
-          const uint32_t mask = low_mask32(L);
-          const uint32_t en = dec_lut[(st << (DEC3_BITS + 1)) + (int)mask + 1 + (int)(peek_at(src, pos) & mask)];
-          const int dn = (int)byte_perm(en, 0u, 0x4442u);
-          al |= en & ((1u << DEC3_BITS) - 1u);
-          ror64_small(al, ah, dn);
-          n += dn;
-          pos += (int)((en >> 24) & 15u);
-          st = (int)(en >> 30);
-        } while (st != 2);
-        rol64(al, ah, n);  // position 0 back to bit 0
-        xl |= al;
-        xh |= ah;
+    if (j < warp_left) {
+      int i = mark_pos(at) >> 5;
+      i = i < nwords ? i : nwords;
+      const uint32_t w0 = src.word(i), w1 = src.word(i + 1), w2 = src.word(i + 2);
+      xl = funnel_r(w0, w1, (int)at);
+      xh = funnel_r(w1, w2, (int)at);
+      at += 64u;
+      if (j < warp_tests) {
+        // the first n bits verbatim (decode.cuh:143-145), then those found up to the next n
+        if (j < tests) at = park.mark(j + 1);
+        xl = (xl & ml) | (fl & ~ml);
+        xh = (xh & mh) | (fh & ~mh);
+        ml = low_mask_sat(mark_n(at));
+        mh = low_mask_sat(mark_n(at) - 32);
+        xl &= ml;
+        xh &= mh;
       }
     }
-    lo[k] = (k & 1) ? ~xl : xl;
-    hi[k] = (k & 1) ? ~xh : xh;
+    lo[7 - j] = (j & 1) ? xl : ~xl;
+    hi[7 - j] = (j & 1) ? xh : ~xh;
+  }
+  // behind planes without tests every coefficient is significant, or the budget is spent
+  m = at;
+  transpose8(lo);
+  transpose8(hi);
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    w[i] = lo[i];
+    w[8 + i] = hi[i];
   }
 }
 
+template <bool NARROW, class WordSrc, class Park>
+CSW_HD void decode_chunk3(const WordSrc& src, Park& park, int maxbits, const uint32_t* dec_lut, uint32_t& m, Found& found,
+                          int& left, uint32_t (&w)[16]) {
+  const int tests = decode_tests3(src, park, maxbits, dec_lut, m, found);
+  decode_rows3<NARROW>(src, park, maxbits, tests, m, found, left, w);
+}
+
+// inv_lift in floating point, where it is exact (decode_block3_float): ten operations become nine
+CSW_HD void inv_lift2(F2& x, F2& y, F2& z, F2& w) {  // two lines at a time
+  const F2 y1 = fma2(w, 0.5f, y);
+  const F2 a = fma2(y1, 0.5f, w), b = fma2(y1, -1.5f, w);
+  const F2 c = fma2(z, -1.0f, x), d = add2(x, z);
+  x = fma2(b, -1.0f, c);
+  y = add2(d, a);
+  z = fma2(a, -1.0f, d);
+  w = add2(c, b);
+}
+CSW_HD void inv_lift1(float& x, float& y, float& z, float& w) {
+  const float y1 = fma1(w, 0.5f, y);
+  const float a = fma1(y1, 0.5f, w), b = fma1(y1, -1.5f, w);
+  const float c = x - z, d = x + z;
+  x = c - b;
+  y = d + a;
+  z = d - a;
+  w = c + b;
+}
+// the lines along z and y, pairs along x
+CSW_HD void inv_xform3_zy(F2 (&q)[32]) {
+#pragma unroll
+  for (int i = 0; i < 8; i++) inv_lift2(q[i], q[i + 8], q[i + 16], q[i + 24]);
+#pragma unroll
+  for (int z = 0; z < 4; z++)
+#pragma unroll
+    for (int x = 0; x < 2; x++) inv_lift2(q[8 * z + x], q[8 * z + x + 2], q[8 * z + x + 4], q[8 * z + x + 6]);
+}
+
+constexpr int perm3_inverse(int p) {
+  int i = 0;
+  while (perm3(i) != p) i++;
+  return i;
+}
+template <int P>
+struct SequencyAt {
+  static constexpr int v = perm3_inverse(P);
+};
+// q <- h * s + t
+template <int... P>
+CSW_HD void floats_of3(const float (&h)[64], float s, float t, F2 (&q)[32], std::integer_sequence<int, P...>) {
+  ((q[P] = fma2(F2{h[SequencyAt<2 * P>::v], h[SequencyAt<2 * P + 1>::v]}, s, F2{t, t})), ...);
+}
+template <int... I>
+CSW_HD void ints_of3(const uint32_t (&u)[64], int lead, uint32_t flip, int (&v)[64], const PipeConsts& kc,
+                     std::integer_sequence<int, I...>) {
+  ((v[PermAt<3, I>::v] = imad((int)kc.nb, kc.mone, (int)((u[I] >> lead) ^ flip))), ...);  // - 0xaaaaaaaa
+}
+
+// The values of a block.
+//
+// Counted from its first plane that is not empty, a block's coefficients are (-1/2)^lead times what
+// they would be if that plane were the top one, so as long as the arithmetic is exact the empty planes
+// are a factor.  It is exact in float32 for most blocks: with K planes read, the lowest of weight
+// 2^p, every intermediate is a multiple of 2^(p - 6) (the inverse lifting halves twice a pass), and of
+// a magnitude that the results bound, since each is a mean of results with weights whose magnitudes add up
+// to one at most (run the lifting backwards).  So when the results stay below 2^(p + 18), 24 bits
+// held everything, and when they stay below 2^31 too the integers of decode.cuh:177-288 would not have
+// wrapped (their shifts lose nothing with p > 5): the same values, to the bit.  The results are checked
+// for that, with a margin for what rounding could have done to larger ones.  A block's scale leaves room
+// for results of 2^30, so p < 12 is not tried; with p of 9 to 11 the first two passes, which have two
+// bits more room, are done this way and the last one in integers.  The products with the block's
+// scale are powers of two, exact within the exponents asked for.
+//
+// What does not fit is left to decode_block3_ints, and so are, once the tests of the first chunk are
+// through, blocks whose planes are so short that more than CHUNKS * 8 of them can be expected.
+struct Block3 {
+  uint32_t e;
+  int lead, start;  // empty planes, where the others begin
+};
 template <class WordSrc>
-CSW_HD void decode_block3_pos(const WordSrc& src, int maxbits, float (&f)[64], const uint32_t* dec_lut,
-                              const PipeConsts& kc) {
+CSW_HD Block3 block_head3(const WordSrc& src, int maxbits) {
   const uint32_t head = src.word(0);
-  // The empty planes common to the warp (at most the first slice) are skipped in one go; a
-  // lane's further ones go through the loop like any other.
-  int lead = 8;
-  if (head & 1u) {
-    const int zeros = leading_empty_planes(head, src.word(1), maxbits - 9);
-    lead = zeros < lead ? zeros : lead;
+  Block3 b;
+  b.e = (head >> 1) & 0xffu;
+  b.lead = leading_empty_planes(head, src.word(1), maxbits - 9);
+  b.start = 9 + b.lead;
+  if (!(head & 1u) || b.lead > 31) {  // a zero block (decode.cuh:240-243), or no plane holds anything
+    b.e = 127;
+    b.lead = 0;
+    b.start = maxbits;
   }
-  lead = warp_min(lead);  // every lane of the warp is here: the tile test before the call is warp-uniform
-  if (!(head & 1u)) {  // zero block
-#pragma unroll
-    for (int i = 0; i < 64; i++) f[i] = 0.0f;
-    return;
+  return b;
+}
+
+// Eight-plane chunks the floating point decoder is given: up to 13 bits a value the planes of a block
+// of noise are 14, and p < 12 takes a block with more than six empty planes.
+CSW_HD int decode3_chunks(int maxbits) { return maxbits <= 832 ? 2 : maxbits <= 1408 ? 3 : 0; }
+
+// What decode_tests3 found of a block's first chunk; tests < 0: nothing yet.
+struct FirstTests3 {
+  int tests;
+  uint32_t m;
+  Found found;
+};
+
+template <class Rest>
+CSW_HD bool over(Rest&& rest) {  // from the start
+  rest(FirstTests3{-1, 0u, {0u, 0u}});
+  return false;
+}
+
+// true: f holds the values.  false: they were left to `rest`, which gets what can be gone on from.  The same
+// for all lanes of the warp, all of which must call.  (`rest` is called where the decision falls: with the
+// state handed back to the caller instead, every call paid 3 us at 256 MiB for keeping it.)
+template <int CHUNKS, class WordSrc, class Park, class Rest>
+CSW_HD bool decode_block3_float(const WordSrc& src, Park& park, int maxbits, float (&f)[64], const uint32_t* dec_lut,
+                                Rest&& rest) {
+  const Block3 blk = block_head3(src, maxbits);
+  uint32_t w0[16], w1[16], w2[16], m = (uint32_t)blk.start;
+  Found found{0u, 0u};
+  const int tests = decode_tests3(src, park, maxbits, dec_lut, m, found);
+  {
+    // a plane takes n + 1 bits and those of the tests
+    const int n = mark_n(m), bits = maxbits - mark_pos(m) - (DEC3_CHUNK - tests) * 64;
+    if (warp_any(bits > (CHUNKS - 1) * DEC3_CHUNK * (9 + n - n / 8))) {
+      rest(FirstTests3{tests, m, found});
+      return false;
+    }
   }
-  const uint32_t e = (head >> 1) & 0xffu;
-  int pos = 9 + lead, n = 0;
-  uint32_t u[64], lo[8], hi[8];
-  // u holds coefficient ^ 0xaaaaaaaa throughout: planes never decoded are zero, i.e. 0xaa bytes.
-  // The first slice is peeled so that these constants are operands of its byte permutes
-  // instead of sixty-four register initialisations carried into a loop.
-  decode_slice3(src, maxbits, dec_lut, lead, pos, n, lo, hi);
+  int planes, left;
+  decode_rows3<false>(src, park, maxbits, tests, m, found, left, w0);
+  planes = left;
+  bool three = false;
+  if (warp_any(left > DEC3_CHUNK)) {
+    decode_chunk3<false>(src, park, maxbits, dec_lut, m, found, left, w1);
+    if (left > 0) planes = DEC3_CHUNK + left;
+    three = warp_any(left > DEC3_CHUNK);
+  } else {
 #pragma unroll
-  for (int i = 0; i < 64; i++) u[i] = 0xaaaaaaaau;
-  bytes_from_planes<0>(lo, 0x4210u, 0x1000u, u);
-  bytes_from_planes<1>(hi, 0x4210u, 0x1000u, u);
-  for (int c = 2; c >= 0 && pos < maxbits; c--) {
-    decode_slice3(src, maxbits, dec_lut, 0, pos, n, lo, hi);
-    const uint32_t sel0 = (0x3210u & ~(0xfu << (4 * c))) | (4u << (4 * c));
-    const uint32_t step = 1u << (4 * c);
-    bytes_from_planes<0>(lo, sel0, step, u);
-    bytes_from_planes<1>(hi, sel0, step, u);
+    for (int i = 0; i < 16; i++) w1[i] = 0xaaaaaaaau;
+  }
+  if (CHUNKS == 2) {
+    if (three) return over(rest);
+  } else if (three) {
+    decode_chunk3<false>(src, park, maxbits, dec_lut, m, found, left, w2);
+    if (left > 0) planes = 2 * DEC3_CHUNK + left;
+    if (warp_any(left > DEC3_CHUNK)) return over(rest);
+  }
+  const bool floats = warp_all(blk.e >= 34 && blk.e <= 225 && planes + blk.lead <= 20);
+  if (!floats && (CHUNKS == 2 || !warp_all(planes + blk.lead <= 23))) return over(rest);
+  // h: the planes as an integer, the first one in bit 15 (or 23), held as a float
+  float h[64], offset = 8388608.0f + 43690.0f;
+  int unit = (floats ? (int)blk.e - 14 : 143) - blk.lead;  // exponent field of the weight of 2^0 of h
+  if (CHUNKS == 2 || !three) {
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
+      const uint32_t a = byte_perm(w1[i], w0[i], 0x5140), b = byte_perm(w1[i], w0[i], 0x7362);
+      const int at = 32 * (i >> 3) + (i & 7);
+      h[at] = u2f(byte_perm(a, 0x4b000000u, 0x7610));  // 2^23 + it
+      h[at + 8] = u2f(byte_perm(a, 0x4b000000u, 0x7632));
+      h[at + 16] = u2f(byte_perm(b, 0x4b000000u, 0x7610));
+      h[at + 24] = u2f(byte_perm(b, 0x4b000000u, 0x7632));
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
+      uint32_t t[4] = {w2[i], w1[i], w0[i], 0u};
+      transpose_bytes4(t);
+      const int at = 32 * (i >> 3) + (i & 7);
+      h[at] = (float)t[0];
+      h[at + 8] = (float)t[1];
+      h[at + 16] = (float)t[2];
+      h[at + 24] = (float)t[3];
+    }
+    offset = 11184810.0f;
+  }
+  float s = u2f(((uint32_t)unit << 23) | ((uint32_t)blk.lead << 31));
+  if (three) s *= 0.00390625f;
+  F2 q[32];
+  floats_of3(h, s, -s * offset, q, std::make_integer_sequence<int, 32>{});
+  inv_xform3_zy(q);
+  float top = 0.0f;
+  if (CHUNKS == 2 || floats) {
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
+      F2 a = q[2 * i], b = q[2 * i + 1];
+      inv_lift1(a.x, a.y, b.x, b.y);
+      top = max_abs3(top, a.x, a.y);
+      top = max_abs3(top, b.x, b.y);
+      f[4 * i] = a.x;
+      f[4 * i + 1] = a.y;
+      f[4 * i + 2] = b.x;
+      f[4 * i + 3] = b.y;
+    }
+    const int room = 34 - planes < 15 + blk.lead ? 34 - planes : 15 + blk.lead;  // 2^(p + 18), 2^31 in units of h
+    return warp_all(top <= u2f(((uint32_t)(unit + room - 1) << 23) | 0x7ff800u)) || over(rest);
+  }
+#pragma unroll
+  for (int i = 0; i < 32; i++) top = max_abs3(top, q[i].x, q[i].y);
+  const int room = 36 - planes < 15 + blk.lead ? 36 - planes : 15 + blk.lead;  // 2^(p + 20)
+  if (!warp_all(top <= u2f(((uint32_t)(unit + room - 1) << 23) | 0x7ff800u))) return over(rest);
+  const float scale = dequant_scale(blk.e);
+#pragma unroll
+  for (int i = 0; i < 16; i++) {
+    int x = f2i_rz(q[2 * i].x), y = f2i_rz(q[2 * i].y), z = f2i_rz(q[2 * i + 1].x), w = f2i_rz(q[2 * i + 1].y);
+    inv_lift(x, y, z, w);
+    mul2(scale, (float)x, (float)y, f[4 * i], f[4 * i + 1]);
+    mul2(scale, (float)z, (float)w, f[4 * i + 2], f[4 * i + 3]);
+  }
+  return true;
+}
+
+template <class WordSrc, class Park>
+CSW_HD void decode_block3_ints(const WordSrc& src, Park& park, int maxbits, float (&f)[64], const uint32_t* dec_lut,
+                               const PipeConsts& kc, const FirstTests3& first) {
+  const Block3 blk = block_head3(src, maxbits);
+  uint32_t w0[16], w1[16], w2[16], w3[16], m = first.m;
+  Found found = first.found;
+  int tests = first.tests, left;
+  if (warp_any(tests < 0)) {
+    m = (uint32_t)blk.start;
+    found = Found{0u, 0u};
+    tests = decode_tests3(src, park, maxbits, dec_lut, m, found);
+  }
+  decode_rows3<true>(src, park, maxbits, tests, m, found, left, w0);
+#pragma unroll
+  for (int i = 0; i < 16; i++) w1[i] = w2[i] = w3[i] = 0xaaaaaaaau;
+  if (warp_any(left > DEC3_CHUNK)) {
+    decode_chunk3<true>(src, park, maxbits, dec_lut, m, found, left, w1);
+    if (warp_any(left > DEC3_CHUNK)) {
+      decode_chunk3<true>(src, park, maxbits, dec_lut, m, found, left, w2);
+      if (warp_any(left > DEC3_CHUNK)) decode_chunk3<true>(src, park, maxbits, dec_lut, m, found, left, w3);
+    }
+  }
+  uint32_t u[64];
+#pragma unroll
+  for (int i = 0; i < 16; i++) {
+    uint32_t t[4] = {w3[i], w2[i], w1[i], w0[i]};
+    transpose_bytes4(t);
+    const int at = 32 * (i >> 3) + (i & 7);
+    u[at] = t[0];
+    u[at + 8] = t[1];
+    u[at + 16] = t[2];
+    u[at + 24] = t[3];
   }
   int v[64];
-  inv_order3_sub(u, v, kc.nb, kc.mone, std::make_integer_sequence<int, 64>{});
-  inv_xform<3>(v);
-  const float w = dequant_scale(e);
+  ints_of3(u, blk.lead, (0xaaaaaaaau >> blk.lead) ^ 0xaaaaaaaau, v, kc, std::make_integer_sequence<int, 64>{});
+  inv_xform3(v);
+  const float scale = dequant_scale(blk.e);
 #pragma unroll
-  for (int i = 0; i < 64; i += 2) mul2(w, (float)v[i], (float)v[i + 1], f[i], f[i + 1]);
+  for (int i = 0; i < 64; i += 2) mul2(scale, (float)v[i], (float)v[i + 1], f[i], f[i + 1]);
 }
+
+#if !defined(__CUDACC__)
+// For host tests: a block given as words, what follows the budget in the last one ignored.
+template <class WordSrc>
+void decode_block3_pos(const WordSrc& src, int maxbits, float (&f)[64], const uint32_t* dec_lut, const PipeConsts& kc) {
+  struct Cut {
+    const WordSrc& src;
+    int maxbits;
+    uint32_t word(int w) const { return 32 * w < maxbits ? src.word(w) & low_mask_sat(maxbits - 32 * w) : 0u; }
+  } cut{src, maxbits};
+  struct Slots {
+    uint32_t marks[DEC3_CHUNK + 2];
+    void put_mark(int j, uint32_t m) { marks[j] = m; }
+    uint32_t mark(int j) const { return marks[j]; }
+  } slots;
+  const int chunks = decode3_chunks(maxbits);
+  const auto rest = [&](const FirstTests3& first) { decode_block3_ints(cut, slots, maxbits, f, dec_lut, kc, first); };
+  if (chunks == 2) decode_block3_float<2>(cut, slots, maxbits, f, dec_lut, rest);
+  else if (chunks == 3) decode_block3_float<3>(cut, slots, maxbits, f, dec_lut, rest);
+  else over(rest);
+}
+#endif
 
 }  // namespace csw

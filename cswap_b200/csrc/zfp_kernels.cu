@@ -6,7 +6,7 @@
 //
 //  * slab kernels for the swap path's view (nx = ny = 32, contiguous, whole
 //    32-bit words per block): one CTA per group of 8 z-slabs (32 KiB, 128
-//    blocks; fewer when the tensor is small), four (encoder) or five (decoder) CTAs per SM, lane = zfp block
+//    blocks; fewer when the tensor is small), four (encoder) or up to six (decoder) CTAs per SM, lane = zfp block
 //    held in registers.  A lane moves its block with sixteen 128-bit accesses
 //    (eight neighbouring lanes cover one 128-byte row segment, so a warp
 //    access touches four whole lines); stream words sit word-major in shared
@@ -42,16 +42,27 @@ namespace {
 constexpr int kThreads = 128;                  // zfp blocks (lanes) per CTA
 constexpr int kSlabFloats = 1024;              // one 32x32 z-slab
 constexpr int kEncCtasPerSm = 4;                // 128 registers per thread: the encoder needs 118
-constexpr int kDecCtasPerSm = 5;                // 96 registers: the decoder spills 16 bytes (generic: 20),
-                                                // and a fifth CTA hides more of its dependent shared-memory reads
+// 3-D decoders: 80 registers are enough for two chunks of planes, 96 for more (no spills); a CTA more hides more of the
+// dependent shared-memory reads (256 MiB at 512 bits 91.7 us with five CTAs, 85.9 with six).  Fields in their own
+// extents need a few registers more and are seldom more than one wave: 31 x 33 x 4096 11.8 us with five, 12.2 with six.
+constexpr int dec_ctas_per_sm(int chunks, bool slabs) { return chunks == 2 && slabs ? 6 : 5; }
 
 // ---- word staging: word w of the block owned by thread t lives at [w * kThreads + t] --
-// Staged stream words of the decoder: rows nwords and nwords + 1 are kept zero
-// so that reads just past a block need no bounds test.
-struct StageWords {
-  const uint32_t* p;  // &stage[threadIdx.x]
-  __device__ __forceinline__ uint32_t word(int w) const { return p[w * kThreads]; }
+// Staged stream words of the 3-D decoder and the slots it parks group tests in: areas of the
+// warp's own, again word-major.
+struct WarpWords {
+  const uint32_t* p;  // of this lane
+  __device__ __forceinline__ uint32_t word(int w) const { return p[w * 32]; }
 };
+struct WarpPark {
+  uint32_t* p;  // of this lane
+  __device__ __forceinline__ void put_mark(int j, uint32_t m) { p[32 * j] = m; }
+  __device__ __forceinline__ uint32_t mark(int j) const { return p[32 * j]; }
+};
+// words of a warp's areas together; store_rows3 takes 512 of them when the block is decoded
+__host__ __device__ constexpr int warp_words3(int nwords) {
+  return nwords > 2 ? 32 * (nwords + DEC3_SPARE_ROWS + DEC3_CHUNK + 2) : 512;
+}
 
 // Staged words and the per-lane expansion queue of the staged encoder, both
 // word-major so that a warp's lanes always hit 32 different banks.
@@ -191,10 +202,9 @@ constexpr DecTable make_dec_table() {
   return t;
 }
 __device__ const DecTable g_dec_table = make_dec_table();
-// 3-D: up to ten stream bits a step (16 KiB; every row with eight took 18).  256 MiB at 256 / 512
-// / 1024 bits 101.2 / 128.1 / 162.5 -> 96.1 / 123.1 / 158.6 us; nine bits 96.8 / 123.4 / 157.6, but
-// 32 MiB at 1024 bits 24.8 against 24.0; eleven (32 KiB: four CTAs per SM at 1024 bits) 99.2 /
-// 131.8 / 176.6.
+// 3-D: up to nine stream bits a step (8 KiB).  A step saved is worth less now that every lane takes its own: 256 MiB at
+// 256 / 512 / 1024 bits with nine 83.9 / 94.4 / 125.0 us, with ten 83.6 / 94.2 / 128.4 (16 KiB leave a CTA less at 1024
+// bits: 178 against 162 for normal values), with eight, six CTAs 83.6 / 93.1 / 125.4 against 82.3 / 92.4 / 124.4.
 struct alignas(16) Dec3Table {
   uint32_t v[DEC3_LUT_SIZE];
 };
@@ -207,50 +217,25 @@ constexpr Dec3Table make_dec3_table() {
 __device__ const Dec3Table g_dec3_table = make_dec3_table();
 }  // namespace
 
-// One CTA per group of 8 z-slabs, lane = block, mirror image of the encoder: a
-// lane pulls its own compressed words into its column of the word-major staging
-// area, parses them by bit position and stores the rebuilt 4x4x4 block with
-// sixteen 128-bit stores.  The only barrier is the one after the table copy.
-__global__ void __launch_bounds__(kThreads, kDecCtasPerSm)
-zfp_decode_slab_kernel(const uint32_t* __restrict__ in, float* __restrict__ out, uint32_t nz, int maxbits, int lsh,
-                       const PipeConsts kc) {
+namespace {
+// the staged words of this thread's lane behind the table, the slots behind the words
+__device__ __forceinline__ uint32_t* decoder3_column(int nwords) {
   extern __shared__ __align__(16) uint32_t smem_words[];
-  const int nwords = maxbits >> 5;
-  uint32_t* stage = smem_words;
-  uint32_t* lut = stage + (nwords + STAGE_SPARE_ROWS) * kThreads;
+  return smem_words + DEC3_LUT_SIZE + (threadIdx.x >> 5) * warp_words3(nwords) + (threadIdx.x & 31);
+}
+__device__ __forceinline__ void decode_ints(int maxbits, float (&f)[64], const PipeConsts& kc, const FirstTests3& first) {
+  extern __shared__ __align__(16) uint32_t smem_words[];
+  const int nwords = (maxbits + 31) >> 5;
+  WarpWords source{decoder3_column(nwords)};
+  WarpPark park{decoder3_column(nwords) + 32 * (nwords + DEC3_SPARE_ROWS)};
+  decode_block3_ints(source, park, maxbits, f, smem_words, kc, first);
+}
 
-  const int tid = threadIdx.x;
-  const uint32_t b = (uint32_t)block_of_thread(lsh);
+// eight neighbouring lanes cover one 128-byte row segment, so every store
+// instruction of a warp writes four full lines: no staging of the output
+__device__ __forceinline__ void store_slab_block(const float (&f)[64], float* out, uint32_t nz, uint32_t b) {
   const int bx = b & 7, by = (b >> 3) & 7;
-  const uint32_t zt = (b >> 6) * 4;  // first slab of my tile
-  uint32_t* col = stage + tid;
-  copy_table<DEC3_LUT_SIZE>(lut, g_dec3_table.v);
-  pdl_wait(in);
-  if (zt < nz) {
-    const uint32_t* src = in + (size_t)b * nwords;
-    if ((nwords & 3) == 0) {
-      for (int w = 0; w < nwords; w += 4) {
-        const uint4 v = __ldg(reinterpret_cast<const uint4*>(src + w));
-        col[w * kThreads] = v.x;
-        col[(w + 1) * kThreads] = v.y;
-        col[(w + 2) * kThreads] = v.z;
-        col[(w + 3) * kThreads] = v.w;
-      }
-    } else {
-      for (int w = 0; w < nwords; w++) col[w * kThreads] = __ldg(src + w);
-    }
-  }
-  // reads just past a block find zeros and need no bounds test
-  for (int w = nwords; w < nwords + STAGE_SPARE_ROWS; w++) col[w * kThreads] = 0u;
-  __syncthreads();  // the table is complete
-  if (zt >= nz) return;
-
-  float f[64];
-  StageWords source{col};
-  decode_block3_pos(source, maxbits, f, lut, kc);
-  if (is_copy(lsh)) return;
-  // eight neighbouring lanes cover one 128-byte row segment, so every store
-  // instruction of a warp writes four full lines: no staging of the output
+  const uint32_t zt = (b >> 6) * 4;  // first slab of the block's tile
   const int vz = nz - zt < 4 ? (int)(nz - zt) : 4;
   float* dst = out + (size_t)zt * kSlabFloats + by * 128 + bx * 4;
 #pragma unroll
@@ -261,6 +246,70 @@ zfp_decode_slab_kernel(const uint32_t* __restrict__ in, float* __restrict__ out,
         *reinterpret_cast<float4*>(dst + z * kSlabFloats + y * 32) =
             make_float4(f[16 * z + 4 * y], f[16 * z + 4 * y + 1], f[16 * z + 4 * y + 2], f[16 * z + 4 * y + 3]);
     }
+}
+// What the floating point decoder leaves over starts again, out of line: in line its code and registers
+// cost the others 12 % (256 MiB at 256 / 512 bits 84.1 / 94.4 us, without it 72 / 85).
+__device__ __noinline__ void decode_slab_ints(float* out, uint32_t nz, int maxbits, int lsh, const PipeConsts kc,
+                                             const FirstTests3 first) {
+  float f[64];
+  decode_ints(maxbits, f, kc, first);
+  if (!is_copy(lsh)) store_slab_block(f, out, nz, (uint32_t)block_of_thread(lsh));
+}
+}  // namespace
+
+// One CTA per group of 8 z-slabs, lane = block, mirror image of the encoder: a
+// lane pulls its own compressed words into its column of the word-major staging
+// area, parses them by bit position and stores the rebuilt 4x4x4 block with
+// sixteen 128-bit stores.  The only barrier is the one after the table copy.
+// CHUNKS: decode3_chunks(maxbits).
+// Bound by instructions issued (about 1780 a warp at 512 bits, issue slots 59 % busy, ALU pipe 64 %); loads and
+// stores alone take 52 of the 86 us.  256 MiB at 256 / 512 / 1024 bits 95.5 / 122.5 / 158.3 -> 77.6 / 86.3 / 125.6 us
+// (tanh of normal values) with each lane at its own pace through the group tests and the inverse transform in
+// exact float32; values smooth enough for every plane to be read, which stay with the integers, 148 / 165
+// / 199 -> 152 / 163 / 208.
+template <int CHUNKS>
+__global__ void __launch_bounds__(kThreads, dec_ctas_per_sm(CHUNKS, true))
+zfp_decode_slab_kernel(const uint32_t* __restrict__ in, float* __restrict__ out, uint32_t nz, int maxbits, int lsh,
+                       const PipeConsts kc) {
+  extern __shared__ __align__(16) uint32_t smem_words[];
+  const int nwords = maxbits >> 5;
+  const uint32_t b = (uint32_t)block_of_thread(lsh);
+  const uint32_t zt = (b >> 6) * 4;  // first slab of my tile
+  uint32_t* col = decoder3_column(nwords);
+  copy_table<DEC3_LUT_SIZE>(smem_words, g_dec3_table.v);
+  pdl_wait(in);
+  if (zt < nz) {
+    const uint32_t* src = in + (size_t)b * nwords;
+    if ((nwords & 3) == 0) {
+      for (int w = 0; w < nwords; w += 4) {
+        const uint4 v = __ldg(reinterpret_cast<const uint4*>(src + w));
+        col[w * 32] = v.x;
+        col[(w + 1) * 32] = v.y;
+        col[(w + 2) * 32] = v.z;
+        col[(w + 3) * 32] = v.w;
+      }
+    } else {
+      for (int w = 0; w < nwords; w++) col[w * 32] = __ldg(src + w);
+    }
+  }
+#pragma unroll
+  for (int w = 0; w < DEC3_SPARE_ROWS; w++) col[(nwords + w) * 32] = 0u;
+  __syncthreads();  // the table is complete
+  if (zt >= nz) return;
+
+  float f[64];
+  const FirstTests3 none{-1, 0u, {0u, 0u}};
+  if constexpr (CHUNKS == 0) {
+    decode_ints(maxbits, f, kc, none);
+  } else {
+    WarpWords source{col};
+    WarpPark park{col + 32 * (nwords + DEC3_SPARE_ROWS)};
+    if (!decode_block3_float<CHUNKS>(source, park, maxbits, f, smem_words, [&](const FirstTests3& first) {
+          decode_slab_ints(out, nz, maxbits, lsh, kc, first);
+        }))
+      return;
+  }
+  if (!is_copy(lsh)) store_slab_block(f, out, nz, b);
 }
 
 // =====================================================================================
@@ -496,67 +545,98 @@ zfp_encode_generic_kernel(const FieldGeom g, const float* __restrict__ in, bool 
   }
 }
 
-template <int DIMS>
-__global__ void __launch_bounds__(kThreads, DIMS == 3 ? kDecCtasPerSm : 8)
+// a decoded 3-D block, every lane of the warp calls
+__device__ __forceinline__ void store_field_block(const FieldGeom& g, float* out, bool vec, uint64_t b, uint64_t nblocks,
+                                                  int nwords, int lsh, const float (&f)[64]) {
+  const BlockAt<3> at(g, b < nblocks ? b : nblocks - 1);
+  const bool valid = b < nblocks && !is_copy(lsh);
+  if (!vec && g.sx == 1) {
+    __syncwarp();  // every lane is done with its words
+    store_rows3(g, out, at, valid, reinterpret_cast<float*>(decoder3_column(nwords) - (threadIdx.x & 31)), f);
+  } else if (valid) {
+    store_block<3>(g, out, vec, at, f);
+  }
+}
+__device__ __noinline__ void decode_field_ints(const FieldGeom& g, float* out, bool vec, uint64_t nblocks, int maxbits,
+                                               int lsh, const PipeConsts kc, const FirstTests3 first) {
+  float f[64];
+  decode_ints(maxbits, f, kc, first);
+  store_field_block(g, out, vec, block_of_thread(lsh), nblocks, (maxbits + 31) >> 5, lsh, f);
+}
+
+// CHUNKS: of 3-D blocks, decode3_chunks(maxbits)
+template <int DIMS, int CHUNKS>
+__global__ void __launch_bounds__(kThreads, DIMS == 3 ? dec_ctas_per_sm(CHUNKS, false) : 8)
 zfp_decode_generic_kernel(const FieldGeom g, const uint32_t* __restrict__ in, float* __restrict__ out, bool vec,
                           int maxbits, uint64_t nblocks, uint64_t total_words, int lsh, const PipeConsts kc) {
   extern __shared__ __align__(16) uint32_t smem_words[];
   const int nwords = (maxbits + 31) >> 5, tid = threadIdx.x;
-  uint32_t* stage = smem_words;
-  uint32_t* lut = stage + (nwords + STAGE_SPARE_ROWS) * kThreads;
-  uint32_t* col = stage + tid;
+  constexpr int kRow = DIMS == 3 ? 32 : kThreads;  // a staged word to the next one of the same lane
+  constexpr int kSpare = DIMS == 3 ? DEC3_SPARE_ROWS : STAGE_SPARE_ROWS;
+  uint32_t* lut = smem_words;
+  uint32_t* col;
   if (DIMS == 1) {
     for (int i = tid; i < DEC1_LUT_SIZE / 8; i += kThreads)
       reinterpret_cast<uint4*>(lut)[i] = __ldg(reinterpret_cast<const uint4*>(g_dec1_table.v) + i);
+    col = lut + DEC1_LUT_SIZE / 2 + tid;
   } else if (DIMS == 2) {
     copy_table<DEC_LUT_SIZE>(lut, g_dec_table.v);
+    col = lut + DEC_LUT_SIZE + tid;
   } else {
     copy_table<DEC3_LUT_SIZE>(lut, g_dec3_table.v);
+    col = decoder3_column(nwords);
   }
   // reads just past a block find zeros and need no bounds test
-  for (int w = nwords; w < nwords + STAGE_SPARE_ROWS; w++) col[w * kThreads] = 0u;
+#pragma unroll
+  for (int w = 0; w < kSpare; w++) col[(nwords + w) * kRow] = 0u;
   __syncthreads();  // the table is complete
   pdl_wait(in);
-  // whole warps go round: the 3-D parser takes a minimum over all lanes
+  // whole warps go round: the 3-D decoder votes
   const uint64_t mine = block_of_thread(lsh), my_lane = tid & ((1u << lsh) - 1u);
   for (uint64_t wb = mine - my_lane; wb < nblocks; wb += (uint64_t)gridDim.x * kThreads) {
     const uint64_t b = wb + my_lane, bit0 = b * (uint64_t)maxbits, w0 = bit0 >> 5;
     const int s = (int)(bit0 & 31);
     if (b >= nblocks) {
       col[0] = 0u;  // an empty block, not stored
+      col[(nwords - 1) * kRow] = 0u;
     } else if ((maxbits & 127) == 0 && (reinterpret_cast<uintptr_t>(in) & 15) == 0) {
       for (int w = 0; w < nwords; w += 4) {
         const uint4 v = __ldg(reinterpret_cast<const uint4*>(in + w0 + w));
-        col[w * kThreads] = v.x;
-        col[(w + 1) * kThreads] = v.y;
-        col[(w + 2) * kThreads] = v.z;
-        col[(w + 3) * kThreads] = v.w;
+        col[w * kRow] = v.x;
+        col[(w + 1) * kRow] = v.y;
+        col[(w + 2) * kRow] = v.z;
+        col[(w + 3) * kRow] = v.w;
       }
     } else {
       uint32_t lo = __ldg(in + w0);
       for (int w = 0; w < nwords; w++) {
         const uint32_t hi = w0 + w + 1 < total_words ? __ldg(in + w0 + w + 1) : 0u;
-        col[w * kThreads] = funnel_r(lo, hi, s);
+        col[w * kRow] = funnel_r(lo, hi, s);
         lo = hi;
       }
+      if (DIMS == 3) col[(nwords - 1) * kRow] &= low_mask32(maxbits - 32 * (nwords - 1));
     }
     float f[1 << (2 * DIMS)];
     if constexpr (DIMS == 3) {
-      StageWords source{col};
-      decode_block3_pos(source, maxbits, f, lut, kc);
+      const FirstTests3 none{-1, 0u, {0u, 0u}};
+      if constexpr (CHUNKS == 0) {
+        decode_ints(maxbits, f, kc, none);
+      } else {
+        WarpWords source{col};
+        WarpPark park{col + 32 * (nwords + DEC3_SPARE_ROWS)};
+        if (!decode_block3_float<CHUNKS>(source, park, maxbits, f, lut, [&](const FirstTests3& first) {
+              decode_field_ints(g, out, vec, nblocks, maxbits, lsh, kc, first);
+            }))
+          return;
+      }
+      store_field_block(g, out, vec, b, nblocks, nwords, lsh, f);
+      return;  // the launcher gives 3-D fields a warp for every group of blocks
     } else {
       ColumnSource source{col};
       if constexpr (DIMS == 2) decode_block2(source, maxbits, f, lut);
       else decode_block1(source, maxbits, f, reinterpret_cast<const uint16_t*>(lut));
+      if (b < nblocks && !is_copy(lsh)) store_block<DIMS>(g, out, vec, BlockAt<DIMS>(g, b), f);
     }
-    const BlockAt<DIMS> at(g, b < nblocks ? b : nblocks - 1);
-    if constexpr (DIMS == 3) {
-      if (!vec && g.sx == 1) {
-        store_rows3(g, out, at, b < nblocks && !is_copy(lsh), reinterpret_cast<float*>(lut + DEC3_LUT_SIZE) + 512 * (tid >> 5), f);
-        continue;
-      }
-    }
-    if (b < nblocks && !is_copy(lsh)) store_block<DIMS>(g, out, vec, at, f);
   }
 }
 
@@ -574,10 +654,10 @@ bool vector_rows(const FieldGeom& g, const void* field) {
 constexpr size_t kDefaultDynamicSmem = 48 * 1024;  // what a kernel may ask for without opting in
 constexpr uint64_t kSchedulersPerSm = 4;
 constexpr int kMostBits = 4096;                    // largest budget the library accepts
-static size_t staged_smem_bytes(int maxbits, bool decode, int dims, bool rowbuf = false) {
+static size_t staged_smem_bytes(int maxbits, bool decode, int dims) {
   const size_t rows = ((size_t)maxbits + 31) / 32 + STAGE_SPARE_ROWS;
-  if (decode && dims == 1) return rows * kThreads * 4 + DEC1_LUT_SIZE * 2;
-  if (decode) return (rows * kThreads + (dims == 3 ? DEC3_LUT_SIZE : DEC_LUT_SIZE)) * 4 + (rowbuf ? kThreads * 16 * 4 : 0);
+  if (decode && dims == 3) return (DEC3_LUT_SIZE + kThreads / 32 * (size_t)warp_words3((maxbits + 31) / 32)) * 4;
+  if (decode) return rows * kThreads * 4 + (dims == 2 ? DEC_LUT_SIZE * 4 : DEC1_LUT_SIZE * 2);
   return (rows + (dims == 3 ? QUEUE_SLOTS * QUEUE_FIELDS : 0)) * kThreads * 4 + (dims == 3 ? ENC3_LUT_SIZE : ENC_LUT_SIZE) * 4;
 }
 // Only the largest budgets need it; the call costs host time on every launch.
@@ -585,7 +665,7 @@ template <class K>
 static cudaError_t allow_smem(K* kernel, size_t smem, bool decode, int dims) {
   if (smem <= kDefaultDynamicSmem) return cudaSuccess;
   return taken(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)staged_smem_bytes(kMostBits, decode, dims, true)));
+                                    (int)staged_smem_bytes(kMostBits, decode, dims)));
 }
 
 static uint64_t slab_blocks(const FieldGeom& g) { return ((uint64_t)g.nz + 3) / 4 * 64; }
@@ -625,11 +705,11 @@ static cudaError_t encode_generic(const FieldGeom& g, const float* in, uint32_t*
                     vector_rows(g, in), out, maxbits, nblocks, (uint64_t)stream_bytes(g, (unsigned)maxbits) / 4, lsh,
                     pipe_consts());
 }
-template <int DIMS>
+template <int DIMS, int CHUNKS>
 static cudaError_t decode_generic(const FieldGeom& g, const uint32_t* in, float* out, int maxbits, uint64_t nblocks,
                                   cudaStream_t stream) {
-  const size_t smem = staged_smem_bytes(maxbits, true, DIMS, DIMS == 3);
-  cudaError_t e = allow_smem(zfp_decode_generic_kernel<DIMS>, smem, true, DIMS);
+  const size_t smem = staged_smem_bytes(maxbits, true, DIMS);
+  cudaError_t e = allow_smem(zfp_decode_generic_kernel<DIMS, CHUNKS>, smem, true, DIMS);
   if (e != cudaSuccess) return e;
   const int lsh = DIMS == 3 ? blocks_per_warp(nblocks) : 5;
   const uint64_t ctas = ctas_of(nblocks, lsh);
@@ -639,7 +719,7 @@ static cudaError_t decode_generic(const FieldGeom& g, const uint32_t* in, float*
   // 210 / 206, 4096 x 4096 64.0 / 54.8.
   const uint64_t full = 8 * (uint64_t)sm_count();
   const uint64_t rounds = DIMS == 3 || ctas < 2 * full ? 1 : ctas / full < 8 ? ctas / full : 8;
-  return pdl_launch(zfp_decode_generic_kernel<DIMS>, (unsigned)((ctas + rounds - 1) / rounds), kThreads, smem, stream,
+  return pdl_launch(zfp_decode_generic_kernel<DIMS, CHUNKS>, (unsigned)((ctas + rounds - 1) / rounds), kThreads, smem, stream,
                     g, in, out, vector_rows(g, out), maxbits, nblocks, (uint64_t)stream_bytes(g, (unsigned)maxbits) / 4, lsh,
                     pipe_consts());
 }
@@ -662,22 +742,32 @@ cudaError_t zfp_encode_launch(const FieldGeom& g, const float* in, void* out, in
                        : encode_generic<1>(g, in, o, maxbits, nblocks, stream);
 }
 
+template <int CHUNKS>
+static cudaError_t decode_slabs(const FieldGeom& g, const uint32_t* in, float* out, int maxbits, cudaStream_t stream) {
+  const size_t smem = staged_smem_bytes(maxbits, true, 3);
+  cudaError_t e = allow_smem(zfp_decode_slab_kernel<CHUNKS>, smem, true, 3);
+  if (e != cudaSuccess) return e;
+  const uint64_t blocks = slab_blocks(g);
+  const int lsh = blocks_per_warp(blocks);
+  return pdl_launch(zfp_decode_slab_kernel<CHUNKS>, ctas_of(blocks, lsh), kThreads, smem, stream, in, out, g.nz, maxbits,
+                    lsh, pipe_consts());
+}
+
 cudaError_t zfp_decode_launch(const FieldGeom& g, const void* in, float* out, int maxbits, cudaStream_t stream) {
   const uint64_t nblocks = geom_blocks(g);
   if (nblocks == 0) return cudaSuccess;
   const uint32_t* i32 = reinterpret_cast<const uint32_t*>(in);
-  if (zfp_slab_eligible(g, out, in, maxbits)) {
-    const size_t smem = staged_smem_bytes(maxbits, true, 3);
-    cudaError_t e = allow_smem(zfp_decode_slab_kernel, smem, true, 3);
-    if (e != cudaSuccess) return e;
-    const uint64_t blocks = slab_blocks(g);
-    const int lsh = blocks_per_warp(blocks);
-    return pdl_launch(zfp_decode_slab_kernel, ctas_of(blocks, lsh), kThreads, smem, stream, i32, out, g.nz, maxbits, lsh,
-                      pipe_consts());
-  }
-  return g.dims == 3   ? decode_generic<3>(g, i32, out, maxbits, nblocks, stream)
-         : g.dims == 2 ? decode_generic<2>(g, i32, out, maxbits, nblocks, stream)
-                       : decode_generic<1>(g, i32, out, maxbits, nblocks, stream);
+  const int chunks = decode3_chunks(maxbits);
+  if (zfp_slab_eligible(g, out, in, maxbits))
+    return chunks == 2   ? decode_slabs<2>(g, i32, out, maxbits, stream)
+           : chunks == 3 ? decode_slabs<3>(g, i32, out, maxbits, stream)
+                         : decode_slabs<0>(g, i32, out, maxbits, stream);
+  if (g.dims == 3)
+    return chunks == 2   ? decode_generic<3, 2>(g, i32, out, maxbits, nblocks, stream)
+           : chunks == 3 ? decode_generic<3, 3>(g, i32, out, maxbits, nblocks, stream)
+                         : decode_generic<3, 0>(g, i32, out, maxbits, nblocks, stream);
+  return g.dims == 2 ? decode_generic<2, 0>(g, i32, out, maxbits, nblocks, stream)
+                     : decode_generic<1, 0>(g, i32, out, maxbits, nblocks, stream);
 }
 
 }  // namespace csw
