@@ -271,11 +271,6 @@ template <int... I>
 CSW_HD void fwd_order2(const int (&v)[16], uint32_t (&u)[16], std::integer_sequence<int, I...>) {
   ((u[I] = int2uint(v[PermAt<2, I>::v])), ...);
 }
-template <int... I>
-CSW_HD void inv_order2(const uint32_t (&u)[16], int (&v)[16], std::integer_sequence<int, I...>) {
-  ((v[PermAt<2, I>::v] = uint2int(u[I])), ...);
-}
-
 // ---- block exponent and cast (encode.cuh:40-71,120-149) ---------------------------
 // Biased exponent field e = emax + 127 (0 for an all-zero block) from the bit
 // pattern of max|v|: frexp's exponent of a normal float with exponent field E
@@ -330,24 +325,6 @@ CSW_HD void planes_of_byte2(const uint32_t (&u)[16], uint32_t sel, uint32_t (&p)
   transpose8(p);
 }
 
-// Inverse: write byte c of each coefficient from eight plane words.
-// sel0 keeps the other three bytes of the destination and takes byte 0 of the
-// second PRMT operand into byte c; adding m << 4c takes byte m instead.
-template <int G, int N>
-CSW_HD void bytes_from_planes(uint32_t (&p)[8], uint32_t sel0, uint32_t step, uint32_t (&u)[N]) {
-  transpose8(p);
-#pragma unroll
-  for (int j = 0; j < 8; j++) {
-    if constexpr (N == 64) {
-#pragma unroll
-      for (int m = 0; m < 4; m++) u[32 * G + 8 * m + j] = byte_perm(u[32 * G + 8 * m + j], p[j], sel0 + m * step);
-    } else {
-      u[j] = byte_perm(u[j], p[j], sel0);
-      u[8 + j] = byte_perm(u[8 + j], p[j], sel0 + step);
-    }
-  }
-}
-
 // ---- coder tables -----------------------------------------------------------------
 // Encoder: entry for the eight positions v of a plane word past the already
 // significant prefix.  Each 0 position codes as '0'; each 1 position codes as
@@ -391,45 +368,6 @@ constexpr CSW_HD uint32_t enc3_lut_entry(uint32_t v) {
   return pat | (len << 22) | (last << 27);
 }
 
-// Decoder: entry for (limit L in 0..8, state, next stream byte).  Simulates the
-// group-test parser of decode.cuh:147-164 over at most L stream bits.
-// State 0: expecting a group-test bit; state 1: inside a unary run (expecting
-// value bits until a one); state 2: negative group test seen, plane finished.
-// L = 0 (no open position left, or the budget is spent) finishes the plane
-// without reading: from state 1 the run's final one is implied.
-// One field per byte, so that each is a single byte-permute away:
-// byte 0: stream bits consumed; byte 1: positions advanced;
-// byte 2: plane bits found, relative to the starting position;
-// byte 3: state afterwards.
-constexpr int DEC_LUT_SIZE = 9 * 2 * 256;
-constexpr CSW_HD int dec_lut_index(int L, int state, uint32_t byte) { return (L * 2 + state) * 256 + (int)byte; }
-constexpr CSW_HD uint32_t dec_lut_entry(int idx) {
-  uint32_t byte = idx & 255;
-  int st = (idx >> 8) & 1, L = idx >> 9;
-  int c = 0, dn = 0;
-  uint32_t pat = 0;
-  if (L == 0) {
-    if (st == 1) { pat = 1u; dn = 1; }
-    st = 2;
-  }
-  while (c < L) {
-    uint32_t bit = (byte >> c) & 1u;
-    c++;
-    if (st == 0) {
-      if (bit) st = 1;
-      else { st = 2; break; }
-    } else {
-      if (bit) { pat |= 1u << dn; st = 0; }
-      dn++;
-    }
-  }
-  return (uint32_t)c | ((uint32_t)dn << 8) | (pat << 16) | ((uint32_t)st << 24);
-}
-CSW_HD int dec_lut_used(uint32_t e) { return (int)(e & 0xffu); }
-CSW_HD int dec_lut_advance(uint32_t e) { return (int)byte_perm(e, 0u, 0x4441u); }
-CSW_HD uint32_t dec_lut_pattern(uint32_t e) { return byte_perm(e, 0u, 0x4442u); }
-CSW_HD int dec_lut_state(uint32_t e) { return (int)(e >> 24); }
-
 // Blocks of four values: a plane is a nibble and its whole code at most eight bits, so one
 // entry holds a plane.  Encoder: entry for (n significant so far, nibble): code in bits
 // 0..7, its length in 8..11, n afterwards in 16..18.  Decoder: entry for (n, next eight stream
@@ -466,22 +404,22 @@ constexpr CSW_HD uint16_t dec1_lut_entry(int idx) {
   return (uint16_t)(x | ((uint32_t)len << 4) | ((uint32_t)n << 8));
 }
 
-// The same for up to nine stream bits, for the 3-D decoder, whose steps are limited by the open
-// positions alone (its words are zero past the budget).  With L < 9 exactly L positions are open,
+// Decoder of the larger blocks: up to nine stream bits of a plane's group tests and runs
+// (decode.cuh:147-164), limited by the open positions alone (its words are zero past the budget).  With L < 9 exactly L positions are open,
 // with L = 9 at least as many; a row of limit L has an entry for each value of L stream bits, behind
 // entry (1 << L) of the state's half.  A run reads one bit less: the last position's one is implied.
 // Bits 0..8: plane bits found; 9: the plane is finished; 10: a run is open (the other half is
 // next; the bits from 9 on are never shifted into what was found); 16..23: stream bits consumed;
 // 24..31: positions advanced.
-constexpr int DEC3_BITS = 9, DEC3_LUT_SIZE = 2 << (DEC3_BITS + 1);
-constexpr uint32_t DEC3_END = 1u << DEC3_BITS, DEC3_RUN = 2u << DEC3_BITS;
-constexpr CSW_HD uint32_t dec3_lut_entry(int idx) {
-  const int half = idx & ((2 << DEC3_BITS) - 1);
-  bool run = (idx >> (DEC3_BITS + 1)) != 0, end = false;
+constexpr int DEC_BITS = 9, DEC_LUT_SIZE = 2 << (DEC_BITS + 1);
+constexpr uint32_t DEC_END = 1u << DEC_BITS, DEC_RUN = 2u << DEC_BITS;
+constexpr CSW_HD uint32_t dec_lut_entry(int idx) {
+  const int half = idx & ((2 << DEC_BITS) - 1);
+  bool run = (idx >> (DEC_BITS + 1)) != 0, end = false;
   int L = 0;
   while ((2 << L) <= half) L++;
   const uint32_t bits = (uint32_t)(half - (1 << L));
-  const int last = L < DEC3_BITS ? L - 1 : 1000;  // the last open position, where it is known
+  const int last = L < DEC_BITS ? L - 1 : 1000;  // the last open position, where it is known
   const int most = run && L > 0 ? L - 1 : L;      // bits to read
   int c = 0, dn = 0;
   uint32_t pat = 0;
@@ -508,7 +446,7 @@ constexpr CSW_HD uint32_t dec3_lut_entry(int idx) {
       }
     }
   }
-  return pat | (end ? DEC3_END : 0u) | (run ? DEC3_RUN : 0u) | ((uint32_t)c << 16) | ((uint32_t)dn << 24);
+  return pat | (end ? DEC_END : 0u) | (run ? DEC_RUN : 0u) | ((uint32_t)c << 16) | ((uint32_t)dn << 24);
 }
 
 // ---- bit emitter ------------------------------------------------------------------
@@ -928,33 +866,6 @@ CSW_HD void encode_block3_staged(const float (&f)[64], int maxbits, Stage& st, c
   }
 }
 
-// ---- decoder: one plane of a small block ----------------------------------------------
-// The code of a plane of 16 coefficients is at most 32 bits: one window
-// of the stream, consumed from the bottom, holds all of it.
-CSW_HD uint32_t decode_plane2(uint32_t win, int& n, int& left, const uint32_t* dec_lut) {
-  constexpr int N = 16;
-  const int m = n < left ? n : left;
-  uint32_t x = win & low_mask_sat(m);
-  win >>= m;
-  left -= m;
-  if (n < N) {
-    int st = 0;
-    do {
-      const int lim = N - st - n;
-      int L = lim < 8 ? lim : 8;
-      L = left < L ? left : L;
-      const uint32_t e = dec_lut[dec_lut_index(L, st, win & 0xffu)];
-      const int used = dec_lut_used(e);
-      x |= dec_lut_pattern(e) << n;
-      n += dec_lut_advance(e);
-      win >>= used;
-      left -= used;
-      st = dec_lut_state(e);
-    } while (st != 2);
-  }
-  return x;
-}
-
 // Leading empty planes of a block whose first two words are given, `budget` bits of which
 // follow the header: while no coefficient is significant a plane is a single '0' bit (the
 // group test of decode.cuh:147 fails at n = 0), so the zeros that follow the header are
@@ -1012,65 +923,27 @@ CSW_HD void decode_block1(WordSource& src, int maxbits, float (&f)[4], const uin
   for (int i = 0; i < 4; i++) f[i] = scale * (float)v[i];
 }
 
-// ---- decoder: 2-D block -------------------------------------------------------------
-// WordSource::get(w) returns the block's w-th 32-bit stream word (0 past the end of the block).
-template <class WordSource>
-CSW_HD void decode_block2(WordSource& src, int maxbits, float (&f)[16], const uint32_t* dec_lut) {
-  const uint32_t head = src.get(0);
-  if (!(head & 1u)) {  // zero block (decode.cuh:240-243)
-#pragma unroll
-    for (int i = 0; i < 16; i++) f[i] = 0.0f;
-    return;
-  }
-  const uint32_t e = (head >> 1) & 0xffu;
-  uint32_t u[16];
-#pragma unroll
-  for (int i = 0; i < 16; i++) u[i] = 0;
-  int left = maxbits - 9, n = 0;
-  const int lead = leading_empty_planes(head, src.get(1), left);
-  left -= lead;
-  for (int c = 3; c >= 0; c--) {
-    uint32_t x[8];
-#pragma unroll
-    for (int k = 7; k >= 0; k--) {
-      x[k] = 0u;
-      if (8 * c + k < 32 - lead && left > 0) {
-        const int pos = maxbits - left;
-        x[k] = decode_plane2(funnel_r(src.get(pos >> 5), src.get((pos >> 5) + 1), pos), n, left, dec_lut);
-      }
-    }
-    bytes_from_planes<0>(x, (0x3210u & ~(0xfu << (4 * c))) | (4u << (4 * c)), 1u << (4 * c), u);
-    if (left <= 0) break;
-  }
-  int v[16];
-  inv_order2(u, v, std::make_integer_sequence<int, 16>{});
-  inv_xform2(v);
-  const float w = dequant_scale(e);
-#pragma unroll
-  for (int i = 0; i < 16; i++) f[i] = w * (float)v[i];
-}
-
-// ---- 3-D decoder (any budget) --------------------------------------------------------
+// ---- decoder: 2-D and 3-D blocks (any budget) ------------------------------------------
 // The values of decode.cuh:232-288.  A warp's lanes decode 32 different blocks, whose group
 // tests lie in different planes and take different numbers of steps, so nothing here goes
 // plane by plane for the warp as a whole:
 //
 //  * Planes are counted from a block's own first one that is not empty (the empty ones ahead
-//    of it are one '0' bit each), and taken in chunks of eight.
+//    of it are one '0' bit each), and taken in chunks, of eight in 3-D and of sixteen in 2-D.
 //  * In a chunk every lane first runs through the group tests of its own planes, as long as
 //    it has coefficients that are not significant, and parks a mark at the end of each: where
 //    the next plane begins and how many of its bits are verbatim.  The loop lasts as long as the lane
-//    with the most steps, not the sum over planes of the longest (15.7 steps against 33.7 at
-//    512 bits, counted on the CPU for tanh of normal values).  What the tests find needs no slots:
-//    a position becomes significant once, so the bits of all planes fit into one word.
-//  * Then the eight planes are put together by all lanes in step - a funnel shift of staged
+//    with the most steps, not the sum over planes of the longest (15.7 steps against 33.7 for
+//    3-D at 512 bits, 11.4 against 25.2 for 2-D at 128, counted on the CPU).  What the tests find
+//    needs no slots: a position becomes significant once, so the bits of all planes fit into one word.
+//  * Then the chunk's planes are put together by all lanes in step - a funnel shift of staged
 //    words, the found bits, masks - and transposed.
 //
 // WordSrc::word(w) returns the block's w-th 32-bit word, with zeros for the bits past the
-// budget and for DEC3_SPARE_ROWS words behind it: a group test that finds no bits ends its plane,
-// as it must, and only a run cut by the budget needs a correction (decode_tests3).
-// Park: mark(j) is the lane's slot j, j <= DEC3_CHUNK + 1.
-constexpr int DEC3_SPARE_ROWS = 4, DEC3_CHUNK = 8;
+// budget and for DEC_SPARE_ROWS words behind it: a group test that finds no bits ends its plane,
+// as it must, and only a run cut by the budget needs a correction (decode_tests).
+// Park: mark(j) is the lane's slot j, j <= chunk + 1.
+constexpr int DEC_SPARE_ROWS = 4, CHUNK3 = 8, CHUNK2 = 16;
 
 // (h:l) rotated left by r, r in 0..64
 CSW_HD void rol64(uint32_t& l, uint32_t& h, int r) {
@@ -1083,38 +956,57 @@ CSW_HD void rol64(uint32_t& l, uint32_t& h, int r) {
 CSW_HD int mark_pos(uint32_t m) { return (int)(m & 0xffffu); }
 CSW_HD int mark_n(uint32_t m) { return (int)(m >> 16); }
 
+struct BlockHead {
+  uint32_t e;
+  int lead, start;  // empty planes, where the others begin
+};
+template <class WordSrc>
+CSW_HD BlockHead block_head(const WordSrc& src, int maxbits) {
+  const uint32_t head = src.word(0);
+  BlockHead b;
+  b.e = (head >> 1) & 0xffu;
+  b.lead = leading_empty_planes(head, src.word(1), maxbits - 9);
+  b.start = 9 + b.lead;
+  if (!(head & 1u) || b.lead > 31) {  // a zero block (decode.cuh:240-243), or no plane holds anything
+    b.e = 127;
+    b.lead = 0;
+    b.start = maxbits;
+  }
+  return b;
+}
+
 // What the group tests of a block have found so far: position p of n is bit 64 - n + p of (hi:lo).
 struct Found {
   uint32_t lo, hi;
 };
 
-// The group tests and unary runs (decode.cuh:147-164) of up to eight planes from `m` on, up to
+// The group tests and unary runs of up to CHUNK planes of a block of N coefficients from `m` on, up to
 // nine stream bits per step.  Returns how many planes had any; m moves behind them.  All lanes of
 // the warp go round together, with a vote at every step: left to itself the compiler makes two
 // loops of this one, the inner one a plane's steps, and the lanes wait at its end.
-template <class WordSrc, class Park>
-CSW_HD int decode_tests3(const WordSrc& src, Park& park, int maxbits, const uint32_t* dec_lut, uint32_t& m, Found& found) {
-  constexpr uint32_t kDone = 64u << 16;  // no open position: steps change nothing
+template <int N, int CHUNK, class WordSrc, class Park>
+CSW_HD int decode_tests(const WordSrc& src, Park& park, int maxbits, const uint32_t* dec_lut, uint32_t& m, Found& found) {
+  constexpr uint32_t kDone = (uint32_t)N << 16;  // no open position: steps change nothing
   int j = 0;
   park.put_mark(0, m);
   uint32_t at = m + (m >> 16), run = 0u;
   if (m >= kDone || mark_pos(m) >= maxbits) at = kDone;
   while (warp_any(at < kDone)) {
-    const int open = 64 - (int)(at >> 16);
-    const uint32_t mask = low_mask32(open < DEC3_BITS ? open : DEC3_BITS);
+    const int open = N - (int)(at >> 16);
+    const uint32_t mask = low_mask32(open < DEC_BITS ? open : DEC_BITS);
     const int w = mark_pos(at) >> 5;
     const uint32_t win = funnel_r(src.word(w), src.word(w + 1), (int)at);
     const uint32_t en = dec_lut[run + mask + 1u + (win & mask)];
     const int dn = (int)(en >> 24);
-    found.lo = funnel_r(found.lo, found.hi, dn);
+    if (N > 32) found.lo = funnel_r(found.lo, found.hi, dn);
     found.hi = funnel_r(found.hi, en, dn);
     at += byte_perm(en, 0u, 0x4342u);
-    run = en & DEC3_RUN;
+    run = en & DEC_RUN;
     park.put_mark(j + 1, at);  // stays when the plane is finished
-    const bool end = (en & DEC3_END) != 0u;
+    const bool end = (en & DEC_END) != 0u;
     j += end ? 1 : 0;
     uint32_t next = at + (at >> 16);  // behind the verbatim bits
-    next = (int)(j == DEC3_CHUNK) | (int)(mark_pos(at) >= maxbits) ? kDone : next;
+    next = (int)(j == CHUNK) | (int)(mark_pos(at) >= maxbits) ? kDone : next;
     next = at >= kDone ? kDone : next;
     at = end ? next : at;
   }
@@ -1132,7 +1024,7 @@ CSW_HD int decode_tests3(const WordSrc& src, Park& park, int maxbits, const uint
 
 // Eight planes, transposed: byte b of w[8 * g + i] holds coefficient 32g + 8b + i (in sequency
 // order), the first plane in its top bit, odd bits complemented (the xor half of the inverse negabinary
-// map).  `tests` of them have group tests, which decode_tests3 found; `m` is what it left, and moves
+// map).  `tests` of them have group tests, which decode_tests found; `m` is what it left, and moves
 // behind the chunk.  left: planes of the block that begin within the budget, from this chunk on (nine when
 // there are more than eight).  NARROW: look out for warps none of whose coefficients from the 32nd on
 // is significant yet.
@@ -1160,13 +1052,13 @@ CSW_HD void decode_rows3(const WordSrc& src, const Park& park, int maxbits, int 
       w[k] = ((xl << (7 - k)) & 0x80808080u) | 0x2a2a2a2au;
       w[8 + k] = ((xh << (7 - k)) & 0x80808080u) | 0x2a2a2a2au;
     }
-    m = at + 64u * DEC3_CHUNK;
+    m = at + 64u * CHUNK3;
     return;
   }
   uint32_t lo[8], hi[8];
   if (NARROW && warp_max(mark_n(m)) <= 32) {
 #pragma unroll
-    for (int j = 0; j < DEC3_CHUNK; j++) {
+    for (int j = 0; j < CHUNK3; j++) {
       uint32_t xl = 0u;
       if (j < warp_tests) {
         int i = mark_pos(at) >> 5;
@@ -1189,7 +1081,7 @@ CSW_HD void decode_rows3(const WordSrc& src, const Park& park, int maxbits, int 
     return;
   }
 #pragma unroll
-  for (int j = 0; j < DEC3_CHUNK; j++) {
+  for (int j = 0; j < CHUNK3; j++) {
     uint32_t xl = 0u, xh = 0u;
     if (j < warp_left) {
       int i = mark_pos(at) >> 5;
@@ -1226,7 +1118,7 @@ CSW_HD void decode_rows3(const WordSrc& src, const Park& park, int maxbits, int 
 template <bool NARROW, class WordSrc, class Park>
 CSW_HD void decode_chunk3(const WordSrc& src, Park& park, int maxbits, const uint32_t* dec_lut, uint32_t& m, Found& found,
                           int& left, uint32_t (&w)[16]) {
-  const int tests = decode_tests3(src, park, maxbits, dec_lut, m, found);
+  const int tests = decode_tests<64, CHUNK3>(src, park, maxbits, dec_lut, m, found);
   decode_rows3<NARROW>(src, park, maxbits, tests, m, found, left, w);
 }
 
@@ -1296,31 +1188,12 @@ CSW_HD void ints_of3(const uint32_t (&u)[64], int lead, uint32_t flip, int (&v)[
 //
 // What does not fit is left to decode_block3_ints, and so are, once the tests of the first chunk are
 // through, blocks whose planes are so short that more than CHUNKS * 8 of them can be expected.
-struct Block3 {
-  uint32_t e;
-  int lead, start;  // empty planes, where the others begin
-};
-template <class WordSrc>
-CSW_HD Block3 block_head3(const WordSrc& src, int maxbits) {
-  const uint32_t head = src.word(0);
-  Block3 b;
-  b.e = (head >> 1) & 0xffu;
-  b.lead = leading_empty_planes(head, src.word(1), maxbits - 9);
-  b.start = 9 + b.lead;
-  if (!(head & 1u) || b.lead > 31) {  // a zero block (decode.cuh:240-243), or no plane holds anything
-    b.e = 127;
-    b.lead = 0;
-    b.start = maxbits;
-  }
-  return b;
-}
-
 // Eight-plane chunks the floating point decoder is given: up to 13 bits a value the planes of a block
 // of noise are 14, and p < 12 takes a block with more than six empty planes.
 CSW_HD int decode3_chunks(int maxbits) { return maxbits <= 832 ? 2 : maxbits <= 1408 ? 3 : 0; }
 
-// What decode_tests3 found of a block's first chunk; tests < 0: nothing yet.
-struct FirstTests3 {
+// What decode_tests found of a block's first chunk; tests < 0: nothing yet.
+struct FirstTests {
   int tests;
   uint32_t m;
   Found found;
@@ -1328,7 +1201,7 @@ struct FirstTests3 {
 
 template <class Rest>
 CSW_HD bool over(Rest&& rest) {  // from the start
-  rest(FirstTests3{-1, 0u, {0u, 0u}});
+  rest(FirstTests{-1, 0u, {0u, 0u}});
   return false;
 }
 
@@ -1338,15 +1211,15 @@ CSW_HD bool over(Rest&& rest) {  // from the start
 template <int CHUNKS, class WordSrc, class Park, class Rest>
 CSW_HD bool decode_block3_float(const WordSrc& src, Park& park, int maxbits, float (&f)[64], const uint32_t* dec_lut,
                                 Rest&& rest) {
-  const Block3 blk = block_head3(src, maxbits);
+  const BlockHead blk = block_head(src, maxbits);
   uint32_t w0[16], w1[16], w2[16], m = (uint32_t)blk.start;
   Found found{0u, 0u};
-  const int tests = decode_tests3(src, park, maxbits, dec_lut, m, found);
+  const int tests = decode_tests<64, CHUNK3>(src, park, maxbits, dec_lut, m, found);
   {
     // a plane takes n + 1 bits and those of the tests
-    const int n = mark_n(m), bits = maxbits - mark_pos(m) - (DEC3_CHUNK - tests) * 64;
-    if (warp_any(bits > (CHUNKS - 1) * DEC3_CHUNK * (9 + n - n / 8))) {
-      rest(FirstTests3{tests, m, found});
+    const int n = mark_n(m), bits = maxbits - mark_pos(m) - (CHUNK3 - tests) * 64;
+    if (warp_any(bits > (CHUNKS - 1) * CHUNK3 * (9 + n - n / 8))) {
+      rest(FirstTests{tests, m, found});
       return false;
     }
   }
@@ -1354,10 +1227,10 @@ CSW_HD bool decode_block3_float(const WordSrc& src, Park& park, int maxbits, flo
   decode_rows3<false>(src, park, maxbits, tests, m, found, left, w0);
   planes = left;
   bool three = false;
-  if (warp_any(left > DEC3_CHUNK)) {
+  if (warp_any(left > CHUNK3)) {
     decode_chunk3<false>(src, park, maxbits, dec_lut, m, found, left, w1);
-    if (left > 0) planes = DEC3_CHUNK + left;
-    three = warp_any(left > DEC3_CHUNK);
+    if (left > 0) planes = CHUNK3 + left;
+    three = warp_any(left > CHUNK3);
   } else {
 #pragma unroll
     for (int i = 0; i < 16; i++) w1[i] = 0xaaaaaaaau;
@@ -1366,8 +1239,8 @@ CSW_HD bool decode_block3_float(const WordSrc& src, Park& park, int maxbits, flo
     if (three) return over(rest);
   } else if (three) {
     decode_chunk3<false>(src, park, maxbits, dec_lut, m, found, left, w2);
-    if (left > 0) planes = 2 * DEC3_CHUNK + left;
-    if (warp_any(left > DEC3_CHUNK)) return over(rest);
+    if (left > 0) planes = 2 * CHUNK3 + left;
+    if (warp_any(left > CHUNK3)) return over(rest);
   }
   const bool floats = warp_all(blk.e >= 34 && blk.e <= 225 && planes + blk.lead <= 20);
   if (!floats && (CHUNKS == 2 || !warp_all(planes + blk.lead <= 23))) return over(rest);
@@ -1435,24 +1308,24 @@ CSW_HD bool decode_block3_float(const WordSrc& src, Park& park, int maxbits, flo
 
 template <class WordSrc, class Park>
 CSW_HD void decode_block3_ints(const WordSrc& src, Park& park, int maxbits, float (&f)[64], const uint32_t* dec_lut,
-                               const PipeConsts& kc, const FirstTests3& first) {
-  const Block3 blk = block_head3(src, maxbits);
+                               const PipeConsts& kc, const FirstTests& first) {
+  const BlockHead blk = block_head(src, maxbits);
   uint32_t w0[16], w1[16], w2[16], w3[16], m = first.m;
   Found found = first.found;
   int tests = first.tests, left;
   if (warp_any(tests < 0)) {
     m = (uint32_t)blk.start;
     found = Found{0u, 0u};
-    tests = decode_tests3(src, park, maxbits, dec_lut, m, found);
+    tests = decode_tests<64, CHUNK3>(src, park, maxbits, dec_lut, m, found);
   }
   decode_rows3<true>(src, park, maxbits, tests, m, found, left, w0);
 #pragma unroll
   for (int i = 0; i < 16; i++) w1[i] = w2[i] = w3[i] = 0xaaaaaaaau;
-  if (warp_any(left > DEC3_CHUNK)) {
+  if (warp_any(left > CHUNK3)) {
     decode_chunk3<true>(src, park, maxbits, dec_lut, m, found, left, w1);
-    if (warp_any(left > DEC3_CHUNK)) {
+    if (warp_any(left > CHUNK3)) {
       decode_chunk3<true>(src, park, maxbits, dec_lut, m, found, left, w2);
-      if (warp_any(left > DEC3_CHUNK)) decode_chunk3<true>(src, park, maxbits, dec_lut, m, found, left, w3);
+      if (warp_any(left > CHUNK3)) decode_chunk3<true>(src, park, maxbits, dec_lut, m, found, left, w3);
     }
   }
   uint32_t u[64];
@@ -1474,25 +1347,167 @@ CSW_HD void decode_block3_ints(const WordSrc& src, Park& park, int maxbits, floa
   for (int i = 0; i < 64; i += 2) mul2(scale, (float)v[i], (float)v[i + 1], f[i], f[i + 1]);
 }
 
+// ---- decoder: 2-D block -------------------------------------------------------------
+// Sixteen planes of sixteen coefficients: byte b of w[i], b < 2, holds coefficient 8b + i in the first
+// eight of them, byte 2 + b in the others; otherwise as decode_rows3.
+template <class WordSrc, class Park>
+CSW_HD void decode_chunk2(const WordSrc& src, Park& park, int maxbits, const uint32_t* dec_lut, uint32_t& m, Found& found,
+                          int& left, uint32_t (&w)[8]) {
+  const int nwords = (maxbits + 31) >> 5;
+  uint32_t at = m;
+  const int tests = decode_tests<16, CHUNK2>(src, park, maxbits, dec_lut, m, found);
+  {
+    const int rest = maxbits - mark_pos(m);
+    left = tests + (rest > 0 ? (mark_n(m) == 16 ? (rest + 15) >> 4 : 1) : 0);
+  }
+  const int warp_tests = warp_max(tests), warp_left = warp_max(left);
+  const uint32_t bits = funnel_l(found.hi, found.hi, mark_n(m));  // position p at bit p
+  uint32_t mask = low_mask32(mark_n(at));
+  uint32_t x[16];
+#pragma unroll
+  for (int j = 0; j < CHUNK2; j++) {
+    x[j] = 0u;
+    if (j < warp_left) {
+      int i = mark_pos(at) >> 5;
+      i = i < nwords ? i : nwords;
+      x[j] = funnel_r(src.word(i), src.word(i + 1), (int)at);
+      at += 16u;
+      if (j < warp_tests) {
+        if (j < tests) at = park.mark(j + 1);
+        x[j] = (x[j] & mask) | (bits & ~mask);
+        mask = low_mask32(mark_n(at));
+        x[j] &= mask;
+      }
+    }
+  }
+  m = at;
+#pragma unroll
+  for (int j = 0; j < 8; j++) {
+    const uint32_t both = byte_perm(x[j], x[8 + j], 0x5410);
+    w[7 - j] = (j & 1) ? both : ~both;
+  }
+  transpose8(w);
+}
+
+constexpr int perm2_inverse(int p) {
+  int i = 0;
+  while (perm2(i) != p) i++;
+  return i;
+}
+template <int P>
+struct SequencyAt2 {
+  static constexpr int v = perm2_inverse(P);
+};
+template <int... P>
+CSW_HD void floats_of2(const float (&h)[16], float s, float t, F2 (&q)[8], std::integer_sequence<int, P...>) {
+  ((q[P] = fma2(F2{h[SequencyAt2<2 * P>::v], h[SequencyAt2<2 * P + 1>::v]}, s, F2{t, t})), ...);
+}
+template <int... I>
+CSW_HD void ints_of2(const uint32_t (&u)[16], int lead, uint32_t flip, int (&v)[16], std::integer_sequence<int, I...>) {
+  ((v[PermAt<2, I>::v] = (int)(((u[I] >> lead) ^ flip) - 0xaaaaaaaau)), ...);
+}
+
+// As the 3-D blocks, with two passes: multiples of 2^(p - 4), so results below 2^(p + 20) are exact
+// and p >= 10 is tried.  What does not fit is little work and done in integers at once.
+template <class WordSrc, class Park>
+CSW_HD void decode_block2(const WordSrc& src, Park& park, int maxbits, float (&f)[16], const uint32_t* dec_lut) {
+  const BlockHead blk = block_head(src, maxbits);
+  uint32_t w0[8], w1[8], m = (uint32_t)blk.start;
+  Found found{0u, 0u};
+  int planes, left;
+  decode_chunk2(src, park, maxbits, dec_lut, m, found, left, w0);
+  planes = left;
+  const bool two = warp_any(left > CHUNK2);
+  if (two) {
+    decode_chunk2(src, park, maxbits, dec_lut, m, found, left, w1);
+    if (left > 0) planes = CHUNK2 + left;
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; i++) w1[i] = 0xaaaaaaaau;
+  }
+  if (warp_all(blk.e >= 40 && blk.e <= 225 && planes <= 24 && planes + blk.lead <= 22)) {
+    const int unit = (int)blk.e - 14 - blk.lead;
+    float h[16], s = u2f(((uint32_t)unit << 23) | ((uint32_t)blk.lead << 31)), offset = 8388608.0f + 43690.0f;
+    if (!two) {
+#pragma unroll
+      for (int i = 0; i < 8; i++) {
+        h[i] = u2f(byte_perm(w0[i], 0x4b000000u, 0x7602));  // 2^23 + it
+        h[8 + i] = u2f(byte_perm(w0[i], 0x4b000000u, 0x7613));
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; i++) {
+        h[i] = (float)(byte_perm(w0[i], w1[i], 0x0024) & 0xffffffu);
+        h[8 + i] = (float)(byte_perm(w0[i], w1[i], 0x1135) & 0xffffffu);
+      }
+      offset = 11184810.0f;
+      s *= 0.00390625f;
+    }
+    F2 q[8];
+    floats_of2(h, s, -s * offset, q, std::make_integer_sequence<int, 8>{});
+    inv_lift2(q[0], q[2], q[4], q[6]);
+    inv_lift2(q[1], q[3], q[5], q[7]);
+    float top = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      F2 a = q[2 * i], b = q[2 * i + 1];
+      inv_lift1(a.x, a.y, b.x, b.y);
+      top = max_abs3(top, a.x, a.y);
+      top = max_abs3(top, b.x, b.y);
+      f[4 * i] = a.x;
+      f[4 * i + 1] = a.y;
+      f[4 * i + 2] = b.x;
+      f[4 * i + 3] = b.y;
+    }
+    const int room = 36 - planes < 15 + blk.lead ? 36 - planes : 15 + blk.lead;  // 2^(p + 20), 2^31 in units of h
+    if (warp_all(top <= u2f(((uint32_t)(unit + room - 1) << 23) | 0x7ff800u))) return;
+  }
+  uint32_t u[16];
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    u[i] = byte_perm(w1[i], w0[i], 0x4602);
+    u[8 + i] = byte_perm(w1[i], w0[i], 0x5713);
+  }
+  int v[16];
+  ints_of2(u, blk.lead, (0xaaaaaaaau >> blk.lead) ^ 0xaaaaaaaau, v, std::make_integer_sequence<int, 16>{});
+  inv_xform2(v);
+  const float scale = dequant_scale(blk.e);
+#pragma unroll
+  for (int i = 0; i < 16; i++) f[i] = scale * (float)v[i];
+}
+
 #if !defined(__CUDACC__)
 // For host tests: a block given as words, what follows the budget in the last one ignored.
+constexpr int DEC3_BITS = DEC_BITS, DEC3_LUT_SIZE = DEC_LUT_SIZE;
+inline uint32_t dec3_lut_entry(int i) { return dec_lut_entry(i); }
+template <class Get>
+struct CutWords {
+  const Get& get;
+  int maxbits;
+  uint32_t word(int w) const { return 32 * w < maxbits ? get(w) & low_mask_sat(maxbits - 32 * w) : 0u; }
+};
+struct HostPark {
+  uint32_t marks[CHUNK2 + 2];
+  void put_mark(int j, uint32_t m) { marks[j] = m; }
+  uint32_t mark(int j) const { return marks[j]; }
+};
 template <class WordSrc>
 void decode_block3_pos(const WordSrc& src, int maxbits, float (&f)[64], const uint32_t* dec_lut, const PipeConsts& kc) {
-  struct Cut {
-    const WordSrc& src;
-    int maxbits;
-    uint32_t word(int w) const { return 32 * w < maxbits ? src.word(w) & low_mask_sat(maxbits - 32 * w) : 0u; }
-  } cut{src, maxbits};
-  struct Slots {
-    uint32_t marks[DEC3_CHUNK + 2];
-    void put_mark(int j, uint32_t m) { marks[j] = m; }
-    uint32_t mark(int j) const { return marks[j]; }
-  } slots;
+  const auto get = [&](int w) { return src.word(w); };
+  CutWords<decltype(get)> cut{get, maxbits};
+  HostPark slots;
   const int chunks = decode3_chunks(maxbits);
-  const auto rest = [&](const FirstTests3& first) { decode_block3_ints(cut, slots, maxbits, f, dec_lut, kc, first); };
+  const auto rest = [&](const FirstTests& first) { decode_block3_ints(cut, slots, maxbits, f, dec_lut, kc, first); };
   if (chunks == 2) decode_block3_float<2>(cut, slots, maxbits, f, dec_lut, rest);
   else if (chunks == 3) decode_block3_float<3>(cut, slots, maxbits, f, dec_lut, rest);
   else over(rest);
+}
+template <class WordSource>
+void decode_block2(WordSource& src, int maxbits, float (&f)[16], const uint32_t* dec_lut) {
+  const auto get = [&](int w) { return src.get(w); };
+  CutWords<decltype(get)> cut{get, maxbits};
+  HostPark slots;
+  decode_block2(cut, slots, maxbits, f, dec_lut);
 }
 #endif
 

@@ -48,7 +48,7 @@ constexpr int kEncCtasPerSm = 4;                // 128 registers per thread: the
 constexpr int dec_ctas_per_sm(int chunks, bool slabs) { return chunks == 2 && slabs ? 6 : 5; }
 
 // ---- word staging: word w of the block owned by thread t lives at [w * kThreads + t] --
-// Staged stream words of the 3-D decoder and the slots it parks group tests in: areas of the
+// Staged stream words of the 2-D and 3-D decoders and the slots they park marks in: areas of the
 // warp's own, again word-major.
 struct WarpWords {
   const uint32_t* p;  // of this lane
@@ -60,8 +60,9 @@ struct WarpPark {
   __device__ __forceinline__ uint32_t mark(int j) const { return p[32 * j]; }
 };
 // words of a warp's areas together; store_rows3 takes 512 of them when the block is decoded
-__host__ __device__ constexpr int warp_words3(int nwords) {
-  return nwords > 2 ? 32 * (nwords + DEC3_SPARE_ROWS + DEC3_CHUNK + 2) : 512;
+__host__ __device__ constexpr int warp_words(int nwords, int dims) {
+  return dims == 2 ? 32 * (nwords + DEC_SPARE_ROWS + CHUNK2 + 2)
+         : nwords > 2 ? 32 * (nwords + DEC_SPARE_ROWS + CHUNK3 + 2) : 512;
 }
 
 // Staged words and the per-lane expansion queue of the staged encoder, both
@@ -191,43 +192,35 @@ zfp_encode_slab_kernel(const float* __restrict__ in, uint32_t* __restrict__ out,
 // slab decoder
 // =====================================================================================
 namespace {
-// The parser tables (2-D; 3-D), evaluated at compile time: a CTA copies its own to shared
-// memory with 128-bit loads instead of rebuilding the entries.
+// The parser table, evaluated at compile time: a CTA copies its own to shared memory with
+// 128-bit loads instead of rebuilding the entries.
+// Up to nine stream bits a step (8 KiB).  A step saved is worth less now that every lane takes its own: 256 MiB at
+// 256 / 512 / 1024 bits with nine 83.9 / 94.4 / 125.0 us, with ten 83.6 / 94.2 / 128.4 (16 KiB leave a CTA less at 1024
+// bits: 178 against 162 for normal values), with eight, six CTAs 83.6 / 93.1 / 125.4 against 82.3 / 92.4 / 124.4.
 struct alignas(16) DecTable {
   uint32_t v[DEC_LUT_SIZE];
 };
 constexpr DecTable make_dec_table() {
   DecTable t{};
-  for (int i = 0; i < DEC_LUT_SIZE; i++) t.v[i] = dec_lut_entry(i);
+  for (int i = 0; i < DEC_LUT_SIZE; i++)
+    if (i & ((2 << DEC_BITS) - 1)) t.v[i] = dec_lut_entry(i);
   return t;
 }
 __device__ const DecTable g_dec_table = make_dec_table();
-// 3-D: up to nine stream bits a step (8 KiB).  A step saved is worth less now that every lane takes its own: 256 MiB at
-// 256 / 512 / 1024 bits with nine 83.9 / 94.4 / 125.0 us, with ten 83.6 / 94.2 / 128.4 (16 KiB leave a CTA less at 1024
-// bits: 178 against 162 for normal values), with eight, six CTAs 83.6 / 93.1 / 125.4 against 82.3 / 92.4 / 124.4.
-struct alignas(16) Dec3Table {
-  uint32_t v[DEC3_LUT_SIZE];
-};
-constexpr Dec3Table make_dec3_table() {
-  Dec3Table t{};
-  for (int i = 0; i < DEC3_LUT_SIZE; i++)
-    if (i & ((2 << DEC3_BITS) - 1)) t.v[i] = dec3_lut_entry(i);
-  return t;
-}
-__device__ const Dec3Table g_dec3_table = make_dec3_table();
 }  // namespace
 
 namespace {
 // the staged words of this thread's lane behind the table, the slots behind the words
-__device__ __forceinline__ uint32_t* decoder3_column(int nwords) {
+template <int DIMS>
+__device__ __forceinline__ uint32_t* decoder_column(int nwords) {
   extern __shared__ __align__(16) uint32_t smem_words[];
-  return smem_words + DEC3_LUT_SIZE + (threadIdx.x >> 5) * warp_words3(nwords) + (threadIdx.x & 31);
+  return smem_words + DEC_LUT_SIZE + (threadIdx.x >> 5) * warp_words(nwords, DIMS) + (threadIdx.x & 31);
 }
-__device__ __forceinline__ void decode_ints(int maxbits, float (&f)[64], const PipeConsts& kc, const FirstTests3& first) {
+__device__ __forceinline__ void decode_ints(int maxbits, float (&f)[64], const PipeConsts& kc, const FirstTests& first) {
   extern __shared__ __align__(16) uint32_t smem_words[];
   const int nwords = (maxbits + 31) >> 5;
-  WarpWords source{decoder3_column(nwords)};
-  WarpPark park{decoder3_column(nwords) + 32 * (nwords + DEC3_SPARE_ROWS)};
+  WarpWords source{decoder_column<3>(nwords)};
+  WarpPark park{decoder_column<3>(nwords) + 32 * (nwords + DEC_SPARE_ROWS)};
   decode_block3_ints(source, park, maxbits, f, smem_words, kc, first);
 }
 
@@ -250,7 +243,7 @@ __device__ __forceinline__ void store_slab_block(const float (&f)[64], float* ou
 // What the floating point decoder leaves over starts again, out of line: in line its code and registers
 // cost the others 12 % (256 MiB at 256 / 512 bits 84.1 / 94.4 us, without it 72 / 85).
 __device__ __noinline__ void decode_slab_ints(float* out, uint32_t nz, int maxbits, int lsh, const PipeConsts kc,
-                                             const FirstTests3 first) {
+                                             const FirstTests first) {
   float f[64];
   decode_ints(maxbits, f, kc, first);
   if (!is_copy(lsh)) store_slab_block(f, out, nz, (uint32_t)block_of_thread(lsh));
@@ -275,8 +268,8 @@ zfp_decode_slab_kernel(const uint32_t* __restrict__ in, float* __restrict__ out,
   const int nwords = maxbits >> 5;
   const uint32_t b = (uint32_t)block_of_thread(lsh);
   const uint32_t zt = (b >> 6) * 4;  // first slab of my tile
-  uint32_t* col = decoder3_column(nwords);
-  copy_table<DEC3_LUT_SIZE>(smem_words, g_dec3_table.v);
+  uint32_t* col = decoder_column<3>(nwords);
+  copy_table<DEC_LUT_SIZE>(smem_words, g_dec_table.v);
   pdl_wait(in);
   if (zt < nz) {
     const uint32_t* src = in + (size_t)b * nwords;
@@ -293,18 +286,18 @@ zfp_decode_slab_kernel(const uint32_t* __restrict__ in, float* __restrict__ out,
     }
   }
 #pragma unroll
-  for (int w = 0; w < DEC3_SPARE_ROWS; w++) col[(nwords + w) * 32] = 0u;
+  for (int w = 0; w < DEC_SPARE_ROWS; w++) col[(nwords + w) * 32] = 0u;
   __syncthreads();  // the table is complete
   if (zt >= nz) return;
 
   float f[64];
-  const FirstTests3 none{-1, 0u, {0u, 0u}};
+  const FirstTests none{-1, 0u, {0u, 0u}};
   if constexpr (CHUNKS == 0) {
     decode_ints(maxbits, f, kc, none);
   } else {
     WarpWords source{col};
-    WarpPark park{col + 32 * (nwords + DEC3_SPARE_ROWS)};
-    if (!decode_block3_float<CHUNKS>(source, park, maxbits, f, smem_words, [&](const FirstTests3& first) {
+    WarpPark park{col + 32 * (nwords + DEC_SPARE_ROWS)};
+    if (!decode_block3_float<CHUNKS>(source, park, maxbits, f, smem_words, [&](const FirstTests& first) {
           decode_slab_ints(out, nz, maxbits, lsh, kc, first);
         }))
       return;
@@ -552,46 +545,46 @@ __device__ __forceinline__ void store_field_block(const FieldGeom& g, float* out
   const bool valid = b < nblocks && !is_copy(lsh);
   if (!vec && g.sx == 1) {
     __syncwarp();  // every lane is done with its words
-    store_rows3(g, out, at, valid, reinterpret_cast<float*>(decoder3_column(nwords) - (threadIdx.x & 31)), f);
+    store_rows3(g, out, at, valid, reinterpret_cast<float*>(decoder_column<3>(nwords) - (threadIdx.x & 31)), f);
   } else if (valid) {
     store_block<3>(g, out, vec, at, f);
   }
 }
 __device__ __noinline__ void decode_field_ints(const FieldGeom& g, float* out, bool vec, uint64_t nblocks, int maxbits,
-                                               int lsh, const PipeConsts kc, const FirstTests3 first) {
+                                               int lsh, const PipeConsts kc, const FirstTests first) {
   float f[64];
   decode_ints(maxbits, f, kc, first);
   store_field_block(g, out, vec, block_of_thread(lsh), nblocks, (maxbits + 31) >> 5, lsh, f);
 }
 
 // CHUNKS: of 3-D blocks, decode3_chunks(maxbits)
+// 2-D: 768 x 4096 at 64 / 128 / 256 bits 11.0 / 13.8 / 16.6 -> 9.4 / 10.7 / 13.7 us with the lanes at their own pace through
+// the group tests, sixteen planes a transpose and the transform in exact float32; 4096 x 4096 48.2 / 63.5 / 79.5 -> 37.3 /
+// 43.0 / 53.7 (and one round of blocks a CTA), smooth values at 128 bits 92.6 -> 81.1.
 template <int DIMS, int CHUNKS>
 __global__ void __launch_bounds__(kThreads, DIMS == 3 ? dec_ctas_per_sm(CHUNKS, false) : 8)
 zfp_decode_generic_kernel(const FieldGeom g, const uint32_t* __restrict__ in, float* __restrict__ out, bool vec,
                           int maxbits, uint64_t nblocks, uint64_t total_words, int lsh, const PipeConsts kc) {
   extern __shared__ __align__(16) uint32_t smem_words[];
   const int nwords = (maxbits + 31) >> 5, tid = threadIdx.x;
-  constexpr int kRow = DIMS == 3 ? 32 : kThreads;  // a staged word to the next one of the same lane
-  constexpr int kSpare = DIMS == 3 ? DEC3_SPARE_ROWS : STAGE_SPARE_ROWS;
+  constexpr int kRow = DIMS > 1 ? 32 : kThreads;  // a staged word to the next one of the same lane
+  constexpr int kSpare = DIMS > 1 ? DEC_SPARE_ROWS : STAGE_SPARE_ROWS;
   uint32_t* lut = smem_words;
   uint32_t* col;
   if (DIMS == 1) {
     for (int i = tid; i < DEC1_LUT_SIZE / 8; i += kThreads)
       reinterpret_cast<uint4*>(lut)[i] = __ldg(reinterpret_cast<const uint4*>(g_dec1_table.v) + i);
     col = lut + DEC1_LUT_SIZE / 2 + tid;
-  } else if (DIMS == 2) {
-    copy_table<DEC_LUT_SIZE>(lut, g_dec_table.v);
-    col = lut + DEC_LUT_SIZE + tid;
   } else {
-    copy_table<DEC3_LUT_SIZE>(lut, g_dec3_table.v);
-    col = decoder3_column(nwords);
+    copy_table<DEC_LUT_SIZE>(lut, g_dec_table.v);
+    col = decoder_column<DIMS>(nwords);
   }
   // reads just past a block find zeros and need no bounds test
 #pragma unroll
   for (int w = 0; w < kSpare; w++) col[(nwords + w) * kRow] = 0u;
   __syncthreads();  // the table is complete
   pdl_wait(in);
-  // whole warps go round: the 3-D decoder votes
+  // whole warps go round: the decoders of the larger blocks vote
   const uint64_t mine = block_of_thread(lsh), my_lane = tid & ((1u << lsh) - 1u);
   for (uint64_t wb = mine - my_lane; wb < nblocks; wb += (uint64_t)gridDim.x * kThreads) {
     const uint64_t b = wb + my_lane, bit0 = b * (uint64_t)maxbits, w0 = bit0 >> 5;
@@ -614,27 +607,32 @@ zfp_decode_generic_kernel(const FieldGeom g, const uint32_t* __restrict__ in, fl
         col[w * kRow] = funnel_r(lo, hi, s);
         lo = hi;
       }
-      if (DIMS == 3) col[(nwords - 1) * kRow] &= low_mask32(maxbits - 32 * (nwords - 1));
+      if (DIMS > 1) col[(nwords - 1) * kRow] &= low_mask32(maxbits - 32 * (nwords - 1));
     }
     float f[1 << (2 * DIMS)];
     if constexpr (DIMS == 3) {
-      const FirstTests3 none{-1, 0u, {0u, 0u}};
+      const FirstTests none{-1, 0u, {0u, 0u}};
       if constexpr (CHUNKS == 0) {
         decode_ints(maxbits, f, kc, none);
       } else {
         WarpWords source{col};
-        WarpPark park{col + 32 * (nwords + DEC3_SPARE_ROWS)};
-        if (!decode_block3_float<CHUNKS>(source, park, maxbits, f, lut, [&](const FirstTests3& first) {
+        WarpPark park{col + 32 * (nwords + DEC_SPARE_ROWS)};
+        if (!decode_block3_float<CHUNKS>(source, park, maxbits, f, lut, [&](const FirstTests& first) {
               decode_field_ints(g, out, vec, nblocks, maxbits, lsh, kc, first);
             }))
           return;
       }
       store_field_block(g, out, vec, b, nblocks, nwords, lsh, f);
-      return;  // the launcher gives 3-D fields a warp for every group of blocks
+      return;  // the launcher gives a 3-D field a warp for every group of blocks
     } else {
-      ColumnSource source{col};
-      if constexpr (DIMS == 2) decode_block2(source, maxbits, f, lut);
-      else decode_block1(source, maxbits, f, reinterpret_cast<const uint16_t*>(lut));
+      if constexpr (DIMS == 2) {
+        WarpWords source{col};
+        WarpPark park{col + 32 * (nwords + DEC_SPARE_ROWS)};
+        decode_block2(source, park, maxbits, f, lut);
+      } else {
+        ColumnSource source{col};
+        decode_block1(source, maxbits, f, reinterpret_cast<const uint16_t*>(lut));
+      }
       if (b < nblocks && !is_copy(lsh)) store_block<DIMS>(g, out, vec, BlockAt<DIMS>(g, b), f);
     }
   }
@@ -656,8 +654,8 @@ constexpr uint64_t kSchedulersPerSm = 4;
 constexpr int kMostBits = 4096;                    // largest budget the library accepts
 static size_t staged_smem_bytes(int maxbits, bool decode, int dims) {
   const size_t rows = ((size_t)maxbits + 31) / 32 + STAGE_SPARE_ROWS;
-  if (decode && dims == 3) return (DEC3_LUT_SIZE + kThreads / 32 * (size_t)warp_words3((maxbits + 31) / 32)) * 4;
-  if (decode) return rows * kThreads * 4 + (dims == 2 ? DEC_LUT_SIZE * 4 : DEC1_LUT_SIZE * 2);
+  if (decode && dims == 1) return rows * kThreads * 4 + DEC1_LUT_SIZE * 2;
+  if (decode) return (DEC_LUT_SIZE + kThreads / 32 * (size_t)warp_words((maxbits + 31) / 32, dims)) * 4;
   return (rows + (dims == 3 ? QUEUE_SLOTS * QUEUE_FIELDS : 0)) * kThreads * 4 + (dims == 3 ? ENC3_LUT_SIZE : ENC_LUT_SIZE) * 4;
 }
 // Only the largest budgets need it; the call costs host time on every launch.
@@ -713,12 +711,12 @@ static cudaError_t decode_generic(const FieldGeom& g, const uint32_t* in, float*
   if (e != cudaSuccess) return e;
   const int lsh = DIMS == 3 ? blocks_per_warp(nblocks) : 5;
   const uint64_t ctas = ctas_of(nblocks, lsh);
-  // 128 small blocks are 8 KiB of field or less, and a CTA begins with a table (18 KiB in 2-D, 2.5 in 1-D): once
-  // every SM has its eight CTAs twice over, a CTA takes up to eight rounds of blocks.  With and without rounds:
-  // 1-D at 32 bits 64 Mi values 275 / 298 us, 16 Mi 73.9 / 75.8, but 4 Mi 23.3 / 20.7; 2-D at 128 bits 8192 x 8192
-  // 210 / 206, 4096 x 4096 64.0 / 54.8.
+  // 128 1-D blocks are 2 KiB of field, and a CTA begins with a table of 2.5: once every SM has its eight CTAs twice
+  // over, a CTA takes up to eight rounds of blocks.  With and without rounds, at 32 bits: 64 Mi values 275 / 298 us, 16 Mi
+  // 73.9 / 75.8, but 4 Mi 23.3 / 20.7.  2-D fields (8 KiB a CTA) are better off without at every size: 4096 x 4096 at
+  // 64 / 128 / 256 bits 43.0 / 49.0 / 62.4 us with rounds and 37.3 / 43.0 / 53.7 without, 8192 x 8192 at 128 bits 165 and 163.
   const uint64_t full = 8 * (uint64_t)sm_count();
-  const uint64_t rounds = DIMS == 3 || ctas < 2 * full ? 1 : ctas / full < 8 ? ctas / full : 8;
+  const uint64_t rounds = DIMS > 1 || ctas < 2 * full ? 1 : ctas / full < 8 ? ctas / full : 8;
   return pdl_launch(zfp_decode_generic_kernel<DIMS, CHUNKS>, (unsigned)((ctas + rounds - 1) / rounds), kThreads, smem, stream,
                     g, in, out, vector_rows(g, out), maxbits, nblocks, (uint64_t)stream_bytes(g, (unsigned)maxbits) / 4, lsh,
                     pipe_consts());

@@ -1,5 +1,5 @@
-"""The 3-D decoder has a floating point path, a mixed one and an integer one, and takes a block's planes in
-chunks of eight: budgets on either side of where the kernels change, block exponents on either side of what the
+"""The 2-D and 3-D decoders have a floating point path, a mixed one (3-D) and an integer one, and take a block's
+planes in chunks of sixteen and eight: budgets on either side of where the kernels change, block exponents on either side of what the
 floating point path takes, values that reach a block's full range, plane counts on either side of
 what 24 bits hold, and bits that no encoder wrote.  All against the oracle, bit for bit."""
 import numpy as np
@@ -20,7 +20,7 @@ def _inputs(n, seed):
     yield (np.sin(0.01 * np.arange(n)) + 1e-4 * t).astype(np.float32)
     yield np.where(rng.random(n) < 0.02, t, 0).astype(np.float32)
     yield util.block_zoo(n, seed)
-    for k in (-127, -100, -94, -93, -92, 97, 98, 99, 127):  # the path takes exponents from -93 to 98
+    for k in (-127, -100, -94, -93, -92, -88, -87, -86, 97, 98, 99, 127):  # taken: exponents from -93 (2-D: -87) to 98
         yield np.ldexp(t, k).astype(np.float32)
 
 
@@ -35,22 +35,22 @@ def _streams(words, seed):
     yield s
 
 
-@pytest.mark.parametrize("maxbits", BUDGETS + [777, 833, 1025, 1409])
-def test_core(core, oracle, maxbits):  # noqa: F811
-    dims = (32, 32, 8)
-    for a in _inputs(32 * 32 * 8, maxbits):
+@pytest.mark.parametrize("dims,maxbits", [((32, 32, 8), b) for b in BUDGETS + [777, 833, 1025, 1409]] +
+                         [((128, 64, 0), b) for b in (64, 128, 200, 256, 272, 384, 512)])
+def test_core(core, oracle, dims, maxbits):  # noqa: F811
+    for a in _inputs(8192, maxbits):
         _run(core, oracle, a, dims, maxbits)
     for s in _streams(oracle.zfp_stream_bytes(*dims, maxbits) // 4, maxbits):
         _check_decode(core, oracle, np.ascontiguousarray(s).view(np.uint64), dims, maxbits)
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("dims", [(32, 32, 24), (31, 30, 9)])
-@pytest.mark.parametrize("maxbits", BUDGETS + [777, 1025, 1409])
+@pytest.mark.parametrize("dims,maxbits", [(d, b) for d in ((32, 32, 24), (31, 30, 9)) for b in BUDGETS + [777, 1025, 1409]] +
+                         [((131, 63, 0), b) for b in (64, 128, 200, 256, 272, 384, 512)])
 def test_kernels(oracle, dims, maxbits):
     import torch
     import cswap_b200 as cs
-    n = dims[0] * dims[1] * dims[2]
+    n = dims[0] * dims[1] * max(dims[2], 1)
     streams = [oracle.zfp_encode(a[:n], *dims, maxbits) for a in _inputs((n + 63) // 64 * 64, maxbits)]
     streams += [np.ascontiguousarray(s).view(np.uint64)
                 for s in _streams(oracle.zfp_stream_bytes(*dims, maxbits) // 4, maxbits)]
