@@ -665,7 +665,9 @@ CSW_HD void encode_block2(const float (&f)[16], int maxbits, WordSink& sink, con
 //    their offsets, one plane after the other, by all lanes in step;
 //  * the expansions (the data-dependent part) are queued per lane and worked off
 //    in one flat loop per eight planes, each lane running through its own queue,
-//    so lanes do not wait for each other plane by plane.
+//    so lanes do not wait for each other plane by plane.  A queue entry is a place, a count of
+//    positions and whether the last one is the block's last; the bits themselves lie one
+//    expansion behind the other in one word, for a position becomes significant once.
 //
 // On sm_100 shifts, logic and compares issue on the integer ALU pipe at half
 // the warp rate while integer multiply-adds go down the (otherwise idle)
@@ -747,8 +749,8 @@ CSW_HD void planes_of_byte_bal(const uint32_t (&u)[64], uint32_t sel, uint32_t (
 }
 
 constexpr int STAGE_SPARE_ROWS = 2;  // words a write may run past the block's last word
-constexpr int QUEUE_SLOTS = 8;       // expansions per lane per eight planes
-constexpr int QUEUE_FIELDS = 3;
+constexpr int QUEUE_SLOTS = 9;       // expansions per lane per eight planes, and the end mark
+constexpr int QUEUE_FIELDS = 1;
 
 // Stage: or_word(w, v) ORs v into the block's w-th staged word (rows
 // 0 .. nwords + STAGE_SPARE_ROWS - 1 exist and rows below nwords start as 0);
@@ -767,6 +769,7 @@ CSW_HD void fwd_order3_add(const int (&v)[64], uint32_t (&u)[64], uint32_t nb, i
   ((u[I] = umad((uint32_t)v[PermAt<3, I>::v], (uint32_t)one, nb)), ...);
 }
 
+// All lanes of the warp call.
 template <class Stage>
 CSW_HD void encode_block3_staged(const float (&f)[64], int maxbits, Stage& st, const uint32_t* enc_lut,
                                  const PipeConsts& kc) {
@@ -774,8 +777,8 @@ CSW_HD void encode_block3_staged(const float (&f)[64], int maxbits, Stage& st, c
 #pragma unroll
   for (int i = 0; i < 64; i++) m = fmaxf(m, fabsf(f[i]));
   const uint32_t e = biased_emax(m);
-  if (e == 0) return;  // all-zero block: the staged words stay zero
-  st.or_word(0, (2u * e + 1u) & 0x1ffu);
+  // an all-zero block's staged words stay zero: its lane has nothing to code, but goes along
+  st.or_word(0, e ? (2u * e + 1u) & 0x1ffu : 0u);
   int v[64];
   {
     const float s = quant_scale(e);
@@ -793,13 +796,15 @@ CSW_HD void encode_block3_staged(const float (&f)[64], int maxbits, Stage& st, c
 
   SigState sg;
   sg.set(0);
-  int off = 9;
+  int off = e ? 9 : maxbits;
   for (int c = 3; c >= 0; c--) {  // planes 8c+7 .. 8c
     const uint32_t sel = (uint32_t)c | ((uint32_t)(4 + c) << 4);
     uint32_t lo[8], hi[8];
     planes_of_byte_bal<0>(u, sel, lo, kc);
     planes_of_byte_bal<1>(u, sel, hi, kc);
     int count = 0;
+    const int from = sg.n;
+    uint32_t fl = 0u, fh = 0u;  // what the expansions code: a position becomes significant once
 #pragma unroll
     for (int k = 7; k >= 0; k--) {
       if (off < maxbits) {
@@ -813,11 +818,10 @@ CSW_HD void encode_block3_staged(const float (&f)[64], int maxbits, Stage& st, c
         if (any) {
           const int top = (int)(hi[k] >> 31);
           const int msb = hi[k] ? 64 - clz32(hi[k]) : 32 - clz32(lo[k]);
+          fl |= above_lo;
+          fh |= above_hi;
           if (off < maxbits) {
-            const uint32_t fl = funnel_r(lo[k], hi[k], n), sh = hi[k] >> (n & 31);
-            st.q_put(count, 0, n < 32 ? fl : sh);
-            st.q_put(count, 1, n < 32 ? sh : 0u);
-            st.q_put(count, 2, (uint32_t)off | ((uint32_t)top << 31));
+            st.q_put(count, 0, (uint32_t)off | ((uint32_t)(msb - n) << 16) | ((uint32_t)top << 31));
             count++;
           }
           off += (msb - n) + popc32(above_lo) + popc32(above_hi) - 2 * top;
@@ -825,44 +829,40 @@ CSW_HD void encode_block3_staged(const float (&f)[64], int maxbits, Stage& st, c
         }
       }
     }
-    // work off this lane's expansions
-    int slot = 0;
-    bool have = count > 0;
-    uint32_t xl = 0, xh = 0;
-    int boff = 0, top = 0;
-    if (have) {
-      xl = st.q_get(0, 0);
-      xh = st.q_get(0, 1);
-      const uint32_t meta = st.q_get(0, 2);
-      boff = (int)(meta & 0x7fffffffu);
-      top = (int)(meta >> 31);
+    st.q_put(count, 0, 0u);
+    // Work off this lane's expansions, with a vote at every step: left to itself the compiler makes
+    // two loops of this one, the inner one an expansion's steps, and the lanes wait at its end.
+    if (from & 32) {
+      fl = fh;
+      fh = 0u;
     }
-    while (have) {
-      const uint32_t en = enc_lut[xl & (ENC3_LUT_SIZE - 1)];
-      xl = funnel_r(xl, xh, ENC3_BITS);
-      xh >>= ENC3_BITS;
-      const bool more = (xl | xh) != 0u;
+    fl = funnel_r(fl, fh, from);
+    fh >>= from & 31;
+    int slot = 0;
+    uint32_t now = st.q_get(0, 0);
+    int boff = (int)(now & 0xffffu), left = (int)((now >> 16) & 0x7fu), top = (int)(now >> 31);
+    while (warp_any(left > 0)) {
+      const bool last = left <= ENC3_BITS;
+      const int take = last ? left : ENC3_BITS;
+      const uint32_t en = enc_lut[fl & low_mask32(take)];
       const int lf = (int)(en >> 27);
-      const int len = more ? (int)((en >> 22) & 0x1fu) : lf - 2 * top;
-      const uint32_t keep = more ? 0x3fffffu : low_mask_sat(lf - 1 - top);
-      const uint32_t pat = en & keep;
+      const int len = last ? lf - 2 * top : (int)((en >> 22) & 0x1fu);
+      const uint32_t pat = en & (last ? low_mask_sat(lf - 1 - top) : 0x3fffffu);
       const int s = boff & 31, w = boff >> 5;
       st.or_word(w, pat << s);
       st.or_word(w + 1, funnel_l(pat, 0u, s));
+      fl = funnel_r(fl, fh, take);
+      fh >>= take;
       boff += len;
-      if (!more || boff >= maxbits) {
-        slot++;
-        have = slot < count;
-        if (have) {
-          xl = st.q_get(slot, 0);
-          xh = st.q_get(slot, 1);
-          const uint32_t meta = st.q_get(slot, 2);
-          boff = (int)(meta & 0x7fffffffu);
-          top = (int)(meta >> 31);
-        }
-      }
+      const bool next = (int)(left > 0) & ((int)last | (int)(boff >= maxbits));
+      left -= take;
+      slot += next ? 1 : 0;
+      now = st.q_get(slot, 0);
+      boff = next ? (int)(now & 0xffffu) : boff;
+      left = next ? (int)((now >> 16) & 0x7fu) : left;
+      top = next ? (int)(now >> 31) : top;
     }
-    if (off >= maxbits) break;
+    if (!warp_any(off < maxbits)) break;
   }
 }
 

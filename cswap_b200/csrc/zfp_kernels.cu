@@ -41,7 +41,8 @@ namespace {
 
 constexpr int kThreads = 128;                  // zfp blocks (lanes) per CTA
 constexpr int kSlabFloats = 1024;              // one 32x32 z-slab
-constexpr int kEncCtasPerSm = 4;                // 128 registers per thread: the encoder needs 118
+constexpr int kEncCtasPerSm = 4;                // 128 registers per thread: the encoder needs 113; five CTAs
+                                                // spill, 256 MiB at 1024 bits 130.6 -> 146.9 us
 // 3-D decoders: 80 registers are enough for two chunks of planes, 96 for more (no spills); a CTA more hides more of the
 // dependent shared-memory reads (256 MiB at 512 bits 91.7 us with five CTAs, 85.9 with six).  Fields in their own
 // extents need a few registers more and are seldom more than one wave: 31 x 33 x 4096 11.8 us with five, 12.2 with six.
@@ -135,6 +136,9 @@ __device__ __forceinline__ int pad_src_z(int z, int vz) { return z < vz ? z : (z
 // 128-byte row segment, so a warp load touches four full lines), codes it into
 // its own column of the word-major staging area and writes its own words out:
 // after the table is built no warp waits for another.
+// Bound by instructions issued (2566 a warp at 512 bits, issue slots 71 % busy).  256 MiB at 256 / 512 / 1024
+// bits 82.0 / 104.0 / 135.8 -> 80.2 / 101.3 / 130.6 us with the expansions' bits in one word and a vote that holds
+// their loop together.
 __global__ void __launch_bounds__(kThreads, kEncCtasPerSm)
 zfp_encode_slab_kernel(const float* __restrict__ in, uint32_t* __restrict__ out, uint32_t nz, int maxbits, int lsh,
                        const PipeConsts kc) {
@@ -494,11 +498,15 @@ zfp_encode_generic_kernel(const FieldGeom g, const float* __restrict__ in, bool 
     for (int w = 0; w < nwords; w++) col[w * kThreads] = 0u;  // coded bits are OR-ed in
   }
   __syncthreads();  // the table is complete
-  if (b < nblocks) {
-    if constexpr (DIMS == 3) {
-      SmemStage st{col, queue + tid};
-      encode_block3_staged(f, maxbits, st, lut, kc);
-    } else {
+  if constexpr (DIMS == 3) {
+    if (b >= nblocks) {
+#pragma unroll
+      for (int i = 0; i < 64; i++) f[i] = 0.0f;
+    }
+    SmemStage st{col, queue + tid};
+    encode_block3_staged(f, maxbits, st, lut, kc);
+  } else {
+    if (b < nblocks) {
       ColumnSink sink{col};
       if constexpr (DIMS == 2) encode_block2(f, maxbits, sink, lut);
       else encode_block1(f, maxbits, sink, lut);
