@@ -657,8 +657,9 @@ bool vector_rows(const FieldGeom& g, const void* field) {
 // =====================================================================================
 // launchers
 // =====================================================================================
-constexpr size_t kDefaultDynamicSmem = 48 * 1024;  // what a kernel may ask for without opting in
+constexpr size_t kDefaultDynamicSmem = 40 * 1024;  // asked for without opting in (48 KiB, static memory included, are allowed)
 constexpr uint64_t kSchedulersPerSm = 4;
+constexpr int kWholeChip = 148;                    // SMs
 constexpr int kMostBits = 4096;                    // largest budget the library accepts
 static size_t staged_smem_bytes(int maxbits, bool decode, int dims) {
   const size_t rows = ((size_t)maxbits + 31) / 32 + STAGE_SPARE_ROWS;
@@ -723,8 +724,10 @@ static cudaError_t decode_generic(const FieldGeom& g, const uint32_t* in, float*
   // over, a CTA takes up to eight rounds of blocks.  With and without rounds, at 32 bits: 64 Mi values 275 / 298 us, 16 Mi
   // 73.9 / 75.8, but 4 Mi 23.3 / 20.7.  2-D fields (8 KiB a CTA) are better off without at every size: 4096 x 4096 at
   // 64 / 128 / 256 bits 43.0 / 49.0 / 62.4 us with rounds and 37.3 / 43.0 / 53.7 without, 8192 x 8192 at 128 bits 165 and 163.
+  // That is a whole chip; a part of one, where it could not be measured, goes round as in 1-D.
   const uint64_t full = 8 * (uint64_t)sm_count();
-  const uint64_t rounds = DIMS > 1 || ctas < 2 * full ? 1 : ctas / full < 8 ? ctas / full : 8;
+  const bool once = DIMS == 3 || (DIMS == 2 && sm_count() >= kWholeChip);
+  const uint64_t rounds = once || ctas < 2 * full ? 1 : ctas / full < 8 ? ctas / full : 8;
   return pdl_launch(zfp_decode_generic_kernel<DIMS, CHUNKS>, (unsigned)((ctas + rounds - 1) / rounds), kThreads, smem, stream,
                     g, in, out, vector_rows(g, out), maxbits, nblocks, (uint64_t)stream_bytes(g, (unsigned)maxbits) / 4, lsh,
                     pipe_consts());
