@@ -12,12 +12,12 @@
 // is not a constant of the library, and every CTA calls it.  What the stream
 // held before is then finished and visible, whatever it was.
 //
-// The exception: sparse_pack_kernel and sparse_onepass_kernel read the call's input
-// before they wait.  That is sound because a kernel of the same call in front of them
+// The exception: sparse_pack_kernel, sparse_pack_sum_kernel and sparse_onepass_kernel read
+// the call's input before they wait.  That is sound because a kernel of the same call in front of them
 // (the counting one; the one that clears the cursor) triggers only behind its own wait,
 // so that whatever produced the input has finished before either can start, also where
 // another kernel stands in between that triggers early (the scan).  A launch of one of
-// the two without such a kernel in front would race with the producer.
+// them without such a kernel in front would race with the producer.
 //
 // pdl_trigger() lets the next kernel of the stream be brought in once all CTAs of
 // this one have started, for chains inside one call whose next kernel has

@@ -176,6 +176,94 @@ sparse_pack_kernel(const uint32_t* __restrict__ in, uint64_t n, uint32_t* __rest
   }
 }
 
+// The same without a scan in between, for kLeastSummed to kMostSummed tiles: a CTA adds up the counts ahead
+// of its tile itself, and the last one to have read them turns them into offsets.  The number of CTAs that
+// have is kept above the thirteen bits of tile 0's count; no CTA waits for another.  A launch
+// less, but a CTA's loads lie in front of its part in the sum: 50 % zeros, with the scan and without, 1 Mi elements
+// 5.94 | 5.22 us, 2 Mi 6.64 | 6.24, 4 Mi 7.77 | 9.53, 8 Mi 13.3 | 15.9; 400 000 elements 5.94 | 6.01.
+constexpr int kCountBits = 13;  // a tile's count is 4096 at most
+constexpr uint32_t kCountMask = (1u << kCountBits) - 1u, kLeastSummed = 128, kMostSummed = 512;
+__global__ void __launch_bounds__(kThreads, 8)
+sparse_pack_sum_kernel(const uint32_t* __restrict__ in, uint64_t n, uint32_t* __restrict__ bitmap, uint32_t* tile_off,
+                       uint32_t* __restrict__ values, uint32_t* __restrict__ nnz_out) {
+  constexpr int kWarps = kThreads / 32, kPer = (int)kMostSummed / kThreads;
+  __shared__ uint32_t warp_cnt[kWarps], warp_sum[kWarps];
+  __shared__ bool last;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t tiles = gridDim.x, tile = tiles - 1 - blockIdx.x;
+  const uint64_t base = (uint64_t)tile * kTile + (uint64_t)warp * (kWordsPerWarp * 32);
+  uint32_t v[kWordsPerWarp], w[kWordsPerWarp];
+#pragma unroll
+  for (int j = 0; j < kWordsPerWarp; j++) {
+    const uint64_t i = base + j * 32 + lane;
+    v[j] = i < n ? __ldcg(in + i) : 0u;
+  }
+  uint32_t mine = 0, cnt = 0;
+#pragma unroll
+  for (int j = 0; j < kWordsPerWarp; j++) {
+    w[j] = __ballot_sync(0xffffffffu, v[j] != 0u);
+    cnt += __popc(w[j]);
+    if (lane == j) mine = w[j];
+  }
+  const uint64_t word0 = base >> 5, nwords = (n + 31) >> 5;
+  pdl_wait();
+  uint32_t ahead = 0;
+#pragma unroll
+  for (int q = 0; q < kPer; q++) {
+    const uint32_t i = q * kThreads + threadIdx.x;
+    if (i < tile) ahead += __ldcg(tile_off + i) & kCountMask;
+  }
+  ahead = __reduce_add_sync(0xffffffffu, ahead);
+  if (lane == 0) {
+    warp_cnt[warp] = cnt;
+    warp_sum[warp] = ahead;
+  }
+  __syncthreads();  // every count that this CTA needs has been read
+  uint32_t order = 0;
+  if (threadIdx.x == 0) order = atomicAdd(tile_off, 1u << kCountBits) >> kCountBits;
+  if (lane < kWordsPerWarp && word0 + lane < nwords) bitmap[word0 + lane] = mine;
+  uint32_t off = 0;
+#pragma unroll
+  for (int i = 0; i < kWarps; i++) off += warp_sum[i] + (i < warp ? warp_cnt[i] : 0u);
+  const uint32_t lt = lanemask_lt();
+#pragma unroll
+  for (int j = 0; j < kWordsPerWarp; j++) {
+    if (v[j] != 0u) values[off + __popc(w[j] & lt)] = v[j];
+    off += __popc(w[j]);
+  }
+  if (threadIdx.x == 0) last = order == tiles - 1;
+  __syncthreads();
+  if (!last) return;
+  uint32_t c[kPer], sum = 0;
+#pragma unroll
+  for (int q = 0; q < kPer; q++) {
+    const uint32_t i = threadIdx.x * kPer + q;
+    c[q] = i < tiles ? __ldcg(tile_off + i) & kCountMask : 0u;
+    sum += c[q];
+  }
+  uint32_t x = sum;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, x, d);
+    if (lane >= d) x += y;
+  }
+  if (lane == 31) warp_sum[warp] = x;
+  __syncthreads();  // the counts have been read by all
+  uint32_t at = x - sum, total = 0;
+#pragma unroll
+  for (int i = 0; i < kWarps; i++) {
+    at += i < warp ? warp_sum[i] : 0u;
+    total += warp_sum[i];
+  }
+#pragma unroll
+  for (int q = 0; q < kPer; q++) {
+    const uint32_t i = threadIdx.x * kPer + q;
+    if (i < tiles) tile_off[i] = at;
+    at += c[q];
+  }
+  if (threadIdx.x == 0) *nnz_out = total;
+}
+
 // ---- small tensors: one cluster --------------------------------------------------------
 // Up to kMaxCluster CTAs of TILES tiles compress the whole tensor: bitmap,
 // counts, offsets and values from one read and one launch.  The CTAs exchange their
@@ -476,6 +564,8 @@ cudaError_t sparse_compress_launch(const float* in, uint64_t n, uint32_t* bitmap
   const bool vec = (reinterpret_cast<uintptr_t>(in) & 15) == 0;
   cudaError_t e = cudaSuccess;
   if (ntiles) e = pdl_launch(sparse_count_kernel, ntiles, kCountThreads, 0, stream, src, n, vec, tile_off);
+  if (e == cudaSuccess && ntiles >= kLeastSummed && ntiles <= kMostSummed)
+    return pdl_launch(sparse_pack_sum_kernel, ntiles, kThreads, 0, stream, src, n, bitmap, tile_off, val, nnz_out);
   if (e == cudaSuccess) e = pdl_launch(block_exclusive_scan_kernel<uint32_t>, 1, 1024, 0, stream, tile_off, ntiles, nnz_out);
   if (e == cudaSuccess && ntiles)
     e = pdl_launch(sparse_pack_kernel, ntiles, kThreads, 0, stream, src, n, bitmap, tile_off, val);
@@ -490,6 +580,7 @@ cudaError_t sparse_compress_preload() {
   if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, sparse_count_kernel);
   if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, block_exclusive_scan_kernel<uint32_t>);
   if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, sparse_pack_kernel);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, sparse_pack_sum_kernel);
   return taken(e);
 }
 

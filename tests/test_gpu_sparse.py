@@ -259,3 +259,26 @@ def test_ordered_compress_with_many_tiles(cs, oracle, tiles):
     a[rng.random(n, dtype=np.float32) < 0.7] = 0.0
     a[4096 * 100:4096 * 103] = 0.0  # empty tiles
     _check_native(cs, oracle, a)
+
+
+@pytest.mark.parametrize("tiles", [127, 128, 129, 257, 511, 512, 513])
+@pytest.mark.parametrize("zeros", [0.0, 0.5, 1.0])
+def test_ordered_compress_where_each_cta_adds_up_the_counts(cs, oracle, tiles, zeros):
+    """Tile counts on either side of the launch rule, the last tile ragged, from no zeros (every count 4096) to
+    nothing else, three calls into one buffer that holds other bytes before."""
+    import torch
+    n = tiles * 4096 - 1234
+    rng = np.random.default_rng(tiles)
+    a = rng.standard_normal(n).astype(np.float32)
+    a[rng.random(n) < zeros] = 0
+    bitmap, values, tile_off, ref_nnz = oracle.sparse_compress(a, threads=oracle.max_threads())
+    L = cs.sparse_layout(n)
+    out = torch.full((L.bound,), 0xFF, dtype=torch.uint8, device="cuda")
+    t = torch.from_numpy(a).cuda()
+    for _ in range(3):
+        _, nnz = cs.sparse_compress(t, out=out)
+    assert int(nnz.item()) == ref_nnz
+    buf = out.cpu().numpy()
+    assert np.array_equal(buf[L.tile_off:L.tile_off + 4 * tiles].view(np.uint32), tile_off)
+    assert np.array_equal(buf[L.bitmap:L.bitmap + 4 * bitmap.size].view(np.uint32), bitmap)
+    assert np.array_equal(buf[L.values:L.values + 4 * ref_nnz].view(np.uint32), values.view(np.uint32))
