@@ -319,7 +319,7 @@ zfp_decode_slab_kernel(const uint32_t* __restrict__ in, float* __restrict__ out,
 // no atomics, no zeroed stream.  (One thread per block reading and writing global
 // memory word by word, with plane-by-plane coders whose lanes wait for each other,
 // took 28.7 + 33.4 us a call for 31 x 33 x 4096 at 512 bits and 22.6 + 26.7 us for
-// 768 x 4096 at 128; these take 11.9 + 14.3 and 11.4 + 13.2.  They are bound as the
+// 768 x 4096 at 128; these take 12.2 + 11.8 and 12.2 + 10.7.  They are bound as the
 // slab kernels are, by the number of instructions a block costs.)
 namespace {
 
