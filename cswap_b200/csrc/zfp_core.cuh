@@ -81,26 +81,41 @@ CSW_HD int f2i_rz(float f) {
   return (int)f;
 #endif
 }
-// true when the predicate holds on every active lane of the warp (host: the one "lane")
-CSW_HD bool warp_all(bool p) {
+// Votes.  A host build runs one lane at a time, alone or, where the tests give it a warp, among the 32 of one.
+#if !defined(__CUDACC__)
+struct HostWarp {
+  virtual bool any(bool p) = 0;
+  virtual int max(int v) = 0;
+};
+inline HostWarp* host_warp = nullptr;
+#endif
+// True when the predicate holds on every lane that happens to be converged here, which CUDA leaves open: for hints only,
+// where it does not matter that lanes of a warp get different answers.
+CSW_HD bool converged_all(bool p) {
 #if defined(__CUDA_ARCH__)
   return __all_sync(__activemask(), p);
 #else
   return p;
 #endif
 }
-// true when it holds on some lane of the warp, all of which must call (host: the one "lane")
+// true when it holds on some lane of the warp, all of which must call
 CSW_HD bool warp_any(bool p) {
 #if defined(__CUDA_ARCH__)
   return __any_sync(0xffffffffu, p);
+#elif !defined(__CUDACC__)
+  return host_warp ? host_warp->any(p) : p;
 #else
   return p;
 #endif
 }
+// true when it holds on every lane of the warp, all of which must call
+CSW_HD bool warp_all(bool p) { return !warp_any(!p); }
 // largest value over the lanes of the warp, all of which must call
 CSW_HD int warp_max(int v) {
 #if defined(__CUDA_ARCH__)
   return __reduce_max_sync(0xffffffffu, v);
+#elif !defined(__CUDACC__)
+  return host_warp ? host_warp->max(v) : v;
 #else
   return v;
 #endif
@@ -526,7 +541,7 @@ struct SigState {  // by mask and shift instructions that saturate: a dozen fewe
 template <class WordSink>
 CSW_HD void encode_plane2(uint32_t x, int& n, Emitter<WordSink>& em, const uint32_t* enc_lut) {
   constexpr int N = 16;
-  if (warp_all(n >= N)) {
+  if (converged_all(n >= N)) {
     em.emit32(x, N);
     return;
   }
@@ -1491,16 +1506,24 @@ struct HostPark {
   void put_mark(int j, uint32_t m) { marks[j] = m; }
   uint32_t mark(int j) const { return marks[j]; }
 };
+// the 3-D decoder as the kernels call it; told(state) whenever the integer decoder is given a block
+template <class WordSrc, class Told>
+void decode_block3_host(const WordSrc& src, HostPark& slots, int maxbits, float (&f)[64], const uint32_t* dec_lut, Told&& told) {
+  const int chunks = decode3_chunks(maxbits);
+  const auto rest = [&](const FirstTests& first) {
+    told(first);
+    decode_block3_ints(src, slots, maxbits, f, dec_lut, pipe_consts(), first);
+  };
+  if (chunks == 2) decode_block3_float<2>(src, slots, maxbits, f, dec_lut, rest);
+  else if (chunks == 3) decode_block3_float<3>(src, slots, maxbits, f, dec_lut, rest);
+  else over(rest);
+}
 template <class WordSrc>
-void decode_block3_pos(const WordSrc& src, int maxbits, float (&f)[64], const uint32_t* dec_lut, const PipeConsts& kc) {
+void decode_block3_pos(const WordSrc& src, int maxbits, float (&f)[64], const uint32_t* dec_lut) {
   const auto get = [&](int w) { return src.word(w); };
   CutWords<decltype(get)> cut{get, maxbits};
   HostPark slots;
-  const int chunks = decode3_chunks(maxbits);
-  const auto rest = [&](const FirstTests& first) { decode_block3_ints(cut, slots, maxbits, f, dec_lut, kc, first); };
-  if (chunks == 2) decode_block3_float<2>(cut, slots, maxbits, f, dec_lut, rest);
-  else if (chunks == 3) decode_block3_float<3>(cut, slots, maxbits, f, dec_lut, rest);
-  else over(rest);
+  decode_block3_host(cut, slots, maxbits, f, dec_lut, [](const FirstTests&) {});
 }
 template <class WordSource>
 void decode_block2(WordSource& src, int maxbits, float (&f)[16], const uint32_t* dec_lut) {

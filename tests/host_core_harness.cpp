@@ -3,10 +3,13 @@
 // plane transposes, table-driven group-test coding) bit for bit against the
 // oracle without a GPU.  Test scaffolding: the shipped library never runs
 // the codec on the host.
+#include <ucontext.h>
+
 #include <cmath>
 #include <cstdint>
 #include <cstring>
 #include <algorithm>
+#include <functional>
 #include <vector>
 
 #include "../cswap_b200/csrc/zfp_field.cuh"
@@ -122,7 +125,7 @@ void decode_field(const csw::FieldGeom& g, const uint32_t* in, int maxbits, floa
     float q[1 << (2 * DIMS)];
     if constexpr (DIMS == 3) {
       PadSource s{rows.data(), nw};
-      csw::decode_block3_pos(s, maxbits, q, dec3_lut().data(), csw::pipe_consts());
+      csw::decode_block3_pos(s, maxbits, q, dec3_lut().data());
     } else {
       VecSource s{rows.data(), nw};
       if constexpr (DIMS == 2) csw::decode_block2(s, maxbits, q, lut.data());
@@ -131,9 +134,109 @@ void decode_field(const csw::FieldGeom& g, const uint32_t* in, int maxbits, floa
     csw::scatter_block<DIMS>(g, out, b, q);
   }
 }
+
+// The 32 lanes of a warp, each on a stack of its own: a lane runs until it votes, and the votes are counted when all 32
+// stand at one.  Lanes that part - one returns while another votes, or they stand at different votes - would wait for
+// each other for good on a GPU; here the warp is given up and run() says so.
+class Warp : public csw::HostWarp {
+ public:
+  Warp() : stacks_(32 * kStack) {}
+  bool run(const std::function<void(int)>& lane) {
+    body_ = &lane;
+    csw::host_warp = this;
+    for (int i = 0; i < 32; i++) {
+      getcontext(&lanes_[i]);
+      lanes_[i].uc_stack.ss_sp = stacks_.data() + i * kStack;
+      lanes_[i].uc_stack.ss_size = kStack;
+      lanes_[i].uc_link = &home_;
+      at_[i] = kRuns;
+      const uintptr_t self = reinterpret_cast<uintptr_t>(this);
+      makecontext(&lanes_[i], reinterpret_cast<void (*)()>(&Warp::enter), 3, (unsigned)(self >> 32), (unsigned)self, i);
+    }
+    bool together = true;
+    while (together) {
+      for (now_ = 0; now_ < 32; now_++) swapcontext(&home_, &lanes_[now_]);
+      for (int i = 1; i < 32; i++) together = together && at_[i] == at_[0];
+      if (at_[0] == kDone) break;
+      result_ = value_[0];
+      for (int i = 1; i < 32; i++) result_ = at_[0] == kAny ? result_ | value_[i] : std::max(result_, value_[i]);
+    }
+    csw::host_warp = nullptr;
+    return together;
+  }
+  bool any(bool p) override { return vote(kAny, p) != 0; }
+  int max(int v) override { return vote(kMax, v); }
+
+ private:
+  enum Where { kRuns, kAny, kMax, kDone };
+  static constexpr size_t kStack = 1 << 17;
+  static void enter(unsigned hi, unsigned lo, int i) {
+    Warp* w = reinterpret_cast<Warp*>(((uintptr_t)hi << 32) | lo);
+    (*w->body_)(i);
+    w->at_[i] = kDone;
+  }
+  int vote(Where kind, int v) {
+    const int i = now_;
+    at_[i] = kind;
+    value_[i] = v;
+    swapcontext(&lanes_[i], &home_);
+    return result_;
+  }
+  const std::function<void(int)>* body_ = nullptr;
+  std::vector<char> stacks_;
+  ucontext_t home_, lanes_[32];
+  Where at_[32];
+  int value_[32], result_ = 0, now_ = 0;
+};
+
+// What the decoders did with a warp's blocks.
+enum Way { kFloatWay, kIntWay, kStartedAgain, kParted, kWays };
+
+// Decodes the 32 blocks from b on as a warp does: lanes behind the last block get an empty one.
+template <int DIMS>
+Way decode_warp(Warp& warp, const csw::FieldGeom& g, const uint32_t* in, int maxbits, float* out, size_t b) {
+  const int nw = (maxbits + 31) / 32;
+  const size_t total = csw::stream_bytes(g, maxbits) / 4, blocks = csw::geom_blocks(g);
+  static std::vector<uint32_t> rows[32];
+  static float q[32][64];
+  Way way = kFloatWay;
+  for (int l = 0; l < 32; l++) {
+    rows[l].assign(nw + csw::DEC_SPARE_ROWS, 0u);
+    for (int w = 0; b + l < blocks && w < nw; w++) {
+      const size_t at = (b + l) * maxbits + 32 * (size_t)w, i = at >> 5;
+      rows[l][w] = csw::funnel_r(in[i], i + 1 < total ? in[i + 1] : 0u, (int)(at & 31));
+    }
+    if (maxbits & 31) rows[l][nw - 1] &= csw::low_mask32(maxbits & 31);
+  }
+  const bool together = warp.run([&](int l) {
+    const PadSource src{rows[l].data(), nw + csw::DEC_SPARE_ROWS};
+    csw::HostPark park;
+    if constexpr (DIMS == 3) {
+      csw::decode_block3_host(src, park, maxbits, q[l], dec3_lut().data(), [&](const csw::FirstTests& first) {
+        way = first.tests < 0 && csw::decode3_chunks(maxbits) ? kStartedAgain : std::max(way, kIntWay);
+      });
+    } else {
+      float (&f)[16] = reinterpret_cast<float (&)[16]>(q[l]);
+      csw::decode_block2(src, park, maxbits, f, dec3_lut().data());
+    }
+  });
+  for (int l = 0; together && l < 32 && b + l < blocks; l++) {
+    if constexpr (DIMS == 3) csw::scatter_block<3>(g, out, b + l, q[l]);
+    else csw::scatter_block<2>(g, out, b + l, reinterpret_cast<float (&)[16]>(q[l]));
+  }
+  return together ? way : kParted;
+}
 }  // namespace
 
 extern "C" {
+// As core_decode, 2-D and 3-D, 32 blocks at a time; ways[] counts the warps by what the decoder did.
+void core_decode_warps(const uint32_t* in, size_t nx, size_t ny, size_t nz, int maxbits, float* out, int* ways) {
+  static Warp warp;
+  const csw::FieldGeom g = csw::make_geom(nx, ny, nz, 0, 0, 0);
+  std::fill(ways, ways + kWays, 0);
+  for (size_t b = 0; b < csw::geom_blocks(g); b += 32)
+    ways[g.dims == 3 ? decode_warp<3>(warp, g, in, maxbits, out, b) : decode_warp<2>(warp, g, in, maxbits, out, b)]++;
+}
 void core_encode(const float* in, size_t nx, size_t ny, size_t nz, int maxbits, uint32_t* out) {
   csw::FieldGeom g = csw::make_geom(nx, ny, nz, 0, 0, 0);
   if (g.dims == 3) encode_field<3>(g, in, maxbits, out);
