@@ -244,13 +244,12 @@ CSW_HD void fwd_lift(int& x, int& y, int& z, int& w) {
   w = wadd(w, y); w >>= 1; y = wsub(y, w);
   w = wadd(w, y >> 1); y = wsub(y, w >> 1);
 }
-CSW_HD int twice_minus(int a, int b) { return (int)(((uint32_t)a << 1) - (uint32_t)b); }
 CSW_HD void inv_lift(int& x, int& y, int& z, int& w) {
-  y = wadd(y, w >> 1); w = wsub(w, y >> 1);
-  y = wadd(y, w); w = twice_minus(w, y);
-  z = wadd(z, x); x = twice_minus(x, z);
-  y = wadd(y, z); z = twice_minus(z, y);
-  w = wadd(w, x); x = twice_minus(x, w);
+  const int a = wadd(y, w >> 1), b = wsub(w, a >> 1), c = wsub(x, z), d = wadd(x, z);
+  x = wadd(wsub(c, b), a);
+  y = wadd(wadd(d, b), a);
+  z = wsub(wsub(d, b), a);
+  w = wsub(wadd(c, b), a);
 }
 
 CSW_HD void fwd_xform2(int (&v)[16]) {
@@ -944,21 +943,21 @@ CSW_HD void decode_block1(WordSource& src, int maxbits, float (&f)[4], const uin
 // plane by plane for the warp as a whole:
 //
 //  * Planes are counted from a block's own first one that is not empty (the empty ones ahead
-//    of it are one '0' bit each), and taken in chunks, of eight in 3-D and of sixteen in 2-D.
-//  * In a chunk every lane first runs through the group tests of its own planes, as long as
+//    of it are one '0' bit each), and taken sixteen at a time.
+//  * Of these every lane first runs through the group tests of its own planes, as long as
 //    it has coefficients that are not significant, and parks a mark at the end of each: where
 //    the next plane begins and how many of its bits are verbatim.  The loop lasts as long as the lane
-//    with the most steps, not the sum over planes of the longest (15.7 steps against 33.7 for
-//    3-D at 512 bits, 11.4 against 25.2 for 2-D at 128, counted on the CPU).  What the tests find
+//    with the most steps, not the sum over planes of the longest (16.2 steps against 33.7 for
+//    3-D at 512 bits, 9.9 against 25.2 for 2-D at 128, counted on the CPU over the benchmark's values).  What the tests find
 //    needs no slots: a position becomes significant once, so the bits of all planes fit into one word.
-//  * Then the chunk's planes are put together by all lanes in step - a funnel shift of staged
-//    words, the found bits, masks - and transposed.
+//  * Then the planes are put together by all lanes in step - a funnel shift of staged
+//    words, the found bits, masks - and transposed, sixteen of 2-D at once and eight of 3-D.
 //
 // WordSrc::word(w) returns the block's w-th 32-bit word, with zeros for the bits past the
 // budget and for DEC_SPARE_ROWS words behind it: a group test that finds no bits ends its plane,
 // as it must, and only a run cut by the budget needs a correction (decode_tests).
-// Park: mark(j) is the lane's slot j, j <= chunk + 1.
-constexpr int DEC_SPARE_ROWS = 4, CHUNK3 = 8, CHUNK2 = 16;
+// Park: mark(j) is the lane's slot j, j < PARK_SLOTS.
+constexpr int DEC_SPARE_ROWS = 4, CHUNK3 = 8, CHUNK2 = 16, PARK_SLOTS = 18;
 
 // (h:l) rotated left by r, r in 0..64
 CSW_HD void rol64(uint32_t& l, uint32_t& h, int r) {
@@ -1037,26 +1036,36 @@ CSW_HD int decode_tests(const WordSrc& src, Park& park, int maxbits, const uint3
   return j;
 }
 
-// Eight planes, transposed: byte b of w[8 * g + i] holds coefficient 32g + 8b + i (in sequency
-// order), the first plane in its top bit, odd bits complemented (the xor half of the inverse negabinary
-// map).  `tests` of them have group tests, which decode_tests found; `m` is what it left, and moves
-// behind the chunk.  left: planes of the block that begin within the budget, from this chunk on (nine when
-// there are more than eight).  NARROW: look out for warps none of whose coefficients from the 32nd on
-// is significant yet.
-template <bool NARROW, class WordSrc, class Park>
-CSW_HD void decode_rows3(const WordSrc& src, const Park& park, int maxbits, int tests, uint32_t& m, const Found& found,
-                         int& left, uint32_t (&w)[16]) {
+// What decode_tests found in planes of a 3-D block, besides the marks: how many had group tests, the place behind them.
+struct Tests3 {
+  int tests;
+  uint32_t m;
+  Found found;
+};
+template <int PLANES, class WordSrc, class Park>
+CSW_HD Tests3 tests_from(const WordSrc& src, Park& park, int maxbits, const uint32_t* dec_lut, uint32_t m, Found found) {
+  Tests3 t{0, m, found};
+  t.tests = decode_tests<64, PLANES>(src, park, maxbits, dec_lut, t.m, t.found);
+  return t;
+}
+// Planes that begin within the budget; many, where more of them have tests than were gone through.
+CSW_HD int planes_behind(const Tests3& t, int maxbits) {
+  const int rest = maxbits - mark_pos(t.m);
+  return t.tests + (rest > 0 ? (mark_n(t.m) == 64 ? (rest + 63) >> 6 : 64) : 0);
+}
+
+// Eight planes from the FIRST one behind a call of decode_tests on, transposed: byte b of w[8 * g + i] holds coefficient
+// 32g + 8b + i (in sequency order), the first plane in its top bit, odd bits complemented (the xor half of the
+// inverse negabinary map).  `at` is the place of the first of them, and moves behind the last; (fh:fl): what was found, position
+// p at bit p.  most_tests, most_planes: of the lanes of the warp.  NARROW: the budget up to which to look
+// out for warps none of whose coefficients from the 32nd on is significant yet.
+template <int FIRST, int NARROW, class WordSrc, class Park>
+CSW_HD void decode_rows3(const WordSrc& src, const Park& park, int maxbits, int tests, int most_tests, int most_planes,
+                         uint32_t fl, uint32_t fh, uint32_t& at, uint32_t (&w)[16]) {
   const int nwords = (maxbits + 31) >> 5;
-  uint32_t at = park.mark(0);
-  {
-    const int rest = maxbits - mark_pos(m);
-    left = tests + (rest > 0 ? (mark_n(m) == 64 ? (rest + 63) >> 6 : 1) : 0);
-  }
-  const int warp_tests = warp_max(tests), warp_left = warp_max(left);
-  uint32_t fl = found.lo, fh = found.hi;
-  rol64(fl, fh, mark_n(m));  // position p at bit p
+  const int warp_tests = most_tests - FIRST, warp_left = most_planes - FIRST;
   uint32_t ml = low_mask_sat(mark_n(at)), mh = low_mask_sat(mark_n(at) - 32);
-  if (warp_left == 1 && warp_tests == 0) {
+  if (warp_left == 1 && warp_tests <= 0) {
     // A plane is left, the usual case behind eight or sixteen of a budget of whole values: no transpose.
     int i = mark_pos(at) >> 5;
     i = i < nwords ? i : nwords;
@@ -1067,11 +1076,11 @@ CSW_HD void decode_rows3(const WordSrc& src, const Park& park, int maxbits, int 
       w[k] = ((xl << (7 - k)) & 0x80808080u) | 0x2a2a2a2au;
       w[8 + k] = ((xh << (7 - k)) & 0x80808080u) | 0x2a2a2a2au;
     }
-    m = at + 64u * CHUNK3;
+    at += 64u * CHUNK3;
     return;
   }
   uint32_t lo[8], hi[8];
-  if (NARROW && warp_max(mark_n(m)) <= 32) {
+  if (maxbits <= NARROW && warp_tests > 0 && warp_max(mark_n(park.mark(tests < FIRST + CHUNK3 ? tests : FIRST + CHUNK3))) <= 32) {
 #pragma unroll
     for (int j = 0; j < CHUNK3; j++) {
       uint32_t xl = 0u;
@@ -1079,7 +1088,7 @@ CSW_HD void decode_rows3(const WordSrc& src, const Park& park, int maxbits, int 
         int i = mark_pos(at) >> 5;
         i = i < nwords ? i : nwords;
         xl = funnel_r(src.word(i), src.word(i + 1), (int)at);
-        if (j < tests) at = park.mark(j + 1);
+        if (FIRST + j < tests) at = park.mark(FIRST + j + 1);
         xl = (xl & ml) | (fl & ~ml);
         ml = low_mask_sat(mark_n(at));
         xl &= ml;
@@ -1092,7 +1101,6 @@ CSW_HD void decode_rows3(const WordSrc& src, const Park& park, int maxbits, int 
       w[i] = lo[i];
       w[8 + i] = 0xaaaaaaaau;
     }
-    m = at;
     return;
   }
 #pragma unroll
@@ -1107,7 +1115,7 @@ CSW_HD void decode_rows3(const WordSrc& src, const Park& park, int maxbits, int 
       at += 64u;
       if (j < warp_tests) {
         // the first n bits verbatim (decode.cuh:143-145), then those found up to the next n
-        if (j < tests) at = park.mark(j + 1);
+        if (FIRST + j < tests) at = park.mark(FIRST + j + 1);
         xl = (xl & ml) | (fl & ~ml);
         xh = (xh & mh) | (fh & ~mh);
         ml = low_mask_sat(mark_n(at));
@@ -1120,7 +1128,6 @@ CSW_HD void decode_rows3(const WordSrc& src, const Park& park, int maxbits, int 
     hi[7 - j] = (j & 1) ? xh : ~xh;
   }
   // behind planes without tests every coefficient is significant, or the budget is spent
-  m = at;
   transpose8(lo);
   transpose8(hi);
 #pragma unroll
@@ -1129,15 +1136,12 @@ CSW_HD void decode_rows3(const WordSrc& src, const Park& park, int maxbits, int 
     w[8 + i] = hi[i];
   }
 }
-
-template <bool NARROW, class WordSrc, class Park>
-CSW_HD void decode_chunk3(const WordSrc& src, Park& park, int maxbits, const uint32_t* dec_lut, uint32_t& m, Found& found,
-                          int& left, uint32_t (&w)[16]) {
-  const int tests = decode_tests<64, CHUNK3>(src, park, maxbits, dec_lut, m, found);
-  decode_rows3<NARROW>(src, park, maxbits, tests, m, found, left, w);
+CSW_HD void empty_rows3(uint32_t (&w)[16]) {
+#pragma unroll
+  for (int i = 0; i < 16; i++) w[i] = 0xaaaaaaaau;
 }
 
-// inv_lift in floating point, where it is exact (decode_block3_float): ten operations become nine
+// inv_lift in floating point, where it is exact (decode_block3): ten operations become nine
 CSW_HD void inv_lift2(F2& x, F2& y, F2& z, F2& w) {  // two lines at a time
   const F2 y1 = fma2(w, 0.5f, y);
   const F2 a = fma2(y1, 0.5f, w), b = fma2(y1, -1.5f, w);
@@ -1181,9 +1185,11 @@ CSW_HD void floats_of3(const float (&h)[64], float s, float t, F2 (&q)[32], std:
   ((q[P] = fma2(F2{h[SequencyAt<2 * P>::v], h[SequencyAt<2 * P + 1>::v]}, s, F2{t, t})), ...);
 }
 template <int... I>
-CSW_HD void ints_of3(const uint32_t (&u)[64], int lead, uint32_t flip, int (&v)[64], const PipeConsts& kc,
-                     std::integer_sequence<int, I...>) {
-  ((v[PermAt<3, I>::v] = imad((int)kc.nb, kc.mone, (int)((u[I] >> lead) ^ flip))), ...);  // - 0xaaaaaaaa
+CSW_HD void ints_of3(const uint32_t (&u)[64], int lead, int (&v)[64], std::integer_sequence<int, I...>) {
+  // the digits move down by `lead`, zeros follow; where that takes the odd ones to even places all are
+  // complemented, and so is the difference: (x ^ 0xaaaaaaaa) - 0xaaaaaaaa or (~x ^ ...) - ...
+  const int sign = (lead & 1) ? -1 : 1, from = (lead & 1) ? 0x55555555 : 0x55555556;
+  ((v[PermAt<3, I>::v] = imad((int)funnel_r(u[I], 0xaaaaaaaau, lead), sign, from)), ...);
 }
 
 // The values of a block.
@@ -1196,73 +1202,73 @@ CSW_HD void ints_of3(const uint32_t (&u)[64], int lead, uint32_t flip, int (&v)[
 // to one at most (run the lifting backwards).  So when the results stay below 2^(p + 18), 24 bits
 // held everything, and when they stay below 2^31 too the integers of decode.cuh:177-288 would not have
 // wrapped (their shifts lose nothing with p > 5): the same values, to the bit.  The results are checked
-// for that, with a margin for what rounding could have done to larger ones.  A block's scale leaves room
-// for results of 2^30, so p < 12 is not tried; with p of 9 to 11 the first two passes, which have two
-// bits more room, are done this way and the last one in integers.  The products with the block's
+// for that, with a margin for what rounding could have done to larger ones.  The products with the block's
 // scale are powers of two, exact within the exponents asked for.
 //
-// What does not fit is left to decode_block3_ints, and so are, once the tests of the first chunk are
-// through, blocks whose planes are so short that more than CHUNKS * 8 of them can be expected.
-// Eight-plane chunks the floating point decoder is given: up to 13 bits a value the planes of a block
-// of noise are 14, and p < 12 takes a block with more than six empty planes.
-CSW_HD int decode3_chunks(int maxbits) { return maxbits <= 832 ? 2 : maxbits <= 1408 ? 3 : 0; }
+// What can fail the check is not tried, as far as the group tests tell: a block's scale leaves room for results of 2^30, so
+// p < 12 (planes + lead > 20) is not, and with p > 26 what the planes below would have added is so much that results beyond
+// 2^31 are common where values reach the top of a block's range.  Failing costs: the block is decoded again from the start
+// (256 MiB at 256 bits, values of +-1 before rounding: 154.7 us with p = 27 tried, 85.8 without).
+//
+// The integers take every block, and get the budgets at which few or only some fit:
+//  * above 832 bits, where p falls below 12.  (256 MiB, normal values: at 896 bits 110.2 us, 100.3 with floats tried up to 1152
+//    bits, but at 1024 bits, where half of the warps fit, 122.3 and 127.1, at 1152 127.0 and 131.8.)
+//  * below 256 bits, where p is mostly above 26.
+enum Way3 { kFloats3, kInts3, kShortInts3 };
+CSW_HD Way3 decode3_way(int maxbits) { return maxbits < 256 ? kShortInts3 : maxbits <= 832 ? kFloats3 : kInts3; }
 
-// What decode_tests found of a block's first chunk; tests < 0: nothing yet.
-struct FirstTests {
-  int tests;
-  uint32_t m;
-  Found found;
-};
+// What became of a warp's blocks, the same for all lanes: for the tests.
+enum Taken3 { kByFloats, kByInts, kByIntsAfterAll };
 
-template <class Rest>
-CSW_HD bool over(Rest&& rest) {  // from the start
-  rest(FirstTests{-1, 0u, {0u, 0u}});
-  return false;
-}
-
-// true: f holds the values.  false: they were left to `rest`, which gets what can be gone on from.  The same
-// for all lanes of the warp, all of which must call.  (`rest` is called where the decision falls: with the
-// state handed back to the caller instead, every call paid 3 us at 256 MiB for keeping it.)
-template <int CHUNKS, class WordSrc, class Park, class Rest>
-CSW_HD bool decode_block3_float(const WordSrc& src, Park& park, int maxbits, float (&f)[64], const uint32_t* dec_lut,
-                                Rest&& rest) {
+// A 3-D block; all lanes of the warp call.  WAY: decode3_way(maxbits).  sink(values) takes them; rest() decodes a block again
+// that the check turned down.
+//
+// What both decoders need is written once, and so are the two rounds of sixteen planes: a warp in one beside a warp in
+// another is the usual case for values that are neither noise nor smooth, and their code together is more than
+// the instruction cache holds.  (With the integers out of line, with a code of their own for the planes: normal
+// values + 10 at 704 bits, where half of the warps fit, 154.4 us against 127.4, all of them noise 97.4 against 98.3;
+// with the second round unrolled smooth values at 512 bits 176.5 against 164.4.)
+// kShortInts3 looks out for warps whose planes have few significant coefficients, or fill one byte (smooth values at 64 bits
+// 99.6 -> 93.2 us, normal ones 70.3 -> 68.3; at 1024 bits it costs, 121.5 -> 126.6).
+template <Way3 WAY, class WordSrc, class Park, class Sink, class Rest>
+CSW_HD Taken3 decode_block3(const WordSrc& src, Park& park, int maxbits, const uint32_t* dec_lut, Sink&& sink,
+                            Rest&& rest) {
+  constexpr int kNarrow = WAY == kShortInts3 ? 255 : 0;
   const BlockHead blk = block_head(src, maxbits);
-  uint32_t w0[16], w1[16], w2[16], m = (uint32_t)blk.start;
+  bool floats = WAY == kFloats3;
+  uint32_t w0[16], w1[16], first0[16], first1[16], at = (uint32_t)blk.start;
   Found found{0u, 0u};
-  const int tests = decode_tests<64, CHUNK3>(src, park, maxbits, dec_lut, m, found);
-  {
-    // a plane takes n + 1 bits and those of the tests
-    const int n = mark_n(m), bits = maxbits - mark_pos(m) - (CHUNK3 - tests) * 64;
-    if (warp_any(bits > (CHUNKS - 1) * CHUNK3 * (9 + n - n / 8))) {
-      rest(FirstTests{tests, m, found});
-      return false;
+  int planes, most_planes;
+  bool second = false;
+  // Sixteen planes, and once more for the others.
+#pragma unroll 1
+  for (;;) {
+    const Tests3 t = tests_from<2 * CHUNK3>(src, park, maxbits, dec_lut, at, found);
+    planes = planes_behind(t, maxbits);
+    if (floats) {
+      const int down = planes + blk.lead;
+      floats = warp_all(blk.e >= 34 && blk.e <= 225 && planes <= 2 * CHUNK3 && ((uint32_t)(down - 6) <= 14u || planes == 0));
+    }
+    const int most_tests = warp_max(t.tests);
+    most_planes = warp_max(planes);
+    found = t.found;
+    uint32_t fl = found.lo, fh = found.hi;
+    rol64(fl, fh, mark_n(t.m));
+    decode_rows3<0, kNarrow>(src, park, maxbits, t.tests, most_tests, most_planes, fl, fh, at, w0);
+    if (most_planes > 8) decode_rows3<8, 0>(src, park, maxbits, t.tests, most_tests, most_planes, fl, fh, at, w1);
+    else empty_rows3(w1);
+    if (floats || second || most_planes <= 16) break;
+    second = true;
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
+      first0[i] = w0[i];
+      first1[i] = w1[i];
     }
   }
-  int planes, left;
-  decode_rows3<false>(src, park, maxbits, tests, m, found, left, w0);
-  planes = left;
-  bool three = false;
-  if (warp_any(left > CHUNK3)) {
-    decode_chunk3<false>(src, park, maxbits, dec_lut, m, found, left, w1);
-    if (left > 0) planes = CHUNK3 + left;
-    three = warp_any(left > CHUNK3);
-  } else {
-#pragma unroll
-    for (int i = 0; i < 16; i++) w1[i] = 0xaaaaaaaau;
-  }
-  if (CHUNKS == 2) {
-    if (three) return over(rest);
-  } else if (three) {
-    decode_chunk3<false>(src, park, maxbits, dec_lut, m, found, left, w2);
-    if (left > 0) planes = 2 * CHUNK3 + left;
-    if (warp_any(left > CHUNK3)) return over(rest);
-  }
-  const bool floats = warp_all(blk.e >= 34 && blk.e <= 225 && planes + blk.lead <= 20);
-  if (!floats && (CHUNKS == 2 || !warp_all(planes + blk.lead <= 23))) return over(rest);
-  // h: the planes as an integer, the first one in bit 15 (or 23), held as a float
-  float h[64], offset = 8388608.0f + 43690.0f;
-  int unit = (floats ? (int)blk.e - 14 : 143) - blk.lead;  // exponent field of the weight of 2^0 of h
-  if (CHUNKS == 2 || !three) {
+  if (floats) {
+    // h: the sixteen planes as an integer, the first one in bit 15, held as a float
+    float h[64];
+    const int unit = (int)blk.e - 14 - blk.lead;  // exponent field of the weight of 2^0 of h
 #pragma unroll
     for (int i = 0; i < 16; i++) {
       const uint32_t a = byte_perm(w1[i], w0[i], 0x5140), b = byte_perm(w1[i], w0[i], 0x7362);
@@ -1272,26 +1278,11 @@ CSW_HD bool decode_block3_float(const WordSrc& src, Park& park, int maxbits, flo
       h[at + 16] = u2f(byte_perm(b, 0x4b000000u, 0x7610));
       h[at + 24] = u2f(byte_perm(b, 0x4b000000u, 0x7632));
     }
-  } else {
-#pragma unroll
-    for (int i = 0; i < 16; i++) {
-      uint32_t t[4] = {w2[i], w1[i], w0[i], 0u};
-      transpose_bytes4(t);
-      const int at = 32 * (i >> 3) + (i & 7);
-      h[at] = (float)t[0];
-      h[at + 8] = (float)t[1];
-      h[at + 16] = (float)t[2];
-      h[at + 24] = (float)t[3];
-    }
-    offset = 11184810.0f;
-  }
-  float s = u2f(((uint32_t)unit << 23) | ((uint32_t)blk.lead << 31));
-  if (three) s *= 0.00390625f;
-  F2 q[32];
-  floats_of3(h, s, -s * offset, q, std::make_integer_sequence<int, 32>{});
-  inv_xform3_zy(q);
-  float top = 0.0f;
-  if (CHUNKS == 2 || floats) {
+    const float s = u2f(((uint32_t)unit << 23) | ((uint32_t)blk.lead << 31));
+    F2 q[32];
+    floats_of3(h, s, -s * (8388608.0f + 43690.0f), q, std::make_integer_sequence<int, 32>{});
+    inv_xform3_zy(q);
+    float top = 0.0f, f[64];
 #pragma unroll
     for (int i = 0; i < 16; i++) {
       F2 a = q[2 * i], b = q[2 * i + 1];
@@ -1303,63 +1294,55 @@ CSW_HD bool decode_block3_float(const WordSrc& src, Park& park, int maxbits, flo
       f[4 * i + 2] = b.x;
       f[4 * i + 3] = b.y;
     }
-    const int room = 34 - planes < 15 + blk.lead ? 34 - planes : 15 + blk.lead;  // 2^(p + 18), 2^31 in units of h
-    return warp_all(top <= u2f(((uint32_t)(unit + room - 1) << 23) | 0x7ff800u)) || over(rest);
-  }
-#pragma unroll
-  for (int i = 0; i < 32; i++) top = max_abs3(top, q[i].x, q[i].y);
-  const int room = 36 - planes < 15 + blk.lead ? 36 - planes : 15 + blk.lead;  // 2^(p + 20)
-  if (!warp_all(top <= u2f(((uint32_t)(unit + room - 1) << 23) | 0x7ff800u))) return over(rest);
-  const float scale = dequant_scale(blk.e);
-#pragma unroll
-  for (int i = 0; i < 16; i++) {
-    int x = f2i_rz(q[2 * i].x), y = f2i_rz(q[2 * i].y), z = f2i_rz(q[2 * i + 1].x), w = f2i_rz(q[2 * i + 1].y);
-    inv_lift(x, y, z, w);
-    mul2(scale, (float)x, (float)y, f[4 * i], f[4 * i + 1]);
-    mul2(scale, (float)z, (float)w, f[4 * i + 2], f[4 * i + 3]);
-  }
-  return true;
-}
-
-template <class WordSrc, class Park>
-CSW_HD void decode_block3_ints(const WordSrc& src, Park& park, int maxbits, float (&f)[64], const uint32_t* dec_lut,
-                               const PipeConsts& kc, const FirstTests& first) {
-  const BlockHead blk = block_head(src, maxbits);
-  uint32_t w0[16], w1[16], w2[16], w3[16], m = first.m;
-  Found found = first.found;
-  int tests = first.tests, left;
-  if (warp_any(tests < 0)) {
-    m = (uint32_t)blk.start;
-    found = Found{0u, 0u};
-    tests = decode_tests<64, CHUNK3>(src, park, maxbits, dec_lut, m, found);
-  }
-  decode_rows3<true>(src, park, maxbits, tests, m, found, left, w0);
-#pragma unroll
-  for (int i = 0; i < 16; i++) w1[i] = w2[i] = w3[i] = 0xaaaaaaaau;
-  if (warp_any(left > CHUNK3)) {
-    decode_chunk3<true>(src, park, maxbits, dec_lut, m, found, left, w1);
-    if (warp_any(left > CHUNK3)) {
-      decode_chunk3<true>(src, park, maxbits, dec_lut, m, found, left, w2);
-      if (warp_any(left > CHUNK3)) decode_chunk3<true>(src, park, maxbits, dec_lut, m, found, left, w3);
+    const int room = 34 - planes < 15 + blk.lead ? 34 - planes : 15 + blk.lead;  // 2^(p + 18)
+    if (warp_all(top <= u2f(((uint32_t)(unit + room - 1) << 23) | 0x7ff800u))) {
+      sink(f);
+      return kByFloats;
     }
+    rest();
+    return kByIntsAfterAll;
   }
   uint32_t u[64];
+  if (second) {
 #pragma unroll
-  for (int i = 0; i < 16; i++) {
-    uint32_t t[4] = {w3[i], w2[i], w1[i], w0[i]};
-    transpose_bytes4(t);
-    const int at = 32 * (i >> 3) + (i & 7);
-    u[at] = t[0];
-    u[at + 8] = t[1];
-    u[at + 16] = t[2];
-    u[at + 24] = t[3];
+    for (int i = 0; i < 16; i++) {
+      uint32_t b[4] = {w1[i], w0[i], first1[i], first0[i]};
+      transpose_bytes4(b);
+      const int j = 32 * (i >> 3) + (i & 7);
+      u[j] = b[0];
+      u[j + 8] = b[1];
+      u[j + 16] = b[2];
+      u[j + 24] = b[3];
+    }
+  } else if (WAY == kShortInts3 && most_planes <= 8) {
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
+      const int j = 32 * (i >> 3) + (i & 7);
+      u[j] = byte_perm(w0[i], 0xaaaaaaaau, 0x0444);
+      u[j + 8] = byte_perm(w0[i], 0xaaaaaaaau, 0x1444);
+      u[j + 16] = byte_perm(w0[i], 0xaaaaaaaau, 0x2444);
+      u[j + 24] = byte_perm(w0[i], 0xaaaaaaaau, 0x3444);
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
+      const uint32_t a = byte_perm(w1[i], w0[i], 0x5140), b = byte_perm(w1[i], w0[i], 0x7362);
+      const int j = 32 * (i >> 3) + (i & 7);
+      u[j] = byte_perm(a, 0xaaaaaaaau, 0x1044);
+      u[j + 8] = byte_perm(a, 0xaaaaaaaau, 0x3244);
+      u[j + 16] = byte_perm(b, 0xaaaaaaaau, 0x1044);
+      u[j + 24] = byte_perm(b, 0xaaaaaaaau, 0x3244);
+    }
   }
   int v[64];
-  ints_of3(u, blk.lead, (0xaaaaaaaau >> blk.lead) ^ 0xaaaaaaaau, v, kc, std::make_integer_sequence<int, 64>{});
+  ints_of3(u, blk.lead, v, std::make_integer_sequence<int, 64>{});
   inv_xform3(v);
   const float scale = dequant_scale(blk.e);
+  float f[64];
 #pragma unroll
   for (int i = 0; i < 64; i += 2) mul2(scale, (float)v[i], (float)v[i + 1], f[i], f[i + 1]);
+  sink(f);
+  return kByInts;
 }
 
 // ---- decoder: 2-D block -------------------------------------------------------------
@@ -1502,28 +1485,28 @@ struct CutWords {
   uint32_t word(int w) const { return 32 * w < maxbits ? get(w) & low_mask_sat(maxbits - 32 * w) : 0u; }
 };
 struct HostPark {
-  uint32_t marks[CHUNK2 + 2];
+  uint32_t marks[PARK_SLOTS];
   void put_mark(int j, uint32_t m) { marks[j] = m; }
   uint32_t mark(int j) const { return marks[j]; }
 };
-// the 3-D decoder as the kernels call it; told(state) whenever the integer decoder is given a block
-template <class WordSrc, class Told>
-void decode_block3_host(const WordSrc& src, HostPark& slots, int maxbits, float (&f)[64], const uint32_t* dec_lut, Told&& told) {
-  const int chunks = decode3_chunks(maxbits);
-  const auto rest = [&](const FirstTests& first) {
-    told(first);
-    decode_block3_ints(src, slots, maxbits, f, dec_lut, pipe_consts(), first);
+// the 3-D decoder as the kernels call it
+template <class WordSrc>
+Taken3 decode_block3_host(const WordSrc& src, HostPark& slots, int maxbits, float (&f)[64], const uint32_t* dec_lut) {
+  const Way3 way = decode3_way(maxbits);
+  const auto sink = [&](const float (&v)[64]) {
+    for (int i = 0; i < 64; i++) f[i] = v[i];
   };
-  if (chunks == 2) decode_block3_float<2>(src, slots, maxbits, f, dec_lut, rest);
-  else if (chunks == 3) decode_block3_float<3>(src, slots, maxbits, f, dec_lut, rest);
-  else over(rest);
+  const auto rest = [&] { decode_block3<kInts3>(src, slots, maxbits, dec_lut, sink, [] {}); };
+  return way == kFloats3 ? decode_block3<kFloats3>(src, slots, maxbits, dec_lut, sink, rest)
+         : way == kInts3 ? decode_block3<kInts3>(src, slots, maxbits, dec_lut, sink, rest)
+                         : decode_block3<kShortInts3>(src, slots, maxbits, dec_lut, sink, rest);
 }
 template <class WordSrc>
 void decode_block3_pos(const WordSrc& src, int maxbits, float (&f)[64], const uint32_t* dec_lut) {
   const auto get = [&](int w) { return src.word(w); };
   CutWords<decltype(get)> cut{get, maxbits};
   HostPark slots;
-  decode_block3_host(cut, slots, maxbits, f, dec_lut, [](const FirstTests&) {});
+  decode_block3_host(cut, slots, maxbits, f, dec_lut);
 }
 template <class WordSource>
 void decode_block2(WordSource& src, int maxbits, float (&f)[16], const uint32_t* dec_lut) {

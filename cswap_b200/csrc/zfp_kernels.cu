@@ -43,10 +43,11 @@ constexpr int kThreads = 128;                  // zfp blocks (lanes) per CTA
 constexpr int kSlabFloats = 1024;              // one 32x32 z-slab
 constexpr int kEncCtasPerSm = 4;                // 128 registers per thread: the encoder needs 113; five CTAs
                                                 // spill, 256 MiB at 1024 bits 130.6 -> 146.9 us
-// 3-D decoders: 80 registers are enough for two chunks of planes, 96 for more (no spills); a CTA more hides more of the
-// dependent shared-memory reads (256 MiB at 512 bits 91.7 us with five CTAs, 85.9 with six).  Fields in their own
-// extents need a few registers more and are seldom more than one wave: 31 x 33 x 4096 11.8 us with five, 12.2 with six.
-constexpr int dec_ctas_per_sm(int chunks, bool slabs) { return chunks == 2 && slabs ? 6 : 5; }
+// 3-D decoders: 80 registers are nearly enough (12 bytes of spills in the floating point one); a CTA more hides more of the
+// dependent shared-memory reads (256 MiB at 512 bits 91.7 us with five CTAs, 85.9 with six; at 1024 bits 125.6 and 123.4).
+// Fields in their own extents need a few registers more and are seldom more than one wave: 31 x 33 x 4096 at 512 bits 11.1 us
+// with five, 11.8 with six.
+constexpr int kSlabDecCtasPerSm = 6, kDecCtasPerSm = 5;
 
 // ---- word staging: word w of the block owned by thread t lives at [w * kThreads + t] --
 // Staged stream words of the 2-D and 3-D decoders and the slots they park marks in: areas of the
@@ -61,10 +62,7 @@ struct WarpPark {
   __device__ __forceinline__ uint32_t mark(int j) const { return p[32 * j]; }
 };
 // words of a warp's areas together; store_rows3 takes 512 of them when the block is decoded
-__host__ __device__ constexpr int warp_words(int nwords, int dims) {
-  return dims == 2 ? 32 * (nwords + DEC_SPARE_ROWS + CHUNK2 + 2)
-         : nwords > 2 ? 32 * (nwords + DEC_SPARE_ROWS + CHUNK3 + 2) : 512;
-}
+__host__ __device__ constexpr int warp_words(int nwords) { return 32 * (nwords + DEC_SPARE_ROWS + PARK_SLOTS); }
 
 // Staged words and the per-lane expansion queue of the staged encoder, both
 // word-major so that a warp's lanes always hit 32 different banks.
@@ -215,19 +213,10 @@ __device__ const DecTable g_dec_table = make_dec_table();
 
 namespace {
 // the staged words of this thread's lane behind the table, the slots behind the words
-template <int DIMS>
 __device__ __forceinline__ uint32_t* decoder_column(int nwords) {
   extern __shared__ __align__(16) uint32_t smem_words[];
-  return smem_words + DEC_LUT_SIZE + (threadIdx.x >> 5) * warp_words(nwords, DIMS) + (threadIdx.x & 31);
+  return smem_words + DEC_LUT_SIZE + (threadIdx.x >> 5) * warp_words(nwords) + (threadIdx.x & 31);
 }
-__device__ __forceinline__ void decode_ints(int maxbits, float (&f)[64], const PipeConsts& kc, const FirstTests& first) {
-  extern __shared__ __align__(16) uint32_t smem_words[];
-  const int nwords = (maxbits + 31) >> 5;
-  WarpWords source{decoder_column<3>(nwords)};
-  WarpPark park{decoder_column<3>(nwords) + 32 * (nwords + DEC_SPARE_ROWS)};
-  decode_block3_ints(source, park, maxbits, f, smem_words, kc, first);
-}
-
 // eight neighbouring lanes cover one 128-byte row segment, so every store
 // instruction of a warp writes four full lines: no staging of the output
 __device__ __forceinline__ void store_slab_block(const float (&f)[64], float* out, uint32_t nz, uint32_t b) {
@@ -244,13 +233,25 @@ __device__ __forceinline__ void store_slab_block(const float (&f)[64], float* ou
             make_float4(f[16 * z + 4 * y], f[16 * z + 4 * y + 1], f[16 * z + 4 * y + 2], f[16 * z + 4 * y + 3]);
     }
 }
-// What the floating point decoder leaves over starts again, out of line: in line its code and registers
-// cost the others 12 % (256 MiB at 256 / 512 bits 84.1 / 94.4 us, without it 72 / 85).
-__device__ __noinline__ void decode_slab_ints(float* out, uint32_t nz, int maxbits, int lsh, const PipeConsts kc,
-                                             const FirstTests first) {
-  float f[64];
-  decode_ints(maxbits, f, kc, first);
-  if (!is_copy(lsh)) store_slab_block(f, out, nz, (uint32_t)block_of_thread(lsh));
+template <Way3 WAY>
+__device__ __forceinline__ void decode_slab_block(float* out, uint32_t nz, int maxbits, int lsh);
+// a block whose results the floating point decoder could not vouch for, from the start
+__device__ __noinline__ void decode_slab_again(float* out, uint32_t nz, int maxbits, int lsh) {
+  decode_slab_block<kInts3>(out, nz, maxbits, lsh);
+}
+template <Way3 WAY>
+__device__ __forceinline__ void decode_slab_block(float* out, uint32_t nz, int maxbits, int lsh) {
+  extern __shared__ __align__(16) uint32_t smem_words[];
+  const int nwords = maxbits >> 5;
+  uint32_t* col = decoder_column(nwords);
+  WarpWords source{col};
+  WarpPark park{col + 32 * (nwords + DEC_SPARE_ROWS)};
+  decode_block3<WAY>(
+      source, park, maxbits, smem_words,
+      [&](const float (&f)[64]) {
+        if (!is_copy(lsh)) store_slab_block(f, out, nz, (uint32_t)block_of_thread(lsh));
+      },
+      [&] { decode_slab_again(out, nz, maxbits, lsh); });
 }
 }  // namespace
 
@@ -258,21 +259,21 @@ __device__ __noinline__ void decode_slab_ints(float* out, uint32_t nz, int maxbi
 // lane pulls its own compressed words into its column of the word-major staging
 // area, parses them by bit position and stores the rebuilt 4x4x4 block with
 // sixteen 128-bit stores.  The only barrier is the one after the table copy.
-// CHUNKS: decode3_chunks(maxbits).
-// Bound by instructions issued (about 1780 a warp at 512 bits, issue slots 59 % busy, ALU pipe 64 %); loads and
-// stores alone take 52 of the 86 us.  256 MiB at 256 / 512 / 1024 bits 95.5 / 122.5 / 158.3 -> 77.6 / 86.3 / 125.6 us
-// (tanh of normal values) with each lane at its own pace through the group tests and the inverse transform in
-// exact float32; values smooth enough for every plane to be read, which stay with the integers, 148 / 165
-// / 199 -> 152 / 163 / 208.
-template <int CHUNKS>
-__global__ void __launch_bounds__(kThreads, dec_ctas_per_sm(CHUNKS, true))
-zfp_decode_slab_kernel(const uint32_t* __restrict__ in, float* __restrict__ out, uint32_t nz, int maxbits, int lsh,
-                       const PipeConsts kc) {
+// WAY: decode3_way(maxbits).
+// Bound by instructions issued (about 1895 a warp at 512 bits); loads and stores alone take 52 of the 86 us.  Against a
+// decoder that goes plane by plane with the slowest lane and lifts in integers, 256 MiB at 256 / 512 / 1024 bits:
+//   tanh of normal values                 95.7 / 122.5 / 158.3 ->  75.2 /  86.1 / 122.3 us
+//   normal values + 10                   117.9 / 133.6 / 167.0 ->  93.2 / 102.3 / 139.0
+//   sines over the field with 3 % noise  129.0 / 148.0 / 179.9 ->  98.7 / 108.0 / 144.1
+//   sines alone                          141.6 / 177.5 / 213.6 -> 136.8 / 164.9 / 187.7
+template <Way3 WAY>
+__global__ void __launch_bounds__(kThreads, kSlabDecCtasPerSm)
+zfp_decode_slab_kernel(const uint32_t* __restrict__ in, float* __restrict__ out, uint32_t nz, int maxbits, int lsh) {
   extern __shared__ __align__(16) uint32_t smem_words[];
   const int nwords = maxbits >> 5;
   const uint32_t b = (uint32_t)block_of_thread(lsh);
   const uint32_t zt = (b >> 6) * 4;  // first slab of my tile
-  uint32_t* col = decoder_column<3>(nwords);
+  uint32_t* col = decoder_column(nwords);
   copy_table<DEC_LUT_SIZE>(smem_words, g_dec_table.v);
   pdl_wait(in);
   if (zt < nz) {
@@ -294,19 +295,7 @@ zfp_decode_slab_kernel(const uint32_t* __restrict__ in, float* __restrict__ out,
   __syncthreads();  // the table is complete
   if (zt >= nz) return;
 
-  float f[64];
-  const FirstTests none{-1, 0u, {0u, 0u}};
-  if constexpr (CHUNKS == 0) {
-    decode_ints(maxbits, f, kc, none);
-  } else {
-    WarpWords source{col};
-    WarpPark park{col + 32 * (nwords + DEC_SPARE_ROWS)};
-    if (!decode_block3_float<CHUNKS>(source, park, maxbits, f, smem_words, [&](const FirstTests& first) {
-          decode_slab_ints(out, nz, maxbits, lsh, kc, first);
-        }))
-      return;
-  }
-  if (!is_copy(lsh)) store_slab_block(f, out, nz, b);
+  decode_slab_block<WAY>(out, nz, maxbits, lsh);
 }
 
 // =====================================================================================
@@ -553,26 +542,41 @@ __device__ __forceinline__ void store_field_block(const FieldGeom& g, float* out
   const bool valid = b < nblocks && !is_copy(lsh);
   if (!vec && g.sx == 1) {
     __syncwarp();  // every lane is done with its words
-    store_rows3(g, out, at, valid, reinterpret_cast<float*>(decoder_column<3>(nwords) - (threadIdx.x & 31)), f);
+    store_rows3(g, out, at, valid, reinterpret_cast<float*>(decoder_column(nwords) - (threadIdx.x & 31)), f);
   } else if (valid) {
     store_block<3>(g, out, vec, at, f);
   }
 }
-__device__ __noinline__ void decode_field_ints(const FieldGeom& g, float* out, bool vec, uint64_t nblocks, int maxbits,
-                                               int lsh, const PipeConsts kc, const FirstTests first) {
-  float f[64];
-  decode_ints(maxbits, f, kc, first);
-  store_field_block(g, out, vec, block_of_thread(lsh), nblocks, (maxbits + 31) >> 5, lsh, f);
+template <Way3 WAY>
+__device__ __forceinline__ void decode_field_block(const FieldGeom& g, float* out, bool vec, uint64_t nblocks, int maxbits,
+                                                   int lsh);
+// the geometry by value: a reference would put it, and the kernel's arguments, on the stack of every call (0.3 us of 6)
+__device__ __noinline__ void decode_field_again(const FieldGeom g, float* out, bool vec, uint64_t nblocks, int maxbits,
+                                                int lsh) {
+  decode_field_block<kInts3>(g, out, vec, nblocks, maxbits, lsh);
+}
+template <Way3 WAY>
+__device__ __forceinline__ void decode_field_block(const FieldGeom& g, float* out, bool vec, uint64_t nblocks, int maxbits,
+                                                   int lsh) {
+  extern __shared__ __align__(16) uint32_t smem_words[];
+  const int nwords = (maxbits + 31) >> 5;
+  uint32_t* col = decoder_column(nwords);
+  WarpWords source{col};
+  WarpPark park{col + 32 * (nwords + DEC_SPARE_ROWS)};
+  decode_block3<WAY>(
+      source, park, maxbits, smem_words,
+      [&](const float (&f)[64]) { store_field_block(g, out, vec, block_of_thread(lsh), nblocks, nwords, lsh, f); },
+      [&] { decode_field_again(g, out, vec, nblocks, maxbits, lsh); });
 }
 
-// CHUNKS: of 3-D blocks, decode3_chunks(maxbits)
+// WAY: of 3-D blocks, decode3_way(maxbits)
 // 2-D: 768 x 4096 at 64 / 128 / 256 bits 11.0 / 13.8 / 16.6 -> 9.4 / 10.7 / 13.7 us with the lanes at their own pace through
 // the group tests, sixteen planes a transpose and the transform in exact float32; 4096 x 4096 48.2 / 63.5 / 79.5 -> 37.3 /
 // 43.0 / 53.7 (and one round of blocks a CTA), smooth values at 128 bits 92.6 -> 81.1.
-template <int DIMS, int CHUNKS>
-__global__ void __launch_bounds__(kThreads, DIMS == 3 ? dec_ctas_per_sm(CHUNKS, false) : 8)
+template <int DIMS, Way3 WAY>
+__global__ void __launch_bounds__(kThreads, DIMS == 3 ? kDecCtasPerSm : 8)
 zfp_decode_generic_kernel(const FieldGeom g, const uint32_t* __restrict__ in, float* __restrict__ out, bool vec,
-                          int maxbits, uint64_t nblocks, uint64_t total_words, int lsh, const PipeConsts kc) {
+                          int maxbits, uint64_t nblocks, uint64_t total_words, int lsh) {
   extern __shared__ __align__(16) uint32_t smem_words[];
   const int nwords = (maxbits + 31) >> 5, tid = threadIdx.x;
   constexpr int kRow = DIMS > 1 ? 32 : kThreads;  // a staged word to the next one of the same lane
@@ -585,7 +589,7 @@ zfp_decode_generic_kernel(const FieldGeom g, const uint32_t* __restrict__ in, fl
     col = lut + DEC1_LUT_SIZE / 2 + tid;
   } else {
     copy_table<DEC_LUT_SIZE>(lut, g_dec_table.v);
-    col = decoder_column<DIMS>(nwords);
+    col = decoder_column(nwords);
   }
   // reads just past a block find zeros and need no bounds test
 #pragma unroll
@@ -619,18 +623,7 @@ zfp_decode_generic_kernel(const FieldGeom g, const uint32_t* __restrict__ in, fl
     }
     float f[1 << (2 * DIMS)];
     if constexpr (DIMS == 3) {
-      const FirstTests none{-1, 0u, {0u, 0u}};
-      if constexpr (CHUNKS == 0) {
-        decode_ints(maxbits, f, kc, none);
-      } else {
-        WarpWords source{col};
-        WarpPark park{col + 32 * (nwords + DEC_SPARE_ROWS)};
-        if (!decode_block3_float<CHUNKS>(source, park, maxbits, f, lut, [&](const FirstTests& first) {
-              decode_field_ints(g, out, vec, nblocks, maxbits, lsh, kc, first);
-            }))
-          return;
-      }
-      store_field_block(g, out, vec, b, nblocks, nwords, lsh, f);
+      decode_field_block<WAY>(g, out, vec, nblocks, maxbits, lsh);
       return;  // the launcher gives a 3-D field a warp for every group of blocks
     } else {
       if constexpr (DIMS == 2) {
@@ -664,7 +657,7 @@ constexpr int kMostBits = 4096;                    // largest budget the library
 static size_t staged_smem_bytes(int maxbits, bool decode, int dims) {
   const size_t rows = ((size_t)maxbits + 31) / 32 + STAGE_SPARE_ROWS;
   if (decode && dims == 1) return rows * kThreads * 4 + DEC1_LUT_SIZE * 2;
-  if (decode) return (DEC_LUT_SIZE + kThreads / 32 * (size_t)warp_words((maxbits + 31) / 32, dims)) * 4;
+  if (decode) return (DEC_LUT_SIZE + kThreads / 32 * (size_t)warp_words((maxbits + 31) / 32)) * 4;
   return (rows + (dims == 3 ? QUEUE_SLOTS * QUEUE_FIELDS : 0)) * kThreads * 4 + (dims == 3 ? ENC3_LUT_SIZE : ENC_LUT_SIZE) * 4;
 }
 // Only the largest budgets need it; the call costs host time on every launch.
@@ -712,11 +705,11 @@ static cudaError_t encode_generic(const FieldGeom& g, const float* in, uint32_t*
                     vector_rows(g, in), out, maxbits, nblocks, (uint64_t)stream_bytes(g, (unsigned)maxbits) / 4, lsh,
                     pipe_consts());
 }
-template <int DIMS, int CHUNKS>
+template <int DIMS, Way3 WAY>
 static cudaError_t decode_generic(const FieldGeom& g, const uint32_t* in, float* out, int maxbits, uint64_t nblocks,
                                   cudaStream_t stream) {
   const size_t smem = staged_smem_bytes(maxbits, true, DIMS);
-  cudaError_t e = allow_smem(zfp_decode_generic_kernel<DIMS, CHUNKS>, smem, true, DIMS);
+  cudaError_t e = allow_smem(zfp_decode_generic_kernel<DIMS, WAY>, smem, true, DIMS);
   if (e != cudaSuccess) return e;
   const int lsh = DIMS == 3 ? blocks_per_warp(nblocks) : 5;
   const uint64_t ctas = ctas_of(nblocks, lsh);
@@ -728,9 +721,8 @@ static cudaError_t decode_generic(const FieldGeom& g, const uint32_t* in, float*
   const uint64_t full = 8 * (uint64_t)sm_count();
   const bool once = DIMS == 3 || (DIMS == 2 && sm_count() >= kWholeChip);
   const uint64_t rounds = once || ctas < 2 * full ? 1 : ctas / full < 8 ? ctas / full : 8;
-  return pdl_launch(zfp_decode_generic_kernel<DIMS, CHUNKS>, (unsigned)((ctas + rounds - 1) / rounds), kThreads, smem, stream,
-                    g, in, out, vector_rows(g, out), maxbits, nblocks, (uint64_t)stream_bytes(g, (unsigned)maxbits) / 4, lsh,
-                    pipe_consts());
+  return pdl_launch(zfp_decode_generic_kernel<DIMS, WAY>, (unsigned)((ctas + rounds - 1) / rounds), kThreads, smem, stream,
+                    g, in, out, vector_rows(g, out), maxbits, nblocks, (uint64_t)stream_bytes(g, (unsigned)maxbits) / 4, lsh);
 }
 
 cudaError_t zfp_encode_launch(const FieldGeom& g, const float* in, void* out, int maxbits, cudaStream_t stream) {
@@ -751,32 +743,32 @@ cudaError_t zfp_encode_launch(const FieldGeom& g, const float* in, void* out, in
                        : encode_generic<1>(g, in, o, maxbits, nblocks, stream);
 }
 
-template <int CHUNKS>
+template <Way3 WAY>
 static cudaError_t decode_slabs(const FieldGeom& g, const uint32_t* in, float* out, int maxbits, cudaStream_t stream) {
   const size_t smem = staged_smem_bytes(maxbits, true, 3);
-  cudaError_t e = allow_smem(zfp_decode_slab_kernel<CHUNKS>, smem, true, 3);
+  cudaError_t e = allow_smem(zfp_decode_slab_kernel<WAY>, smem, true, 3);
   if (e != cudaSuccess) return e;
   const uint64_t blocks = slab_blocks(g);
   const int lsh = blocks_per_warp(blocks);
-  return pdl_launch(zfp_decode_slab_kernel<CHUNKS>, ctas_of(blocks, lsh), kThreads, smem, stream, in, out, g.nz, maxbits,
-                    lsh, pipe_consts());
+  return pdl_launch(zfp_decode_slab_kernel<WAY>, ctas_of(blocks, lsh), kThreads, smem, stream, in, out, g.nz, maxbits,
+                    lsh);
 }
 
 cudaError_t zfp_decode_launch(const FieldGeom& g, const void* in, float* out, int maxbits, cudaStream_t stream) {
   const uint64_t nblocks = geom_blocks(g);
   if (nblocks == 0) return cudaSuccess;
   const uint32_t* i32 = reinterpret_cast<const uint32_t*>(in);
-  const int chunks = decode3_chunks(maxbits);
+  const Way3 way = decode3_way(maxbits);
   if (zfp_slab_eligible(g, out, in, maxbits))
-    return chunks == 2   ? decode_slabs<2>(g, i32, out, maxbits, stream)
-           : chunks == 3 ? decode_slabs<3>(g, i32, out, maxbits, stream)
-                         : decode_slabs<0>(g, i32, out, maxbits, stream);
+    return way == kFloats3 ? decode_slabs<kFloats3>(g, i32, out, maxbits, stream)
+           : way == kInts3 ? decode_slabs<kInts3>(g, i32, out, maxbits, stream)
+                           : decode_slabs<kShortInts3>(g, i32, out, maxbits, stream);
   if (g.dims == 3)
-    return chunks == 2   ? decode_generic<3, 2>(g, i32, out, maxbits, nblocks, stream)
-           : chunks == 3 ? decode_generic<3, 3>(g, i32, out, maxbits, nblocks, stream)
-                         : decode_generic<3, 0>(g, i32, out, maxbits, nblocks, stream);
-  return g.dims == 2 ? decode_generic<2, 0>(g, i32, out, maxbits, nblocks, stream)
-                     : decode_generic<1, 0>(g, i32, out, maxbits, nblocks, stream);
+    return way == kFloats3 ? decode_generic<3, kFloats3>(g, i32, out, maxbits, nblocks, stream)
+           : way == kInts3 ? decode_generic<3, kInts3>(g, i32, out, maxbits, nblocks, stream)
+                           : decode_generic<3, kShortInts3>(g, i32, out, maxbits, nblocks, stream);
+  return g.dims == 2 ? decode_generic<2, kInts3>(g, i32, out, maxbits, nblocks, stream)
+                     : decode_generic<1, kInts3>(g, i32, out, maxbits, nblocks, stream);
 }
 
 }  // namespace csw

@@ -212,9 +212,8 @@ Way decode_warp(Warp& warp, const csw::FieldGeom& g, const uint32_t* in, int max
     const PadSource src{rows[l].data(), nw + csw::DEC_SPARE_ROWS};
     csw::HostPark park;
     if constexpr (DIMS == 3) {
-      csw::decode_block3_host(src, park, maxbits, q[l], dec3_lut().data(), [&](const csw::FirstTests& first) {
-        way = first.tests < 0 && csw::decode3_chunks(maxbits) ? kStartedAgain : std::max(way, kIntWay);
-      });
+      static const Way ways[] = {kFloatWay, kIntWay, kStartedAgain};
+      way = ways[csw::decode_block3_host(src, park, maxbits, q[l], dec3_lut().data())];
     } else {
       float (&f)[16] = reinterpret_cast<float (&)[16]>(q[l]);
       csw::decode_block2(src, park, maxbits, f, dec3_lut().data());

@@ -74,3 +74,45 @@ def test_2d_warps_of_blocks_that_differ(core, oracle, maxbits):  # noqa: F811
         decode(core, oracle, oracle.zfp_encode(a, *dims, maxbits), dims, maxbits)
     for s in util.arbitrary_streams(oracle.zfp_stream_bytes(*dims, maxbits) // 4, maxbits):
         decode(core, oracle, s, dims, maxbits)
+
+
+def values_between_noise_and_smooth(n, seed):
+    g = util.normal(n, seed)
+    i = np.arange(n)
+    smooth = 1.7 * np.sin(0.11 * (i % 32) + 0.07 * (i // 32 % 32) + 0.05 * (i // 1024) + 0.3)
+    yield from ((f"normal+{k}", g + k) for k in (0, 3, 10, 30, 100))
+    yield from ((f"smooth+{k}", smooth + k * g) for k in (0, 0.001, 0.01, 0.03, 0.1))
+    yield from ((f"tanh*{k}", np.tanh(k * g)) for k in (1, 2, 3))
+    yield "signs", 0.9999 * np.sign(g)
+    yield "channels", (g.reshape(-1, 1024) + 4 * util.normal(n // 1024, seed + 1)[:, None]).reshape(-1)
+    yield "relu", np.maximum(g - 1.28, 0)
+    yield "constant in parts", np.maximum(0.05 * g + 0.5 + smooth, 0)
+
+
+@pytest.mark.parametrize("maxbits", [64, 192, 256, 300, 512, 704, 832, 864, 1024, 1152, 1216, 1280, 1408, 2048])
+def test_no_block_is_decoded_twice(core, oracle, maxbits):  # noqa: F811
+    """Which decoder a warp's blocks get is told from their group tests: none of these values are tried by the floating point
+    decoder and then decoded again, but for a few warps whose results come close to 2^31."""
+    dims = (32, 32, 32)
+    for name, a in values_between_noise_and_smooth(32 * 1024, maxbits):
+        ways = decode(core, oracle, oracle.zfp_encode(np.ascontiguousarray(a, dtype=np.float32), *dims, maxbits), dims, maxbits)
+        assert ways[AGAIN] <= sum(ways) // 8, (name, ways)
+
+
+def test_each_way_is_taken(core, oracle):  # noqa: F811
+    """Blocks whose planes and leading empty planes leave 24 bits enough go by floating point, what they do not
+    fit and the smooth ones by integers; bits that no encoder wrote give results beyond 2^31, and are decoded twice."""
+    dims = (32, 32, 32)
+    values = {name: np.ascontiguousarray(a, dtype=np.float32) for name, a in values_between_noise_and_smooth(32 * 1024, 1)}
+    way = {}
+    for name, maxbits in (("normal+0", 512), ("normal+30", 512), ("smooth+0.03", 256), ("constant in parts", 512),
+                          ("smooth+0", 512), ("normal+100", 832), ("normal+0", 1024), ("normal+0", 192)):
+        way[name, maxbits] = decode(core, oracle, oracle.zfp_encode(values[name], *dims, maxbits), dims, maxbits)
+    for key in (("normal+0", 512), ("normal+30", 512), ("smooth+0.03", 256), ("constant in parts", 512)):
+        assert way[key][INTS] == way[key][AGAIN] == 0, (key, way)
+    for key in (("smooth+0", 512), ("normal+100", 832), ("normal+0", 1024), ("normal+0", 192)):
+        assert way[key][FLOATS] == way[key][AGAIN] == 0, (key, way)
+    bits, more = (util.arbitrary_streams(oracle.zfp_stream_bytes(*dims, 288) // 4, seed)[0] for seed in (1, 10))
+    bits |= more  # three ones in four
+    bits[0::9] = (bits[0::9] & ~np.uint32(0x1FF)) | np.uint32((130 << 1) | 1)
+    assert decode(core, oracle, bits, dims, 288)[AGAIN] > 0
