@@ -14,7 +14,7 @@ LIB = os.path.join(HERE, "libcswap_b200.so")
 ROOT = os.path.dirname(HERE)
 SOURCES = ["zfp_kernels.cu", "sparse_kernels.cu", "cswap_abi.cu", "swap_manager.cu", "cost_model.cu",
            "sparse_static.cu"]
-HEADERS = ["pdl.cuh", "zfp_core.cuh", "zfp_field.cuh", "zfp_kernels.h", "sparse_kernels.h", "internal.h",
+HEADERS = ["pdl.cuh", "zfp_core.cuh", "zfp_field.cuh", "zfp_kernels.h", "sparse_kernels.h", "tile_counts.cuh", "internal.h",
            os.path.join("..", "..", "include", "cswap_b200.h"), os.path.join("..", "..", "include", "cswap_compat.h")]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC"]

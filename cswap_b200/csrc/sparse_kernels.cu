@@ -34,6 +34,7 @@
 
 #include "pdl.cuh"
 #include "sparse_kernels.h"
+#include "tile_counts.cuh"
 
 namespace csw {
 
@@ -177,12 +178,11 @@ sparse_pack_kernel(const uint32_t* __restrict__ in, uint64_t n, uint32_t* __rest
 }
 
 // The same without a scan in between, for kLeastSummed to kMostSummed tiles: a CTA adds up the counts ahead
-// of its tile itself, and the last one to have read them turns them into offsets.  The number of CTAs that
-// have is kept above the thirteen bits of tile 0's count; no CTA waits for another.  A launch
-// less, but a CTA's loads lie in front of its part in the sum: 50 % zeros, with the scan and without, 1 Mi elements
-// 5.94 | 5.22 us, 2 Mi 6.64 | 6.24, 4 Mi 7.77 | 9.53, 8 Mi 13.3 | 15.9; 400 000 elements 5.94 | 6.01.
-constexpr int kCountBits = 13;  // a tile's count is 4096 at most
-constexpr uint32_t kCountMask = (1u << kCountBits) - 1u, kLeastSummed = 128, kMostSummed = 512;
+// of its tile itself, and the last one to have read them turns them into offsets (tile_counts.cuh); no CTA waits
+// for another.  A launch less, but a CTA's loads lie in front of its part in the sum: 50 % zeros, with the scan and without, 1 Mi elements
+// 5.94 | 5.22 us, 2 Mi 6.64 | 6.24, 4 Mi 7.77 | 9.53, 8 Mi 13.3 | 15.9; 400 000 elements 5.94 | 6.01.  Where the host's
+// part of a call is the longer one the launch counts whole, 1 Mi 8.27 | 6.38; in a graph it is nearly free, 4.93 | 5.09.
+constexpr uint32_t kLeastSummed = 128, kMostSummed = 512;
 __global__ void __launch_bounds__(kThreads, 8)
 sparse_pack_sum_kernel(const uint32_t* __restrict__ in, uint64_t n, uint32_t* __restrict__ bitmap, uint32_t* tile_off,
                        uint32_t* __restrict__ values, uint32_t* __restrict__ nnz_out) {
@@ -211,7 +211,7 @@ sparse_pack_sum_kernel(const uint32_t* __restrict__ in, uint64_t n, uint32_t* __
 #pragma unroll
   for (int q = 0; q < kPer; q++) {
     const uint32_t i = q * kThreads + threadIdx.x;
-    if (i < tile) ahead += __ldcg(tile_off + i) & kCountMask;
+    if (i < tile) ahead += tile_count(tile_off + i);
   }
   ahead = __reduce_add_sync(0xffffffffu, ahead);
   if (lane == 0) {
@@ -219,8 +219,8 @@ sparse_pack_sum_kernel(const uint32_t* __restrict__ in, uint64_t n, uint32_t* __
     warp_sum[warp] = ahead;
   }
   __syncthreads();  // every count that this CTA needs has been read
-  uint32_t order = 0;
-  if (threadIdx.x == 0) order = atomicAdd(tile_off, 1u << kCountBits) >> kCountBits;
+  bool arrived_last = false;
+  if (threadIdx.x == 0) arrived_last = last_to_arrive(tile_off, tiles);
   if (lane < kWordsPerWarp && word0 + lane < nwords) bitmap[word0 + lane] = mine;
   uint32_t off = 0;
 #pragma unroll
@@ -231,14 +231,14 @@ sparse_pack_sum_kernel(const uint32_t* __restrict__ in, uint64_t n, uint32_t* __
     if (v[j] != 0u) values[off + __popc(w[j] & lt)] = v[j];
     off += __popc(w[j]);
   }
-  if (threadIdx.x == 0) last = order == tiles - 1;
+  if (threadIdx.x == 0) last = arrived_last;
   __syncthreads();
   if (!last) return;
   uint32_t c[kPer], sum = 0;
 #pragma unroll
   for (int q = 0; q < kPer; q++) {
     const uint32_t i = threadIdx.x * kPer + q;
-    c[q] = i < tiles ? __ldcg(tile_off + i) & kCountMask : 0u;
+    c[q] = i < tiles ? tile_count(tile_off + i) : 0u;
     sum += c[q];
   }
   uint32_t x = sum;
