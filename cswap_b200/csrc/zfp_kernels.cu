@@ -42,7 +42,7 @@ namespace {
 constexpr int kThreads = 128;                  // zfp blocks (lanes) per CTA
 constexpr int kSlabFloats = 1024;              // one 32x32 z-slab
 constexpr int kEncCtasPerSm = 4;                // 128 registers per thread: the encoder needs 113; five CTAs
-                                                // spill, 256 MiB at 1024 bits 130.6 -> 146.9 us
+                                                // spill, 256 MiB at 1024 bits 130.6 -> 146.9 us (before the queue was read ahead)
 // 3-D decoders: 80 registers are nearly enough (12 bytes of spills in the floating point one); a CTA more hides more of the
 // dependent shared-memory reads (256 MiB at 512 bits 91.7 us with five CTAs, 85.9 with six; at 1024 bits 125.6 and 123.4).
 // Fields in their own extents need a few registers more and are seldom more than one wave: 31 x 33 x 4096 at 512 bits 11.1 us
@@ -135,8 +135,8 @@ __device__ __forceinline__ int pad_src_z(int z, int vz) { return z < vz ? z : (z
 // its own column of the word-major staging area and writes its own words out:
 // after the table is built no warp waits for another.
 // Bound by instructions issued (2566 a warp at 512 bits, issue slots 71 % busy).  256 MiB at 256 / 512 / 1024
-// bits 82.0 / 104.0 / 135.8 -> 80.2 / 101.3 / 130.6 us with the expansions' bits in one word and a vote that holds
-// their loop together.
+// bits 82.0 / 104.0 / 135.8 -> 79.9 / 100.1 / 129.4 us with the expansions' bits in one word, a vote that holds
+// their loop together, and the queue read one entry ahead.
 __global__ void __launch_bounds__(kThreads, kEncCtasPerSm)
 zfp_encode_slab_kernel(const float* __restrict__ in, uint32_t* __restrict__ out, uint32_t nz, int maxbits, int lsh,
                        const PipeConsts kc) {
