@@ -670,12 +670,13 @@ static cudaError_t allow_smem(K* kernel, size_t smem, bool decode, int dims) {
 
 static uint64_t slab_blocks(const FieldGeom& g) { return ((uint64_t)g.nz + 3) / 4 * 64; }
 // log2 of the blocks a warp takes.  While every scheduler of the device has at most one
-// warp, a call lasts as long as one warp does, and a warp waits, plane by plane, for
-// the one of its blocks with the most group tests: the fewer blocks, the shorter.  So blocks
-// are spread until there is a warp for each of the schedulers, 4 x 148.  64 KiB at 512 bits
-// 5.4 -> 4.4 us (encode) and 7.3 -> 5.2 (decode), 1 MiB at 1024 bits 6.4 -> 5.8 and 8.7 -> 7.8.
-// From two warps a scheduler on the copies cost more issue slots than they save: 4 MiB with
-// 16 blocks a warp 5.6 -> 6.6 and 7.3 -> 7.8.
+// warp, a call lasts as long as one warp does, and a warp takes the steps of the one of its
+// blocks with the most group tests: the fewer blocks, the shorter.  So blocks are spread until there
+// is a warp for each of the schedulers, 4 x 148.  64 KiB at 512 bits 4.70 -> 4.39 us (encode) and 4.56 -> 4.26
+// (decode), at 1024 bits 5.65 -> 4.95 and 6.33 -> 5.17; 1 MiB at 1024 bits 5.88 -> 5.42 and 6.42 -> 6.47, the decoder's
+// tests being no longer most of its time there.  From two warps a scheduler on the copies cost
+// more issue slots than they save: 1 MiB at 512 bits with 4 blocks a warp in place of 8 4.67 -> 6.03 and 4.92 -> 5.49, 4 MiB
+// with 16 in place of 32 5.05 -> 6.28 and 5.00 -> 5.80.
 static int blocks_per_warp(uint64_t nblocks) {
   const uint64_t schedulers = kSchedulersPerSm * (unsigned)sm_count();
   int lsh = 0;
