@@ -134,7 +134,7 @@ __device__ __forceinline__ int pad_src_z(int z, int vz) { return z < vz ? z : (z
 // 128-byte row segment, so a warp load touches four full lines), codes it into
 // its own column of the word-major staging area and writes its own words out:
 // after the table is built no warp waits for another.
-// Bound by instructions issued (2566 a warp at 512 bits, issue slots 71 % busy).  256 MiB at 256 / 512 / 1024
+// Bound by instructions issued (2558 a warp at 512 bits, ALU pipe 66 % busy).  256 MiB at 256 / 512 / 1024
 // bits 82.0 / 104.0 / 135.8 -> 79.9 / 100.1 / 129.4 us with the expansions' bits in one word, a vote that holds
 // their loop together, and the queue read one entry ahead.
 __global__ void __launch_bounds__(kThreads, kEncCtasPerSm)
@@ -260,7 +260,7 @@ __device__ __forceinline__ void decode_slab_block(float* out, uint32_t nz, int m
 // area, parses them by bit position and stores the rebuilt 4x4x4 block with
 // sixteen 128-bit stores.  The only barrier is the one after the table copy.
 // WAY: decode3_way(maxbits).
-// Bound by instructions issued (about 1895 a warp at 512 bits); loads and stores alone take 52 of the 86 us.  Against a
+// Bound by instructions issued (1895 a warp at 512 bits, ALU pipe 57 % busy); loads and stores alone take 52 of the 86 us.  Against a
 // decoder that goes plane by plane with the slowest lane and lifts in integers, 256 MiB at 256 / 512 / 1024 bits:
 //   tanh of normal values                 95.7 / 122.5 / 158.3 ->  75.2 /  86.1 / 122.3 us
 //   normal values + 10                   117.9 / 133.6 / 167.0 ->  93.2 / 102.3 / 139.0
@@ -308,7 +308,7 @@ zfp_decode_slab_kernel(const uint32_t* __restrict__ in, float* __restrict__ out,
 // no atomics, no zeroed stream.  (One thread per block reading and writing global
 // memory word by word, with plane-by-plane coders whose lanes wait for each other,
 // took 28.7 + 33.4 us a call for 31 x 33 x 4096 at 512 bits and 22.6 + 26.7 us for
-// 768 x 4096 at 128; these take 12.2 + 11.8 and 12.2 + 10.7.  They are bound as the
+// 768 x 4096 at 128; these take 11.8 + 10.7 and 11.9 + 10.3.  They are bound as the
 // slab kernels are, by the number of instructions a block costs.)
 namespace {
 
