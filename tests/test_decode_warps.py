@@ -116,3 +116,21 @@ def test_each_way_is_taken(core, oracle):  # noqa: F811
     bits |= more  # three ones in four
     bits[0::9] = (bits[0::9] & ~np.uint32(0x1FF)) | np.uint32((130 << 1) | 1)
     assert decode(core, oracle, bits, dims, 288)[AGAIN] > 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("maxbits", [32, 64, 224, 255, 256, 288, 704, 832, 833, 864, 1024, 1440, 2048, 4096])
+def test_kernels_on_warps_that_differ(oracle, maxbits):
+    """Budgets on either side of where the kernel changes, warps that go different ways, in the swap path's view and with
+    ragged edges."""
+    import torch
+    import cswap_b200 as cs
+    for dims in ((32, 32, 32), (31, 30, 17)):
+        n = dims[0] * dims[1] * dims[2]
+        fields = [a for _, a in values_between_noise_and_smooth(32 * 1024, maxbits)] + [mixed_field(s, 16)[0] for s in range(2)]
+        streams = [oracle.zfp_encode(np.ascontiguousarray(a[:n], dtype=np.float32), *dims, maxbits) for a in fields]
+        streams += [np.ascontiguousarray(s).view(np.uint64)
+                    for s in util.arbitrary_streams(oracle.zfp_stream_bytes(*dims, maxbits) // 4, maxbits)]
+        for s in streams:
+            got = cs.zfp_decompress(torch.from_numpy(s.view(np.uint8).copy()).cuda(), n, maxbits, dims).cpu().numpy()
+            assert np.array_equal(got.view(np.uint32), oracle.zfp_decode(s, *dims, maxbits).view(np.uint32))
